@@ -15,26 +15,24 @@
 //     m, n < 65536).  A warp reads 32 consecutive values and 32 consecutive
 //     indices per step: coalesced, no per-row pointers, no divergence.
 //   * `count` instances, each naming a matrix; b, c, l, u in FP64 (internal
-//     order; KKT and re-centring); per column one packed record {scaled cost,
-//     lower, upper, Halpern anchor} and per row one {scaled rhs, dual lower
-//     bound, anchor} in the solve's precision (16 bytes each in FP32: one
-//     vector load); iterates x, y and the check-point copies xt, yt.  All
-//     concatenated at x_off[i] / y_off[i]; warm starts and answers are mapped
+//     order; KKT and re-centring); column and row records of the scaled problem in
+//     the solve's precision, one 32-column (row) block after another (col_rec,
+//     row_rec); iterates x, y and the check-point copies xt, yt.  All
+//     concatenated at per-instance offsets; warm starts and answers are mapped
 //     between external and internal order on the device.
 // Execution
-//   * one CTA owns one instance at a time (persistent grid, work queue sorted by
-//     nnz descending = longest-first) -- or, in the paired form for batches whose
-//     instances share one matrix, two instances iterated in lockstep so that each
-//     SELL load feeds both.  When a CTA takes an instance it copies its matrix's
+//   * one CTA owns a group of NI instances at a time (persistent grid, work queue
+//     sorted by nnz descending = longest-first): NI = 1 for any batch, 2 or 4 for
+//     batches whose instances share one matrix, iterated in lockstep so that each
+//     SELL load feeds all of them.  When a CTA takes a group it copies its matrix's
 //     slice pointers into a shared-memory table.  The gathered operands of both SpMVs --
 //     y (also the dual iterate) for A^T y and xh for A xh -- live in shared
-//     memory; x and the packed records stay in global memory, touched only by
-//     their owning thread.  A PDHG iteration is: primal phase (one thread per
+//     memory, interleaved over the group; x follows from xh, so a plain iteration
+//     reads only the records and the matrix.  A PDHG iteration is: primal phase (one thread per
 //     column, one warp per column slice) | barrier | dual phase (one thread per
-//     row) | barrier.  A slice longer than kLongSlice entries per lane is summed
-//     by the whole warp over the CSR copy instead (one dense row cannot stall
-//     its slice).  Control scalars are private copies in every thread; the CTA
-//     only meets in shared memory at restart-check iterations.
+//     row) | barrier.  Rows longer than kLongSlice are summed by whole warps over
+//     the CSR copy instead (one dense row cannot stall its slice).  Control scalars
+//     and step sizes live in shared memory; restart checks are out of line.
 //   * precision MT (float = mixed, double = FP64) is the type of the scaled
 //     matrix values, the packed records, the iterates and the SpMV sums.  FP64 is
 //     kept for the scaling factors, the squared-residual sums, the KKT of the
@@ -50,13 +48,16 @@
 //   * a launch runs every active instance for up to `chunk` iterations; a
 //     compaction kernel drops finished instances; [chunk, compact] x 2 is
 //     captured as a CUDA graph and replayed until no instance is active.
-//   * CTA size, SELL entry order (one entry or a pair per lane load), form
-//     (single or paired) and chunk length come from an autotuner that times the
-//     candidates on a sample of the batch (cached on disk).
+//   * CTA size, SELL entry order (one entry or a pair per lane load), instances per
+//     CTA and chunk length come from an autotuner that times the candidates on a
+//     sample of the batch (cached on disk); between replays the host picks the form
+//     with the least rounds of resident CTAs x time per round for the instances
+//     still active, and a wide single form for the tail.
 #include <cub/cub.cuh>
 
 #include <algorithm>
 #include <type_traits>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -81,6 +82,18 @@ struct InstCtrl {
     int pad;
 };
 
+// A tuned launch shape of the chunk kernel.
+struct TuneCfg {
+    int threads = 256, chunk = 2048, w = 1;  // CTA size, iterations per chunk launch, SELL entries per lane load (1 or 2)
+    int ni = 1;                              // instances per CTA: 1, or 2 or 4 (groups, batches of one shared matrix)
+    // the forms a solve chooses between by the number of instances still active: instances
+    // per CTA 1, 2, 4 with their CTA sizes (0: not available) and microseconds per iteration
+    // of one round of resident CTAs
+    int form_th[3] = {0, 0, 0};
+    double form_us[3] = {0, 0, 0};
+};
+constexpr int kFormNi[3] = {1, 2, 4};
+
 struct BatchWork {
     int nmat = 0, count = 0;
     int64_t tot_m = 0, tot_n = 0, nnz = 0, inst_m = 0, inst_n = 0;
@@ -101,7 +114,8 @@ struct BatchWork {
     std::vector<int32_t> h_mat_m, h_mat_n;
     // instances
     DBuf<int32_t> inst_mat;
-    DBuf<int64_t> x_off, y_off;
+    DBuf<int64_t> x_off, y_off;    // of an instance's vectors
+    DBuf<int64_t> xp_off, yp_off;  // of its column / row records (whole slices), in values
     DBuf<double> b, c, lb, ub, bnorm, cnorm;
     DBuf<uint8_t> is_eq;
     // packed records and iterates, sized for FP64 and reinterpreted for FP32; dx, dy hold
@@ -113,15 +127,14 @@ struct BatchWork {
     DBuf<int32_t> active, active2, counters;  // counters[0]=head, [1]=active count
     std::vector<int32_t> h_inst_mat, order;
     int max_m = 0, max_n = 0;
+    int max_len = 0;  // longest row or column of any matrix
     // results of the last solve: per-instance control blocks (host) and the answers
     // in the original space, external order (device, FP64), with the primal weights
     std::vector<InstCtrl> hc;
     DBuf<double> ox, oy, oom;
     bool solved = false;
-    int tuned_threads[2] = {0, 0};  // block size per precision (0 = not tuned yet)
-    int tuned_chunk[2] = {2048, 2048};  // iterations per chunk launch per precision
-    int tuned_w[2] = {1, 1};        // SELL entry order per precision
-    int tuned_ni[2] = {1, 1};       // instances per CTA per precision (2: paired form)
+    bool tuned[2] = {false, false};
+    TuneCfg tuned_cfg[2];           // per precision
     int ell_w = 1;                  // entry order the SELL copies hold now
     DBuf<int32_t> list;             // instances re-initialised by a subset solve
     // active-instance trace of the last solve: host time (ms from the first graph launch of
@@ -140,16 +153,14 @@ namespace {
 
 constexpr int kLongSlice = 128;  // entries per lane above which a slice is summed warp-cooperatively
 
-// Packed per-column / per-row parameters of the scaled (and, when re-centred,
-// shifted) problem in the solve's precision.
-template <typename T>
-struct alignas(4 * sizeof(T)) ColP {
-    T c, l, u, a;  // cost, lower bound, upper bound, Halpern anchor
-};
-template <typename T>
-struct alignas(4 * sizeof(T)) RowP {
-    T b, lo, a, pad;  // rhs, lower bound of the dual (-inf on equality rows), anchor
-};
+// Column and row records of the scaled (and, when re-centred, shifted) problem in the
+// solve's precision, in blocks of one 32-column / 32-row slice: cost, lower bound, upper
+// bound, Halpern anchor (4 x 32 values) per column slice; rhs, lower bound of the dual
+// (-inf on equality rows), anchor (3 x 32) per row slice.  A warp reads each part it
+// needs as one contiguous 128- or 256-byte run, and a re-centred solve, whose anchors are
+// 0, does not read that part at all.
+__host__ __device__ __forceinline__ size_t col_rec(int j) { return (size_t)(j >> 5) * 128 + (j & 31); }
+__host__ __device__ __forceinline__ size_t row_rec(int i) { return (size_t)(i >> 5) * 96 + (i & 31); }
 
 struct BArgs {
     // matrices
@@ -166,7 +177,8 @@ struct BArgs {
     const int32_t *r_ext, *c_ext;
     // instances
     const int32_t* inst_mat;
-    const int64_t *x_off, *y_off;
+    const int64_t *x_off, *y_off;    // vectors
+    const int64_t *xp_off, *yp_off;  // column / row records
     const double *b, *c, *lb, *ub;
     double *bnorm, *cnorm;  // written by the init kernel
     const uint8_t* is_eq;
@@ -264,65 +276,6 @@ __device__ __forceinline__ VT ell_dot_vg(const VT* __restrict__ v, const uint16_
     return s;
 }
 
-template <typename MT, int W>
-__device__ __forceinline__ MT ell_dot(const MT* __restrict__ v, const uint16_t* __restrict__ ix, int len,
-                                      const MT* __restrict__ g) {
-    return ell_dot_vg<MT, MT, W>(v, ix, len, g);
-}
-
-// ell_dot for two instances of one matrix: every value and index load of the slice
-// feeds a gather from each instance's operand (g0, g1) and two independent sums, each
-// in the entry order of ell_dot (the same results as two ell_dot calls).
-template <typename MT, int W>
-__device__ __forceinline__ void ell_dot2(const MT* __restrict__ v, const uint16_t* __restrict__ ix, int len,
-                                         const MT* __restrict__ g0, const MT* __restrict__ g1, MT& s0, MT& s1) {
-    constexpr int B = sizeof(MT) == 4 ? 8 : 4;
-    MT a0 = (MT)0, a1 = (MT)0;
-    if constexpr (W == 1) {
-        for (int q = 0; q < len; q += B) {
-            MT vv[B];
-            unsigned ii[B];
-#pragma unroll
-            for (int u = 0; u < B; ++u) {
-                const bool h = q + u < len;
-                vv[u] = h ? v[(q + u) * 32] : (MT)0;
-                ii[u] = h ? (unsigned)ix[(q + u) * 32] : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < B; ++u)
-                if (q + u < len) {
-                    a0 += vv[u] * g0[ii[u]];
-                    a1 += vv[u] * g1[ii[u]];
-                }
-        }
-    } else {
-        typedef typename std::conditional<sizeof(MT) == 4, float2, double2>::type MT2;
-        constexpr int P = B / 2;
-        const int np = len >> 1;
-        for (int t = 0; t < np; t += P) {
-            MT2 vv[P];
-            unsigned ii[P];
-#pragma unroll
-            for (int u = 0; u < P; ++u) {
-                const bool h = t + u < np;
-                vv[u] = h ? *reinterpret_cast<const MT2*>(v + (t + u) * 64) : MT2{(MT)0, (MT)0};
-                ii[u] = h ? *reinterpret_cast<const unsigned*>(ix + (t + u) * 64) : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < P; ++u)
-                if (t + u < np) {
-                    const unsigned lo = ii[u] & 0xFFFFu, hi = ii[u] >> 16;
-                    a0 += vv[u].x * g0[lo];
-                    a1 += vv[u].x * g1[lo];
-                    a0 += vv[u].y * g0[hi];
-                    a1 += vv[u].y * g1[hi];
-                }
-        }
-    }
-    s0 = a0;
-    s1 = a1;
-}
-
 // Entries of a CTA's slice table (column slices, then row slices; even, so what follows
 // it in shared memory stays 16-byte aligned).
 __host__ __device__ __forceinline__ int slice_tab_len(int nrs, int ncs) { return (nrs + ncs + 1) & ~1; }
@@ -368,21 +321,18 @@ __device__ MT long_slice_dot(const MT* __restrict__ vals, const int32_t* __restr
 // on inequality rows -- from the original FP64 matrix, with zero anchors (the
 // iterates restart at the centre).  Called by every thread of the owning CTA.
 template <typename MT>
-__device__ void rebuild_shifted(const BArgs& a, int m, int n, int64_t ro, int64_t co, int64_t xo, int64_t yo) {
-    ColP<MT>* colp = (ColP<MT>*)a.colp;
-    RowP<MT>* rowp = (RowP<MT>*)a.rowp;
+__device__ void rebuild_shifted(const BArgs& a, int m, int n, int64_t ro, int64_t co, int64_t xo, int64_t yo,
+                                int64_t xp, int64_t yp) {
     for (int i = threadIdx.x; i < m; i += blockDim.x) {
         const int64_t gi = ro + i;
         double s = 0.0;
         for (int e = a.rowptr[gi]; e < a.rowptr[gi + 1]; ++e) s += a.vals[e] * a.xbar[xo + a.colidx[e] - co];
         const double dri = a.dr[gi];
         a.axbar[yo + i] = s;
-        RowP<MT> r;
-        r.b = (MT)(dri * (a.b[yo + i] - s));
-        r.lo = a.is_eq[yo + i] ? (MT)(-INFINITY) : (MT)(-a.ybar[yo + i] / dri);
-        r.a = (MT)0;
-        r.pad = (MT)0;
-        rowp[yo + i] = r;
+        MT* r = (MT*)a.rowp + yp + row_rec(i);
+        r[0] = (MT)(dri * (a.b[yo + i] - s));
+        r[32] = a.is_eq[yo + i] ? (MT)(-INFINITY) : (MT)(-a.ybar[yo + i] / dri);
+        r[64] = (MT)0;
     }
     for (int j = threadIdx.x; j < n; j += blockDim.x) {
         const int64_t gj = co + j;
@@ -390,35 +340,33 @@ __device__ void rebuild_shifted(const BArgs& a, int m, int n, int64_t ro, int64_
         for (int e = a.t_rowptr[gj]; e < a.t_rowptr[gj + 1]; ++e) s += a.t_vals[e] * a.ybar[yo + a.t_colidx[e] - ro];
         const double dcj = a.dc[gj], xb = a.xbar[xo + j];
         a.atybar[xo + j] = s;
-        ColP<MT> p;
-        p.c = (MT)(dcj * (a.c[xo + j] + s));
-        p.l = (MT)((a.lb[xo + j] - xb) / dcj);
-        p.u = (MT)((a.ub[xo + j] - xb) / dcj);
-        p.a = (MT)0;
-        colp[xo + j] = p;
+        MT* p = (MT*)a.colp + xp + col_rec(j);
+        p[0] = (MT)(dcj * (a.c[xo + j] + s));
+        p[32] = (MT)((a.lb[xo + j] - xb) / dcj);
+        p[64] = (MT)((a.ub[xo + j] - xb) / dcj);
+        p[96] = (MT)0;
     }
 }
 
 // Restart of one instance after its check decided so, by every thread of the owning
 // CTA (ys: its dual iterate in shared memory): z <- anchor <- T(z), or, re-centred,
 // T(z) becomes the new FP64 centre and the shifted problem is rebuilt around it.
-template <typename MT>
-__device__ __forceinline__ void restart_instance(const BArgs& a, int m, int n, int64_t ro, int64_t co, int64_t xo,
-                                              int64_t yo, MT* ys) {
+// Element i of the dual iterate is ys[YS i].
+template <typename MT, int YS>
+__device__ __noinline__ void restart_instance(const BArgs& a, int m, int n, int64_t ro, int64_t co, int64_t xo,
+                                              int64_t yo, int64_t xp, int64_t yp, MT* ys) {
     const int tid = threadIdx.x, nt = blockDim.x;
-    ColP<MT>* colp = (ColP<MT>*)a.colp;
-    RowP<MT>* rowp = (RowP<MT>*)a.rowp;
     MT *xg = (MT*)a.x, *xtg = (MT*)a.xt, *ytg = (MT*)a.yt;
     if (!a.recenter) {
         for (int j = tid; j < n; j += nt) {
             const MT v = xtg[xo + j];
             xg[xo + j] = v;
-            colp[xo + j].a = v;
+            ((MT*)a.colp)[xp + col_rec(j) + 96] = v;
         }
         for (int i = tid; i < m; i += nt) {
             const MT v = ytg[yo + i];
-            ys[i] = v;
-            rowp[yo + i].a = v;
+            ys[YS * i] = v;
+            ((MT*)a.rowp)[yp + row_rec(i) + 64] = v;
         }
     } else {
         for (int j = tid; j < n; j += nt) {
@@ -428,11 +376,11 @@ __device__ __forceinline__ void restart_instance(const BArgs& a, int m, int n, i
         }
         for (int i = tid; i < m; i += nt) {
             a.ybar[yo + i] += a.dr[ro + i] * (double)ytg[yo + i];
-            ys[i] = (MT)0;
+            ys[YS * i] = (MT)0;
             ytg[yo + i] = (MT)0;
         }
         __syncthreads();
-        rebuild_shifted<MT>(a, m, n, ro, co, xo, yo);
+        rebuild_shifted<MT>(a, m, n, ro, co, xo, yo, xp, yp);
     }
 }
 
@@ -608,453 +556,649 @@ __device__ __noinline__ void check_instance(const BArgs& a, int inst, int m, int
     }
 }
 
-// Body of the persistent chunk kernel; launched as k_batch_chunk (the tuned CTA
-// size, up to 512 threads, two CTAs per SM) while many instances are active and as
-// k_batch_chunk_wide (1024 threads, one CTA per SM) once no more than one instance
-// per SM is left, so the last, slowest instances iterate with twice the threads.
-template <typename MT, int W>
-__device__ __forceinline__ void batch_chunk_body(const BArgs& a, int chunk) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ double red[32 * 7];
-    __shared__ InstCtrl sc;
-    __shared__ int s_q;
-    __shared__ int s_flags[2];  // 0: done, 1: restart
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-    const MT* sv = (const MT*)a.sv;
-    const MT* stv = (const MT*)a.stv;
-    const MT* rev = (const MT*)a.r_ev;
-    const MT* cev = (const MT*)a.c_ev;
-    ColP<MT>* colp = (ColP<MT>*)a.colp;
-    RowP<MT>* rowp = (RowP<MT>*)a.rowp;
-    MT *xg = (MT*)a.x, *xtg = (MT*)a.xt, *yg = (MT*)a.y, *ytg = (MT*)a.yt;
-    MT *dxg = (MT*)a.dx, *dyg = (MT*)a.dy;
-    const bool rays = a.eps_inf > 0.0;
-    const int active_count = a.counters[1];
-    const MT rho = (MT)a.rho, one_rho = (MT)(1.0 + a.rho);
-    while (true) {
-        if (tid == 0) s_q = atomicAdd(&a.counters[0], 1);
-        __syncthreads();
-        const int q = s_q;
-        if (q >= active_count) break;
-        const int inst = a.active[q];
-        const int mat = a.inst_mat[inst];
-        const int m = a.mat_m[mat], n = a.mat_n[mat];
-        const int64_t ro = a.mat_row_off[mat], co = a.mat_col_off[mat];
-        const int64_t xo = a.x_off[inst], yo = a.y_off[inst];
-        const int64_t* rsp = a.r_sptr + a.mat_rs_off[mat];
-        const int64_t* csp = a.c_sptr + a.mat_cs_off[mat];
-        const int nrs = (m + 31) >> 5, ncs = (n + 31) >> 5;
-        const double eta = a.mat_eta[mat];
-        int2* tab = (int2*)smem_raw;  // column slices, then row slices
-        MT* ys = (MT*)(tab + slice_tab_len(nrs, ncs));
-        MT* xhs = ys + ((m + 3) & ~3);
-        fill_slice_tab(tab, csp, ncs, rsp, nrs);
-        if (tid == 0) sc = a.ictrl[inst];
-        for (int i = tid; i < m; i += nt) ys[i] = yg[yo + i];
-        __syncthreads();
-        long long kk = sc.k, total = sc.total;
-        bool first = sc.first != 0;
-        double om = sc.omega;
-        __syncthreads();  // every thread holds its copy before thread 0 writes sc again
-        bool done = false;
-        for (int it = 0; it < chunk && !done; ++it) {
-            const bool check = ((total + 1) % a.K) == 0;
-            const bool stats = first || check;
-            const MT tau = (MT)(eta / om), sigma = (MT)(eta * om);
-            const MT wk = (MT)((kk + 1.0) / (kk + 2.0)), wa = (MT)(1.0 / (kk + 2.0));
-            double acc[4] = {0, 0, 0, 0};  // |x - T(x)|^2 and |y - T(y)|^2 (first or check), distances to anchors
-            // ---- primal phase: one thread per column, gathers y from shared memory; slices
-            // (longest first) are dealt to the warps boustrophedon-wise, which evens out the
-            // warps' load round trips before the barrier
-            for (int r = 0, sl = warp; sl < ncs; ++r, sl = snake_slice(r, warp, nwarps)) {
-                const int j = (sl << 5) + lane;
-                const bool valid = j < n;
-                ColP<MT> p;
-                MT x0 = (MT)0;
-                if (valid) {
-                    p = colp[xo + j];
-                    x0 = xg[xo + j];
-                }
-                const int2 t = tab[sl];
-                const int p0 = t.x, len = t.y;
-                const MT s = len <= kLongSlice
-                                 ? ell_dot<MT, W>(cev + p0 + W * lane, a.c_eidx + p0 + W * lane, len, ys)
-                                 : long_slice_dot<MT>(stv, a.t_rowptr, a.t_colidx, co + (sl << 5), min(32, n - (sl << 5)),
-                                                      ro, ys, lane);
-                if (valid) {
-                    const MT xt = clampT(x0 - tau * (p.c + s), p.l, p.u);
-                    xhs[j] = (MT)2 * xt - x0;
-                    xg[xo + j] = wk * (one_rho * xt - rho * x0) + wa * p.a;
-                    if (stats) {
-                        const double d = (double)x0 - (double)xt;
-                        acc[0] += d * d;
-                    }
-                    if (check) {
-                        xtg[xo + j] = xt;
-                        if (rays) dxg[xo + j] = xt - x0;
-                        const double e = (double)xt - (double)p.a;
-                        acc[1] += e * e;
-                    }
-                }
-            }
-            __syncthreads();
-            // ---- dual phase: one thread per row, gathers xh from shared memory
-            for (int r = 0, sl = warp; sl < nrs; ++r, sl = snake_slice(r, warp, nwarps)) {
-                const int i = (sl << 5) + lane;
-                const bool valid = i < m;
-                RowP<MT> p;
-                if (valid) p = rowp[yo + i];
-                const int2 t = tab[ncs + sl];
-                const int p0 = t.x, len = t.y;
-                const MT s = len <= kLongSlice
-                                 ? ell_dot<MT, W>(rev + p0 + W * lane, a.r_eidx + p0 + W * lane, len, xhs)
-                                 : long_slice_dot<MT>(sv, a.rowptr, a.colidx, ro + (sl << 5), min(32, m - (sl << 5)),
-                                                      co, xhs, lane);
-                if (valid) {
-                    const MT y0 = ys[i];
-                    MT yt = y0 + sigma * (s - p.b);
-                    if (yt < p.lo) yt = p.lo;  // NaN stays NaN
-                    ys[i] = wk * (one_rho * yt - rho * y0) + wa * p.a;
-                    if (stats) {
-                        const double d = (double)y0 - (double)yt;
-                        acc[2] += d * d;
-                    }
-                    if (check) {
-                        ytg[yo + i] = yt;
-                        if (rays) {  // a dual ray candidate keeps y >= 0 on <= rows (p.lo = -inf on = rows)
-                            MT d = yt - y0;
-                            if (p.lo != (MT)(-INFINITY) && d < (MT)0) d = (MT)0;
-                            dyg[yo + i] = d;
-                        }
-                        const double e = (double)yt - (double)p.a;
-                        acc[3] += e * e;
-                    }
-                }
-            }
-            kk += 1;
-            total += 1;
-            if (!stats) {
-                __syncthreads();
-                continue;
-            }
-            block_sums<4>(acc, red);
-            const bool was_first = first;
-            first = false;
-            if (!check) {  // first iteration after a (re)start: the restart reference residual
-                if (tid == 0) {
-                    sc.r0 = sqrt(om * acc[0] + acc[2] / om);
-                    sc.rprev = sc.r0;
-                }
-                __syncthreads();
-                continue;
-            }
-            double r_now = 0, dxa = 0, dya = 0;
-            if (tid == 0) {
-                r_now = sqrt(om * acc[0] + acc[2] / om);
-                if (was_first) {
-                    sc.r0 = r_now;
-                    sc.rprev = r_now;
-                }
-                dxa = sqrt(acc[1]);
-                dya = sqrt(acc[3]);
-            }
-            __syncthreads();  // xt / yt of this iteration are in global memory
-            check_instance<MT, W>(a, inst, m, n, ro, co, xo, yo, total, kk, om, r_now, dxa, dya, sc, s_flags, red,
-                                  tab, xhs);
-            __syncthreads();
-            done = s_flags[0] != 0;
-            om = sc.omega;
-            if (s_flags[1]) {
-                kk = 0;
-                first = true;
-                restart_instance<MT>(a, m, n, ro, co, xo, yo, ys);
-            }
-            __syncthreads();
-        }
-        // store the dual iterate and the control block
-        for (int i = tid; i < m; i += nt) yg[yo + i] = ys[i];
-        if (tid == 0) {
-            sc.k = kk;
-            sc.total = total;
-            sc.first = first ? 1 : 0;
-            a.ictrl[inst] = sc;
-        }
-        __syncthreads();
+// The NI operands of gather index i: element i of instance k is stored at NI i + k, so one
+// 4-, 8- or 16-byte shared-memory load serves all NI instances.
+template <typename MT, int NI>
+__device__ __forceinline__ void ld_group(const MT* __restrict__ g, unsigned i, MT (&t)[NI]) {
+    if constexpr (NI == 1) {
+        t[0] = g[i];
+    } else if constexpr (sizeof(MT) == 4 && NI == 4) {
+        const float4 q = reinterpret_cast<const float4*>(g)[i];
+        t[0] = q.x; t[1] = q.y; t[2] = q.z; t[3] = q.w;
+    } else if constexpr (sizeof(MT) == 4) {
+        static_assert(NI == 2, "a group holds 1, 2 or 4 instances");
+        const float2 q = reinterpret_cast<const float2*>(g)[i];
+        t[0] = q.x; t[1] = q.y;
+    } else {
+        static_assert(NI == 2, "an FP64 group holds 1 or 2 instances");
+        const double2 q = reinterpret_cast<const double2*>(g)[i];
+        t[0] = q.x; t[1] = q.y;
+    }
+}
+template <typename MT, int NI>
+__device__ __forceinline__ void st_group(MT* g, int i, const MT (&t)[NI]) {
+    if constexpr (NI == 1)
+        g[i] = t[0];
+    else if constexpr (sizeof(MT) == 4 && NI == 4)
+        reinterpret_cast<float4*>(g)[i] = make_float4(t[0], t[1], t[2], t[3]);
+    else if constexpr (sizeof(MT) == 4)
+        reinterpret_cast<float2*>(g)[i] = make_float2(t[0], t[1]);
+    else
+        reinterpret_cast<double2*>(g)[i] = make_double2(t[0], t[1]);
+}
+
+// One row summed by the whole warp over the CSR copy, for the NI interleaved operands of a
+// group (each entry is read once); every lane returns the sums.
+template <typename MT, int NI>
+__device__ __forceinline__ void long_row_group(const MT* __restrict__ vals, const int32_t* __restrict__ idx, int e0,
+                                               int e1, int64_t off, const MT* __restrict__ g, int lane, MT (&s)[NI]) {
+#pragma unroll
+    for (int k = 0; k < NI; ++k) s[k] = (MT)0;
+#pragma unroll 4
+    for (int e = e0 + lane; e < e1; e += 32) {
+        const MT v = vals[e];
+        MT t[NI];
+        ld_group<MT, NI>(g, (unsigned)(idx[e] - off), t);
+#pragma unroll
+        for (int k = 0; k < NI; ++k) s[k] += v * t[k];
+    }
+#pragma unroll
+    for (int k = 0; k < NI; ++k)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+}
+
+// The rows of one slice (long_slice_dot for a group): lane r returns the sums of row first + r.
+template <typename MT, int NI>
+__device__ __forceinline__ void long_slice_group(const MT* __restrict__ vals, const int32_t* __restrict__ ptr,
+                                                 const int32_t* __restrict__ idx, int64_t first, int cnt, int64_t off,
+                                                 const MT* __restrict__ g, int lane, MT (&mine)[NI]) {
+#pragma unroll 1
+    for (int r = 0; r < cnt; ++r) {
+        MT s[NI];
+        long_row_group<MT, NI>(vals, idx, ptr[first + r], ptr[first + r + 1], off, g, lane, s);
+#pragma unroll
+        for (int k = 0; k < NI; ++k)
+            if (lane == r) mine[k] = s[k];
     }
 }
 
-template <typename MT, int W>
-__global__ void __launch_bounds__(512, 2) k_batch_chunk(const __grid_constant__ BArgs a, int chunk) {
-    batch_chunk_body<MT, W>(a, chunk);
+// One batch of a lane's entries of a slice (entries q .. q + B - 1 of its len), loaded
+// before it is needed: the iteration loop issues the next batch (of this slice, or the
+// first one of the warp's next slice) before it gathers for the current one, so the L2
+// round trip of the matrix stream overlaps the gathers.
+template <typename VT, int W, int B>
+struct EllBatch {
+    VT v[B];
+    unsigned i[W == 1 ? B : B / 2];
+    __device__ __forceinline__ void load_at(const VT* __restrict__ pv, const uint16_t* __restrict__ pi, int u) {
+        if constexpr (W == 1) {
+            v[u] = pv[u * 32];
+            i[u] = pi[u * 32];
+        } else if (!(u & 1)) {
+            typedef typename std::conditional<sizeof(VT) == 4, float2, double2>::type VT2;
+            const VT2 t = *reinterpret_cast<const VT2*>(pv + u * 32);
+            v[u] = t.x;
+            v[u + 1] = t.y;
+            i[u / 2] = *reinterpret_cast<const unsigned*>(pi + u * 32);
+        }
+    }
+    // pv, pi: the lane's first entry; lengths are even
+    __device__ __forceinline__ void load(const VT* __restrict__ pv, const uint16_t* __restrict__ pi, int q, int len) {
+        pv += q * 32;
+        pi += q * 32;
+        if (q + B <= len) {
+#pragma unroll
+            for (int u = 0; u < B; ++u) load_at(pv, pi, u);
+        } else {
+#pragma unroll
+            for (int u = 0; u < B; ++u)
+                if (q + (u & ~1) < len) load_at(pv, pi, u);
+        }
+    }
+    template <int NI>
+    __device__ __forceinline__ void add_at(int u, const VT* __restrict__ g, VT (&s)[NI]) const {
+        const unsigned idx = W == 1 ? i[u] : ((u & 1) ? i[u / 2] >> 16 : i[u / 2] & 0xFFFFu);
+        VT t[NI];
+        ld_group<VT, NI>(g, idx, t);
+#pragma unroll
+        for (int k = 0; k < NI; ++k) s[k] += v[u] * t[k];
+    }
+    // s[k] += entry * g[NI index + k], in entry order
+    template <int NI>
+    __device__ __forceinline__ void add(int q, int len, const VT* __restrict__ g, VT (&s)[NI]) const {
+        if (q + B <= len) {
+#pragma unroll
+            for (int u = 0; u < B; ++u) add_at<NI>(u, g, s);
+        } else {
+#pragma unroll
+            for (int u = 0; u < B; u += 2) {
+                if (q + u >= len) break;
+                add_at<NI>(u, g, s);
+                add_at<NI>(u + 1, g, s);
+            }
+        }
+    }
+};
+
+// One instance of a group: what the iterations need of it, in shared memory.
+template <typename MT>
+struct alignas(16) GroupInst {
+    MT par[2][4];  // tau, sigma and the Halpern weights wk, wa of the even / odd iterations
+    long long xo, yo, xp, yp;  // offsets of its vectors and of its column / row records
+    int inst;                  // -1: an empty slot of the last group
+    int stat;                  // this iteration gives its restart reference residual (1) or is its check (2)
+};
+
+// Parameters of an instance's next iteration (one thread per instance).
+template <typename MT>
+__device__ __forceinline__ void group_params(GroupInst<MT>& g, const InstCtrl& sc, int slot, double eta) {
+    g.par[slot][0] = (MT)(eta / sc.omega);
+    g.par[slot][1] = (MT)(eta * sc.omega);
+    g.par[slot][2] = (MT)((sc.k + 1.0) / (sc.k + 2.0));
+    g.par[slot][3] = (MT)(1.0 / (sc.k + 2.0));
 }
 
-template <typename MT, int W>
-__global__ void __launch_bounds__(1024, 1) k_batch_chunk_wide(const __grid_constant__ BArgs a, int chunk) {
-    batch_chunk_body<MT, W>(a, chunk);
+// Iteration (counted within this launch, from `it` on) of the next reference residual or
+// check of any live instance; INT_MAX when none is live.
+template <typename MT, int NI>
+__device__ __forceinline__ int group_next_stat(const GroupInst<MT>* gi, const InstCtrl* sc, int it, int K) {
+    int nx = INT_MAX;
+#pragma unroll
+    for (int k = 0; k < NI; ++k)
+        if (gi[k].inst >= 0 && !sc[k].done) nx = min(nx, sc[k].first ? it : it + (K - 1) - (int)(sc[k].total % K));
+    return nx;
 }
 
-// Paired form of the chunk kernel for a batch whose instances all share one matrix
-// (a parametric family): a CTA takes two consecutive entries of the active list and
-// iterates both instances in lockstep, so every SELL value and index load of the
-// shared matrix feeds both instances' gathers (ell_dot2) -- the matrix bytes per
-// instance-iteration halve and each warp carries two independent sums per load.
-// Shared memory holds y and xh of both instances.  Per instance everything is as in
-// batch_chunk_body, with the same thread-to-column/row assignment and arithmetic, so
-// the iterates and decisions are those of the single form bit for bit.  An instance
-// that finishes leaves its partner to iterate alone (single gathers) until the chunk
-// ends; the compaction between chunks re-pairs the survivors.
-template <typename MT, int W>
-__device__ __forceinline__ void batch_pair_body(const BArgs& a, int chunk) {
+// The matrix a CTA iterates on.  Dynamic shared memory holds the slice table (column slices,
+// then row slices), the interleaved dual iterates ys and the extrapolated primal points xh;
+// they are addressed from the array itself, by offsets, so that every access is known to be
+// to shared memory.
+struct GroupView {
+    int m, n, ncs, nrs;
+    int ys_off, xh_off;  // bytes
+    int nlc, nlr;        // long column / row slices (they come first)
+    int64_t ro, co;
+    double eta;
+};
+// Bytes of the per-instance blocks in front of the slice table.
+template <typename MT>
+__host__ __device__ constexpr int group_head(int ni) {
+    return (int)((ni * (sizeof(GroupInst<MT>) + sizeof(InstCtrl)) + 15) & ~(size_t)15);
+}
+template <typename T>
+__device__ __forceinline__ T* smem_at(int off) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ double red[32 * 7];
-    __shared__ InstCtrl sc[2];
+    return reinterpret_cast<T*>(smem_raw + off);
+}
+
+// x of the next iteration from this one's extrapolation h = 2 T(x) - x (reflection 1):
+// wk h + wa anchor.
+template <typename MT>
+__device__ __forceinline__ MT halpern_point(MT wk, MT h, MT wa, MT anchor) {
+    if constexpr (sizeof(MT) == 4) return __fmaf_rn(wk, h, __fmul_rn(wa, anchor));
+    else return __fma_rn(wk, h, __dmul_rn(wa, anchor));
+}
+
+// What a plain iteration reads of the launch's arguments, passed by value.
+template <typename MT>
+struct IterPtrs {
+    const MT *c_ev, *r_ev, *colp, *rowp;
+    const uint16_t *c_eidx, *r_eidx;
+    const BArgs* a;  // everything else (long slices, general iterations)
+    MT rho, one_rho;
+    bool anchors;  // re-centred iterates restart at 0: no anchors
+};
+
+// The slices with rows (columns) longer than kLongSlice in a plain iteration: their rows are
+// dealt to all warps of the CTA, each summed by a whole warp over the CSR copy, so a dense
+// row stalls neither its slice nor one warp.  Out of line and outside the slice loop, which
+// then holds no call.
+template <typename MT, int NI, bool PRIMAL>
+__device__ __noinline__ void long_slices(const IterPtrs<MT> ip, int slot, const GroupView gv) {
+    const BArgs& a = *ip.a;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const GroupInst<MT>* gi = smem_at<GroupInst<MT>>(0);
+    MT *ys = smem_at<MT>(gv.ys_off), *xh = smem_at<MT>(gv.xh_off);
+    const int rows = PRIMAL ? min(gv.n, gv.nlc << 5) : min(gv.m, gv.nlr << 5);
+#pragma unroll 1
+    for (int i = warp; i < rows; i += nwarps) {
+        MT s[NI], v[NI];
+        if (PRIMAL)
+            long_row_group<MT, NI>((const MT*)a.stv, a.t_colidx, a.t_rowptr[gv.co + i], a.t_rowptr[gv.co + i + 1], gv.ro,
+                                   ys, lane, s);
+        else
+            long_row_group<MT, NI>((const MT*)a.sv, a.colidx, a.rowptr[gv.ro + i], a.rowptr[gv.ro + i + 1], gv.co, xh,
+                                   lane, s);
+        if (lane != 0) continue;
+        ld_group<MT, NI>(PRIMAL ? xh : ys, i, v);
+#pragma unroll
+        for (int k = 0; k < NI; ++k) {
+            const MT* par = gi[k].par[slot];
+            if (PRIMAL) {
+                const MT* q = ip.colp + gi[k].xp + col_rec(i);
+                const MT x0 = halpern_point<MT>(gi[k].par[slot ^ 1][2], v[k], gi[k].par[slot ^ 1][3],
+                                                ip.anchors ? q[96] : (MT)0);
+                v[k] = (MT)2 * clampT(x0 - par[0] * (q[0] + s[k]), q[32], q[64]) - x0;
+            } else {
+                const MT* q = ip.rowp + gi[k].yp + row_rec(i);
+                MT yt = v[k] + par[1] * (s[k] - q[0]);
+                if (yt < q[32]) yt = q[32];
+                v[k] = halpern_point<MT>(par[2], ip.one_rho * yt - ip.rho * v[k], par[3], ip.anchors ? q[64] : (MT)0);
+            }
+        }
+        st_group<MT, NI>(PRIMAL ? xh : ys, i, v);
+    }
+}
+
+// One PDHG iteration of a group of NI instances of one matrix.
+// GEN = false: a plain iteration with reflection 1.  x is not in memory: it is
+// wk h + wa anchor of the previous iteration's xh, which is still in shared memory, so a
+// column costs its record (c, l, u; the anchor only where it is not 0) and no more.
+// GEN = true: any iteration.  ldx / stx: x is read from / written to memory (around a
+// check, which overwrites xh, at the ends of a launch, and always when the reflection is
+// not 1); gi[].stat names the instances whose residual sums are taken (into acc, per warp)
+// and whose T(z) and displacement are stored for the check.
+template <typename MT, int W, int NI, int B, bool GEN, bool PIPE, bool LONG>
+__device__ __forceinline__ void iteration_body(const IterPtrs<MT> ip, int slot, const GroupView gv,
+                                               double (*acc)[NI][4], bool ldx, bool stx) {
+    const BArgs& a = *ip.a;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const MT rho = ip.rho, one_rho = ip.one_rho;
+    const bool rays = GEN && a.eps_inf > 0.0;
+    GroupInst<MT>* gi = smem_at<GroupInst<MT>>(0);
+    InstCtrl* sc = smem_at<InstCtrl>(NI * (int)sizeof(GroupInst<MT>));
+    const int2* tab = smem_at<const int2>(group_head<MT>(NI));
+    MT* ys = smem_at<MT>(gv.ys_off);
+    MT* xh = smem_at<MT>(gv.xh_off);
+    double st[NI][2];
+    if (GEN)
+#pragma unroll
+        for (int k = 0; k < NI; ++k) st[k][0] = st[k][1] = 0.0;
+    if (LONG && gv.nlc > 0) long_slices<MT, NI, true>(ip, slot, gv);
+    // ---- primal phase: one thread per column, gathers y.  Slices (longest first) are dealt
+    // to the warps boustrophedon-wise, which evens out their work before the barrier.
+    {
+        const MT* ev = ip.c_ev + W * lane;
+        const uint16_t* ei = ip.c_eidx + W * lane;
+        const MT* rec[NI];
+        MT tau[NI], wk[NI], wa[NI];
+#pragma unroll
+        for (int k = 0; k < NI; ++k) {
+            rec[k] = ip.colp + gi[k].xp + lane;
+            tau[k] = gi[k].par[slot][0];
+            wk[k] = gi[k].par[slot ^ 1][2];  // of the previous iteration
+            wa[k] = gi[k].par[slot ^ 1][3];
+        }
+        EllBatch<MT, W, B> cur, nxt;
+        int r = 0, sl = warp;
+        if (LONG)
+            while (sl < gv.nlc) sl = snake_slice(++r, warp, nwarps);  // done by long_slices
+        int2 t = sl < gv.ncs ? tab[sl] : make_int2(0, 0);
+        if (PIPE) cur.load(ev + t.x, ei + t.x, 0, t.y);
+#pragma unroll 1
+        for (; sl < gv.ncs; ++r) {
+            const int j = (sl << 5) + lane;
+            const bool valid = j < gv.n;
+            MT c[NI], l[NI], u[NI], an[NI];
+#pragma unroll
+            for (int k = 0; k < NI; ++k) {  // records are padded to whole slices
+                const MT* q = rec[k] + (size_t)sl * 128;
+                c[k] = q[0];
+                l[k] = q[32];
+                u[k] = q[64];
+                an[k] = ip.anchors ? q[96] : (MT)0;
+            }
+            const int sl2 = snake_slice(r + 1, warp, nwarps);
+            const int2 t2 = sl2 < gv.ncs ? tab[sl2] : make_int2(0, 0);
+            MT s[NI];
+#pragma unroll
+            for (int k = 0; k < NI; ++k) s[k] = (MT)0;
+            if (!GEN || t.y <= kLongSlice) {
+                int q = 0;
+                if (PIPE) {
+#pragma unroll 1
+                    for (; q + B < t.y; q += B) {
+                        nxt.load(ev + t.x, ei + t.x, q + B, t.y);
+                        cur.template add<NI>(q, t.y, ys, s);
+                        cur = nxt;
+                    }
+                    nxt.load(ev + t2.x, ei + t2.x, 0, t2.y);
+                    cur.template add<NI>(q, t.y, ys, s);
+                } else {
+#pragma unroll 1
+                    for (; q < t.y; q += B) {
+                        cur.load(ev + t.x, ei + t.x, q, t.y);
+                        cur.template add<NI>(q, t.y, ys, s);
+                    }
+                }
+            } else {
+                long_slice_group<MT, NI>((const MT*)a.stv, a.t_rowptr, a.t_colidx, gv.co + (sl << 5),
+                                         min(32, gv.n - (sl << 5)), gv.ro, ys, lane, s);
+            }
+            if (valid) {
+                MT h[NI];
+                if (!GEN || !ldx) ld_group<MT, NI>(xh, j, h);
+#pragma unroll
+                for (int k = 0; k < NI; ++k) {
+                    const MT x0 = (GEN && ldx) ? ((const MT*)a.x)[gi[k].xo + j]
+                                               : halpern_point<MT>(wk[k], h[k], wa[k], an[k]);
+                    const MT xt = clampT(x0 - tau[k] * (c[k] + s[k]), l[k], u[k]);
+                    h[k] = (MT)2 * xt - x0;
+                    if (GEN) {
+                        const int stat = gi[k].stat;
+                        if (stx && gi[k].inst >= 0 && !sc[k].done)
+                            ((MT*)a.x)[gi[k].xo + j] = halpern_point<MT>(gi[k].par[slot][2], one_rho * xt - rho * x0,
+                                                                         gi[k].par[slot][3], an[k]);
+                        if (stat) {
+                            const double d = (double)x0 - (double)xt;
+                            st[k][0] += d * d;
+                        }
+                        if (stat == 2) {
+                            ((MT*)a.xt)[gi[k].xo + j] = xt;
+                            if (rays) ((MT*)a.dx)[gi[k].xo + j] = xt - x0;
+                            const double e = (double)xt - (double)an[k];
+                            st[k][1] += e * e;
+                        }
+                    }
+                }
+                st_group<MT, NI>(xh, j, h);
+            }
+            if (PIPE) cur = nxt;
+            t = t2;
+            sl = sl2;
+        }
+    }
+    if (GEN)
+#pragma unroll
+        for (int k = 0; k < NI; ++k) {
+            st[k][0] = warp_sum(st[k][0]);
+            st[k][1] = warp_sum(st[k][1]);
+            if (lane == 0) {
+                acc[warp][k][0] = st[k][0];
+                acc[warp][k][1] = st[k][1];
+            }
+            st[k][0] = st[k][1] = 0.0;
+        }
+    __syncthreads();
+    if (LONG && gv.nlr > 0) long_slices<MT, NI, false>(ip, slot, gv);
+    // ---- dual phase: one thread per row, gathers xh
+    {
+        const MT* ev = ip.r_ev + W * lane;
+        const uint16_t* ei = ip.r_eidx + W * lane;
+        const MT* rec[NI];
+        MT sigma[NI], wk[NI], wa[NI];
+#pragma unroll
+        for (int k = 0; k < NI; ++k) {
+            rec[k] = ip.rowp + gi[k].yp + lane;
+            sigma[k] = gi[k].par[slot][1];
+            wk[k] = gi[k].par[slot][2];
+            wa[k] = gi[k].par[slot][3];
+        }
+        // the next iteration's parameters, in the slot whose last reads are behind the barrier
+        if (tid < NI && !sc[tid].done) {
+            sc[tid].k += 1;
+            sc[tid].total += 1;
+            group_params<MT>(gi[tid], sc[tid], slot ^ 1, gv.eta);
+        }
+        EllBatch<MT, W, B> cur, nxt;
+        int r = 0, sl = warp;
+        if (LONG)
+            while (sl < gv.nlr) sl = snake_slice(++r, warp, nwarps);
+        int2 t = sl < gv.nrs ? tab[gv.ncs + sl] : make_int2(0, 0);
+        if (PIPE) cur.load(ev + t.x, ei + t.x, 0, t.y);
+#pragma unroll 1
+        for (; sl < gv.nrs; ++r) {
+            const int i = (sl << 5) + lane;
+            const bool valid = i < gv.m;
+            MT b[NI], lo[NI], an[NI];
+#pragma unroll
+            for (int k = 0; k < NI; ++k) {
+                const MT* q = rec[k] + (size_t)sl * 96;
+                b[k] = q[0];
+                lo[k] = q[32];
+                an[k] = ip.anchors ? q[64] : (MT)0;
+            }
+            const int sl2 = snake_slice(r + 1, warp, nwarps);
+            const int2 t2 = sl2 < gv.nrs ? tab[gv.ncs + sl2] : make_int2(0, 0);
+            MT s[NI];
+#pragma unroll
+            for (int k = 0; k < NI; ++k) s[k] = (MT)0;
+            if (!GEN || t.y <= kLongSlice) {
+                int q = 0;
+                if (PIPE) {
+#pragma unroll 1
+                    for (; q + B < t.y; q += B) {
+                        nxt.load(ev + t.x, ei + t.x, q + B, t.y);
+                        cur.template add<NI>(q, t.y, xh, s);
+                        cur = nxt;
+                    }
+                    nxt.load(ev + t2.x, ei + t2.x, 0, t2.y);
+                    cur.template add<NI>(q, t.y, xh, s);
+                } else {
+#pragma unroll 1
+                    for (; q < t.y; q += B) {
+                        cur.load(ev + t.x, ei + t.x, q, t.y);
+                        cur.template add<NI>(q, t.y, xh, s);
+                    }
+                }
+            } else {
+                long_slice_group<MT, NI>((const MT*)a.sv, a.rowptr, a.colidx, gv.ro + (sl << 5),
+                                         min(32, gv.m - (sl << 5)), gv.co, xh, lane, s);
+            }
+            if (valid) {
+                MT y0[NI], h[NI];
+                ld_group<MT, NI>(ys, i, y0);
+#pragma unroll
+                for (int k = 0; k < NI; ++k) {
+                    MT yt = y0[k] + sigma[k] * (s[k] - b[k]);
+                    if (yt < lo[k]) yt = lo[k];  // NaN stays NaN
+                    h[k] = halpern_point<MT>(wk[k], one_rho * yt - rho * y0[k], wa[k], an[k]);
+                    if (GEN) {
+                        const int stat = gi[k].stat;
+                        if (stat) {
+                            const double d = (double)y0[k] - (double)yt;
+                            st[k][0] += d * d;
+                        }
+                        if (stat == 2) {
+                            ((MT*)a.yt)[gi[k].yo + i] = yt;
+                            if (rays) {  // a dual ray candidate keeps y >= 0 on <= rows (lo = -inf on = rows)
+                                MT d = yt - y0[k];
+                                if (lo[k] != (MT)(-INFINITY) && d < (MT)0) d = (MT)0;
+                                ((MT*)a.dy)[gi[k].yo + i] = d;
+                            }
+                            const double e = (double)yt - (double)an[k];
+                            st[k][1] += e * e;
+                        }
+                    }
+                }
+                st_group<MT, NI>(ys, i, h);
+            }
+            if (PIPE) cur = nxt;
+            t = t2;
+            sl = sl2;
+        }
+    }
+    if (GEN)
+#pragma unroll
+        for (int k = 0; k < NI; ++k) {
+            st[k][0] = warp_sum(st[k][0]);
+            st[k][1] = warp_sum(st[k][1]);
+            if (lane == 0) {
+                acc[warp][k][2] = st[k][0];
+                acc[warp][k][3] = st[k][1];
+            }
+        }
+    __syncthreads();
+}
+
+// The general one is out of line: its FP64 sums stay out of the plain loop's registers.
+template <typename MT, int W, int NI, int B, bool PIPE, bool LONG>
+__device__ __forceinline__ void plain_iteration(const IterPtrs<MT> ip, int slot, const GroupView gv) {
+    iteration_body<MT, W, NI, B, false, PIPE, LONG>(ip, slot, gv, nullptr, false, false);
+}
+template <typename MT, int W, int NI, int B>
+__device__ __noinline__ void general_iteration(const IterPtrs<MT> ip, int slot, const GroupView gv,
+                                               double (*acc)[NI][4], bool ldx, bool stx) {
+    iteration_body<MT, W, NI, B, true, false, false>(ip, slot, gv, acc, ldx, stx);
+}
+
+// The chunk kernel: a CTA takes NI consecutive entries of the active list at a time and
+// iterates them in lockstep for up to `chunk` iterations.  NI = 1 serves any batch.
+// NI = 2 or 4 serve a batch whose instances all share one matrix (a parametric family, the
+// nodes of a branch-and-bound search): every SELL value and index load feeds NI instances,
+// and one vector gather reads the operands of all of them.  Per instance the arithmetic and
+// the thread-to-column/row assignment do not depend on NI, so at one CTA size the
+// iterates, statuses and iteration counts are the same bit for bit in every form.  An
+// instance that finishes leaves its slot idle until the chunk ends; the compaction between
+// chunks regroups the survivors.
+// MAXT, MINB: the largest CTA size of this instantiation and the CTAs per SM it leaves
+// registers for.  PIPE: the next batch of entries is loaded ahead (groups: one CTA per SM,
+// 128 registers; a single instance at 64 registers is faster without).  LONG: the batch has
+// rows longer than kLongSlice (kept apart because a call in the plain loop costs registers).
+//
+// Bound: shared-memory wavefronts of the random gathers (16-byte gathers of 4 instances: 8.7
+// wavefronts per 32 entries against 4 without conflicts) and the L2 latency in front of
+// them.  2,000 x 8,000, 47,984 nonzeros, 1,184 instances, checks every 256 iterations, ns per
+// instance-iteration (before: one scalar gather per instance, x and 16-byte records in
+// memory): FP32 NI = 1 118 -> 92, NI = 2 103 -> 64, NI = 4 49 (10.6 k of 14.4 k SM cycles are
+// L1 wavefronts; L2 hit rate 94 % because the records without x and anchors fit); FP64 NI = 1
+// 182 -> 139, NI = 2 160 -> 114.
+template <typename MT, int W, int NI, int MAXT, int MINB, bool PIPE, bool LONG>
+__global__ void __launch_bounds__(MAXT, MINB) k_batch_chunk(const __grid_constant__ BArgs a, int chunk) {
+    constexpr int B = sizeof(MT) == 4 ? 8 : 4;
+    constexpr int kWarps = MAXT / 32;
+    __shared__ double red[kWarps * 7];
+    __shared__ double acc[kWarps][NI][4];
     __shared__ int s_q;
-    __shared__ int s_flags[2][2];  // per instance -- 0: done, 1: restart
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-    const MT* sv = (const MT*)a.sv;
-    const MT* stv = (const MT*)a.stv;
-    const MT* rev = (const MT*)a.r_ev;
-    const MT* cev = (const MT*)a.c_ev;
-    ColP<MT>* colp = (ColP<MT>*)a.colp;
-    RowP<MT>* rowp = (RowP<MT>*)a.rowp;
-    MT *xg = (MT*)a.x, *xtg = (MT*)a.xt, *yg = (MT*)a.y, *ytg = (MT*)a.yt;
-    MT *dxg = (MT*)a.dx, *dyg = (MT*)a.dy;
-    const bool rays = a.eps_inf > 0.0;
+    __shared__ int s_flags[2];  // 0: done, 1: restart
+    const int tid = threadIdx.x, nt = blockDim.x, nwarps = nt >> 5;
+    MT* yg = (MT*)a.y;
     const int active_count = a.counters[1];
-    const MT rho = (MT)a.rho, one_rho = (MT)(1.0 + a.rho);
-    // the one matrix of the batch
-    const int m = a.mat_m[0], n = a.mat_n[0];
-    const int64_t ro = a.mat_row_off[0], co = a.mat_col_off[0];
-    const int64_t* rsp = a.r_sptr + a.mat_rs_off[0];
-    const int64_t* csp = a.c_sptr + a.mat_cs_off[0];
-    const int nrs = (m + 31) >> 5, ncs = (n + 31) >> 5;
-    const double eta = a.mat_eta[0];
-    const int m4 = (m + 3) & ~3, stride = m4 + max((n + 3) & ~3, m4);  // xh region also stages y at checks
-    int2* tab = (int2*)smem_raw;  // column slices, then row slices (built once: one matrix)
-    MT* ysb[2] = {(MT*)(tab + slice_tab_len(nrs, ncs)), (MT*)(tab + slice_tab_len(nrs, ncs)) + stride};
-    MT* xhb[2] = {ysb[0] + m4, ysb[1] + m4};
-    fill_slice_tab(tab, csp, ncs, rsp, nrs);
+    const bool plain_x = a.rho == 1.0;  // x follows from xh
+    GroupInst<MT>* gi = smem_at<GroupInst<MT>>(0);
+    InstCtrl* sc = smem_at<InstCtrl>(NI * (int)sizeof(GroupInst<MT>));
+    int2* tab = smem_at<int2>(group_head<MT>(NI));
+    const IterPtrs<MT> ip{(const MT*)a.c_ev, (const MT*)a.r_ev, (const MT*)a.colp, (const MT*)a.rowp, a.c_eidx,
+                          a.r_eidx, &a, (MT)a.rho, (MT)(1.0 + a.rho), !a.recenter};
+    GroupView gv;
+    int cur_mat = -1;
     while (true) {
-        if (tid == 0) s_q = atomicAdd(&a.counters[0], 2);
+        if (tid == 0) s_q = atomicAdd(&a.counters[0], NI);
         __syncthreads();
         const int q = s_q;
         if (q >= active_count) break;
-        const bool has2 = q + 1 < active_count;
-        int inst[2];
-        inst[0] = a.active[q];
-        inst[1] = has2 ? a.active[q + 1] : inst[0];
-        bool live[2] = {true, has2};
-        int64_t xo[2], yo[2];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            xo[k] = a.x_off[inst[k]];
-            yo[k] = a.y_off[inst[k]];
+        const int mat = NI > 1 ? 0 : a.inst_mat[a.active[q]];
+        if (mat != cur_mat) {
+            cur_mat = mat;
+            gv.m = a.mat_m[mat];
+            gv.n = a.mat_n[mat];
+            gv.ro = a.mat_row_off[mat];
+            gv.co = a.mat_col_off[mat];
+            gv.nrs = (gv.m + 31) >> 5;
+            gv.ncs = (gv.n + 31) >> 5;
+            gv.eta = a.mat_eta[mat];
+            gv.ys_off = group_head<MT>(NI) + (int)sizeof(int2) * slice_tab_len(gv.nrs, gv.ncs);
+            gv.xh_off = gv.ys_off + (int)sizeof(MT) * NI * ((gv.m + 3) & ~3);  // at a check: stages max(n, m) elements
+            fill_slice_tab(tab, a.c_sptr + a.mat_cs_off[mat], gv.ncs, a.r_sptr + a.mat_rs_off[mat], gv.nrs);
         }
-        if (tid == 0) sc[0] = a.ictrl[inst[0]];
-        if (tid == 1 && has2) sc[1] = a.ictrl[inst[1]];
-#pragma unroll
-        for (int k = 0; k < 2; ++k)
-            if (live[k])
-                for (int i = tid; i < m; i += nt) ysb[k][i] = yg[yo[k] + i];
+        if (tid < NI) {
+            GroupInst<MT>& g = gi[tid];
+            const bool real = q + tid < active_count;
+            const int inst = a.active[real ? q + tid : q];
+            sc[tid] = a.ictrl[inst];
+            g.inst = real ? inst : -1;
+            g.xo = a.x_off[inst];  // an empty slot reads the first instance's vectors and writes nothing
+            g.yo = a.y_off[inst];
+            g.xp = a.xp_off[inst];
+            g.yp = a.yp_off[inst];
+            group_params<MT>(g, sc[tid], 0, gv.eta);
+        }
+        MT* ys = smem_at<MT>(gv.ys_off);
         __syncthreads();
-        long long kk[2], total[2];
-        bool first[2];
-        double om[2];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int src = live[k] ? k : 0;
-            kk[k] = sc[src].k;
-            total[k] = sc[src].total;
-            first[k] = sc[src].first != 0;
-            om[k] = sc[src].omega;
+        for (int k = 0; k < NI; ++k)
+            for (int i = tid; i < gv.m; i += nt) ys[NI * i + k] = gi[k].inst >= 0 ? yg[gi[k].yo + i] : (MT)0;
+        if (LONG) {
+            gv.nlc = gv.nlr = 0;
+            while (gv.nlc < gv.ncs && tab[gv.nlc].y > kLongSlice) ++gv.nlc;
+            while (gv.nlr < gv.nrs && tab[gv.ncs + gv.nlr].y > kLongSlice) ++gv.nlr;
         }
-        __syncthreads();  // every thread holds its copies before thread 0 writes sc again
-        for (int it = 0; it < chunk && (live[0] || live[1]); ++it) {
-            bool check[2], stats[2];
-            MT tau[2], sigma[2], wk[2], wa[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                check[k] = live[k] && ((total[k] + 1) % a.K) == 0;
-                stats[k] = live[k] && (first[k] || check[k]);
-                tau[k] = (MT)(eta / om[k]);
-                sigma[k] = (MT)(eta * om[k]);
-                wk[k] = (MT)((kk[k] + 1.0) / (kk[k] + 2.0));
-                wa[k] = (MT)(1.0 / (kk[k] + 2.0));
-            }
-            const bool both = live[0] && live[1];
-            const bool solo1 = !live[0];  // the one live instance when not both
-            const MT* ys_solo = solo1 ? ysb[1] : ysb[0];
-            const MT* xh_solo = solo1 ? xhb[1] : xhb[0];
-            double acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-            // ---- primal phase
-            for (int r = 0, sl = warp; sl < ncs; ++r, sl = snake_slice(r, warp, nwarps)) {
-                const int j = (sl << 5) + lane;
-                const bool valid = j < n;
-                ColP<MT> p[2];
-                MT x0[2] = {(MT)0, (MT)0};
-#pragma unroll
-                for (int k = 0; k < 2; ++k)
-                    if (valid && live[k]) {
-                        p[k] = colp[xo[k] + j];
-                        x0[k] = xg[xo[k] + j];
-                    }
-                const int2 tb = tab[sl];
-                const int p0 = tb.x, len = tb.y;
-                MT s[2] = {(MT)0, (MT)0};
-                if (len <= kLongSlice) {
-                    if (both)
-                        ell_dot2<MT, W>(cev + p0 + W * lane, a.c_eidx + p0 + W * lane, len, ysb[0], ysb[1], s[0], s[1]);
-                    else {
-                        const MT t = ell_dot<MT, W>(cev + p0 + W * lane, a.c_eidx + p0 + W * lane, len, ys_solo);
-                        s[0] = solo1 ? (MT)0 : t;
-                        s[1] = solo1 ? t : (MT)0;
-                    }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 2; ++k)
-                        if (live[k])
-                            s[k] = long_slice_dot<MT>(stv, a.t_rowptr, a.t_colidx, co + (sl << 5),
-                                                      min(32, n - (sl << 5)), ro, ysb[k], lane);
-                }
-#pragma unroll
-                for (int k = 0; k < 2; ++k)
-                    if (valid && live[k]) {
-                        const MT xt = clampT(x0[k] - tau[k] * (p[k].c + s[k]), p[k].l, p[k].u);
-                        xhb[k][j] = (MT)2 * xt - x0[k];
-                        xg[xo[k] + j] = wk[k] * (one_rho * xt - rho * x0[k]) + wa[k] * p[k].a;
-                        if (stats[k]) {
-                            const double d = (double)x0[k] - (double)xt;
-                            acc[k][0] += d * d;
-                        }
-                        if (check[k]) {
-                            xtg[xo[k] + j] = xt;
-                            if (rays) dxg[xo[k] + j] = xt - x0[k];
-                            const double e = (double)xt - (double)p[k].a;
-                            acc[k][1] += e * e;
-                        }
-                    }
+        int next_stat = group_next_stat<MT, NI>(gi, sc, 0, a.K);
+        bool ldx = true;
+        __syncthreads();
+        for (int it = 0; it < chunk && next_stat != INT_MAX; ++it) {
+            if (!ldx && plain_x)
+                for (const int stop = min(next_stat, chunk - 1); it < stop; ++it)
+                    plain_iteration<MT, W, NI, B, PIPE, LONG>(ip, it & 1, gv);
+            const int slot = it & 1;
+            const bool stats = it == next_stat;
+            if (tid < NI) {
+                const InstCtrl& c = sc[tid];
+                gi[tid].stat = (!stats || gi[tid].inst < 0 || c.done) ? 0 : ((c.total + 1) % a.K == 0 ? 2 : (c.first ? 1 : 0));
             }
             __syncthreads();
-            // ---- dual phase
-            for (int r = 0, sl = warp; sl < nrs; ++r, sl = snake_slice(r, warp, nwarps)) {
-                const int i = (sl << 5) + lane;
-                const bool valid = i < m;
-                RowP<MT> p[2];
+            bool check = false;
 #pragma unroll
-                for (int k = 0; k < 2; ++k)
-                    if (valid && live[k]) p[k] = rowp[yo[k] + i];
-                const int2 tb = tab[ncs + sl];
-                const int p0 = tb.x, len = tb.y;
-                MT s[2] = {(MT)0, (MT)0};
-                if (len <= kLongSlice) {
-                    if (both)
-                        ell_dot2<MT, W>(rev + p0 + W * lane, a.r_eidx + p0 + W * lane, len, xhb[0], xhb[1], s[0], s[1]);
-                    else {
-                        const MT t = ell_dot<MT, W>(rev + p0 + W * lane, a.r_eidx + p0 + W * lane, len, xh_solo);
-                        s[0] = solo1 ? (MT)0 : t;
-                        s[1] = solo1 ? t : (MT)0;
-                    }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 2; ++k)
-                        if (live[k])
-                            s[k] = long_slice_dot<MT>(sv, a.rowptr, a.colidx, ro + (sl << 5), min(32, m - (sl << 5)),
-                                                      co, xhb[k], lane);
-                }
-#pragma unroll
-                for (int k = 0; k < 2; ++k)
-                    if (valid && live[k]) {
-                        const MT y0 = ysb[k][i];
-                        MT yt = y0 + sigma[k] * (s[k] - p[k].b);
-                        if (yt < p[k].lo) yt = p[k].lo;  // NaN stays NaN
-                        ysb[k][i] = wk[k] * (one_rho * yt - rho * y0) + wa[k] * p[k].a;
-                        if (stats[k]) {
-                            const double d = (double)y0 - (double)yt;
-                            acc[k][2] += d * d;
-                        }
-                        if (check[k]) {
-                            ytg[yo[k] + i] = yt;
-                            if (rays) {
-                                MT d = yt - y0;
-                                if (p[k].lo != (MT)(-INFINITY) && d < (MT)0) d = (MT)0;
-                                dyg[yo[k] + i] = d;
-                            }
-                            const double e = (double)yt - (double)p[k].a;
-                            acc[k][3] += e * e;
-                        }
-                    }
+            for (int k = 0; k < NI; ++k) check |= gi[k].stat == 2;
+            const bool stx = check || !plain_x || it + 1 == chunk;
+            general_iteration<MT, W, NI, B>(ip, slot, gv, acc, ldx, stx);
+            ldx = check || !plain_x;
+            if (!stats) continue;
+            // the sums of every instance, over the warps in order
+            if (tid < 4 * NI) {
+                double t = 0.0;
+                for (int w = 0; w < nwarps; ++w) t += acc[w][tid >> 2][tid & 3];
+                acc[0][tid >> 2][tid & 3] = t;
             }
-#pragma unroll
-            for (int k = 0; k < 2; ++k)
-                if (live[k]) {
-                    kk[k] += 1;
-                    total[k] += 1;
-                }
-            if (!stats[0] && !stats[1]) {
-                __syncthreads();
-                continue;
-            }
+            __syncthreads();
             // ---- per instance: restart reference residual, or the check and its decisions
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                if (!stats[k]) continue;
-                block_sums<4>(acc[k], red);
-                const bool was_first = first[k];
-                first[k] = false;
-                if (!check[k]) {
-                    if (tid == 0) {
-                        sc[k].r0 = sqrt(om[k] * acc[k][0] + acc[k][2] / om[k]);
-                        sc[k].rprev = sc[k].r0;
-                    }
-                    __syncthreads();
-                    continue;
-                }
+            for (int k = 0; k < NI; ++k) {
+                const int stat = gi[k].stat;
+                if (!stat) continue;
                 double r_now = 0, dxa = 0, dya = 0;
+                const double om = sc[k].omega;
+                const long long kk = sc[k].k, total = sc[k].total;
+                __syncthreads();  // every thread holds its copy of the instance's state
                 if (tid == 0) {
-                    r_now = sqrt(om[k] * acc[k][0] + acc[k][2] / om[k]);
-                    if (was_first) {
+                    r_now = sqrt(om * acc[0][k][0] + acc[0][k][2] / om);
+                    if (sc[k].first) {
                         sc[k].r0 = r_now;
                         sc[k].rprev = r_now;
+                        sc[k].first = 0;
                     }
-                    dxa = sqrt(acc[k][1]);
-                    dya = sqrt(acc[k][3]);
+                    dxa = sqrt(acc[0][k][1]);
+                    dya = sqrt(acc[0][k][3]);
                 }
-                __syncthreads();
-                check_instance<MT, W>(a, inst[k], m, n, ro, co, xo[k], yo[k], total[k], kk[k], om[k], r_now, dxa,
-                                      dya, sc[k], s_flags[k], red, tab, xhb[k]);
-                __syncthreads();
-                live[k] = s_flags[k][0] == 0;
-                om[k] = sc[k].omega;
-                if (s_flags[k][1]) {
-                    kk[k] = 0;
-                    first[k] = true;
-                    restart_instance<MT>(a, m, n, ro, co, xo[k], yo[k], ysb[k]);
+                if (stat == 2) {
+                    check_instance<MT, W>(a, gi[k].inst, gv.m, gv.n, gv.ro, gv.co, gi[k].xo, gi[k].yo, total, kk, om,
+                                          r_now, dxa, dya, sc[k], s_flags, red, tab, smem_at<MT>(gv.xh_off));
+                    __syncthreads();
+                    const bool restart = s_flags[1] != 0;
+                    if (tid == 0) {
+                        if (restart) {
+                            sc[k].k = 0;
+                            sc[k].first = 1;
+                        }
+                        group_params<MT>(gi[k], sc[k], slot ^ 1, gv.eta);
+                    }
+                    if (restart)
+                        restart_instance<MT, NI>(a, gv.m, gv.n, gv.ro, gv.co, gi[k].xo, gi[k].yo, gi[k].xp, gi[k].yp,
+                                                 ys + k);
+                    __syncthreads();
                 }
-                __syncthreads();
             }
+            __syncthreads();
+            next_stat = group_next_stat<MT, NI>(gi, sc, it + 1, a.K);
         }
         // store the dual iterates and the control blocks
 #pragma unroll
-        for (int k = 0; k < 2; ++k)
-            if (k == 0 || has2)
-                for (int i = tid; i < m; i += nt) yg[yo[k] + i] = ysb[k][i];
-#pragma unroll
-        for (int k = 0; k < 2; ++k)
-            if (tid == k && (k == 0 || has2)) {
-                sc[k].k = kk[k];
-                sc[k].total = total[k];
-                sc[k].first = first[k] ? 1 : 0;
-                a.ictrl[inst[k]] = sc[k];
-            }
+        for (int k = 0; k < NI; ++k)
+            if (gi[k].inst >= 0)
+                for (int i = tid; i < gv.m; i += nt) yg[gi[k].yo + i] = ys[NI * i + k];
+        if (tid < NI && gi[tid].inst >= 0) a.ictrl[gi[tid].inst] = sc[tid];
         __syncthreads();
     }
-}
-
-template <typename MT, int W>
-__global__ void __launch_bounds__(512, 1) k_batch_pair(const __grid_constant__ BArgs a, int chunk) {
-    batch_pair_body<MT, W>(a, chunk);
 }
 
 // Order-preserving compaction of the active list (one CTA).
@@ -1292,14 +1436,13 @@ __global__ void k_batch_init(BArgs a, int count, const int32_t* __restrict__ lis
                              const double* __restrict__ y0, const double* __restrict__ omega0,
                              const long long* __restrict__ base0) {
     __shared__ double red[32 * 4];
-    ColP<MT>* colp = (ColP<MT>*)a.colp;
-    RowP<MT>* rowp = (RowP<MT>*)a.rowp;
     MT *xg = (MT*)a.x, *xtg = (MT*)a.xt, *yg = (MT*)a.y, *ytg = (MT*)a.yt;
     for (int q = blockIdx.x; q < count; q += gridDim.x) {
         const int inst = list ? list[q] : q;
         const int k = a.inst_mat[inst];
         const int m = a.mat_m[k], n = a.mat_n[k];
         const int64_t ro = a.mat_row_off[k], co = a.mat_col_off[k], xo = a.x_off[inst], yo = a.y_off[inst];
+        const int64_t xp = a.xp_off[inst], yp = a.yp_off[inst];
         double acc[4] = {0, 0, 0, 0};  // ||b||^2, ||c||^2, ||b_s||^2, ||c_s||^2
         for (int j = threadIdx.x; j < n; j += blockDim.x) {
             const double d = a.dc[co + j];
@@ -1313,12 +1456,11 @@ __global__ void k_batch_init(BArgs a, int count, const int32_t* __restrict__ lis
                 const MT vs = (MT)(v / d);
                 xg[xo + j] = vs;
                 xtg[xo + j] = vs;
-                ColP<MT> p;
-                p.c = (MT)(cj * d);
-                p.l = (MT)(lj / d);
-                p.u = (MT)(uj / d);
-                p.a = vs;
-                colp[xo + j] = p;
+                MT* p = (MT*)a.colp + xp + col_rec(j);
+                p[0] = (MT)(cj * d);
+                p[32] = (MT)(lj / d);
+                p[64] = (MT)(uj / d);
+                p[96] = vs;
             }
             acc[1] += cj * cj;
             acc[3] += (cj * d) * (cj * d);
@@ -1337,12 +1479,10 @@ __global__ void k_batch_init(BArgs a, int count, const int32_t* __restrict__ lis
                 const MT vs = (MT)(v / d);
                 yg[yo + i] = vs;
                 ytg[yo + i] = vs;
-                RowP<MT> r;
-                r.b = (MT)(bi * d);
-                r.lo = eq ? (MT)(-INFINITY) : (MT)0;
-                r.a = vs;
-                r.pad = (MT)0;
-                rowp[yo + i] = r;
+                MT* r = (MT*)a.rowp + yp + row_rec(i);
+                r[0] = (MT)(bi * d);
+                r[32] = eq ? (MT)(-INFINITY) : (MT)0;
+                r[64] = vs;
             }
             acc[0] += bi * bi;
             acc[2] += (bi * d) * (bi * d);
@@ -1362,7 +1502,7 @@ __global__ void k_batch_init(BArgs a, int count, const int32_t* __restrict__ lis
         }
         if (a.recenter) {
             __syncthreads();  // the centre of this instance is complete
-            rebuild_shifted<MT>(a, m, n, ro, co, xo, yo);
+            rebuild_shifted<MT>(a, m, n, ro, co, xo, yo, xp, yp);
         }
         __syncthreads();
     }
@@ -1386,17 +1526,14 @@ __global__ void k_batch_unscale(BArgs a, int count, const double* __restrict__ x
 }
 
 // ------------------------------------------------------------------ host side
-struct TuneCfg {
-    int threads, chunk, w;  // CTA size, iterations per chunk launch, SELL entries per lane load (1 or 2)
-    int ni;                 // instances per CTA: 1, or 2 (paired form, batches of one shared matrix)
-};
 
 // Candidate shapes of the autotuner: CTA sizes, SELL entry orders and instances per CTA
-// (2 only when every instance shares one matrix).  B2P_BATCH_SHAPE="threads,w,ni" pins
-// all three (the chunk length is still tuned); a pinned pair on a batch of several
-// matrices falls back to one instance per CTA.
+// (more than 1 only when every instance shares one matrix; 4 only in FP32).
+// B2P_BATCH_SHAPE="threads,w,ni" pins all three (the chunk length is still tuned); a pinned
+// group on a batch of several matrices falls back to one instance per CTA.
 struct ShapeChoices {
-    std::vector<int> threads{128, 256, 512}, w{1, 2}, ni{1, 2};
+    std::vector<int> threads{128, 256, 512}, w{1, 2}, ni{1, 2, 4};
+    bool pinned = false;
 };
 
 ShapeChoices shape_choices(BatchWork* w) {
@@ -1405,11 +1542,12 @@ ShapeChoices shape_choices(BatchWork* w) {
     if (!can_pair) c.ni = {1};
     const char* e = std::getenv("B2P_BATCH_SHAPE");
     int th = 0, ww = 0, ni = 0;
-    if (e && std::sscanf(e, "%d,%d,%d", &th, &ww, &ni) == 3 && (th == 128 || th == 256 || th == 512) &&
-        (ww == 1 || ww == 2) && (ni == 1 || ni == 2)) {
+    if (e && std::sscanf(e, "%d,%d,%d", &th, &ww, &ni) == 3 && (th == 128 || th == 256 || th == 512 || th == 1024) &&
+        (ww == 1 || ww == 2) && (ni == 1 || ni == 2 || ni == 4)) {
         c.threads = {th};
         c.w = {ww};
         c.ni = {can_pair ? ni : 1};
+        c.pinned = true;
     }
     return c;
 }
@@ -1427,7 +1565,7 @@ std::string batch_key(BatchWork* w, int precision) {
     double nnz_col = (double)w->nnz / std::max<int64_t>(w->tot_n, 1);
     std::ostringstream os;
     const char* f = std::getenv("B2P_BATCH_SHAPE");
-    os << "batch6" << (f && *f ? std::string("_s") + f : std::string()) << "_p" << precision << "_c" << (int)std::log2(std::max(1, w->count)) << "_m"
+    os << "batch7" << (f && *f ? std::string("_s") + f : std::string()) << "_p" << precision << "_c" << (int)std::log2(std::max(1, w->count)) << "_m"
        << (int)std::log2(mean_m + 1) << "_n" << (int)std::log2(mean_n + 1) << "_k" << (int)std::lround(nnz_col) << "_M"
        << w->max_m << "_N" << w->max_n << "_shared" << (w->nmat == 1 && w->count > 1);
     return os.str();
@@ -1441,7 +1579,8 @@ bool cache_lookup(const std::string& key, TuneCfg* out) {
         std::string k;
         TuneCfg c;
         if (!(is >> k) || k != key) continue;
-        if (is >> c.threads >> c.chunk >> c.w >> c.ni) {
+        if (is >> c.threads >> c.chunk >> c.w >> c.ni >> c.form_th[0] >> c.form_us[0] >> c.form_th[1] >> c.form_us[1] >>
+            c.form_th[2] >> c.form_us[2]) {
             *out = c;
             return true;
         }
@@ -1457,7 +1596,9 @@ void cache_store(const std::string& key, const TuneCfg& c) {
         if (std::system(cmd.c_str()) != 0) return;
     }
     std::ofstream f(p, std::ios::app);
-    f << key << " " << c.threads << " " << c.chunk << " " << c.w << " " << c.ni << "\n";
+    f << key << " " << c.threads << " " << c.chunk << " " << c.w << " " << c.ni;
+    for (int i = 0; i < 3; ++i) f << " " << c.form_th[i] << " " << c.form_us[i];
+    f << "\n";
 }
 
 template <typename MT>
@@ -1494,6 +1635,8 @@ BArgs make_args(BatchWork* w, const b2p_params* p, const int32_t* active) {
     a.inst_mat = w->inst_mat.p;
     a.x_off = w->x_off.p;
     a.y_off = w->y_off.p;
+    a.xp_off = w->xp_off.p;
+    a.yp_off = w->yp_off.p;
     a.b = w->b.p;
     a.c = w->c.p;
     a.lb = w->lb.p;
@@ -1536,14 +1679,35 @@ BArgs make_args(BatchWork* w, const b2p_params* p, const int32_t* active) {
 size_t smem_bytes(BatchWork* w, size_t mt_size, int ni = 1) {
     const size_t tab = sizeof(int2) * slice_tab_len((w->max_m + 31) >> 5, (w->max_n + 31) >> 5);
     const size_t m4 = (size_t)((w->max_m + 3) & ~3), n4 = (size_t)((w->max_n + 3) & ~3);
-    return tab + mt_size * ni * (m4 + std::max(n4, m4)) + 16;  // y, then xh (which also stages y at checks)
+    const size_t head = mt_size == 4 ? group_head<float>(ni) : group_head<double>(ni);
+    return head + tab + mt_size * ni * (m4 + std::max(n4, m4)) + 16;  // y, then xh (which also stages y at checks)
 }
 
-// The chunk kernel of a tuned shape.
+// CTA size of the tail form: one warp per slice of the largest instance, a power of two from
+// 128 to 1024 threads (a warp without a slice only lengthens the barriers).
+int tail_threads(BatchWork* w) {
+    const int slices = (std::max(w->max_m, w->max_n) + 31) >> 5;
+    int th = 128;
+    while (th < 1024 && th / 32 < slices) th *= 2;
+    return th;
+}
+
+// The chunk kernel of a shape (null: there is none).
+template <typename MT, int W, bool LONG>
+void (*chunk_kernel_w(int ni, int threads))(const BArgs, int) {
+    const bool wide = threads > 512;
+    if (ni == 1) return wide ? k_batch_chunk<MT, W, 1, 1024, 1, false, LONG> : k_batch_chunk<MT, W, 1, 512, 2, false, LONG>;
+    if (wide) return nullptr;
+    if (ni == 2) return k_batch_chunk<MT, W, 2, 512, 1, true, LONG>;
+    if constexpr (sizeof(MT) == 4)
+        if (ni == 4) return k_batch_chunk<MT, W, 4, 512, 1, true, LONG>;
+    return nullptr;
+}
 template <typename MT>
-void (*chunk_kernel(int w, int ni))(const BArgs, int) {
-    if (ni == 2) return w == 2 ? k_batch_pair<MT, 2> : k_batch_pair<MT, 1>;
-    return w == 2 ? k_batch_chunk<MT, 2> : k_batch_chunk<MT, 1>;
+void (*chunk_kernel(const BatchWork* bw, int w, int ni, int threads))(const BArgs, int) {
+    if (bw->max_len > kLongSlice)
+        return w == 2 ? chunk_kernel_w<MT, 2, true>(ni, threads) : chunk_kernel_w<MT, 1, true>(ni, threads);
+    return w == 2 ? chunk_kernel_w<MT, 2, false>(ni, threads) : chunk_kernel_w<MT, 1, false>(ni, threads);
 }
 
 template <typename MT>
@@ -1584,9 +1748,11 @@ int refill_ell(Ctx* ctx, BatchWork* w, int W) {
 // compaction that follows); the chunk is the shortest power of two from 256 to 8192
 // whose fixed cost is at most 2 % of its iterations -- shorter chunks drop finished
 // instances sooner, so the tail of an uneven batch is cut finer.  Each block size is
-// tried with both SELL entry orders (one entry or a pair per lane load) and, when every
-// instance shares one matrix, in the single and the paired form (two instances per
-// CTA).  Instance state is re-initialised afterwards by the caller.
+// tried with one instance per CTA and both SELL entry orders (one entry or a pair per lane
+// load), and, when every instance shares one matrix, with groups of 2 and 4 instances (pair
+// order only: their gathers are vectors, so fewer loads always won).  Of the chosen entry
+// order the fastest size of every form is kept with its time per round of resident CTAs.
+// Instance state is re-initialised afterwards by the caller.
 template <typename MT>
 int autotune(Ctx* ctx, BatchWork* w, const b2p_params* p, TuneCfg* best) {
     std::string key = batch_key(w, sizeof(MT) == 8 ? 0 : 1);
@@ -1604,16 +1770,19 @@ int autotune(Ctx* ctx, BatchWork* w, const b2p_params* p, TuneCfg* best) {
     tp.eps_infeasible = 0.0;
     const int trial_iters = 128;
     float best_ms = 1e30f;
-    *best = {256, 2048, 1, 1};
+    *best = TuneCfg();
     int max_smem = 0;
     B2P_CUDA(ctx, cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     // one trial launch of `iters` iterations over the sample with `th` threads, entry order W
     // and ni instances per CTA (ms; < 0: the shape does not fit)
-    auto trial = [&](int th, int W, int ni, int iters, float* ms) -> int {
+    auto trial = [&](int th, int W, int ni, int iters, float* ms, int* rounds) -> int {
         *ms = -1.0f;
-        auto fn = chunk_kernel<MT>(W, ni);
+        auto fn = chunk_kernel<MT>(w, W, ni, th);
+        if (!fn) return B2P_OK;
         const size_t sm = smem_bytes(w, sizeof(MT), ni);
-        if (sm > (size_t)max_smem) return B2P_OK;
+        cudaFuncAttributes fa;
+        B2P_CUDA(ctx, cudaFuncGetAttributes(&fa, fn));
+        if (sm + fa.sharedSizeBytes > (size_t)max_smem) return B2P_OK;
         B2P_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         int st = refill_ell(ctx, w, W);
         if (st) return st;
@@ -1625,7 +1794,9 @@ int autotune(Ctx* ctx, BatchWork* w, const b2p_params* p, TuneCfg* best) {
         int per_sm = 0;
         B2P_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, th, sm));
         if (per_sm < 1) return B2P_OK;
-        int grid = std::min((sample + ni - 1) / ni, ctx->sm_count * per_sm);
+        const int groups = (sample + ni - 1) / ni, slots = ctx->sm_count * per_sm;
+        const int grid = std::min(groups, slots);
+        *rounds = (groups + slots - 1) / slots;
         cudaEventRecord(ctx->ev0, s);
         fn<<<grid, th, sm, s>>>(a, iters);
         k_batch_compact<<<1, 1024, 0, s>>>(w->ictrl.p, dids.p, w->active2.p, w->counters.p);
@@ -1637,12 +1808,25 @@ int autotune(Ctx* ctx, BatchWork* w, const b2p_params* p, TuneCfg* best) {
         return B2P_OK;
     };
     const ShapeChoices choices = shape_choices(w);
-    for (int ni : choices.ni)
-        for (int W : choices.w)
+    int rounds = 1;
+    int form_th[3][3] = {};  // [form][entry order]
+    float form_ms[3][3], form_us[3][3] = {};
+    for (auto& r : form_ms)
+        for (float& v : r) v = 1e30f;
+    for (int f = 0; f < 3; ++f) {
+        const int ni = kFormNi[f];
+        if (std::find(choices.ni.begin(), choices.ni.end(), ni) == choices.ni.end()) continue;
+        for (int W : choices.w) {
+            if (ni > 1 && W == 1 && !choices.pinned) continue;
             for (int th : choices.threads) {
                 float ms = 0.0f;
-                int st = trial(th, W, ni, 4 * trial_iters, &ms);
+                int st = trial(th, W, ni, 4 * trial_iters, &ms, &rounds);
                 if (st) return st;
+                if (ms >= 0.0f && ms < form_ms[f][W]) {
+                    form_ms[f][W] = ms;
+                    form_us[f][W] = 1e3f * ms / (4 * trial_iters * rounds);
+                    form_th[f][W] = th;
+                }
                 if (ms >= 0.0f && ms < best_ms) {
                     best_ms = ms;
                     best->threads = th;
@@ -1650,12 +1834,18 @@ int autotune(Ctx* ctx, BatchWork* w, const b2p_params* p, TuneCfg* best) {
                     best->ni = ni;
                 }
             }
+        }
+    }
+    for (int f = 0; f < 3; ++f) {
+        best->form_th[f] = form_th[f][best->w];
+        best->form_us[f] = form_us[f][best->w];
+    }
     if (best_ms >= 1e30f) {
         ctx->err = "batch: no chunk-kernel shape fits this batch";
         return B2P_INVALID_ARGUMENT;
     }
     float t1 = 0.0f;
-    int st = trial(best->threads, best->w, best->ni, trial_iters, &t1);
+    int st = trial(best->threads, best->w, best->ni, trial_iters, &t1, &rounds);
     if (st) return st;
     const double per_iter = std::max(1e-9, (double)(best_ms - t1) / (3.0 * trial_iters));
     const double fixed = std::max(0.0, (double)t1 - trial_iters * per_iter);
@@ -1688,12 +1878,9 @@ int batch_run(Ctx* ctx, BatchWork* w, const b2p_params* p, const double* x0_dev,
         }
     }
     w->recenter = false;  // autotune trials run without re-centring
-    TuneCfg cfg = {256, 2048, 1, 1};
-    if (w->tuned_threads[prec] > 0) {
-        cfg.threads = w->tuned_threads[prec];
-        cfg.chunk = w->tuned_chunk[prec];
-        cfg.w = w->tuned_w[prec];
-        cfg.ni = w->tuned_ni[prec];
+    TuneCfg cfg;
+    if (w->tuned[prec]) {
+        cfg = w->tuned_cfg[prec];
     } else {
         if (subset) {
             ctx->err = "subset solve before a full solve of this precision";
@@ -1701,10 +1888,8 @@ int batch_run(Ctx* ctx, BatchWork* w, const b2p_params* p, const double* x0_dev,
         }
         int st = autotune<MT>(ctx, w, p, &cfg);
         if (st) return st;
-        w->tuned_threads[prec] = cfg.threads;
-        w->tuned_chunk[prec] = cfg.chunk;
-        w->tuned_w[prec] = cfg.w;
-        w->tuned_ni[prec] = cfg.ni;
+        w->tuned[prec] = true;
+        w->tuned_cfg[prec] = cfg;
     }
     {
         int st = refill_ell(ctx, w, cfg.w);
@@ -1756,77 +1941,116 @@ int batch_run(Ctx* ctx, BatchWork* w, const b2p_params* p, const double* x0_dev,
     B2P_CUDA(ctx, cudaMemcpyAsync(w->active.p, act.data(), sizeof(int32_t) * n_act, cudaMemcpyHostToDevice, s));
     int32_t cnt[2] = {0, n_act};
     B2P_CUDA(ctx, cudaMemcpyAsync(w->counters.p, cnt, sizeof(cnt), cudaMemcpyHostToDevice, s));
-    const size_t sm_main = smem_bytes(w, sizeof(MT), cfg.ni);
-    auto fn = chunk_kernel<MT>(cfg.w, cfg.ni);
-    B2P_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_main));
-    int per_sm = 0;
-    B2P_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, cfg.threads, sm_main));
-    if (per_sm < 1) {
-        ctx->err = "batch instance too large for one CTA's shared memory";
-        return B2P_INVALID_ARGUMENT;
-    }
-    const int grid = ctx->sm_count * per_sm;
-    const size_t sm = smem_bytes(w, sizeof(MT));  // the wide (single) form
     BArgs a1 = make_args<MT>(w, p, w->active.p);
     BArgs a2 = make_args<MT>(w, p, w->active2.p);
-    // the wide form for the tail: 1024 threads, one CTA per SM
-    auto fnw = cfg.w == 2 ? k_batch_chunk_wide<MT, 2> : k_batch_chunk_wide<MT, 1>;
-    B2P_CUDA(ctx, cudaFuncSetAttribute(fnw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    int per_sm_w = 0;
-    B2P_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_w, fnw, 1024, sm));
-    const bool have_wide = per_sm_w >= 1;
-    const int grid_w = ctx->sm_count * std::max(per_sm_w, 1);
-    // one graph = two chunk launches with compaction (ping-pong active lists); a second
-    // graph does the same with the wide kernel.  The guard releases the graphs, their
-    // executables and the pinned counter copy on every way out of this function.
+    // The forms of this solve: the tuned ones by instances per CTA, and for the tail, when no
+    // more than one instance per SM is left, one CTA per SM as wide as the largest instance has
+    // rows or columns to occupy.
+    struct Form {
+        void (*fn)(const BArgs, int) = nullptr;
+        int ni = 1, threads = 0, slots = 0;  // instances per CTA, CTA size, resident CTAs
+        size_t smem = 0;
+        double us = 0.0;
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+    };
+    // the graphs, their executables and the pinned counter copy are released on every way out
     struct Owned {
-        cudaGraph_t graph[2] = {nullptr, nullptr};
-        cudaGraphExec_t exec[2] = {nullptr, nullptr};
+        Form form[4];
         int32_t* host_cnt = nullptr;
         ~Owned() {
-            for (int g = 0; g < 2; ++g) {
-                if (exec[g]) cudaGraphExecDestroy(exec[g]);
-                if (graph[g]) cudaGraphDestroy(graph[g]);
+            for (Form& f : form) {
+                if (f.exec) cudaGraphExecDestroy(f.exec);
+                if (f.graph) cudaGraphDestroy(f.graph);
             }
             if (host_cnt) cudaFreeHost(host_cnt);
         }
     } own;
-    cudaGraph_t& graph = own.graph[0];
-    cudaGraph_t& graph_w = own.graph[1];
-    cudaGraphExec_t& exec = own.exec[0];
-    cudaGraphExec_t& exec_w = own.exec[1];
-    for (int g = 0; g < (have_wide ? 2 : 1); ++g) {
+    int max_smem = 0;
+    B2P_CUDA(ctx, cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    auto open_form = [&](Form& f, int ni, int threads, double us) -> int {
+        auto fn = chunk_kernel<MT>(w, cfg.w, ni, threads);
+        const size_t sm = smem_bytes(w, sizeof(MT), ni);
+        if (!fn) return B2P_OK;
+        cudaFuncAttributes fa;
+        B2P_CUDA(ctx, cudaFuncGetAttributes(&fa, fn));
+        if (sm + fa.sharedSizeBytes > (size_t)max_smem) return B2P_OK;
+        B2P_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        int per_sm = 0;
+        B2P_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, sm));
+        if (per_sm < 1) return B2P_OK;
+        f.fn = fn;
+        f.ni = ni;
+        f.threads = threads;
+        f.slots = ctx->sm_count * per_sm;
+        f.smem = sm;
+        f.us = us;
+        return B2P_OK;
+    };
+    for (int f = 0; f < 3; ++f)
+        if (cfg.form_th[f] > 0) {
+            int st = open_form(own.form[f], kFormNi[f], cfg.form_th[f], cfg.form_us[f]);
+            if (st) return st;
+        }
+    {
+        int st = open_form(own.form[3], 1, tail_threads(w), 0.0);
+        if (st) return st;
+    }
+    bool any = false;
+    for (const Form& f : own.form) any = any || f.fn != nullptr;
+    if (!any) {
+        ctx->err = "batch instance too large for one CTA's shared memory";
+        return B2P_INVALID_ARGUMENT;
+    }
+    // the form for `n` active instances: the tail form for up to one instance per SM, else the
+    // one with the least rounds x time per round
+    auto pick_form = [&](int n) -> Form& {
+        if (own.form[3].fn && n <= ctx->sm_count) return own.form[3];
+        Form* best = nullptr;
+        double best_us = 0.0;
+        for (int i = 0; i < 3; ++i) {
+            Form& f = own.form[i];
+            if (!f.fn) continue;
+            const int groups = (n + f.ni - 1) / f.ni;
+            const double us = ((groups + f.slots - 1) / f.slots) * std::max(f.us, 1e-3);
+            if (!best || us < best_us) {
+                best = &f;
+                best_us = us;
+            }
+        }
+        return best ? *best : own.form[3];
+    };
+    // one graph = two chunk launches with compaction (ping-pong active lists), captured when
+    // the form is first picked
+    auto capture = [&](Form& f) -> int {
+        if (f.exec) return B2P_OK;
         B2P_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        if (g == 0) fn<<<grid, cfg.threads, sm_main, s>>>(a1, cfg.chunk);
-        else fnw<<<grid_w, 1024, sm, s>>>(a1, cfg.chunk);
+        f.fn<<<f.slots, f.threads, f.smem, s>>>(a1, cfg.chunk);
         k_batch_compact<<<1, 1024, 0, s>>>(w->ictrl.p, w->active.p, w->active2.p, w->counters.p);
-        if (g == 0) fn<<<grid, cfg.threads, sm_main, s>>>(a2, cfg.chunk);
-        else fnw<<<grid_w, 1024, sm, s>>>(a2, cfg.chunk);
+        f.fn<<<f.slots, f.threads, f.smem, s>>>(a2, cfg.chunk);
         k_batch_compact<<<1, 1024, 0, s>>>(w->ictrl.p, w->active2.p, w->active.p, w->counters.p);
-        cudaGraph_t& gr = g == 0 ? graph : graph_w;
-        cudaGraphExec_t& ex = g == 0 ? exec : exec_w;
-        cudaError_t ce = cudaStreamEndCapture(s, &gr);
+        cudaError_t ce = cudaStreamEndCapture(s, &f.graph);
         if (ce != cudaSuccess) {
-            gr = nullptr;
+            f.graph = nullptr;
             ctx->err = std::string("batch graph capture: ") + cudaGetErrorString(ce);
             return B2P_EXECUTION_FAILED;
         }
-        ce = cudaGraphInstantiate(&ex, gr, 0);
+        ce = cudaGraphInstantiate(&f.exec, f.graph, 0);
         if (ce != cudaSuccess) {
-            ex = nullptr;
+            f.exec = nullptr;
             ctx->err = std::string("batch graph instantiate: ") + cudaGetErrorString(ce);
             return B2P_EXECUTION_FAILED;
         }
-    }
+        return B2P_OK;
+    };
     int32_t*& host_cnt = own.host_cnt;
     B2P_CUDA(ctx, cudaMallocHost(&host_cnt, 2 * sizeof(int32_t)));
+    host_cnt[1] = n_act;
     const int64_t max_graphs = p->max_iterations / (2LL * cfg.chunk) + 3;
     int64_t graphs = 0;
     bool timed_out = false;
     const double tl = p->time_limit_s * 1000.0;
     cudaEventRecord(ctx->ev0, s);
-    // no more than one instance per SM left: the wide form
-    bool wide = have_wide && n_act <= ctx->sm_count;
     const double trace_base = subset && !w->trace_ms.empty() ? w->trace_ms.back() : 0.0;
     if (!subset) {
         w->trace_ms.clear();
@@ -1836,14 +2060,18 @@ int batch_run(Ctx* ctx, BatchWork* w, const b2p_params* p, const double* x0_dev,
     w->trace_ms.push_back(trace_base);
     w->trace_active.push_back(n_act);
     while (graphs < max_graphs) {
-        B2P_CUDA(ctx, cudaGraphLaunch(wide ? exec_w : exec, s));
+        Form& form = pick_form(host_cnt[1]);
+        {
+            int st = capture(form);
+            if (st) return st;
+        }
+        B2P_CUDA(ctx, cudaGraphLaunch(form.exec, s));
         graphs++;
         B2P_CUDA(ctx, cudaMemcpyAsync(host_cnt, w->counters.p, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         B2P_CUDA(ctx, cudaStreamSynchronize(s));
         w->trace_ms.push_back(trace_base + now_ms() - t_loop);
         w->trace_active.push_back(host_cnt[1]);
         if (host_cnt[1] == 0) break;
-        if (have_wide && host_cnt[1] <= ctx->sm_count) wide = true;
         if (tl > 0 && now_ms() - t_start > tl) {
             timed_out = true;
             break;
@@ -2015,7 +2243,9 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
                 clen[cidx]++;
             }
             rlen[i] = rp[i + 1] - rp[i];
+            w->max_len = std::max(w->max_len, rlen[i]);
         }
+        for (int j = 0; j < n; ++j) w->max_len = std::max(w->max_len, clen[j]);
         rord.resize(m);
         cord.resize(n);
         std::iota(rord.begin(), rord.end(), 0);
@@ -2059,8 +2289,8 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
     w->h_mat_m.assign(mat_m, mat_m + nmat);
     w->h_mat_n.assign(mat_n, mat_n + nmat);
     // instances
-    std::vector<int64_t> xoff(count), yoff(count);
-    int64_t IN = 0, IM = 0;
+    std::vector<int64_t> xoff(count), yoff(count), xpoff(count), ypoff(count);
+    int64_t IN = 0, IM = 0, IC = 0, IR = 0;
     std::vector<int64_t> inst_nnz(count);
     for (int i = 0; i < count; ++i) {
         int k = inst_mat[i];
@@ -2070,8 +2300,12 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
         }
         xoff[i] = IN;
         yoff[i] = IM;
+        xpoff[i] = IC;
+        ypoff[i] = IR;
         IN += mat_n[k];
         IM += mat_m[k];
+        IC += (int64_t)col_rec((mat_n[k] + 31) & ~31);
+        IR += (int64_t)row_rec((mat_m[k] + 31) & ~31);
         inst_nnz[i] = mat_nnz_off[k + 1] - mat_nnz_off[k];
     }
     w->inst_n = IN;
@@ -2108,11 +2342,11 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
     B2P_CUDA(ctx, w->c_ev32.reserve(c_pad));
     B2P_CUDA(ctx, w->mat_eta.reserve(nmat));
     B2P_CUDA(ctx, w->inst_mat.reserve(count));
-    for (auto* bf : {&w->x_off, &w->y_off}) B2P_CUDA(ctx, bf->reserve(count));
+    for (auto* bf : {&w->x_off, &w->y_off, &w->xp_off, &w->yp_off}) B2P_CUDA(ctx, bf->reserve(count));
     for (auto* bf : {&w->c, &w->lb, &w->ub, &w->x, &w->xt}) B2P_CUDA(ctx, bf->reserve(IN));
     for (auto* bf : {&w->b, &w->y, &w->yt}) B2P_CUDA(ctx, bf->reserve(IM));
-    B2P_CUDA(ctx, w->colp.reserve(4 * IN));
-    B2P_CUDA(ctx, w->rowp.reserve(4 * IM));
+    B2P_CUDA(ctx, w->colp.reserve(IC));
+    B2P_CUDA(ctx, w->rowp.reserve(IR));
     B2P_CUDA(ctx, w->is_eq.reserve(IM));
     for (auto* bf : {&w->bnorm, &w->cnorm}) B2P_CUDA(ctx, bf->reserve(count));
     B2P_CUDA(ctx, w->ictrl.reserve(count));
@@ -2134,6 +2368,8 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
     B2P_CUDA(ctx, cudaMemcpyAsync(w->inst_mat.p, inst_mat, sizeof(int32_t) * count, cudaMemcpyHostToDevice, s));
     B2P_CUDA(ctx, cudaMemcpyAsync(w->x_off.p, xoff.data(), sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
     B2P_CUDA(ctx, cudaMemcpyAsync(w->y_off.p, yoff.data(), sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
+    B2P_CUDA(ctx, cudaMemcpyAsync(w->xp_off.p, xpoff.data(), sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
+    B2P_CUDA(ctx, cudaMemcpyAsync(w->yp_off.p, ypoff.data(), sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
     {
         // per-instance vectors arrive in external order: stage, then permute on the device
         DBuf<double> sb, scv, sl, su;
@@ -2222,7 +2458,7 @@ int b2p_batch_solve(void* p, const b2p_params* params, const double* x0, const d
     }
     bool timed_out = false;
     float kms = 0.0f;
-    TuneCfg cfg = {0, 0};
+    TuneCfg cfg;
     int st = pp->precision == B2P_FP64
                  ? batch_run<double>(ctx, w, pp, x0 ? dx0.p : nullptr, y0 ? dy0.p : nullptr, omega0 ? dom.p : nullptr,
                                      nullptr, &timed_out, &kms, &cfg)
@@ -2318,7 +2554,7 @@ int b2p_batch_solve_learned(void* p, const b2p_params* params, const float* feat
     const bool f64 = pp->precision == B2P_FP64;
     bool timed_out = false;
     float kms = 0.0f, kms2 = 0.0f;
-    TuneCfg cfg = {0, 0};
+    TuneCfg cfg;
     st = f64 ? batch_run<double>(ctx, w, pp, dx0.p, dy0.p, dom.p, nullptr, &timed_out, &kms, &cfg)
              : batch_run<float>(ctx, w, pp, dx0.p, dy0.p, dom.p, nullptr, &timed_out, &kms, &cfg);
     if (st) return st;
