@@ -53,6 +53,7 @@
 //     sample of the batch (cached on disk); between replays the host picks the form
 //     with the least rounds of resident CTAs x time per round for the instances
 //     still active, and a wide single form for the tail.
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -151,6 +152,8 @@ void batch_free(Ctx* ctx) {
 
 namespace {
 
+constexpr int kPowerCluster = 16384;  // entries from which a matrix's power iteration runs on a cluster
+constexpr int kPowerCtas = 8;
 constexpr int kLongSlice = 128;  // entries per lane above which a slice is summed warp-cooperatively
 
 // Column and row records of the scaled (and, when re-centred, shifted) problem in the
@@ -1293,26 +1296,34 @@ __global__ void k_batch_scale_vals(int64_t tot_m, int64_t tot_n, const int32_t* 
     }
 }
 
-// sigma_max(A_s)^2 per matrix by power iteration (CTA per matrix, stops at rel change 1e-7)
+// Start entry j of the power iteration: in (0.5, 1.5), splitmix64 of j.
+__device__ __forceinline__ double power_start(int j) {
+    unsigned long long z = (unsigned long long)j * 0x9E3779B97F4A7C15ull + 0x1234567ull;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    z ^= z >> 31;
+    return 0.5 + (double)(z >> 11) * (1.0 / 9007199254740992.0);
+}
+
+// sigma_max(A_s)^2 per matrix by power iteration (stops at rel change 1e-7).  Two kernels
+// share the matrices: this one takes those of fewer than cluster_from entries, one CTA
+// each -- a batch of many matrices fills the GPU that way.
 __global__ void k_batch_power(int nmat, const int32_t* __restrict__ mat_m, const int32_t* __restrict__ mat_n,
                               const int64_t* __restrict__ row_off, const int64_t* __restrict__ col_off,
                               const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colidx,
                               const double* __restrict__ sv64, const int32_t* __restrict__ t_rowptr,
                               const int32_t* __restrict__ t_colidx, const double* __restrict__ stv64, double* pv,
-                              double* pu, double safety, double* __restrict__ eta_out) {
+                              double* pu, double safety, int cluster_from, double* __restrict__ eta_out) {
     __shared__ double red[32];
     __shared__ double s_norm, s_prev;
     __shared__ int s_stop;
     for (int k = blockIdx.x; k < nmat; k += gridDim.x) {
         const int m = mat_m[k], n = mat_n[k];
         const int64_t ro = row_off[k], co = col_off[k];
+        if (rowptr[ro + m] - rowptr[ro] >= cluster_from) continue;
         double part = 0.0;
         for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            unsigned long long z = (unsigned long long)j * 0x9E3779B97F4A7C15ull + 0x1234567ull;
-            z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-            z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-            z ^= z >> 31;
-            double v = 0.5 + (double)(z >> 11) * (1.0 / 9007199254740992.0);
+            const double v = power_start(j);
             pv[co + j] = v;
             part += v * v;
         }
@@ -1355,6 +1366,113 @@ __global__ void k_batch_power(int nmat, const int32_t* __restrict__ mat_m, const
         }
         __syncthreads();
     }
+}
+
+// The matrices of at least kPowerCluster entries, where a batch has few of them: a cluster of
+// kPowerCtas CTAs each.  One CTA's
+// step is a chain of dependent loads over its whole share of rows and columns (41 us a step
+// on a 2,000 x 8,000 matrix of 47,984 entries, up to 1,000 steps); eight CTAs walk an eighth
+// of it between two cluster barriers (9 us a step: 41 -> 9.2 ms for the planning matrix).  Rows and columns are
+// summed over the FP64 SELL copies (entry order W = 1), one lane each, in the order of the
+// one-CTA kernel; the vectors live in L2 (loads bypass L1, which other CTAs' stores do not
+// reach).  The kernel's clusters loop over the matrices; every CTA of a cluster makes the
+// same decisions from the same sums.
+__global__ void __cluster_dims__(kPowerCtas, 1, 1) __launch_bounds__(512)
+k_batch_power_cluster(int nmat, const int32_t* __restrict__ mat_m, const int32_t* __restrict__ mat_n,
+                      const int64_t* __restrict__ row_off, const int64_t* __restrict__ col_off,
+                      const int32_t* __restrict__ rowptr, const int64_t* __restrict__ rs_off,
+                      const int64_t* __restrict__ cs_off, const int64_t* __restrict__ r_sptr,
+                      const int64_t* __restrict__ c_sptr, const uint16_t* __restrict__ r_eidx,
+                      const uint16_t* __restrict__ c_eidx, const double* __restrict__ r_ev,
+                      const double* __restrict__ c_ev, double* pv, double* pu, double safety,
+                      double* __restrict__ eta_out) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ double red[32];
+    __shared__ double part[2];  // this CTA's share of ||v||^2, by step parity
+    const int rank = (int)cl.block_rank();
+    const int lane = threadIdx.x & 31, warp = rank * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int warps = kPowerCtas * (blockDim.x >> 5);
+    // the whole cluster's ||v||^2 from the CTAs' shares, in rank order
+    auto total = [&](double share, int slot) -> double {
+        double w[1] = {share};
+        block_sums<1>(w, red);
+        if (threadIdx.x == 0) part[slot] = w[0];
+        cl.sync();
+        double t = 0.0;
+        for (int r = 0; r < kPowerCtas; ++r) t += *cl.map_shared_rank(&part[slot], r);
+        return t;
+    };
+    // entries of one row (column) of a slice, 8 in flight
+    auto dot = [&](const double* __restrict__ v, const uint16_t* __restrict__ ix, int len, const double* g) -> double {
+        double s = 0.0;
+        for (int q = 0; q < len; q += 8) {
+            double vv[8];
+            unsigned ii[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const bool h = q + u < len;
+                vv[u] = h ? v[(q + u) * 32] : 0.0;
+                ii[u] = h ? (unsigned)ix[(q + u) * 32] : 0u;
+            }
+            double gg[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) gg[u] = q + u < len ? __ldcg(g + ii[u]) : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (q + u < len) s += vv[u] * gg[u];
+        }
+        return s;
+    };
+    for (int k = blockIdx.x / kPowerCtas; k < nmat; k += gridDim.x / kPowerCtas) {
+        const int m = mat_m[k], n = mat_n[k];
+        const int64_t ro = row_off[k], co = col_off[k];
+        if (rowptr[ro + m] - rowptr[ro] < kPowerCluster) continue;
+        const int64_t* rsp = r_sptr + rs_off[k];
+        const int64_t* csp = c_sptr + cs_off[k];
+        const int nrs = (m + 31) >> 5, ncs = (n + 31) >> 5;
+        double sum = 0.0;
+        for (int sl = warp; sl < ncs; sl += warps) {
+            const int j = (sl << 5) + lane;
+            if (j < n) {
+                const double v = power_start(j);
+                pv[co + j] = v;
+                sum += v * v;
+            }
+        }
+        double norm = sqrt(total(sum, 0)), prev = 0.0;
+        for (int t = 0; t < 1000; ++t) {
+            const double inv = 1.0 / norm;
+            for (int sl = warp; sl < nrs; sl += warps) {
+                const int i = (sl << 5) + lane;
+                const int64_t p0 = rsp[sl];
+                const double s = dot(r_ev + p0 + lane, r_eidx + p0 + lane, (int)((rsp[sl + 1] - p0) >> 5), pv + co);
+                if (i < m) pu[ro + i] = s * inv;
+            }
+            cl.sync();
+            sum = 0.0;
+            for (int sl = warp; sl < ncs; sl += warps) {
+                const int j = (sl << 5) + lane;
+                const int64_t p0 = csp[sl];
+                const double s = dot(c_ev + p0 + lane, c_eidx + p0 + lane, (int)((csp[sl + 1] - p0) >> 5), pu + ro);
+                if (j < n) {
+                    pv[co + j] = s;
+                    sum += s * s;
+                }
+            }
+            const double nn = sqrt(total(sum, (t + 1) & 1));
+            const bool stop = nn <= 0.0 || fabs(nn - prev) <= 1e-7 * nn;
+            prev = nn;
+            norm = nn > 0.0 ? nn : 1.0;
+            if (stop) break;
+        }
+        if (rank == 0 && threadIdx.x == 0) {
+            const double sig = sqrt(fmax(prev, 0.0));
+            eta_out[k] = sig > 0.0 ? safety / sig : 1.0;
+        }
+        cl.sync();  // every CTA has read the shares before the next matrix writes them
+    }
+    cl.sync();  // no CTA leaves while another may still read its shares
 }
 
 // SELL-32 copy of one orientation, CTA per matrix: every lane slot of every slice
@@ -2198,6 +2316,8 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
         w->max_n = std::max(w->max_n, mat_n[k]);
     }
     const int64_t nnz = mat_nnz_off[nmat];
+    int big = 0;  // matrices whose power iteration is worth a cluster
+    for (int k = 0; k < nmat; ++k) big += mat_nnz_off[k + 1] - mat_nnz_off[k] >= kPowerCluster;
     if (nnz > INT32_MAX || tm > INT32_MAX || tn > INT32_MAX) {
         ctx->err = "b2p_batch_upload: batch exceeds 32-bit index range";
         return B2P_INVALID_ARGUMENT;
@@ -2404,15 +2524,26 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
     k_batch_scale_vals<<<grid_for(std::max(tm, tn), 256, ctx->sm_count), 256, 0, s>>>(
         tm, tn, w->rowptr.p, w->colidx.p, w->vals.p, w->t_rowptr.p, w->t_colidx.p, w->t_vals.p, w->dr.p, w->dc.p,
         w->sv64.p, w->sv32.p, w->stv64.p, w->stv32.p);
-    k_batch_power<<<gmat, 256, 0, s>>>(nmat, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->rowptr.p,
-                                        w->colidx.p, w->sv64.p, w->t_rowptr.p, w->t_colidx.p, w->stv64.p, w->pv.p,
-                                        w->pu.p, 0.998, w->mat_eta.p);
     k_fill_ell<<<gmat, 256, 0, s>>>(1, nmat, w->mat_m.p, w->mat_row_off.p, w->mat_col_off.p, w->mat_rs_off.p, w->r_sptr.p,
                                      w->rowptr.p, w->colidx.p, w->sv64.p, w->sv32.p, w->r_eidx.p, w->r_ev64.p,
                                      w->r_ev32.p);
     k_fill_ell<<<gmat, 256, 0, s>>>(1, nmat, w->mat_n.p, w->mat_col_off.p, w->mat_row_off.p, w->mat_cs_off.p, w->c_sptr.p,
                                      w->t_rowptr.p, w->t_colidx.p, w->stv64.p, w->stv32.p, w->c_eidx.p, w->c_ev64.p,
                                      w->c_ev32.p);
+    // clusters only while all big matrices' clusters are resident at once (two 512-thread CTAs
+    // per SM): 304 big matrices of 1,024 take 130 ms longer on clusters than one CTA each
+    const int clusters = 2 * ctx->sm_count / kPowerCtas;
+    const bool use_clusters = big > 0 && big <= clusters;
+    k_batch_power<<<gmat, 256, 0, s>>>(nmat, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->rowptr.p,
+                                        w->colidx.p, w->sv64.p, w->t_rowptr.p, w->t_colidx.p, w->stv64.p, w->pv.p,
+                                        w->pu.p, 0.998, use_clusters ? kPowerCluster : INT_MAX, w->mat_eta.p);
+    if (use_clusters) {
+        k_batch_power_cluster<<<std::min(nmat, clusters) * kPowerCtas, 512, 0, s>>>(
+            nmat, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->rowptr.p, w->mat_rs_off.p,
+            w->mat_cs_off.p, w->r_sptr.p, w->c_sptr.p, w->r_eidx.p, w->c_eidx.p, w->r_ev64.p, w->c_ev64.p, w->pv.p,
+            w->pu.p, 0.998, w->mat_eta.p);
+        ctx->launches += 1;
+    }
     B2P_LAUNCH(ctx);
     ctx->launches += 5;
     B2P_CUDA(ctx, cudaStreamSynchronize(s));
