@@ -318,6 +318,7 @@ int b2p_ctx_destroy(void* p) {
     if (!ctx) return B2P_INVALID_ARGUMENT;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    ref_free(ctx);
     halpern_free(ctx);
     batch_free(ctx);
     mlp_free(ctx);

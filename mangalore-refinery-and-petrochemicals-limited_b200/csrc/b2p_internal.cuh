@@ -81,6 +81,7 @@ struct DevLP {
     int max_row_len = 0, max_col_len = 0;
 };
 
+struct RefWork;       // ref_engine.cu
 struct HalpernWork;   // halpern_engine.cu
 struct BatchWork;     // batch_engine.cu
 struct MlpState;      // mlp.cu
@@ -103,6 +104,7 @@ struct Ctx {
     DBuf<int32_t> s_flag;
     // CUB temp storage for setup-only sorts / scans
     DBuf<uint8_t> cub_tmp;
+    RefWork* rw = nullptr;
     HalpernWork* hw = nullptr;
     BatchWork* bw = nullptr;
     MlpState* mlp = nullptr;
@@ -130,6 +132,7 @@ int halpern_engine_solve(Ctx* ctx, const b2p_params* p, const double* x0, const 
                          double* x_out, double* y_out);
 int halpern_kernel_timing(Ctx* ctx, const b2p_params* p, int reps, double* primal_ms, double* dual_ms,
                           double* primal_bytes, double* dual_bytes);
+void ref_free(Ctx* ctx);
 void halpern_free(Ctx* ctx);
 void batch_free(Ctx* ctx);
 void mlp_free(Ctx* ctx);

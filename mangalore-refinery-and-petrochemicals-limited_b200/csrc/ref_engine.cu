@@ -6,15 +6,22 @@
 // row for A x), so x^k, y^k, the convergence checks, the iteration count and
 // the status are bit-identical to the compiled reference.
 //
-// Layout: one thread per column (primal step over the CSR of A^T) and one
-// thread per row (dual step over the CSR of A).  The check_frequency
-// iterations between two convergence checks are captured once as a CUDA graph
-// (2 kernels per iteration + 2 check kernels) and replayed; the host reads back
-// four doubles per check.
+// Layout: one thread per column (primal step over A^T) and one thread per row
+// (dual step over A), each over a copy of the matrix in slices of 32 rows, entry q
+// of the slice's lanes side by side (Sell below): a warp reads 32 consecutive values
+// and indices per step while every lane still sums its own row in order.
+// An LP small enough for one cluster of CTAs runs whole in one launch
+// (k_ref_cluster): its vectors live in shared memory, and the convergence checks are
+// decided on the device.  A larger one takes two kernels per iteration, captured in a CUDA
+// graph of kGraphIters iterations; the host reads back four doubles per check.
+#include <cub/cub.cuh>
+
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "b2p_internal.cuh"
+#include "cluster.cuh"
 
 namespace b2p {
 
@@ -25,6 +32,12 @@ __device__ __forceinline__ double ref_clamp(double v, double lo, double hi) {
     return (v < lo) ? lo : ((hi < v) ? hi : v);
 }
 
+constexpr int kBatch = 16;       // entries in flight per row: the two-kernel form (few warps per SM)
+constexpr int kBatchSmall = 8;   // ... and the cluster form
+constexpr int kGraphIters = 20;  // plain iterations per captured graph
+// LPs of at most this many entries (and whose vectors fit shared memory) run on one cluster
+constexpr int64_t kClusterNnz = 49152;
+
 // Slots of the per-check reduction block.
 enum { R_DPRIMAL = 0, R_DDUAL, R_VIOL_X, R_VIOL_AVG, R_BOUND, R_COUNT };
 
@@ -33,6 +46,86 @@ struct RefState {
     unsigned long long* red;  // R_COUNT slots (bit patterns of non-negative doubles)
     long long* iter;          // device iteration counter (== avg_count)
 };
+
+// One orientation of the matrix by slices of 32 rows in their natural order: entry q of
+// row 32 s + l at off[s] + 32 q + l, slices padded to their longest row and to a multiple
+// of kPad entries.  A padding entry has value 0 and the index one past the gathered vector, where
+// a 0 is stored: it adds +0 to a sum that started from +0, which leaves every sum as it was
+// (such a sum is never -0), whatever the iterates hold.  off null: the CSR arrays (a slice with
+// one very long row would pad the others to it).
+struct Sell {
+    const int64_t* off;
+    const int32_t* ptr;  // CSR row pointers
+    const int32_t* idx;
+    const double* val;
+};
+constexpr int kPad = 2;
+
+// Sum over row i in entry order, products and sums rounded separately.  The products of a
+// batch are independent; only the additions are a chain.
+template <int B, bool SLICED>
+__device__ __forceinline__ double row_sum(const Sell& S, int i, const double* g) {
+    double w = 0.0;
+    if constexpr (!SLICED) {
+        for (int k = S.ptr[i]; k < S.ptr[i + 1]; ++k) w += S.val[k] * g[S.idx[k]];
+        return w;
+    }
+    const int64_t p0 = __ldg(S.off + (i >> 5));
+    int len = (int)((__ldg(S.off + (i >> 5) + 1) - p0) >> 5);
+    const double* v = S.val + p0 + (i & 31);
+    const int32_t* ix = S.idx + p0 + (i & 31);
+    auto batch = [&](auto size) {
+        constexpr int N = decltype(size)::value;
+        double vv[N], gg[N];
+        int ii[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            vv[u] = __ldg(v + u * 32);
+            ii[u] = __ldg(ix + u * 32);
+        }
+#pragma unroll
+        for (int u = 0; u < N; ++u) gg[u] = g[ii[u]];
+#pragma unroll
+        for (int u = 0; u < N; ++u) w += vv[u] * gg[u];
+        v += N * 32;
+        ix += N * 32;
+        len -= N;
+    };
+#pragma unroll 1
+    while (len >= B) batch(std::integral_constant<int, B>());
+    if constexpr (B > 8)
+        if (len >= 8) batch(std::integral_constant<int, 8>());
+    if (len >= 4) batch(std::integral_constant<int, 4>());
+    if (len >= kPad) batch(std::integral_constant<int, kPad>());
+    return w;
+}
+
+// padded length of every slice, x 32 lanes (the offsets are their sums)
+__global__ void k_ref_slice_len(int rows, const int32_t* __restrict__ ptr, int64_t* __restrict__ off) {
+    const int nsl = (rows + 31) >> 5;
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nsl; s += gridDim.x * blockDim.x) {
+        int mx = 0;
+        for (int i = s << 5; i < min(rows, (s + 1) << 5); ++i) mx = max(mx, ptr[i + 1] - ptr[i]);
+        off[s + 1] = 32ll * ((mx + kPad - 1) / kPad * kPad);
+        if (s == 0) off[0] = 0;
+    }
+}
+
+// every lane slot of every slice; `other`: the length of the gathered vector
+__global__ void k_ref_slice_fill(int rows, int other, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+                                 const double* __restrict__ val, const int64_t* __restrict__ off,
+                                 int32_t* __restrict__ oidx, double* __restrict__ oval) {
+    const int padded = (rows + 31) & ~31;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < padded; i += gridDim.x * blockDim.x) {
+        const int64_t base = off[i >> 5] + (i & 31);
+        const int slen = (int)((off[(i >> 5) + 1] - off[i >> 5]) >> 5);
+        const int p0 = i < rows ? ptr[i] : 0, len = i < rows ? ptr[i + 1] - p0 : 0;
+        for (int q = 0; q < slen; ++q) {
+            oidx[base + 32ll * q] = q < len ? idx[p0 + q] : other;
+            oval[base + 32ll * q] = q < len ? val[p0 + q] : 0.0;
+        }
+    }
+}
 
 // first_order_solver.cpp:103-128
 __global__ void k_ref_steps(int m, int n, const int32_t* __restrict__ rowptr, const double* __restrict__ vals,
@@ -54,7 +147,7 @@ __global__ void k_ref_steps(int m, int n, const int32_t* __restrict__ rowptr, co
 // first_order_solver.cpp:130-151
 __global__ void k_ref_init(int m, int n, const double* __restrict__ lb, const double* __restrict__ ub,
                            double* __restrict__ x, double* __restrict__ y, double* __restrict__ x_sum,
-                           long long* iter, unsigned long long* red) {
+                           double* __restrict__ x_hat, double* __restrict__ x_avg, long long* iter, unsigned long long* red) {
     int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     const double inf = INFINITY;
     for (int j = tid; j < n; j += stride) {
@@ -67,6 +160,8 @@ __global__ void k_ref_init(int m, int n, const double* __restrict__ lb, const do
     }
     for (int i = tid; i < m; i += stride) y[i] = 0.0;
     if (tid == 0) {
+        y[m] = 0.0;  // where the padding of the sliced copies points
+        x[n] = x_hat[n] = x_avg[n] = 0.0;
         *iter = 0;
         for (int r = 0; r < R_COUNT; ++r) red[r] = 0ull;
     }
@@ -74,15 +169,12 @@ __global__ void k_ref_init(int m, int n, const double* __restrict__ lb, const do
 
 // Steps A-C (first_order_solver.cpp:163-180): A^T y, projected primal step,
 // ergodic sum, extrapolation.  x_prev == x at entry, so x_hat = 2 x_new - x.
-template <bool CHECK>
-__global__ void __launch_bounds__(256) k_ref_primal(int n, const int32_t* __restrict__ t_rowptr,
-                                                    const int32_t* __restrict__ t_colidx,
-                                                    const double* __restrict__ t_vals, const double* __restrict__ c,
+template <bool CHECK, bool SLICED>
+__global__ void __launch_bounds__(128) k_ref_primal(int n, Sell At, const double* __restrict__ c,
                                                     const double* __restrict__ lb, const double* __restrict__ ub,
                                                     RefState st) {
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        double w = 0.0;
-        for (int k = t_rowptr[j]; k < t_rowptr[j + 1]; ++k) w += t_vals[k] * st.y[t_colidx[k]];
+        double w = row_sum<kBatch, SLICED>(At, j, st.y);
         double xj = st.x[j];
         double grad = c[j] + w;
         double next_x = xj - st.tau[j] * grad;
@@ -95,15 +187,12 @@ __global__ void __launch_bounds__(256) k_ref_primal(int n, const int32_t* __rest
 }
 
 // Steps D-E (first_order_solver.cpp:183-192): A x_hat, dual step, sign projection.
-template <bool CHECK>
-__global__ void __launch_bounds__(256) k_ref_dual(int m, const int32_t* __restrict__ rowptr,
-                                                  const int32_t* __restrict__ colidx, const double* __restrict__ vals,
-                                                  const double* __restrict__ b, const uint8_t* __restrict__ is_eq,
-                                                  RefState st) {
+template <bool CHECK, bool SLICED>
+__global__ void __launch_bounds__(128) k_ref_dual(int m, Sell A, const double* __restrict__ b,
+                                                  const uint8_t* __restrict__ is_eq, RefState st) {
     int tid = blockIdx.x * blockDim.x + threadIdx.x;
     for (int i = tid; i < m; i += gridDim.x * blockDim.x) {
-        double v = 0.0;
-        for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) v += vals[k] * st.x_hat[colidx[k]];
+        double v = row_sum<kBatch, SLICED>(A, i, st.x_hat);
         double yi = st.y[i];
         double next_y = yi + st.sigma[i] * (v - b[i]);
         // std::max(0.0, next_y) == (0.0 < next_y) ? next_y : 0.0
@@ -127,13 +216,11 @@ __global__ void k_ref_check_cols(int n, const double* __restrict__ lb, const dou
 }
 
 // Step F, row part (first_order_solver.cpp:199-206, 219-225): max row violation of x and x_avg.
-__global__ void k_ref_check_rows(int m, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colidx,
-                                 const double* __restrict__ vals, const double* __restrict__ b,
-                                 const uint8_t* __restrict__ is_eq, RefState st) {
+template <bool SLICED>
+__global__ void __launch_bounds__(128) k_ref_check_rows(int m, Sell A, const double* __restrict__ b,
+                                                        const uint8_t* __restrict__ is_eq, RefState st) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-        double ax = 0.0, aa = 0.0;
-        for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) ax += vals[k] * st.x[colidx[k]];
-        for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) aa += vals[k] * st.x_avg[colidx[k]];
+        double ax = row_sum<kBatch, SLICED>(A, i, st.x), aa = row_sum<kBatch, SLICED>(A, i, st.x_avg);
         double d1 = ax - b[i], d2 = aa - b[i];
         double v1 = (!is_eq[i]) ? ((0.0 < d1) ? d1 : 0.0) : fabs(d1);
         double v2 = (!is_eq[i]) ? ((0.0 < d2) ? d2 : 0.0) : fabs(d2);
@@ -152,66 +239,411 @@ double bits_to_double(unsigned long long b) {
     return d;
 }
 
+// The whole run of an LP whose vectors fit shared memory, on one cluster: each CTA owns a
+// range of column and row slices with their vectors, copies of y and x_hat (which at a check
+// hold x and then x_avg) are in every CTA, and the owned part of the matrix is in shared
+// memory too where it fits (MAT_SMEM, 16-bit indices).  The check of every interval (steps F,
+// :195-246) is decided here by the host loop's own comparisons.  Runs until convergence,
+// failure, or iteration `stop`.
+//
+// Bound: latency -- the additions of a row (8.6 cycles each), shared-memory gathers, and the
+// cluster barrier behind the remote stores (about 1 us a phase).  us per iteration, before ->
+// now (two kernels in a graph -> this): 60 x 200 7.9 -> 0.95 and 300 x 1,000 9.0 -> 2.7 (one
+// CTA / cluster), 1,000 x 3,000 10.0 -> 3.9, 2,000 x 6,000 10.1 -> 5.2.  From 3,000 x 9,000 on
+// (54,000 entries) the stores into eight copies cost as much as kernel boundaries: 8.5 here, 8.5
+// with two kernels (12.2 before, over CSR), so the line is drawn at 49,152 entries.
+struct RefOutcome {
+    long long iter;
+    int converged, failed;
+    double viol_x, viol_avg, bound, dprimal, ddual;
+};
+
+// Shared memory of one CTA (bytes from the start of the dynamic array), the same in all.
+struct RefLayout {
+    int cols, rows;      // most owned columns / rows of any CTA
+    int y, xh, x, xsum, tau, c, lb, ub, sigma, b, eq, cval, rval, cidx, ridx, total;
+};
+
+// entries in shared memory by slices: entry q of lane l of the CTA's slice s at off + 32 q + l
+template <bool MAT_SMEM>
+struct SliceView {
+    const double* val;
+    const void* idx;  // uint16_t in shared memory, int32_t in global memory
+    __device__ __forceinline__ double sum(int64_t p0, int len, int lane, const double* g) const {
+        double w = 0.0;
+        const double* v = val + p0 + lane;
+        const uint16_t* i16 = (const uint16_t*)idx + p0 + lane;
+        const int32_t* i32 = (const int32_t*)idx + p0 + lane;
+        auto batch = [&](auto size) {
+            constexpr int N = decltype(size)::value;
+            double vv[N], gg[N];
+            int ii[N];
+#pragma unroll
+            for (int u = 0; u < N; ++u) {
+                vv[u] = MAT_SMEM ? v[u * 32] : __ldg(v + u * 32);
+                ii[u] = MAT_SMEM ? (int)i16[u * 32] : __ldg(i32 + u * 32);
+            }
+#pragma unroll
+            for (int u = 0; u < N; ++u) gg[u] = g[ii[u]];
+#pragma unroll
+            for (int u = 0; u < N; ++u) w += vv[u] * gg[u];
+            v += N * 32;
+            i16 += N * 32;
+            i32 += N * 32;
+            len -= N;
+        };
+#pragma unroll 1
+        while (len >= kBatchSmall) batch(std::integral_constant<int, kBatchSmall>());
+        if (len >= 4) batch(std::integral_constant<int, 4>());
+        if (len >= kPad) batch(std::integral_constant<int, kPad>());
+        return w;
+    }
+};
+
+template <int NC, bool MAT_SMEM>
+__global__ void __launch_bounds__(kClusterThreads, 1)
+k_ref_cluster(int m, int n, Sell A, Sell At, const double* __restrict__ c, const double* __restrict__ lb,
+              const double* __restrict__ ub, const double* __restrict__ b, const uint8_t* __restrict__ is_eq, RefState st,
+              RefLayout lay, long long stop, long long max_it, long long cf, double tol, RefOutcome* out) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ __align__(16) unsigned char sh[];
+    __shared__ unsigned long long red[R_COUNT];
+    auto at = [&](int off) { return reinterpret_cast<double*>(sh + off); };
+    double *ys = at(lay.y), *xh = at(lay.xh), *xs = at(lay.x), *sums = at(lay.xsum), *ts = at(lay.tau), *cs = at(lay.c);
+    double *ls = at(lay.lb), *us = at(lay.ub), *ss = at(lay.sigma), *bs = at(lay.b);
+    uint8_t* eq = sh + lay.eq;
+    const int rank = (int)cl.block_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    const int ncs = (n + 31) >> 5, nrs = (m + 31) >> 5;
+    const int c0 = cluster_slice<NC>(ncs, rank), c1 = cluster_slice<NC>(ncs, rank + 1);
+    const int r0 = cluster_slice<NC>(nrs, rank), r1 = cluster_slice<NC>(nrs, rank + 1);
+    const ClusterVec<double, NC> yc(cl, ys), xc(cl, xh);
+    // full copies, owned vectors, owned part of the matrix
+    for (int i = tid; i <= m; i += blockDim.x) ys[i] = st.y[i];
+    if (tid == 0) xh[n] = 0.0;
+    for (int j = (c0 << 5) + tid; j < min(n, c1 << 5); j += blockDim.x) {
+        const int o = j - (c0 << 5);
+        xs[o] = st.x[j];
+        sums[o] = st.x_sum[j];
+        ts[o] = st.tau[j];
+        cs[o] = c[j];
+        ls[o] = lb[j];
+        us[o] = ub[j];
+    }
+    for (int i = (r0 << 5) + tid; i < min(m, r1 << 5); i += blockDim.x) {
+        const int o = i - (r0 << 5);
+        ss[o] = st.sigma[i];
+        bs[o] = b[i];
+        eq[o] = is_eq[i];
+    }
+    const int64_t cb = At.off[c0], rb = A.off[r0];
+    SliceView<MAT_SMEM> cv{At.val, At.idx}, rv{A.val, A.idx};
+    if (MAT_SMEM) {
+        double *vc = at(lay.cval), *vr = at(lay.rval);
+        uint16_t *ic = (uint16_t*)(sh + lay.cidx), *ir = (uint16_t*)(sh + lay.ridx);
+        for (int e = tid; e < (int)(At.off[c1] - cb); e += blockDim.x) {
+            vc[e] = At.val[cb + e];
+            ic[e] = (uint16_t)At.idx[cb + e];
+        }
+        for (int e = tid; e < (int)(A.off[r1] - rb); e += blockDim.x) {
+            vr[e] = A.val[rb + e];
+            ir[e] = (uint16_t)A.idx[rb + e];
+        }
+        cv = SliceView<MAT_SMEM>{vc - cb, ic - cb};
+        rv = SliceView<MAT_SMEM>{vr - rb, ir - rb};
+    }
+    cluster_phase<NC>(cl);
+    long long it = out->iter;
+    bool finished = out->converged || out->failed;
+    // max row violation of the vector whose copies are in xh, into slot
+    auto violation = [&](int slot) {
+        for (int sl = r0 + warp; sl < r1; sl += nw) {
+            const int64_t p0 = A.off[sl];
+            const double v = rv.sum(p0, (int)((A.off[sl + 1] - p0) >> 5), lane, xh);
+            const int i = (sl << 5) + lane, o = i - (r0 << 5);
+            if (i < m) {
+                const double d = v - bs[o];
+                atomic_max_nonneg(&red[slot], (!eq[o]) ? ((0.0 < d) ? d : 0.0) : fabs(d));
+            }
+        }
+    };
+    while (it < stop && !finished) {
+        const long long check_at = min(it - it % cf + cf, max_it);  // the interval ends on a check
+        for (; it < check_at; ++it) {
+            const bool check = it + 1 == check_at;
+            if (check) {
+                if (tid < R_COUNT) red[tid] = 0ull;
+                __syncthreads();
+            }
+            for (int sl = c0 + warp; sl < c1; sl += nw) {
+                const int64_t p0 = __ldg(At.off + sl);
+                const double w = cv.sum(p0, (int)((__ldg(At.off + sl + 1) - p0) >> 5), lane, ys);
+                const int j = (sl << 5) + lane, o = j - (c0 << 5);
+                if (j < n) {
+                    double xj = xs[o];
+                    double grad = cs[o] + w;
+                    double next_x = xj - ts[o] * grad;
+                    double new_x = ref_clamp(next_x, ls[o], us[o]);
+                    if (check) atomic_max_nonneg(&red[R_DPRIMAL], fabs(new_x - xj));
+                    sums[o] += new_x;
+                    xc.store(j, 2.0 * new_x - xj);
+                    xs[o] = new_x;
+                }
+            }
+            cluster_phase<NC>(cl);
+            for (int sl = r0 + warp; sl < r1; sl += nw) {
+                const int64_t p0 = __ldg(A.off + sl);
+                const double v = rv.sum(p0, (int)((__ldg(A.off + sl + 1) - p0) >> 5), lane, xh);
+                const int i = (sl << 5) + lane, o = i - (r0 << 5);
+                if (i < m) {
+                    double yi = ys[i];
+                    double next_y = yi + ss[o] * (v - bs[o]);
+                    double new_y = (!eq[o]) ? ((0.0 < next_y) ? next_y : 0.0) : next_y;
+                    if (check) atomic_max_nonneg(&red[R_DDUAL], fabs(new_y - yi));
+                    yc.store(i, new_y);
+                }
+            }
+            cluster_phase<NC>(cl);
+        }
+        for (int j = (c0 << 5) + tid; j < min(n, c1 << 5); j += blockDim.x) {
+            const int o = j - (c0 << 5);
+            const double xj = xs[o];
+            if (xj < ls[o] - 1e-12) atomic_max_nonneg(&red[R_BOUND], ls[o] - xj);
+            if (xj > us[o] + 1e-12) atomic_max_nonneg(&red[R_BOUND], xj - us[o]);
+            xc.store(j, xj);
+        }
+        cluster_phase<NC>(cl);
+        violation(R_VIOL_X);
+        cluster_phase<NC>(cl);
+        for (int j = (c0 << 5) + tid; j < min(n, c1 << 5); j += blockDim.x) {
+            const int o = j - (c0 << 5);
+            const double a = ref_clamp(sums[o] / (double)it, ls[o], us[o]);
+            st.x_avg[j] = a;
+            xc.store(j, a);
+        }
+        cluster_phase<NC>(cl);
+        violation(R_VIOL_AVG);
+        cluster_phase<NC>(cl);
+        double v[R_COUNT];
+#pragma unroll
+        for (int q = 0; q < R_COUNT; ++q) {
+            unsigned long long mx = 0ull;
+            for (int r = 0; r < NC; ++r) mx = max(mx, *cl.map_shared_rank(&red[q], r));
+            v[q] = __longlong_as_double((long long)mx);
+        }
+        const double best = (v[R_VIOL_AVG] < v[R_VIOL_X]) ? v[R_VIOL_AVG] : v[R_VIOL_X];
+        const bool failed = isnan(best) || best > 1e15;
+        const bool converged =
+            !failed && best <= tol && v[R_BOUND] <= tol && v[R_DPRIMAL] <= 1e-7 && v[R_DDUAL] <= 1e-7 && it >= 100;
+        finished = failed || converged;
+        cluster_phase<NC>(cl);  // every CTA has read the others' maxima
+        if (rank == 0 && tid == 0) {
+            out->iter = it;
+            out->failed = failed;
+            out->converged = converged;
+            out->viol_x = v[R_VIOL_X];
+            out->viol_avg = v[R_VIOL_AVG];
+            out->bound = v[R_BOUND];
+            out->dprimal = v[R_DPRIMAL];
+            out->ddual = v[R_DDUAL];
+        }
+    }
+    for (int i = (r0 << 5) + tid; i < min(m, r1 << 5); i += blockDim.x) st.y[i] = ys[i];
+    for (int j = (c0 << 5) + tid; j < min(n, c1 << 5); j += blockDim.x) {
+        st.x[j] = xs[j - (c0 << 5)];
+        st.x_sum[j] = sums[j - (c0 << 5)];
+    }
+    cluster_phase<NC>(cl);  // no CTA leaves while another may still store into its copies
+}
+
+// Shared-memory layout for an m x n LP whose largest owned parts hold `ce` / `re` padded entries
+// (0: the matrix stays in global memory).
+template <int NC>
+RefLayout ref_layout(int m, int n, int64_t ce, int64_t re) {
+    RefLayout L;
+    const int ncs = (n + 31) >> 5, nrs = (m + 31) >> 5;
+    L.cols = L.rows = 0;
+    for (int r = 0; r < NC; ++r) {
+        L.cols = std::max(L.cols, 32 * (cluster_slice<NC>(ncs, r + 1) - cluster_slice<NC>(ncs, r)));
+        L.rows = std::max(L.rows, 32 * (cluster_slice<NC>(nrs, r + 1) - cluster_slice<NC>(nrs, r)));
+    }
+    int64_t o = 0;
+    auto take = [&](int64_t bytes) {
+        const int64_t at = o;
+        o = (o + bytes + 15) & ~15ll;
+        return (int)std::min<int64_t>(at, 1 << 30);
+    };
+    L.y = take(8ll * (m + 1));
+    L.xh = take(8ll * (n + 1));
+    for (int* f : {&L.x, &L.xsum, &L.tau, &L.c, &L.lb, &L.ub}) *f = take(8ll * L.cols);
+    for (int* f : {&L.sigma, &L.b}) *f = take(8ll * L.rows);
+    L.eq = take(L.rows);
+    L.cval = take(8 * ce);
+    L.rval = take(8 * re);
+    L.cidx = take(2 * ce);
+    L.ridx = take(2 * re);
+    L.total = (int)std::min<int64_t>(o, 1 << 30);
+    return L;
+}
+
+// Grow-only device buffers of the engine, kept by the context between solves.
 struct RefBuffers {
     DBuf<double> tau, sigma, x, y, x_hat, x_sum, x_avg;
     DBuf<unsigned long long> red;
     DBuf<long long> iter;
+    DBuf<RefOutcome> outcome;
+    DBuf<int64_t> off, t_off;
+    DBuf<int32_t> idx, t_idx;
+    DBuf<double> val, t_val;
 };
 
+// The sliced copy of one orientation, or the CSR arrays where padding would cost more than
+// three times the entries.
+int build_sell(Ctx* ctx, int rows, int other, int64_t nnz, const int32_t* ptr, const int32_t* idx, const double* val,
+               DBuf<int64_t>& off, DBuf<int32_t>& oidx, DBuf<double>& oval, Sell* S, std::vector<int64_t>* h_off) {
+    cudaStream_t s = ctx->stream;
+    const int nsl = (rows + 31) >> 5;
+    *S = Sell{nullptr, ptr, idx, val};
+    B2P_CUDA(ctx, off.reserve(nsl + 1));
+    k_ref_slice_len<<<grid_for(nsl, 128, ctx->sm_count), 128, 0, s>>>(rows, ptr, off.p);
+    B2P_LAUNCH(ctx);
+    size_t tmp = 0;
+    B2P_CUDA(ctx, cub::DeviceScan::InclusiveSum(nullptr, tmp, off.p + 1, off.p + 1, nsl, s));
+    B2P_CUDA(ctx, ctx->cub_tmp.reserve(tmp));
+    tmp = ctx->cub_tmp.bytes();
+    B2P_CUDA(ctx, cub::DeviceScan::InclusiveSum(ctx->cub_tmp.p, tmp, off.p + 1, off.p + 1, nsl, s));
+    // the offsets of an LP that may run on a cluster are wanted on the host, else only the total
+    const size_t want = nnz <= kClusterNnz ? (size_t)nsl + 1 : 1;
+    h_off->resize(want);
+    B2P_CUDA(ctx, cudaMemcpyAsync(h_off->data(), off.p + nsl + 1 - want, sizeof(int64_t) * want, cudaMemcpyDeviceToHost, s));
+    B2P_CUDA(ctx, cudaStreamSynchronize(s));
+    const int64_t total = h_off->back();
+    ctx->launches += 2;
+    if (total > 3 * nnz + 4096) return B2P_OK;
+    B2P_CUDA(ctx, oidx.reserve(total));
+    B2P_CUDA(ctx, oval.reserve(total));
+    k_ref_slice_fill<<<grid_for(rows + 31, 128, ctx->sm_count), 128, 0, s>>>(rows, other, ptr, idx, val, off.p, oidx.p,
+                                                                            oval.p);
+    B2P_LAUNCH(ctx);
+    ctx->launches += 1;
+    *S = Sell{off.p, ptr, oidx.p, oval.p};
+    return B2P_OK;
+}
+
 }  // namespace
+
+struct RefWork {
+    RefBuffers b;
+};
+
+void ref_free(Ctx* ctx) {
+    delete ctx->rw;
+    ctx->rw = nullptr;
+}
 
 int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out, double* y_out) {
     DevLP& L = ctx->lp;
     const int m = L.m, n = L.n;
     cudaStream_t s = ctx->stream;
-    RefBuffers B;
+    if (!ctx->rw) ctx->rw = new RefWork();
+    RefBuffers& B = ctx->rw->b;
     B2P_CUDA(ctx, B.tau.reserve(n));
     B2P_CUDA(ctx, B.sigma.reserve(m));
-    B2P_CUDA(ctx, B.x.reserve(n));
-    B2P_CUDA(ctx, B.y.reserve(m));
-    B2P_CUDA(ctx, B.x_hat.reserve(n));
+    B2P_CUDA(ctx, B.x.reserve((size_t)n + 1));
+    B2P_CUDA(ctx, B.y.reserve((size_t)m + 1));
+    B2P_CUDA(ctx, B.x_hat.reserve((size_t)n + 1));
     B2P_CUDA(ctx, B.x_sum.reserve(n));
-    B2P_CUDA(ctx, B.x_avg.reserve(n));
+    B2P_CUDA(ctx, B.x_avg.reserve((size_t)n + 1));
     B2P_CUDA(ctx, B.red.reserve(R_COUNT));
     B2P_CUDA(ctx, B.iter.reserve(1));
     RefState st{B.tau.p, B.sigma.p, B.x.p, B.y.p, B.x_hat.p, B.x_sum.p, B.x_avg.p, B.red.p, B.iter.p};
 
-    const int TB = 256;
+    const int TB = 128;
     unsigned gn = grid_for(n, TB, ctx->sm_count), gm = grid_for(m, TB, ctx->sm_count);
     unsigned gmn = grid_for(std::max(m, n), TB, ctx->sm_count);
     k_ref_steps<<<gmn, TB, 0, s>>>(m, n, L.rowptr.p, L.vals.p, L.t_rowptr.p, L.t_vals.p, p->adaptive_step_size,
                                    p->primal_step_size, p->dual_step_size, st.tau, st.sigma);
-    k_ref_init<<<gmn, TB, 0, s>>>(m, n, L.lb.p, L.ub.p, st.x, st.y, st.x_sum, st.iter, st.red);
+    k_ref_init<<<gmn, TB, 0, s>>>(m, n, L.lb.p, L.ub.p, st.x, st.y, st.x_sum, st.x_hat, st.x_avg, st.iter, st.red);
     B2P_LAUNCH(ctx);
     ctx->launches += 2;
+    Sell A, At;
+    std::vector<int64_t> h_off, h_toff;
+    int bst = build_sell(ctx, m, n, L.nnz, L.rowptr.p, L.colidx.p, L.vals.p, B.off, B.idx, B.val, &A, &h_off);
+    if (bst) return bst;
+    bst = build_sell(ctx, n, m, L.nnz, L.t_rowptr.p, L.t_colidx.p, L.t_vals.p, B.t_off, B.t_idx, B.t_val, &At, &h_toff);
+    if (bst) return bst;
 
+    auto primal = [&](auto check) {
+        constexpr bool C = decltype(check)::value;
+        if (At.off) k_ref_primal<C, true><<<gn, TB, 0, s>>>(n, At, L.c.p, L.lb.p, L.ub.p, st);
+        else k_ref_primal<C, false><<<gn, TB, 0, s>>>(n, At, L.c.p, L.lb.p, L.ub.p, st);
+    };
+    auto dual = [&](auto check) {
+        constexpr bool C = decltype(check)::value;
+        if (A.off) k_ref_dual<C, true><<<gm, TB, 0, s>>>(m, A, L.b.p, L.is_eq.p, st);
+        else k_ref_dual<C, false><<<gm, TB, 0, s>>>(m, A, L.b.p, L.is_eq.p, st);
+    };
+    auto check_xs = [&]() {
+        k_ref_check_cols<<<gn, TB, 0, s>>>(n, L.lb.p, L.ub.p, st);
+        if (A.off) k_ref_check_rows<true><<<gm, TB, 0, s>>>(m, A, L.b.p, L.is_eq.p, st);
+        else k_ref_check_rows<false><<<gm, TB, 0, s>>>(m, A, L.b.p, L.is_eq.p, st);
+    };
     auto plain_iter = [&]() {
-        k_ref_primal<false><<<gn, TB, 0, s>>>(n, L.t_rowptr.p, L.t_colidx.p, L.t_vals.p, L.c.p, L.lb.p, L.ub.p, st);
-        k_ref_dual<false><<<gm, TB, 0, s>>>(m, L.rowptr.p, L.colidx.p, L.vals.p, L.b.p, L.is_eq.p, st);
+        primal(std::false_type());
+        dual(std::false_type());
     };
     auto check_iter = [&]() {
         k_ref_clear<<<1, 32, 0, s>>>(st.red);
-        k_ref_primal<true><<<gn, TB, 0, s>>>(n, L.t_rowptr.p, L.t_colidx.p, L.t_vals.p, L.c.p, L.lb.p, L.ub.p, st);
-        k_ref_dual<true><<<gm, TB, 0, s>>>(m, L.rowptr.p, L.colidx.p, L.vals.p, L.b.p, L.is_eq.p, st);
-        k_ref_check_cols<<<gn, TB, 0, s>>>(n, L.lb.p, L.ub.p, st);
-        k_ref_check_rows<<<gm, TB, 0, s>>>(m, L.rowptr.p, L.colidx.p, L.vals.p, L.b.p, L.is_eq.p, st);
+        primal(std::true_type());
+        dual(std::true_type());
+        check_xs();
     };
 
     const int64_t max_it = p->max_iterations;
     const int64_t cf = std::min<int64_t>(p->check_frequency, 100);  // first_order_solver.cpp:156
-    // One check interval = cf-1 plain iterations + 1 check iteration, captured once.
+    int max_smem = 0;
+    B2P_CUDA(ctx, cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    max_smem -= 1024;  // static part
+    // One CTA where the vectors and the matrix fit its shared memory (no cluster barrier), else a
+    // cluster where the vectors do, with the owned parts of the matrix in shared memory if
+    // they fit as well.
+    RefLayout lay{};
+    int form = 0;  // 1: one CTA, 2: cluster with the matrix in shared memory, 3: cluster without
+    if (A.off && At.off && L.nnz <= kClusterNnz && m < 65535 && n < 65535) {
+        const int ncs = (n + 31) >> 5, nrs = (m + 31) >> 5;
+        lay = ref_layout<1>(m, n, h_toff[ncs], h_off[nrs]);
+        if (lay.total <= max_smem) form = 1;
+        if (!form) {
+            int64_t ce = 0, re = 0;
+            for (int r = 0; r < kClusterCtas; ++r) {
+                ce = std::max(ce, h_toff[cluster_slice<kClusterCtas>(ncs, r + 1)] - h_toff[cluster_slice<kClusterCtas>(ncs, r)]);
+                re = std::max(re, h_off[cluster_slice<kClusterCtas>(nrs, r + 1)] - h_off[cluster_slice<kClusterCtas>(nrs, r)]);
+            }
+            lay = ref_layout<kClusterCtas>(m, n, ce, re);
+            if (lay.total <= max_smem) form = 2;
+        }
+        if (!form) {
+            lay = ref_layout<kClusterCtas>(m, n, 0, 0);
+            if (lay.total <= max_smem) form = 3;
+        }
+    }
+    const bool small = form != 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    if (max_it >= cf) {
+    if (!small && max_it >= kGraphIters && cf > kGraphIters) {
         B2P_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        for (int64_t k = 0; k < cf - 1; ++k) plain_iter();
-        check_iter();
+        for (int k = 0; k < kGraphIters; ++k) plain_iter();
         cudaError_t ce = cudaStreamEndCapture(s, &graph);
         if (ce != cudaSuccess) {
             ctx->err = std::string("graph capture: ") + cudaGetErrorString(ce);
             return B2P_EXECUTION_FAILED;
         }
-        B2P_CUDA(ctx, cudaGraphInstantiate(&exec, graph, 0));
+        ce = cudaGraphInstantiate(&exec, graph, 0);
+        if (ce != cudaSuccess) {
+            cudaGraphDestroy(graph);
+            ctx->err = std::string("graph instantiate: ") + cudaGetErrorString(ce);
+            return B2P_EXECUTION_FAILED;
+        }
     }
     struct GraphGuard {
         cudaGraph_t g;
@@ -227,18 +659,54 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
     bool converged = false, failed = false;
     double cons_viol = 0.0, bound_viol = 0.0, dpr = 0.0, ddu = 0.0;
     cudaEventRecord(ctx->ev0, s);
-    while (iter < max_it) {
+    if (small) {
+        B2P_CUDA(ctx, B.outcome.reserve(1));
+        B2P_CUDA(ctx, cudaMemsetAsync(B.outcome.p, 0, sizeof(RefOutcome), s));
+        auto fn = form == 1 ? k_ref_cluster<1, true>
+                            : (form == 2 ? k_ref_cluster<kClusterCtas, true> : k_ref_cluster<kClusterCtas, false>);
+        B2P_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, lay.total));
+        cudaLaunchConfig_t lc{};
+        cudaLaunchAttribute dims;
+        dims.id = cudaLaunchAttributeClusterDimension;
+        dims.val.clusterDim.x = form == 1 ? 1 : kClusterCtas;
+        dims.val.clusterDim.y = dims.val.clusterDim.z = 1;
+        lc.gridDim = dim3(form == 1 ? 1 : kClusterCtas);
+        lc.blockDim = dim3(kClusterThreads);
+        lc.dynamicSmemBytes = lay.total;
+        lc.stream = s;
+        lc.attrs = &dims;
+        lc.numAttrs = 1;
+        // one launch runs up to 100,000 iterations (a fraction of a second)
+        while (iter < max_it && !converged && !failed) {
+            const int64_t stop = std::min<int64_t>(iter + 100000, max_it);
+            B2P_CUDA(ctx, cudaLaunchKernelEx(&lc, fn, m, n, A, At, (const double*)L.c.p, (const double*)L.lb.p,
+                                             (const double*)L.ub.p, (const double*)L.b.p, (const uint8_t*)L.is_eq.p, st, lay,
+                                             (long long)stop, (long long)max_it, (long long)cf, p->feasibility_tolerance,
+                                             B.outcome.p));
+            B2P_LAUNCH(ctx);
+            ctx->launches += 1;
+            RefOutcome o;
+            B2P_CUDA(ctx, cudaMemcpyAsync(&o, B.outcome.p, sizeof(o), cudaMemcpyDeviceToHost, s));
+            B2P_CUDA(ctx, cudaStreamSynchronize(s));
+            iter = o.iter;
+            converged = o.converged != 0;
+            failed = o.failed != 0;
+            cons_viol = (o.viol_avg < o.viol_x) ? o.viol_avg : o.viol_x;
+            bound_viol = o.bound;
+            dpr = o.dprimal;
+            ddu = o.ddual;
+        }
+        B2P_CUDA(ctx, cudaMemcpyAsync(st.iter, &iter, sizeof(iter), cudaMemcpyHostToDevice, s));
+    }
+    while (!small && iter < max_it) {
         int64_t next_check = std::min<int64_t>((iter / cf + 1) * cf, max_it);
         int64_t span = next_check - iter;
-        if (span == cf && exec) {
-            B2P_CUDA(ctx, cudaGraphLaunch(exec, s));
-            ctx->launches += 2 * cf + 3;
-        } else {
-            for (int64_t k = 0; k < span - 1; ++k) plain_iter();
-            check_iter();
-            B2P_LAUNCH(ctx);
-            ctx->launches += 2 * span + 3;
-        }
+        int64_t k = 0;
+        for (; exec && k + kGraphIters <= span - 1; k += kGraphIters) B2P_CUDA(ctx, cudaGraphLaunch(exec, s));
+        for (; k < span - 1; ++k) plain_iter();
+        check_iter();
+        B2P_LAUNCH(ctx);
+        ctx->launches += 2 * span + 3;
         iter = next_check;
         B2P_CUDA(ctx, cudaMemcpyAsync(host_red, st.red, sizeof(host_red), cudaMemcpyDeviceToHost, s));
         B2P_CUDA(ctx, cudaStreamSynchronize(s));
@@ -272,8 +740,7 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
         // first_order_solver.cpp:261-279: the ergodic average replaces x only when the
         // loop did not converge and its violation is no worse than the last check's.
         k_ref_clear<<<1, 32, 0, s>>>(st.red);
-        k_ref_check_cols<<<gn, TB, 0, s>>>(n, L.lb.p, L.ub.p, st);
-        k_ref_check_rows<<<gm, TB, 0, s>>>(m, L.rowptr.p, L.colidx.p, L.vals.p, L.b.p, L.is_eq.p, st);
+        check_xs();
         B2P_LAUNCH(ctx);
         ctx->launches += 3;
         B2P_CUDA(ctx, cudaMemcpyAsync(host_red, st.red, sizeof(host_red), cudaMemcpyDeviceToHost, s));
