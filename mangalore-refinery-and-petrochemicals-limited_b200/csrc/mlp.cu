@@ -9,8 +9,10 @@
 //     (M = 128, N = 128, K = 16 per instruction, BF16 x BF16 -> FP32) reading
 //     both operands from shared memory through UMMA descriptors; the accumulator
 //     lives in 128 TMEM columns; tcgen05.commit frees a stage when its MMAs finish;
-//   * all 4 warps: tcgen05.ld (32 lanes x 16 columns per load) of their TMEM lane
-//     quarter, then the FP32 store of the tile.
+//   * all 8 warps: tcgen05.ld (32 lanes x 16 columns per load) of half their TMEM lane
+//     quarter into the (now free) shared memory, then row by row the coalesced store of
+//     the tile -- or, for the output layer in training, the loss and its gradient
+//     straight from the tile (LossEpi), so the layer's output never reaches memory.
 // No cluster, no multicast.  Every mbarrier wait is bounded: on timeout the
 // kernel records an error code and leaves without touching the output.
 // Transposed operands are materialised by small transpose kernels so the MMA
@@ -35,6 +37,32 @@
 
 namespace b2p {
 
+// The result of a GEMM as its consumer reads it: one array, or the partial sums of a split-K
+// one, added in a fixed order (deterministic).
+struct GemmOut {
+    const float* p;
+    int splits;
+    size_t stride;
+    __device__ __forceinline__ float get(size_t o) const {
+        if (splits == 1) return p[o];
+        float acc = 0.0f;
+        for (int z = 0; z < splits; ++z) acc += p[z * stride + o];
+        return acc;
+    }
+    __device__ __forceinline__ float4 get4(size_t o) const {  // elements o .. o + 3, 16-byte aligned
+        if (splits == 1) return *reinterpret_cast<const float4*>(p + o);
+        float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int z = 0; z < splits; ++z) {
+            const float4 q = *reinterpret_cast<const float4*>(p + z * stride + o);
+            acc.x += q.x;
+            acc.y += q.y;
+            acc.z += q.z;
+            acc.w += q.w;
+        }
+        return acc;
+    }
+};
+
 struct MlpState {
     int in = 0, hid = 0, out = 0, outp = 0;  // outp: out rounded up to a multiple of 8
     int maxb = 0;                           // batch capacity of the activation buffers
@@ -54,9 +82,13 @@ struct MlpState {
     DBuf<long long> dstep;
     // split-K partial sums of the GEMMs whose output tiles alone would leave most SMs idle
     DBuf<float> ws;
+    // those of the gradients of W1 and W2, kept until Adam reads them
+    DBuf<float> ws1, ws2;
+    GemmOut g1{}, g2{}, g3{};  // the gradients of the last backward pass
     // one training epoch captured as a CUDA graph (for this data-set size and batch)
     cudaGraphExec_t epoch_exec = nullptr;
     int epoch_n = 0, epoch_batch = 0;
+    std::vector<const void*> epoch_bufs;  // the buffers it works on (a larger request elsewhere may have moved them)
     long long epoch_launches = 0;  // kernels one replay launches
     ~MlpState() {
         if (epoch_exec) cudaGraphExecDestroy(epoch_exec);
@@ -163,14 +195,37 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 // columns each -- so one CTA's epilogue overlaps the other's main loop and a 256 x 10,008
 // output fits in one wave.
 constexpr int GBM = 128, GBN = 128, GBK = 64, GSTAGES = 3;
+constexpr int GWARPS = 8;  // one produces, one issues the MMAs, all of them run the epilogue
 constexpr int GTILE_A = GBM * GBK * 2, GTILE_B = GBN * GBK * 2;
 constexpr size_t GEMM_SMEM = 1024 + GSTAGES * (GTILE_A + GTILE_B) + 256;
 
+constexpr int kTileLd = GBN + 1;  // floats per row of the staged tile: conflict-free along rows and columns
+static_assert(GBM * kTileLd * 4 <= GSTAGES * (GTILE_A + GTILE_B), "the staged tile fits the operand ring");
+
+// Epilogue of the output layer in training: Y = tile + bias; squared error against T on the valid
+// rows / real columns; dY = 2 (Y - T) / (valid * out) as BF16 and its transpose.  Row r's
+// targets are T + perm[r] * out (perm null: T + r * out).
+struct LossEpi {
+    const float* bias;
+    const float* T;
+    const int32_t* perm;
+    __nv_bfloat16 *dY, *dYt;  // rows x outp, outp x rows (ld_t)
+    double* loss;
+    int valid, out, outp, ld_t;
+};
+
 // C[M,N] = A[M,K] . B[N,K]^T ; A, B through tensor maps; C FP32 row-major, ldc elements.
 // Split-K: CTA z of gridDim.z sums k-blocks [z kbs, (z + 1) kbs) into C + z split_stride.
-__global__ void __launch_bounds__(128, 2)
+// LOSS: the loss epilogue instead of the store of C.
+//
+// The epilogue bounds the large products here: a lane's row of the tile stored straight from TMEM
+// is 128 scalar stores of 32 scattered 4-byte pieces each.  Staged through shared memory every
+// store is a 128-byte run.  10,008 x 1,024 x 1,000: 76 -> 33 us; 1,000 x 10,008 x 1,024 with its
+// loss: 84 + 54 (+ 31 for gathering the targets) -> 79 us; 1,000 x 1,024 x 1,024: 17 -> 8 us.
+template <bool LOSS>
+__global__ void __launch_bounds__(GWARPS * 32, 2)
 k_gemm_tn_bf16(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, float* __restrict__ C,
-               int M, int N, int K, int ldc, int kbs, size_t split_stride, int* err) {
+               int M, int N, int K, int ldc, int kbs, size_t split_stride, const LossEpi le, int* err) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // SW128 tiles: 1024-aligned
     uint8_t* sA = base;
@@ -233,22 +288,102 @@ k_gemm_tn_bf16(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         umma_commit(accum);
     }
     __syncwarp();
-    // epilogue: warp w owns TMEM lanes (= tile rows) 32w .. 32w+31
+    if constexpr (LOSS)
+        if (warp >= 2)  // the tile's targets on their way to L2 while the products run
+            for (int r = m0 + (tid - 64); r < min(m0 + GBM, le.valid); r += 32 * (GWARPS - 2)) {
+                const float* src = le.T + (size_t)(le.perm ? __ldg(le.perm + r) : r) * le.out + n0;
+                for (int c = 0; c < min(GBN, le.out - n0); c += 32)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(src + c));
+            }
+    // epilogue: warp w reads TMEM lanes (= tile rows) 32 (w % 4) .. + 31, one half of the columns
     const bool acc_ok = mbar_wait(accum, 0, err, 3);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (acc_ok && ok) {
-        const int row = m0 + warp * 32 + lane;
+    const bool good = __all_sync(0xffffffffu, acc_ok && ok);
+    float* tile = reinterpret_cast<float*>(base);  // every MMA has read the ring by now
+    if (good) {
 #pragma unroll 1
-        for (int c = 0; c < GBN / 16; ++c) {
+        for (int c = warp / 4 * (GBN / 32); c < (warp / 4 + 1) * (GBN / 32); ++c) {
             float v[16];
-            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c * 16), v);
-            if (row < M) {
-                float* dst = C + (size_t)row * ldc + n0 + c * 16;
+            tmem_ld16(tmem + ((uint32_t)(warp % 4 * 32) << 16) + (uint32_t)(c * 16), v);
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (n0 + c * 16 + i < N) dst[i] = v[i];
+            for (int i = 0; i < 16; ++i) tile[(warp % 4 * 32 + lane) * kTileLd + c * 16 + i] = v[i];
+        }
+    }
+    __syncthreads();
+    if (good) {
+        const int rows = min(GBM, M - m0), cols = min(GBN, N - n0);
+        double part = 0.0;
+        if constexpr (!LOSS) {
+#pragma unroll 4
+            for (int r = warp; r < rows; r += GWARPS) {
+                const float* t = tile + r * kTileLd;
+                float* dst = C + (size_t)(m0 + r) * ldc + n0;
+#pragma unroll
+                for (int q = 0; q < GBN; q += 32)
+                    if (q + lane < cols) dst[q + lane] = t[q + lane];
+            }
+        } else {
+            // lane l holds the target row of the warp's l-th row; the targets of kRows rows are loaded
+            // before the first is used
+            constexpr int kRows = 8;
+            const int mine = lane < GBM / GWARPS ? m0 + warp + GWARPS * lane : le.valid;
+            const int trow = mine < le.valid ? (le.perm ? __ldg(le.perm + mine) : mine) : -1;
+            const float scale = 2.0f / ((float)le.valid * (float)le.out);
+            float bias[GBN / 32];
+#pragma unroll
+            for (int q = 0; q < GBN / 32; ++q) bias[q] = q * 32 + lane < cols ? __ldg(le.bias + n0 + q * 32 + lane) : 0.0f;
+#pragma unroll 1
+            for (int k = 0; warp + GWARPS * k < rows; k += kRows) {
+                float T[kRows][GBN / 32];
+#pragma unroll
+                for (int u = 0; u < kRows; ++u) {
+                    const int tr = __shfl_sync(0xffffffffu, trow, k + u);
+                    const float* src = le.T + (size_t)max(tr, 0) * le.out + n0;
+#pragma unroll
+                    for (int q = 0; q < GBN / 32; ++q) {
+                        const int c = q * 32 + lane;
+                        T[u][q] = tr >= 0 && n0 + c < le.out ? __ldg(src + c) : 0.0f;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kRows; ++u) {
+                    const int r = warp + GWARPS * (k + u);
+                    if (r >= rows) break;
+                    const bool live = m0 + r < le.valid;
+                    float* t = tile + r * kTileLd;
+                    __nv_bfloat16* dst = le.dY + (size_t)(m0 + r) * le.outp + n0;
+#pragma unroll
+                    for (int q = 0; q < GBN / 32; ++q) {
+                        const int c = q * 32 + lane;
+                        if (c < cols) {
+                            float g = 0.0f;
+                            if (live && n0 + c < le.out) {
+                                const float d = t[c] + bias[q] - T[u][q];
+                                part += (double)d * d;
+                                g = scale * d;
+                            }
+                            const __nv_bfloat16 h = __float2bfloat16(g);
+                            dst[c] = h;
+                            t[c] = __bfloat162float(h);
+                        }
+                    }
+                }
             }
         }
+        if constexpr (LOSS) {
+            __syncthreads();
+#pragma unroll 4
+            for (int c = warp; c < cols; c += GWARPS) {
+                __nv_bfloat16* dst = le.dYt + (size_t)(n0 + c) * le.ld_t + m0;
+#pragma unroll
+                for (int q = 0; q < GBM; q += 32)
+                    if (q + lane < rows) dst[q + lane] = __float2bfloat16(tile[(q + lane) * kTileLd + c]);
+            }
+            part = warp_sum(part);
+            if (lane == 0 && part != 0.0) atomicAdd(le.loss, part);
+        }
+    } else if (LOSS) {
+        __syncthreads();  // the other warps meet here between their two passes
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -302,10 +437,11 @@ __global__ void k_splitk_reduce(int M, int N, int ldc, int splits, size_t stride
 
 // C[M,N] = A[M,K] B[N,K]^T; all leading dimensions multiples of 8.  With a workspace, a GEMM
 // whose output tiles would occupy fewer than half of the SMs and whose K spans at least
-// 8 k-blocks is split along K (each split >= 4 k-blocks), the partial tiles summed by
-// k_splitk_reduce.
+// 8 k-blocks is split along K (each split >= 4 k-blocks); the partial tiles are summed by the
+// consumer of *out (ldc == N), or by k_splitk_reduce into C where out is null.  le: the loss
+// epilogue instead of C.
 int gemm_tn(Ctx* ctx, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, float* C, int ldc, int M, int N,
-            int K, int* err, DBuf<float>* ws = nullptr) {
+            int K, int* err, DBuf<float>* ws = nullptr, GemmOut* out = nullptr, const LossEpi* le = nullptr) {
     CUtensorMap ta, tb;
     if (!make_map(&ta, A, M, K, lda, GBM) || !make_map(&tb, B, N, K, ldb, GBN)) {
         ctx->err = "gemm: tensor map rejected (alignment) or driver entry point missing";
@@ -313,7 +449,8 @@ int gemm_tn(Ctx* ctx, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, i
     }
     static bool attr = false;
     if (!attr) {
-        B2P_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tn_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM));
+        B2P_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tn_bf16<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM));
+        B2P_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tn_bf16<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM));
         attr = true;
     }
     const int tiles = ((N + GBN - 1) / GBN) * ((M + GBM - 1) / GBM);
@@ -323,15 +460,17 @@ int gemm_tn(Ctx* ctx, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, i
     const int kbs = (nkb + splits - 1) / splits;
     splits = (nkb + kbs - 1) / kbs;  // every split gets at least one k-block
     const size_t stride = (size_t)M * ldc;
-    float* out = C;
+    float* dst = C;
     if (splits > 1) {
         B2P_CUDA(ctx, ws->reserve(stride * splits));
-        out = ws->p;
+        dst = ws->p;
     }
+    if (out) *out = GemmOut{dst, splits, stride};
     dim3 grid((N + GBN - 1) / GBN, (M + GBM - 1) / GBM, splits);
-    k_gemm_tn_bf16<<<grid, 128, GEMM_SMEM, ctx->stream>>>(ta, tb, out, M, N, K, ldc, kbs, stride, err);
+    if (le) k_gemm_tn_bf16<true><<<grid, GWARPS * 32, GEMM_SMEM, ctx->stream>>>(ta, tb, dst, M, N, K, ldc, kbs, stride, *le, err);
+    else k_gemm_tn_bf16<false><<<grid, GWARPS * 32, GEMM_SMEM, ctx->stream>>>(ta, tb, dst, M, N, K, ldc, kbs, stride, LossEpi{}, err);
     ctx->launches += 1;
-    if (splits > 1) {
+    if (splits > 1 && !out) {
         k_splitk_reduce<<<grid_for((long long)M * N, 256, ctx->sm_count, 8), 256, 0, ctx->stream>>>(M, N, ldc, splits,
                                                                                                    stride, ws->p, C);
         ctx->launches += 1;
@@ -404,89 +543,164 @@ __global__ void k_transpose_bf16(int rows, int cols, const __nv_bfloat16* __rest
 
 // Z = G + bias (FP32 kept for the backward GELU'), H = GELU(Z) as BF16 and its transpose;
 // rows >= valid are zeroed.
-__global__ void k_bias_gelu(int rows, int valid, int cols, const float* __restrict__ G, const float* __restrict__ bias,
+__global__ void k_bias_gelu(int rows, int valid, int cols, const GemmOut G, const float* __restrict__ bias,
                             float* __restrict__ Z, __nv_bfloat16* __restrict__ H, __nv_bfloat16* __restrict__ Ht,
                             int ld_t) {
     tile_pass(rows, cols, H, cols, Ht, ld_t, [&](int r, int c) {
         const size_t i = (size_t)r * cols + c;
-        const float z = r < valid ? G[i] + bias[c] : 0.0f;
+        const float z = r < valid ? G.get(i) + bias[c] : 0.0f;
         if (Z) Z[i] = z;
         return __float2bfloat16(r < valid ? gelu(z) : 0.0f);
     });
 }
 
-// Y = G + b3; squared error against T on the valid rows / real columns; dY = 2 (Y - T) / (valid * out)
-__global__ void k_out_loss(int rows, int valid, int out, int outp, const float* __restrict__ G,
-                           const float* __restrict__ bias, const float* __restrict__ T, float* __restrict__ Y,
-                           __nv_bfloat16* __restrict__ dY, __nv_bfloat16* __restrict__ dYt, int ld_t, double* loss,
-                           bool want_grad) {
-    double part = 0.0;
-    const float scale = 2.0f / ((float)valid * (float)out);
-    tile_pass(rows, outp, want_grad ? dY : nullptr, outp, want_grad ? dYt : nullptr, ld_t, [&](int r, int c) {
-        const size_t i = (size_t)r * outp + c;
-        const float y = G[i] + bias[c];
-        if (Y) Y[i] = y;
-        float g = 0.0f;
-        if (r < valid && c < out && T) {
-            const float d = y - T[(size_t)r * out + c];
-            part += (double)d * d;
-            g = scale * d;
-        }
-        return __float2bfloat16(g);
-    });
-    if (loss) {
-        part = warp_sum(part);
-        if ((threadIdx.x & 31) == 0 && part != 0.0) atomicAdd(loss, part);
-    }
+// Y = G + b3 (inference)
+__global__ void k_bias_out(int rows, int outp, const float* __restrict__ G, const float* __restrict__ bias,
+                           float* __restrict__ Y) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)rows * outp;
+         i += (long long)gridDim.x * blockDim.x)
+        Y[i] = G[i] + bias[i % outp];
 }
 
 // dZ = G * GELU'(Z) (BF16 + transpose), rows >= valid zeroed
-__global__ void k_gelu_back(int rows, int valid, int cols, const float* __restrict__ G, const float* __restrict__ Z,
+__global__ void k_gelu_back(int rows, int valid, int cols, const GemmOut G, const float* __restrict__ Z,
                             __nv_bfloat16* __restrict__ dZ, __nv_bfloat16* __restrict__ dZt, int ld_t) {
     tile_pass(rows, cols, dZ, cols, dZt, ld_t, [&](int r, int c) {
         const size_t i = (size_t)r * cols + c;
-        return __float2bfloat16(r < valid ? G[i] * gelu_grad(Z[i]) : 0.0f);
+        return __float2bfloat16(r < valid ? G.get(i) * gelu_grad(Z[i]) : 0.0f);
     });
 }
 
-// db[c] = sum over rows of a BF16 gradient (FP32 accumulation); one thread per column
-__global__ void k_colsum(int rows, int cols, const __nv_bfloat16* __restrict__ D, float* __restrict__ db) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < cols; c += gridDim.x * blockDim.x) {
-        float s = 0.0f;
-        for (int r = 0; r < rows; ++r) s += __bfloat162float(D[(size_t)r * cols + c]);
-        db[c] = s;
+// db[c] = sum over rows of a BF16 gradient, rows in order (FP32).  A CTA takes 64 columns: all
+// threads load 64 rows of them ahead into shared memory, one thread per column adds them
+// up, so only the additions are a chain (1,000 x 10,008: 78 us with one thread walking each
+// column in memory -> 14).  cols is even.
+constexpr int kSumCols = 64, kSumRows = 64;
+__global__ void __launch_bounds__(256) k_colsum(int rows, int cols, const __nv_bfloat16* __restrict__ D,
+                                                float* __restrict__ db) {
+    __shared__ __nv_bfloat162 t[kSumRows][kSumCols / 2 + 1];
+    const int c0 = blockIdx.x * kSumCols, cp = threadIdx.x & 31, r0 = threadIdx.x >> 5;
+    const bool in = c0 + 2 * cp < cols;
+    __nv_bfloat162 v[kSumRows / 8];
+    auto load = [&](int base) {
+#pragma unroll
+        for (int k = 0; k < kSumRows / 8; ++k) {
+            const int r = base + r0 + 8 * k;
+            v[k] = in && r < rows ? *reinterpret_cast<const __nv_bfloat162*>(D + (size_t)r * cols + c0 + 2 * cp)
+                                  : __floats2bfloat162_rn(0.0f, 0.0f);
+        }
+    };
+    load(0);
+    float s = 0.0f;
+    for (int base = 0; base < rows; base += kSumRows) {
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kSumRows / 8; ++k) t[r0 + 8 * k][cp] = v[k];
+        __syncthreads();
+        if (base + kSumRows < rows) load(base + kSumRows);
+        if (threadIdx.x < kSumCols) {
+            const __nv_bfloat16* col = reinterpret_cast<const __nv_bfloat16*>(&t[0][0]) + threadIdx.x;
+            constexpr int ld = 2 * (kSumCols / 2 + 1);
+            const int n = min(kSumRows, rows - base);
+            if (n == kSumRows) {
+                float q[kSumRows];
+#pragma unroll
+                for (int r = 0; r < kSumRows; ++r) q[r] = __bfloat162float(col[r * ld]);
+#pragma unroll
+                for (int r = 0; r < kSumRows; ++r) s += q[r];
+            } else {
+                for (int r = 0; r < n; ++r) s += __bfloat162float(col[r * ld]);
+            }
+        }
+    }
+    if (threadIdx.x < kSumCols && c0 + (int)threadIdx.x < cols) db[c0 + threadIdx.x] = s;
+}
+
+// Adam on one weight: the new value; mi, vi become the new moments.  c1, c2: 1 - beta^t.  The
+// roundings are written out: a training run is not to depend on how a kernel contracts them.
+__device__ __forceinline__ float adam_value(float w, float g, float& mi, float& vi, float lr, float c1, float c2) {
+    mi = __fmaf_rn(0.1f, g, __fmul_rn(0.9f, mi));
+    vi = __fmaf_rn(__fmul_rn(0.001f, g), g, __fmul_rn(0.999f, vi));
+    return w - lr * (mi / c1) / (sqrtf(vi / c2) + 1e-8f);
+}
+
+// Adam of the three bias vectors.
+struct BiasAdam {
+    int n;
+    float* w;
+    const float* g;
+    float *m, *v;
+};
+__global__ void k_adam_vec(BiasAdam b1, BiasAdam b2, BiasAdam b3, const float* __restrict__ hyper) {
+    const int total = b1.n + b2.n + b3.n;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const BiasAdam& b = i < b1.n ? b1 : (i < b1.n + b2.n ? b2 : b3);
+        const int k = i < b1.n ? i : (i < b1.n + b2.n ? i - b1.n : i - b1.n - b2.n);
+        float mi = b.m[k], vi = b.v[k];
+        b.w[k] = adam_value(b.w[k], b.g[k], mi, vi, hyper[0], hyper[1], hyper[2]);
+        b.m[k] = mi;
+        b.v[k] = vi;
     }
 }
 
-// One Adam update of element i; hyper = {learning rate, 1 - beta1^t, 1 - beta2^t}.
-__device__ __forceinline__ float adam_update(size_t i, float* __restrict__ w, const float* __restrict__ g,
-                                             float* __restrict__ m, float* __restrict__ v, const float* hyper) {
-    const float gi = g[i];
-    const float mi = 0.9f * m[i] + 0.1f * gi;
-    const float vi = 0.999f * v[i] + 0.001f * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float wi = w[i] - hyper[0] * (mi / hyper[1]) / (sqrtf(vi / hyper[2]) + 1e-8f);
-    w[i] = wi;
-    return wi;
-}
-
-// Adam of a bias vector (n elements).
-__global__ void k_adam_vec(int n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                           float* __restrict__ v, const float* __restrict__ hyper) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) adam_update(i, w, g, m, v, hyper);
-}
-
-// Adam on FP32 master weights (rows x cols, ld == cols) for the first live_rows rows, then
-// their BF16 copy and its transpose (cols x rows, ld_t); hyper null: no update, copies only.
-__global__ void k_adam(int rows, int cols, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, const float* __restrict__ hyper, __nv_bfloat16* __restrict__ wh,
-                       __nv_bfloat16* __restrict__ wt, int ld_t, int live_rows) {
-    tile_pass(rows, cols, wh, cols, wt, ld_t, [&](int r, int c) {
-        const size_t i = (size_t)r * cols + c;
-        const float wi = (hyper && r < live_rows) ? adam_update(i, w, g, m, v, hyper) : w[i];
-        return __float2bfloat16(wi);
-    });
+// Adam on FP32 master weights (rows x cols, ld == cols, cols a multiple of 4) for the first
+// live_rows rows, then their BF16 copy and its transpose (cols x rows, ld_t); hyper null: no
+// update, copies only.  Bound: HBM (32 bytes per weight).  Tiles of 32 x 128, four columns per
+// thread: all 16-byte loads of a tile are issued before the first is used (10,008 x 1,024:
+// 75 us with 4-byte accesses on 32 x 32 tiles -> 67).
+__global__ void __launch_bounds__(256) k_adam(int rows, int cols, float* __restrict__ w, const GemmOut g,
+                                              float* __restrict__ m, float* __restrict__ v,
+                                              const float* __restrict__ hyper, __nv_bfloat16* __restrict__ wh,
+                                              __nv_bfloat16* __restrict__ wt, int ld_t, int live_rows) {
+    __shared__ __nv_bfloat16 t[128][34];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tiles_c = (cols + 127) / 128, tiles = tiles_c * ((rows + 31) / 32);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int r0 = tile / tiles_c * 32, c0 = tile % tiles_c * 128, c = c0 + 4 * lane;
+        float4 wi[4], gi[4], mi[4], vi[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int r = r0 + warp + 8 * k;
+            const size_t i = (size_t)r * cols + c;
+            if (r >= rows || c >= cols) continue;
+            wi[k] = *reinterpret_cast<const float4*>(w + i);
+            if (hyper && r < live_rows) {
+                gi[k] = g.get4(i);
+                mi[k] = *reinterpret_cast<const float4*>(m + i);
+                vi[k] = *reinterpret_cast<const float4*>(v + i);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int r = r0 + warp + 8 * k;
+            const size_t i = (size_t)r * cols + c;
+            if (r >= rows || c >= cols) continue;
+            if (hyper && r < live_rows) {
+                const float lr = hyper[0], c1 = hyper[1], c2 = hyper[2];
+                wi[k].x = adam_value(wi[k].x, gi[k].x, mi[k].x, vi[k].x, lr, c1, c2);
+                wi[k].y = adam_value(wi[k].y, gi[k].y, mi[k].y, vi[k].y, lr, c1, c2);
+                wi[k].z = adam_value(wi[k].z, gi[k].z, mi[k].z, vi[k].z, lr, c1, c2);
+                wi[k].w = adam_value(wi[k].w, gi[k].w, mi[k].w, vi[k].w, lr, c1, c2);
+                *reinterpret_cast<float4*>(w + i) = wi[k];
+                *reinterpret_cast<float4*>(m + i) = mi[k];
+                *reinterpret_cast<float4*>(v + i) = vi[k];
+            }
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(wi[k].x, wi[k].y), hi = __floats2bfloat162_rn(wi[k].z, wi[k].w);
+            uint2 q;
+            q.x = *reinterpret_cast<const unsigned*>(&lo);
+            q.y = *reinterpret_cast<const unsigned*>(&hi);
+            *reinterpret_cast<uint2*>(wh + i) = q;
+            t[4 * lane][warp + 8 * k] = lo.x;
+            t[4 * lane + 1][warp + 8 * k] = lo.y;
+            t[4 * lane + 2][warp + 8 * k] = hi.x;
+            t[4 * lane + 3][warp + 8 * k] = hi.y;
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int k = warp; k < 128; k += 8)
+            if (c0 + k < cols && r0 + lane < rows) wt[(size_t)(c0 + k) * ld_t + r0 + lane] = t[k][lane];
+        __syncthreads();
+    }
 }
 
 // Start of an Adam step on the device: t += 1, the bias corrections of step t, and the
@@ -594,6 +808,10 @@ unsigned tile_grid(Ctx* ctx, long long rows, long long cols) {
     return grid_for(((rows + 31) / 32) * ((cols + 31) / 32) * 256, 256, ctx->sm_count, 8);
 }
 const dim3 kTileBlock(32, kTileThreadsY);
+// grid of k_adam: its tiles, at most four CTAs per SM
+unsigned adam_grid(Ctx* ctx, long long rows, long long cols) {
+    return grid_for(((rows + 31) / 32) * ((cols + 127) / 128) * 256, 256, ctx->sm_count, 4);
+}
 
 int check_err(Ctx* ctx, MlpState* s) {
     int e = 0;
@@ -622,69 +840,83 @@ int reserve_batch(Ctx* ctx, MlpState* s, int rows) {
     return B2P_OK;
 }
 
-// Forward for `rows` (multiple of 8) rows already in Xh/Xt; valid rows carry data.
-int forward(Ctx* ctx, MlpState* s, int rows, int valid, bool keep) {
-    const int in = s->in, h = s->hid, op = s->outp;
+// Hidden layers for `rows` (multiple of 8) rows already in Xh/Xt; valid rows carry data.
+int forward_hidden(Ctx* ctx, MlpState* s, int rows, int valid, bool keep) {
+    const int in = s->in, h = s->hid;
     cudaStream_t st = ctx->stream;
     int r;
-    if ((r = gemm_tn(ctx, s->Xh.p, in, s->W1h.p, in, s->G.p, h, rows, h, in, s->err.p, &s->ws))) return r;
-    k_bias_gelu<<<tile_grid(ctx, rows, h), kTileBlock, 0, st>>>(rows, valid, h, s->G.p, s->b1.p, s->Z1.p, s->H1.p,
+    GemmOut g;
+    if ((r = gemm_tn(ctx, s->Xh.p, in, s->W1h.p, in, s->G.p, h, rows, h, in, s->err.p, &s->ws, &g))) return r;
+    k_bias_gelu<<<tile_grid(ctx, rows, h), kTileBlock, 0, st>>>(rows, valid, h, g, s->b1.p, s->Z1.p, s->H1.p,
                                                                     keep ? s->H1t.p : nullptr, rows);
-    if ((r = gemm_tn(ctx, s->H1.p, h, s->W2h.p, h, s->G.p, h, rows, h, h, s->err.p, &s->ws))) return r;
-    k_bias_gelu<<<tile_grid(ctx, rows, h), kTileBlock, 0, st>>>(rows, valid, h, s->G.p, s->b2.p, s->Z2.p, s->H2.p,
+    if ((r = gemm_tn(ctx, s->H1.p, h, s->W2h.p, h, s->G.p, h, rows, h, h, s->err.p, &s->ws, &g))) return r;
+    k_bias_gelu<<<tile_grid(ctx, rows, h), kTileBlock, 0, st>>>(rows, valid, h, g, s->b2.p, s->Z2.p, s->H2.p,
                                                                     keep ? s->H2t.p : nullptr, rows);
-    if ((r = gemm_tn(ctx, s->H2.p, h, s->W3h.p, h, s->G.p, op, rows, op, h, s->err.p))) return r;
     B2P_LAUNCH(ctx);
     ctx->launches += 2;
     return B2P_OK;
 }
 
-// Loss and gradients of one batch (rows padded to 8; X, T already on the device in Xf/Tf)
-int backward(Ctx* ctx, MlpState* s, int rows, int valid) {
-    const int in = s->in, h = s->hid, op = s->outp, out = s->out;
+// Forward pass of inference: the output layer without its bias in G.
+int forward(Ctx* ctx, MlpState* s, int rows, int valid) {
+    const int h = s->hid, op = s->outp;
+    int r = forward_hidden(ctx, s, rows, valid, false);
+    if (r) return r;
+    return gemm_tn(ctx, s->H2.p, h, s->W3h.p, h, s->G.p, op, rows, op, h, s->err.p);
+}
+
+// Output layer, loss and gradients of one batch (rows padded to 8; X staged, the hidden layers
+// done with keep).  T, perm: the targets (LossEpi).  The gradients of W1 and W2 are left as
+// their GEMMs made them (s->g1, s->g2) for Adam, or summed into gW1 / gW2 (reduce).
+int backward(Ctx* ctx, MlpState* s, int rows, int valid, const float* T, const int32_t* perm, bool reduce) {
+    const int in = s->in, h = s->hid, op = s->outp;
     cudaStream_t st = ctx->stream;
     int r;
-    k_out_loss<<<tile_grid(ctx, rows, op), kTileBlock, 0, st>>>(rows, valid, out, op, s->G.p, s->b3.p, s->Tf.p,
-                                                                    s->Y.p, s->dY.p, s->dYt.p, rows, s->loss.p, true);
-    k_colsum<<<ew_grid(ctx, op), 256, 0, st>>>(rows, op, s->dY.p, s->gb3.p);
+    GemmOut g;
+    const LossEpi le{s->b3.p, T, perm, s->dY.p, s->dYt.p, s->loss.p, valid, s->out, op, rows};
+    if ((r = gemm_tn(ctx, s->H2.p, h, s->W3h.p, h, nullptr, op, rows, op, h, s->err.p, nullptr, nullptr, &le))) return r;
+    k_colsum<<<(op + kSumCols - 1) / kSumCols, 256, 0, st>>>(rows, op, s->dY.p, s->gb3.p);
     // dW3 = dY^T H2 : [op, h]
-    if ((r = gemm_tn(ctx, s->dYt.p, rows, s->H2t.p, rows, s->gW3.p, h, op, h, rows, s->err.p))) return r;
+    if ((r = gemm_tn(ctx, s->dYt.p, rows, s->H2t.p, rows, s->gW3.p, h, op, h, rows, s->err.p, nullptr, &s->g3))) return r;
     // dH2 = dY W3 : [rows, h]  (B = W3^T stored [h][op])
-    if ((r = gemm_tn(ctx, s->dY.p, op, s->W3t.p, op, s->G.p, h, rows, h, op, s->err.p, &s->ws))) return r;
-    k_gelu_back<<<tile_grid(ctx, rows, h), kTileBlock, 0, st>>>(rows, valid, h, s->G.p, s->Z2.p, s->dZ.p, s->dZt.p,
-                                                                    rows);
-    k_colsum<<<ew_grid(ctx, h), 256, 0, st>>>(rows, h, s->dZ.p, s->gb2.p);
-    if ((r = gemm_tn(ctx, s->dZt.p, rows, s->H1t.p, rows, s->gW2.p, h, h, h, rows, s->err.p, &s->ws))) return r;
-    if ((r = gemm_tn(ctx, s->dZ.p, h, s->W2t.p, h, s->G.p, h, rows, h, h, s->err.p, &s->ws))) return r;
+    if ((r = gemm_tn(ctx, s->dY.p, op, s->W3t.p, op, s->G.p, h, rows, h, op, s->err.p, &s->ws, &g))) return r;
+    k_gelu_back<<<tile_grid(ctx, rows, h), kTileBlock, 0, st>>>(rows, valid, h, g, s->Z2.p, s->dZ.p, s->dZt.p, rows);
+    k_colsum<<<(h + kSumCols - 1) / kSumCols, 256, 0, st>>>(rows, h, s->dZ.p, s->gb2.p);
+    if ((r = gemm_tn(ctx, s->dZt.p, rows, s->H1t.p, rows, s->gW2.p, h, h, h, rows, s->err.p, &s->ws2,
+                     reduce ? nullptr : &s->g2)))
+        return r;
+    if ((r = gemm_tn(ctx, s->dZ.p, h, s->W2t.p, h, s->G.p, h, rows, h, h, s->err.p, &s->ws, &g))) return r;
     // dZ1 reuses the dZ buffers
-    k_gelu_back<<<tile_grid(ctx, rows, h), kTileBlock, 0, st>>>(rows, valid, h, s->G.p, s->Z1.p, s->dZ.p, s->dZt.p,
-                                                                    rows);
-    k_colsum<<<ew_grid(ctx, h), 256, 0, st>>>(rows, h, s->dZ.p, s->gb1.p);
-    if ((r = gemm_tn(ctx, s->dZt.p, rows, s->Xt.p, rows, s->gW1.p, in, h, in, rows, s->err.p, &s->ws))) return r;
+    k_gelu_back<<<tile_grid(ctx, rows, h), kTileBlock, 0, st>>>(rows, valid, h, g, s->Z1.p, s->dZ.p, s->dZt.p, rows);
+    k_colsum<<<(h + kSumCols - 1) / kSumCols, 256, 0, st>>>(rows, h, s->dZ.p, s->gb1.p);
+    if ((r = gemm_tn(ctx, s->dZt.p, rows, s->Xt.p, rows, s->gW1.p, in, h, in, rows, s->err.p, &s->ws1,
+                     reduce ? nullptr : &s->g1)))
+        return r;
     B2P_LAUNCH(ctx);
-    ctx->launches += 6;
+    ctx->launches += 5;
     return B2P_OK;
 }
 
-// One Adam step of all parameters; lr >= 0 sets the learning rate, a negative lr keeps the
-// one in device memory (the captured training epoch sets it before each replay).
+// One Adam step of all parameters with the gradients of the last backward pass; lr >= 0 sets
+// the learning rate, a negative lr keeps the one in device memory (the captured training epoch
+// sets it before each replay).
 int adam_step(Ctx* ctx, MlpState* s, float lr) {
     s->step += 1;
     const int in = s->in, h = s->hid, op = s->outp;
     cudaStream_t st = ctx->stream;
     const float* hy = s->hyper.p;
     k_adam_begin<<<1, 1, 0, st>>>(s->dstep.p, s->hyper.p, lr);
-    k_adam<<<tile_grid(ctx, h, in), kTileBlock, 0, st>>>(h, in, s->W1.p, s->gW1.p, s->m1.p, s->v1.p, hy, s->W1h.p,
-                                                         s->W1t.p, h, h);
-    k_adam<<<tile_grid(ctx, h, h), kTileBlock, 0, st>>>(h, h, s->W2.p, s->gW2.p, s->m2.p, s->v2.p, hy, s->W2h.p,
-                                                        s->W2t.p, h, h);
-    k_adam<<<tile_grid(ctx, op, h), kTileBlock, 0, st>>>(op, h, s->W3.p, s->gW3.p, s->m3.p, s->v3.p, hy, s->W3h.p,
-                                                         s->W3t.p, op, s->out);
-    k_adam_vec<<<ew_grid(ctx, h), 256, 0, st>>>(h, s->b1.p, s->gb1.p, s->mb1.p, s->vb1.p, hy);
-    k_adam_vec<<<ew_grid(ctx, h), 256, 0, st>>>(h, s->b2.p, s->gb2.p, s->mb2.p, s->vb2.p, hy);
-    k_adam_vec<<<ew_grid(ctx, s->out), 256, 0, st>>>(s->out, s->b3.p, s->gb3.p, s->mb3.p, s->vb3.p, hy);
+    k_adam<<<adam_grid(ctx, h, in), 256, 0, st>>>(h, in, s->W1.p, s->g1, s->m1.p, s->v1.p, hy, s->W1h.p, s->W1t.p, h,
+                                                         h);
+    k_adam<<<adam_grid(ctx, h, h), 256, 0, st>>>(h, h, s->W2.p, s->g2, s->m2.p, s->v2.p, hy, s->W2h.p, s->W2t.p, h,
+                                                        h);
+    k_adam<<<adam_grid(ctx, op, h), 256, 0, st>>>(op, h, s->W3.p, s->g3, s->m3.p, s->v3.p, hy, s->W3h.p, s->W3t.p, op,
+                                                         s->out);
+    k_adam_vec<<<ew_grid(ctx, 2 * h + s->out), 256, 0, st>>>(
+        BiasAdam{h, s->b1.p, s->gb1.p, s->mb1.p, s->vb1.p}, BiasAdam{h, s->b2.p, s->gb2.p, s->mb2.p, s->vb2.p},
+        BiasAdam{s->out, s->b3.p, s->gb3.p, s->mb3.p, s->vb3.p}, hy);
     B2P_LAUNCH(ctx);
-    ctx->launches += 7;
+    ctx->launches += 5;
     return B2P_OK;
 }
 
@@ -705,11 +937,11 @@ int stage_batch(Ctx* ctx, MlpState* s, const float* X, const float* T, int valid
 int refresh_bf16(Ctx* ctx, MlpState* s) {
     const int in = s->in, h = s->hid, op = s->outp;
     cudaStream_t st = ctx->stream;
-    k_adam<<<tile_grid(ctx, h, in), kTileBlock, 0, st>>>(h, in, s->W1.p, s->gW1.p, s->m1.p, s->v1.p, nullptr, s->W1h.p,
+    k_adam<<<adam_grid(ctx, h, in), 256, 0, st>>>(h, in, s->W1.p, GemmOut{}, s->m1.p, s->v1.p, nullptr, s->W1h.p,
                                                          s->W1t.p, h, 0);
-    k_adam<<<tile_grid(ctx, h, h), kTileBlock, 0, st>>>(h, h, s->W2.p, s->gW2.p, s->m2.p, s->v2.p, nullptr, s->W2h.p,
+    k_adam<<<adam_grid(ctx, h, h), 256, 0, st>>>(h, h, s->W2.p, GemmOut{}, s->m2.p, s->v2.p, nullptr, s->W2h.p,
                                                         s->W2t.p, h, 0);
-    k_adam<<<tile_grid(ctx, op, h), kTileBlock, 0, st>>>(op, h, s->W3.p, s->gW3.p, s->m3.p, s->v3.p, nullptr, s->W3h.p,
+    k_adam<<<adam_grid(ctx, op, h), 256, 0, st>>>(op, h, s->W3.p, GemmOut{}, s->m3.p, s->v3.p, nullptr, s->W3h.p,
                                                          s->W3t.p, op, 0);
     B2P_LAUNCH(ctx);
     ctx->launches += 3;
@@ -818,9 +1050,8 @@ int mlp_predict_warm(Ctx* ctx, const float* feat_host, int count, int n, int m, 
         k_to_bf16<<<tile_grid(ctx, rows, in), kTileBlock, 0, st>>>(rows, in, s->Xf.p, in, s->Xh.p, in, s->Xt.p, rows);
         B2P_LAUNCH(ctx);
         ctx->launches += 2;
-        if ((r = forward(ctx, s, rows, valid, false))) return r;
-        k_out_loss<<<tile_grid(ctx, rows, s->outp), kTileBlock, 0, st>>>(
-            rows, valid, s->out, s->outp, s->G.p, s->b3.p, nullptr, s->Y.p, nullptr, nullptr, 0, nullptr, false);
+        if ((r = forward(ctx, s, rows, valid))) return r;
+        k_bias_out<<<ew_grid(ctx, (long long)rows * s->outp), 256, 0, st>>>(rows, s->outp, s->G.p, s->b3.p, s->Y.p);
         k_denorm_warm<<<ew_grid(ctx, (long long)valid * s->out), 256, 0, st>>>(valid, s->outp, n, m, s->Y.p,
                                                                               s->out_mean.p, s->out_std.p, off, x0, y0,
                                                                               om);
@@ -904,8 +1135,8 @@ int b2p_mlp_train_epoch(void* p, const float* X, const float* Y, int N, int batc
         const int valid = std::min(batch, N - off);
         const int rows = (valid + 7) & ~7;
         if ((r = stage_batch(ctx, s, X + (size_t)off * s->in, Y + (size_t)off * s->out, valid, rows))) return r;
-        if ((r = forward(ctx, s, rows, valid, true))) return r;
-        if ((r = backward(ctx, s, rows, valid))) return r;
+        if ((r = forward_hidden(ctx, s, rows, valid, true))) return r;
+        if ((r = backward(ctx, s, rows, valid, s->Tf.p, nullptr, false))) return r;
         if ((r = adam_step(ctx, s, lr))) return r;
     }
     double loss = 0.0;
@@ -932,9 +1163,8 @@ int b2p_mlp_infer(void* p, const float* X, int N, float* Y_out) {
         const int valid = std::min(chunk, N - off);
         const int rows = (valid + 7) & ~7;
         if ((r = stage_batch(ctx, s, X + (size_t)off * s->in, nullptr, valid, rows))) return r;
-        if ((r = forward(ctx, s, rows, valid, false))) return r;
-        k_out_loss<<<tile_grid(ctx, rows, s->outp), kTileBlock, 0, ctx->stream>>>(
-            rows, valid, s->out, s->outp, s->G.p, s->b3.p, nullptr, s->Y.p, nullptr, nullptr, 0, nullptr, false);
+        if ((r = forward(ctx, s, rows, valid))) return r;
+        k_bias_out<<<ew_grid(ctx, (long long)rows * s->outp), 256, 0, ctx->stream>>>(rows, s->outp, s->G.p, s->b3.p, s->Y.p);
         B2P_LAUNCH(ctx);
         ctx->launches += 1;
         B2P_CUDA(ctx, cudaMemcpy2DAsync(Y_out + (size_t)off * s->out, sizeof(float) * s->out, s->Y.p,
@@ -983,8 +1213,8 @@ int b2p_mlp_gradient(void* p, const float* X, const float* Y, int N, float* loss
     if (r) return r;
     B2P_CUDA(ctx, cudaMemsetAsync(s->loss.p, 0, sizeof(double), ctx->stream));
     if ((r = stage_batch(ctx, s, X, Y, N, rows))) return r;
-    if ((r = forward(ctx, s, rows, N, true))) return r;
-    if ((r = backward(ctx, s, rows, N))) return r;
+    if ((r = forward_hidden(ctx, s, rows, N, true))) return r;
+    if ((r = backward(ctx, s, rows, N, s->Tf.p, nullptr, true))) return r;
     double loss = 0.0;
     B2P_CUDA(ctx, cudaMemcpyAsync(&loss, s->loss.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     if ((r = check_err(ctx, s))) return r;
@@ -1029,20 +1259,22 @@ int b2p_mlp_train(void* p, int epochs, int batch, float lr_start, float lr_end, 
             const int rows = (valid + 7) & ~7;
             k_gather_rows<<<ew_grid(ctx, (long long)rows * in), 256, 0, st>>>(valid, rows, in, s->perm.p + off, s->DX.p,
                                                                               s->Xf.p);
-            k_gather_rows<<<ew_grid(ctx, (long long)rows * out), 256, 0, st>>>(valid, rows, out, s->perm.p + off,
-                                                                               s->DT.p, s->Tf.p);
             k_to_bf16<<<tile_grid(ctx, rows, in), kTileBlock, 0, st>>>(rows, in, s->Xf.p, in, s->Xh.p, in, s->Xt.p,
                                                                         rows);
             B2P_LAUNCH(ctx);
-            ctx->launches += 3;
-            if ((q = forward(ctx, s, rows, valid, true))) return q;
-            if ((q = backward(ctx, s, rows, valid))) return q;
+            ctx->launches += 2;
+            if ((q = forward_hidden(ctx, s, rows, valid, true))) return q;
+            if ((q = backward(ctx, s, rows, valid, s->DT.p, s->perm.p + off, false))) return q;
             if ((q = adam_step(ctx, s, -1.0f))) return q;
         }
         return B2P_OK;
     };
+    auto buffers = [&]() -> std::vector<const void*> {
+        return {s->Xf.p, s->Xh.p, s->Z1.p, s->H1.p, s->dY.p, s->dZ.p, s->G.p, s->ws.p, s->ws1.p, s->ws2.p, s->DX.p, s->DT.p,
+                s->perm.p};
+    };
     const int steps_per_epoch = (N + batch - 1) / batch;
-    if (!s->epoch_exec || s->epoch_n != N || s->epoch_batch != batch) {
+    if (!s->epoch_exec || s->epoch_bufs != buffers() || s->epoch_n != N || s->epoch_batch != batch) {
         if (s->epoch_exec) {
             cudaGraphExecDestroy(s->epoch_exec);
             s->epoch_exec = nullptr;
@@ -1050,8 +1282,9 @@ int b2p_mlp_train(void* p, int epochs, int batch, float lr_start, float lr_end, 
         // outside the capture: kernel attributes and the split-K workspace of every GEMM shape
         // (one forward / backward of a full batch; no parameter changes)
         const int rows0 = (std::min(batch, N) + 7) & ~7;
-        if ((r = forward(ctx, s, rows0, std::min(batch, N), true))) return r;
-        if ((r = backward(ctx, s, rows0, std::min(batch, N)))) return r;
+        if ((r = forward_hidden(ctx, s, rows0, std::min(batch, N), true))) return r;
+        B2P_CUDA(ctx, cudaMemcpyAsync(s->perm.p, order.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice, st));
+        if ((r = backward(ctx, s, rows0, std::min(batch, N), s->DT.p, s->perm.p, false))) return r;
         B2P_CUDA(ctx, cudaStreamSynchronize(st));
         const long long launches0 = ctx->launches, step0 = s->step;
         cudaGraph_t graph = nullptr;
@@ -1076,6 +1309,7 @@ int b2p_mlp_train(void* p, int epochs, int batch, float lr_start, float lr_end, 
         s->epoch_launches = ctx->launches - launches0;
         ctx->launches = launches0;  // counted per replay below
         s->step = step0;
+        s->epoch_bufs = buffers();
         s->epoch_n = N;
         s->epoch_batch = batch;
     }
