@@ -117,6 +117,7 @@ struct HalpernWork {
     Sell sr_all[3], sc_all[3];
     Sell* sr = &sr_all[0];
     Sell* sc = &sc_all[0];
+    Sell kr, kc;  // FP64 copies in pair order for the power iteration and the KKT checks
     bool sell_r = false, sell_c = false;  // tuned: SELL (true) or CSR kernel per side
     // tuned gather windows of the SELL kernels (smem 0 = none): grid, shared memory
     // bytes and the per-CTA windows built for that grid
@@ -180,6 +181,72 @@ __device__ __forceinline__ double block_sum_to(double v, double* slot) {
 template <typename T>
 __device__ __forceinline__ T clampT(T v, T lo, T hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
+// Block sums of NV values in one pass, added to their slots by NV threads side by side.
+template <int NV>
+__device__ __forceinline__ void block_sums_to(double (&v)[NV], double* const (&slot)[NV]) {
+    __shared__ double sh[32][NV];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q] = warp_sum(v[q]);
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) sh[w][q] = v[q];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+        if ((int)threadIdx.x == q) {
+            double t = 0.0;
+            for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += sh[i][q];
+            if (t != 0.0) atomicAdd(slot[q], t);
+        }
+}
+
+// Sums of slice sl's rows over a copy in pair order (W = 2), for NV gathered vectors of one
+// type: 32 / C lanes per row take every (32 / C)-th pair, four pairs in flight each, and
+// meet in a shuffle; the lanes below C return the rows' sums.
+template <int C, int NV, typename GT>
+__device__ __forceinline__ void sell_pair_dot(const int64_t* __restrict__ off, const int32_t* __restrict__ idx,
+                                              const double* __restrict__ val, int sl, int lane,
+                                              const GT* const (&g)[NV], double (&s)[NV]) {
+    constexpr int LPR = 32 / C, U = 4;
+    const int64_t p0 = off[sl];
+    const int np = (int)((off[sl + 1] - p0) / (2 * C));  // pairs per row
+    const int rl = lane % C, sub = lane / C;
+    const double2* vp = reinterpret_cast<const double2*>(val + p0) + rl;
+    const int2* ip = reinterpret_cast<const int2*>(idx + p0) + rl;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) s[k] = 0.0;
+    for (int q = sub; q < np; q += U * LPR) {
+        double2 v[U];
+        int2 c[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int qq = q + u * LPR;
+            const bool h = qq < np;
+            v[u] = h ? __ldg(vp + (int64_t)qq * C) : make_double2(0.0, 0.0);
+            c[u] = h ? __ldg(ip + (int64_t)qq * C) : make_int2(-1, -1);
+        }
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            GT a[U], b[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                a[u] = c[u].x >= 0 ? g[k][c[u].x] : (GT)0;
+                b[u] = c[u].y >= 0 ? g[k][c[u].y] : (GT)0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                s[k] += v[u].x * (double)a[u];
+                s[k] += v[u].y * (double)b[u];
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+#pragma unroll
+        for (int o = C; o < 32; o <<= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+}
+
 // ------------------------------------------------------------------ scaling (FP64, setup)
 __global__ void k_fill(int64_t n, double v, double* __restrict__ a) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) a[i] = v;
@@ -237,47 +304,73 @@ __global__ void k_scale_vecs(int m, int n, const double* __restrict__ b, const d
 }
 
 // ------------------------------------------------------------------ power iteration (FP64)
-// u = A_s v / nv ; v is normalised by the norm stored in *nv (1 on the first pass).
-__global__ void k_pow_rows(int m, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                           const double* __restrict__ v64, const double* __restrict__ v, const double* __restrict__ nv,
-                           double* __restrict__ u) {
-    double inv = 1.0 / *nv;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int k = ptr[i]; k < ptr[i + 1]; ++k) s += v64[k] * v[idx[k]];
-        u[i] = s * inv;
+// Power iteration and KKT checks read their own FP64 copy of each orientation (Sell kr, kc):
+// pair order, slice height by the number of rows.  One thread per CSR row read uncoalesced; L
+// lanes per CSR row spent three dependent loads on each row of a few entries.  us per launch,
+// before -> now: 100k x 400k, 4.0M nonzeros, power rows 45 -> 22, columns 25 -> 19; 204k x 1M,
+// 8.0M nonzeros, FP32 iterates with certificates, KKT rows 153 -> 64, columns 190 -> 54.  What is
+// left is the gathers: one L1 lookup per entry and SM cycle is 14 us for 4.0M of them.
+// One step: u = A_s v / ||v||, w = A_s^T u, ||w||^2 -> nrm2[t + 1] (nrm2[t] holds ||v||^2, so
+// ||w|| estimates sigma_max^2).  Both run over the check copies, one warp per slice.
+template <int C>
+__global__ void __launch_bounds__(256) k_pow_rows(int m, const int64_t* __restrict__ off, const int32_t* __restrict__ idx,
+                                                  const double* __restrict__ val, const double* __restrict__ v,
+                                                  const double* __restrict__ nrm2, double* __restrict__ u) {
+    const double nn = sqrt(*nrm2), inv = 1.0 / (nn > 0 ? nn : 1.0);
+    const int lane = threadIdx.x & 31, nsl = (m + C - 1) / C;
+    for (int sl = blockIdx.x * 8 + (threadIdx.x >> 5); sl < nsl; sl += gridDim.x * 8) {
+        double s[1];
+        const double* g[1] = {v};
+        sell_pair_dot<C, 1>(off, idx, val, sl, lane, g, s);
+        const int i = sl * C + lane;
+        if (lane < C && i < m) u[i] = s[0] * inv;
     }
 }
 
-__global__ void k_pow_cols(int n, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                           const double* __restrict__ v64, const double* __restrict__ u, double* __restrict__ w,
-                           double* __restrict__ nrm2) {
+template <int C>
+__global__ void __launch_bounds__(256) k_pow_cols(int n, const int64_t* __restrict__ off, const int32_t* __restrict__ idx,
+                                                  const double* __restrict__ val, const double* __restrict__ u,
+                                                  double* __restrict__ w, double* __restrict__ nrm2) {
     double part = 0.0;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int k = ptr[j]; k < ptr[j + 1]; ++k) s += v64[k] * u[idx[k]];
-        w[j] = s;
-        part += s * s;
+    const int lane = threadIdx.x & 31, nsl = (n + C - 1) / C;
+    for (int sl = blockIdx.x * 8 + (threadIdx.x >> 5); sl < nsl; sl += gridDim.x * 8) {
+        double s[1];
+        const double* g[1] = {u};
+        sell_pair_dot<C, 1>(off, idx, val, sl, lane, g, s);
+        const int j = sl * C + lane;
+        if (lane < C && j < n) {
+            w[j] = s[0];
+            part += s[0] * s[0];
+        }
     }
     block_sum_to(part, nrm2);
 }
 
-__global__ void k_pow_finish(double* __restrict__ nrm2, double* __restrict__ nv, double* __restrict__ hist, int t) {
-    double nn = sqrt(*nrm2);
-    hist[t] = nn;          // ||A^T A v|| with ||v|| = 1  ->  sigma_max^2
-    *nv = nn > 0 ? nn : 1.0;
-    *nrm2 = 0.0;
-}
-
-__global__ void k_pow_init(int n, double* __restrict__ v) {
+// start vector; ||v||^2 -> nrm2[0]
+__global__ void k_pow_init(int n, double* __restrict__ v, double* __restrict__ nrm2) {
+    double part = 0.0;
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         // deterministic pseudo-random start (splitmix64), entries in (0.5, 1.5)
         unsigned long long z = (unsigned long long)j * 0x9E3779B97F4A7C15ull + 0x1234567ull;
         z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
         z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
         z ^= z >> 31;
-        v[j] = 0.5 + (double)(z >> 11) * (1.0 / 9007199254740992.0);
+        const double q = 0.5 + (double)(z >> 11) * (1.0 / 9007199254740992.0);
+        v[j] = q;
+        part += q * q;
     }
+    block_sum_to(part, nrm2);
+}
+
+// ||a||^2 -> out[0], ||b||^2 -> out[1] (zeroed by the caller)
+__global__ void k_norms2(int na, const double* __restrict__ a, int nb, const double* __restrict__ b,
+                         double* __restrict__ out) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, st = gridDim.x * blockDim.x;
+    double v[2] = {0.0, 0.0};
+    for (int i = tid; i < na; i += st) v[0] += a[i] * a[i];
+    for (int i = tid; i < nb; i += st) v[1] += b[i] * b[i];
+    double* const slots[2] = {out, out + 1};
+    block_sums_to<2>(v, slots);
 }
 
 // ------------------------------------------------------------------ iterate init
@@ -833,71 +926,58 @@ struct KktMap {
 };
 
 // rows: primal residual, b.y, the objective-error sum |y| viol; with xd / yd (the
-// displacement T(z) - z), A xd for the primal ray and the row terms of the dual ray
-template <int L, typename ZT>
-__global__ void __launch_bounds__(TB) k_kkt_rows(int m, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                                                 const double* __restrict__ v64, const ZT* __restrict__ xt,
+// displacement T(z) - z), A xd for the primal ray and the row terms of the dual ray.  Both
+// kernels run over the FP64 check copies, one warp per slice (lane < C: one row each).
+template <int C, typename ZT>
+__global__ void __launch_bounds__(TB) k_kkt_rows(int m, const int64_t* __restrict__ off, const int32_t* __restrict__ idx,
+                                                 const double* __restrict__ val, const ZT* __restrict__ xt,
                                                  const ZT* __restrict__ yt, const double* __restrict__ b,
                                                  const uint8_t* __restrict__ is_eq, const double* __restrict__ dr,
                                                  KktMap map, const double* __restrict__ xd,
                                                  const double* __restrict__ yd, Ctrl* ctrl) {
     if (ctrl->done) return;
     const double ps = ctrl->pscale, ds = ctrl->dscale;
-    const int lane = threadIdx.x & 31, sub = lane & (L - 1), rpw = 32 / L;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x & 31, nsl = (m + C - 1) / C;
     const bool rays = xd != nullptr;
-    double p2 = 0.0, by = 0.0, est = 0.0, prv = 0.0, drb = 0.0, drm = 0.0, ysv = 0.0;
-    for (int base = warp * rpw; base < m; base += nw * rpw) {
-        int r = base + lane / L;
-        bool valid = r < m;
-        double s = 0.0, sd = 0.0;
-        if (valid)
-            for (int k = ptr[r] + sub; k < ptr[r + 1]; k += L) {
-                s += v64[k] * (double)xt[idx[k]];
-                if (rays) sd += v64[k] * xd[idx[k]];
-            }
-#pragma unroll
-        for (int o = L / 2; o > 0; o >>= 1) {
-            s += __shfl_xor_sync(0xffffffffu, s, o);
-            sd += __shfl_xor_sync(0xffffffffu, sd, o);
+    double a[7] = {0, 0, 0, 0, 0, 0, 0};  // |rp|^2, b.y, sum |y| viol, y < 0, |A dx viol|^2, b.dy, sum |b dy|
+    for (int sl = blockIdx.x * (TB / 32) + (threadIdx.x >> 5); sl < nsl; sl += gridDim.x * (TB / 32)) {
+        double s[1], sd[1] = {0.0};
+        const ZT* g[1] = {xt};
+        sell_pair_dot<C, 1>(off, idx, val, sl, lane, g, s);
+        if (rays) {
+            const double* gd[1] = {xd};
+            sell_pair_dot<C, 1>(off, idx, val, sl, lane, gd, sd);
         }
-        if (valid && sub == 0) {
-            const bool eq = is_eq[r] != 0;
-            double ax = (map.axbar ? map.axbar[r] : 0.0) + ps * (s / dr[r]);
-            double rp = ax - b[r];
-            if (!eq) rp = fmax(rp, 0.0);
-            p2 += rp * rp;
-            const double yv = (map.ybar ? map.ybar[r] : 0.0) + ds * (dr[r] * (double)yt[r]);
-            by += b[r] * yv;
-            est += fabs(yv) * fabs(rp);
-            if (!eq && yv < 0.0) ysv += yv * yv;  // y >= 0 on <= rows: part of the dual residual
-            if (rays) {
-                const double adx = sd / dr[r];  // (A dx)_r, original space
-                const double v = eq ? adx : fmax(adx, 0.0);
-                prv += v * v;
-                const double dyo = dr[r] * yd[r];
-                drb += b[r] * dyo;
-                drm += fabs(b[r] * dyo);
-            }
+        const int r = sl * C + lane;
+        if (lane >= C || r >= m) continue;
+        const bool eq = is_eq[r] != 0;
+        double ax = (map.axbar ? map.axbar[r] : 0.0) + ps * (s[0] / dr[r]);
+        double rp = ax - b[r];
+        if (!eq) rp = fmax(rp, 0.0);
+        a[0] += rp * rp;
+        const double yv = (map.ybar ? map.ybar[r] : 0.0) + ds * (dr[r] * (double)yt[r]);
+        a[1] += b[r] * yv;
+        a[2] += fabs(yv) * fabs(rp);
+        if (!eq && yv < 0.0) a[3] += yv * yv;  // y >= 0 on <= rows: part of the dual residual
+        if (rays) {
+            const double adx = sd[0] / dr[r];  // (A dx)_r, original space
+            const double v = eq ? adx : fmax(adx, 0.0);
+            a[4] += v * v;
+            const double dyo = dr[r] * yd[r];
+            a[5] += b[r] * dyo;
+            a[6] += fabs(b[r] * dyo);
         }
     }
-    block_sum_to(p2, &ctrl->acc[A_PRES2]);
-    block_sum_to(by, &ctrl->acc[A_BY]);
-    block_sum_to(est, &ctrl->acc[A_EST]);
-    block_sum_to(ysv, &ctrl->acc[A_DRES2]);
-    if (rays) {
-        block_sum_to(prv, &ctrl->acc[A_PRV2]);
-        block_sum_to(drb, &ctrl->acc[A_DRB]);
-        block_sum_to(drm, &ctrl->acc[A_DRM]);
-    }
+    double* const slots[7] = {&ctrl->acc[A_PRES2], &ctrl->acc[A_BY],  &ctrl->acc[A_EST], &ctrl->acc[A_DRES2],
+                              &ctrl->acc[A_PRV2],  &ctrl->acc[A_DRB], &ctrl->acc[A_DRM]};
+    block_sums_to<7>(a, slots);
 }
 
-// columns: reduced cost g = c + A^T y, bound multipliers lambda, dual residual, c.x and the bound terms
 // columns: reduced cost g = c + A^T y, bound multipliers lambda, dual residual, c.x and the bound
 // terms; with xd / yd, the column terms of the primal ray and A^T yd for the dual ray
-template <int L, typename ZT>
-__global__ void __launch_bounds__(TB) k_kkt_cols(int n, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                                                 const double* __restrict__ v64, const ZT* __restrict__ yt,
+template <int C, typename ZT>
+__global__ void __launch_bounds__(TB) k_kkt_cols(int n, const int64_t* __restrict__ off, const int32_t* __restrict__ idx,
+                                                 const double* __restrict__ val, const ZT* __restrict__ yt,
                                                  const ZT* __restrict__ xt, const double* __restrict__ c,
                                                  const double* __restrict__ lb, const double* __restrict__ ub,
                                                  const double* __restrict__ dc, KktMap map,
@@ -905,60 +985,48 @@ __global__ void __launch_bounds__(TB) k_kkt_cols(int n, const int32_t* __restric
                                                  Ctrl* ctrl) {
     if (ctrl->done) return;
     const double ps = ctrl->pscale, ds = ctrl->dscale;
-    const int lane = threadIdx.x & 31, sub = lane & (L - 1), rpw = 32 / L;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x & 31, nsl = (n + C - 1) / C;
     const bool rays = yd != nullptr;
-    double d2 = 0.0, pc = 0.0, lam_t = 0.0, prv = 0.0, prc = 0.0, prm = 0.0, drl = 0.0, drm = 0.0, drv = 0.0;
-    for (int base = warp * rpw; base < n; base += nw * rpw) {
-        int j = base + lane / L;
-        bool valid = j < n;
-        double s = 0.0, sd = 0.0;
-        if (valid)
-            for (int k = ptr[j] + sub; k < ptr[j + 1]; k += L) {
-                s += v64[k] * (double)yt[idx[k]];
-                if (rays) sd += v64[k] * yd[idx[k]];
-            }
-#pragma unroll
-        for (int o = L / 2; o > 0; o >>= 1) {
-            s += __shfl_xor_sync(0xffffffffu, s, o);
-            sd += __shfl_xor_sync(0xffffffffu, sd, o);
+    // |rd|^2, c.x, bound term, |dx recession viol|^2, c.dx, sum |c dx|, bound term of A^T dy, sum |terms|, |viol|^2
+    double a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    for (int sl = blockIdx.x * (TB / 32) + (threadIdx.x >> 5); sl < nsl; sl += gridDim.x * (TB / 32)) {
+        double s[1], sd[1] = {0.0};
+        const ZT* g1[1] = {yt};
+        sell_pair_dot<C, 1>(off, idx, val, sl, lane, g1, s);
+        if (rays) {
+            const double* gd[1] = {yd};
+            sell_pair_dot<C, 1>(off, idx, val, sl, lane, gd, sd);
         }
-        if (valid && sub == 0) {
-            double g = c[j] + (map.atybar ? map.atybar[j] : 0.0) + ds * (s / dc[j]);
-            bool fl = isfinite(lb[j]), fu = isfinite(ub[j]);
-            double lam = (fl && fu) ? g : (fl ? fmax(g, 0.0) : (fu ? fmin(g, 0.0) : 0.0));
-            double rd = g - lam;
-            d2 += rd * rd;
-            double x = (map.xbar ? map.xbar[j] : 0.0) + ps * (dc[j] * (double)xt[j]);
-            pc += c[j] * x;
-            if (lam > 0.0) lam_t += lam * lb[j];
-            else if (lam < 0.0) lam_t += lam * ub[j];
-            if (rays) {
-                const double dxo = dc[j] * xd[j];
-                prc += c[j] * dxo;
-                prm += fabs(c[j] * dxo);
-                const double bv = (fl && dxo < 0.0 ? -dxo : 0.0) + (fu && dxo > 0.0 ? dxo : 0.0);
-                prv += bv * bv;
-                const double at = sd / dc[j];  // (A^T dy)_j, original space
-                const double t = at > 0.0 ? (fl ? at * lb[j] : 0.0) : (at < 0.0 ? (fu ? at * ub[j] : 0.0) : 0.0);
-                drl += t;
-                drm += fabs(t);
-                const double av = (!fl && at > 0.0 ? at : 0.0) + (!fu && at < 0.0 ? -at : 0.0);
-                drv += av * av;
-            }
+        const int j = sl * C + lane;
+        if (lane >= C || j >= n) continue;
+        const double cj = c[j], lj = lb[j], uj = ub[j], dcj = dc[j];
+        double g = cj + (map.atybar ? map.atybar[j] : 0.0) + ds * (s[0] / dcj);
+        const bool fl = isfinite(lj), fu = isfinite(uj);
+        double lam = (fl && fu) ? g : (fl ? fmax(g, 0.0) : (fu ? fmin(g, 0.0) : 0.0));
+        double rd = g - lam;
+        a[0] += rd * rd;
+        double x = (map.xbar ? map.xbar[j] : 0.0) + ps * (dcj * (double)xt[j]);
+        a[1] += cj * x;
+        if (lam > 0.0) a[2] += lam * lj;
+        else if (lam < 0.0) a[2] += lam * uj;
+        if (rays) {
+            const double dxo = dcj * xd[j];
+            a[4] += cj * dxo;
+            a[5] += fabs(cj * dxo);
+            const double bv = (fl && dxo < 0.0 ? -dxo : 0.0) + (fu && dxo > 0.0 ? dxo : 0.0);
+            a[3] += bv * bv;
+            const double at = sd[0] / dcj;  // (A^T dy)_j, original space
+            const double t = at > 0.0 ? (fl ? at * lj : 0.0) : (at < 0.0 ? (fu ? at * uj : 0.0) : 0.0);
+            a[6] += t;
+            a[7] += fabs(t);
+            const double av = (!fl && at > 0.0 ? at : 0.0) + (!fu && at < 0.0 ? -at : 0.0);
+            a[8] += av * av;
         }
     }
-    block_sum_to(d2, &ctrl->acc[A_DRES2]);
-    block_sum_to(pc, &ctrl->acc[A_PC]);
-    block_sum_to(lam_t, &ctrl->acc[A_LAM]);
-    if (rays) {
-        block_sum_to(prv, &ctrl->acc[A_PRV2]);
-        block_sum_to(prc, &ctrl->acc[A_PRC]);
-        block_sum_to(prm, &ctrl->acc[A_PRM]);
-        block_sum_to(drl, &ctrl->acc[A_DRL]);
-        block_sum_to(drm, &ctrl->acc[A_DRM]);
-        block_sum_to(drv, &ctrl->acc[A_DRV2]);
-    }
+    double* const slots[9] = {&ctrl->acc[A_DRES2], &ctrl->acc[A_PC],  &ctrl->acc[A_LAM],
+                              &ctrl->acc[A_PRV2],  &ctrl->acc[A_PRC], &ctrl->acc[A_PRM],
+                              &ctrl->acc[A_DRL],   &ctrl->acc[A_DRM], &ctrl->acc[A_DRV2]};
+    block_sums_to<9>(a, slots);
 }
 
 // One thread: termination, restart and primal-weight decisions for the chunk just run.
@@ -1153,19 +1221,31 @@ void launch_iter(int mode, int L, int R, unsigned grid, int tb, cudaStream_t s, 
     else launch_iter_LR<VT, GT, 1, M_PLAIN, PRIMAL>(L, grid, tb, s, a, it);
 }
 
+// CTAs of a kernel over the slices of a check copy, one warp each, at most one resident wave
+unsigned slice_grid(const Sell& S, int sm_count) { return grid_for(S.slices * 32, TB, sm_count, 8); }
+
 template <typename MT>
-void launch_kkt(int Lr, int Lc, unsigned gr, unsigned gc, cudaStream_t s, const DevLP& lp, HalpernWork* w,
-                const KktMap& map, Ctrl* ctrl) {
+void launch_kkt(Ctx* ctx, const DevLP& lp, HalpernWork* w, const KktMap& map, Ctrl* ctrl) {
+    cudaStream_t s = ctx->stream;
     const double* xd = w->rays ? w->xd.p : nullptr;
     const double* yd = w->rays ? w->yd.p : nullptr;
     const MT* xt = (const MT*)w->xt.p;
     const MT* yt = (const MT*)w->yt.p;
-#define KR(LL) k_kkt_rows<LL, MT><<<gr, TB, 0, s>>>(lp.m, lp.rowptr.p, lp.colidx.p, w->sv64.p, xt, yt, lp.b.p, lp.is_eq.p, w->dr.p, map, xd, yd, ctrl)
-#define KC(LL) k_kkt_cols<LL, MT><<<gc, TB, 0, s>>>(lp.n, lp.t_rowptr.p, lp.t_colidx.p, w->stv64.p, yt, xt, lp.c.p, lp.lb.p, lp.ub.p, w->dc.p, map, xd, yd, ctrl)
-    switch (Lr) { case 1: KR(1); break; case 2: KR(2); break; case 4: KR(4); break; case 8: KR(8); break; case 16: KR(16); break; default: KR(32); }
-    switch (Lc) { case 1: KC(1); break; case 2: KC(2); break; case 4: KC(4); break; case 8: KC(8); break; case 16: KC(16); break; default: KC(32); }
-#undef KR
-#undef KC
+    const unsigned gr = slice_grid(w->kr, ctx->sm_count), gc = slice_grid(w->kc, ctx->sm_count);
+    auto rows = [&](auto fn) {
+        fn<<<gr, TB, 0, s>>>(lp.m, w->kr.off.p, w->kr.idx.p, w->kr.v64.p, xt, yt, lp.b.p, lp.is_eq.p, w->dr.p, map, xd, yd,
+                             ctrl);
+    };
+    auto cols = [&](auto fn) {
+        fn<<<gc, TB, 0, s>>>(lp.n, w->kc.off.p, w->kc.idx.p, w->kc.v64.p, yt, xt, lp.c.p, lp.lb.p, lp.ub.p, w->dc.p, map, xd,
+                             yd, ctrl);
+    };
+    if (w->kr.C == 32) rows(k_kkt_rows<32, MT>);
+    else if (w->kr.C == 16) rows(k_kkt_rows<16, MT>);
+    else rows(k_kkt_rows<8, MT>);
+    if (w->kc.C == 32) cols(k_kkt_cols<32, MT>);
+    else if (w->kc.C == 16) cols(k_kkt_cols<16, MT>);
+    else cols(k_kkt_cols<8, MT>);
 }
 
 // Scaling, scaled copies and ||A_s||_2 (FP64, once per uploaded LP and ruiz count).
@@ -1205,36 +1285,36 @@ int power_sigma2(Ctx* ctx, HalpernWork* w, double* sigma2) {
     DevLP& L = w->ilp;
     cudaStream_t s = ctx->stream;
     const int m = L.m, n = L.n;
-    unsigned gm = grid_for(m, TB, ctx->sm_count), gn = grid_for(n, TB, ctx->sm_count, 4);
-    double* scal = w->pw.p;  // [0] ||w||^2 accumulator, [1] ||v||, [2..17] history of ||A^T A v|| / ||v||
+    const unsigned gr = slice_grid(w->kr, ctx->sm_count), gc = slice_grid(w->kc, ctx->sm_count);
     const int kMax = 512, kRound = 16;
-    k_pow_init<<<gn, TB, 0, s>>>(n, w->pv.p);
-    k_fill<<<1, 32, 0, s>>>(2, 0.0, scal);
+    double* nrm2 = w->pw.p;  // [t]: the squared norm of the vector step t starts from
+    B2P_CUDA(ctx, cudaMemsetAsync(nrm2, 0, sizeof(double) * (kMax + 1), s));
+    k_pow_init<<<grid_for(n, TB, ctx->sm_count, 4), TB, 0, s>>>(n, w->pv.p, nrm2);
     B2P_LAUNCH(ctx);
-    // ||v|| of the start vector (once, on the host)
-    {
-        std::vector<double> hv(n);
-        B2P_CUDA(ctx, cudaMemcpyAsync(hv.data(), w->pv.p, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-        B2P_CUDA(ctx, cudaStreamSynchronize(s));
-        double nn = 0;
-        for (double v : hv) nn += v * v;
-        nn = std::sqrt(nn);
-        B2P_CUDA(ctx, cudaMemcpyAsync(scal + 1, &nn, sizeof(double), cudaMemcpyHostToDevice, s));
-    }
-    double hist[kRound];
+    ctx->launches += 1;
+    auto rows = [&](auto fn, int t) {
+        fn<<<gr, TB, 0, s>>>(m, w->kr.off.p, w->kr.idx.p, w->kr.v64.p, w->pv.p, nrm2 + t, w->pu.p);
+    };
+    auto cols = [&](auto fn, int t) {
+        fn<<<gc, TB, 0, s>>>(n, w->kc.off.p, w->kc.idx.p, w->kc.v64.p, w->pu.p, w->pv.p, nrm2 + t + 1);
+    };
     double est = 0.0;
     for (int t = 0; t < kMax; t += kRound) {
-        for (int q = 0; q < kRound; ++q) {
-            k_pow_rows<<<gm, TB, 0, s>>>(m, L.rowptr.p, L.colidx.p, w->sv64.p, w->pv.p, scal + 1, w->pu.p);
-            k_pow_cols<<<gn, TB, 0, s>>>(n, L.t_rowptr.p, L.t_colidx.p, w->stv64.p, w->pu.p, w->pv.p, scal);
-            k_pow_finish<<<1, 1, 0, s>>>(scal, scal + 1, scal + 2, q);
+        for (int q = t; q < t + kRound; ++q) {
+            if (w->kr.C == 32) rows(k_pow_rows<32>, q);
+            else if (w->kr.C == 16) rows(k_pow_rows<16>, q);
+            else rows(k_pow_rows<8>, q);
+            if (w->kc.C == 32) cols(k_pow_cols<32>, q);
+            else if (w->kc.C == 16) cols(k_pow_cols<16>, q);
+            else cols(k_pow_cols<8>, q);
         }
         B2P_LAUNCH(ctx);
-        ctx->launches += 3 * kRound;
-        B2P_CUDA(ctx, cudaMemcpyAsync(hist, scal + 2, sizeof(hist), cudaMemcpyDeviceToHost, s));
+        ctx->launches += 2 * kRound;
+        double last[2];  // ||A^T A v|| with ||v|| = 1  ->  sigma_max^2, of the round's last two steps
+        B2P_CUDA(ctx, cudaMemcpyAsync(last, nrm2 + t + kRound - 1, sizeof(last), cudaMemcpyDeviceToHost, s));
         B2P_CUDA(ctx, cudaStreamSynchronize(s));
-        est = hist[kRound - 1];
-        double prev = hist[kRound - 2];
+        const double prev = std::sqrt(last[0]);
+        est = std::sqrt(last[1]);
         if (est > 0 && std::fabs(est - prev) <= 1e-7 * est) break;
     }
     *sigma2 = est;
@@ -1331,6 +1411,7 @@ int build_internal(Ctx* ctx, HalpernWork* w) {
     I.max_row_len = U.max_row_len;
     I.max_col_len = U.max_col_len;
     for (int k = 0; k < 3; ++k) w->sr_all[k].idx_ready = w->sc_all[k].idx_ready = false;
+    w->kr.idx_ready = w->kc.idx_ready = false;
     w->sr = &w->sr_all[0];
     w->sc = &w->sc_all[0];
     B2P_CUDA(ctx, cudaStreamSynchronize(s));
@@ -1341,7 +1422,7 @@ int build_internal(Ctx* ctx, HalpernWork* w) {
 // Slice layout and indices of a SELL copy (once per upload): vector width W = 4 or 2
 // when its padding costs at most 3 % over W = 1, which pads only to each slice's
 // longest row.
-int build_sell_layout(Ctx* ctx, Sell& S, int rows, const int32_t* ptr, const int32_t* idx, int C) {
+int build_sell_layout(Ctx* ctx, Sell& S, int rows, const int32_t* ptr, const int32_t* idx, int C, int force_W = 0) {
     cudaStream_t s = ctx->stream;
     const int nsl = (rows + C - 1) / C;
     DBuf<int32_t> slen;
@@ -1359,7 +1440,8 @@ int build_sell_layout(Ctx* ctx, Sell& S, int rows, const int32_t* ptr, const int
     const int pad_pct = 3;  // padding allowed for the wider vectors, percent of the W = 1 layout
     const int64_t t1 = padded_total(1);
     int W = 1;
-    if (padded_total(4) <= t1 + t1 * pad_pct / 100) W = 4;
+    if (force_W) W = force_W;
+    else if (padded_total(4) <= t1 + t1 * pad_pct / 100) W = 4;
     else if (padded_total(2) <= t1 + t1 * pad_pct / 100) W = 2;
     std::vector<int64_t> off(nsl + 1, 0);
     for (int i = 0; i < nsl; ++i) off[i + 1] = off[i] + (int64_t)C * ((h[i] + W - 1) / W * W);
@@ -1759,8 +1841,6 @@ int run_chunks(Ctx* ctx, HalpernWork* w, const b2p_params* p, double time_limit_
     unsigned grR = iter_grid(m, Lr, Rr, Tr, ctx->sm_count), gcR = iter_grid(n, Lc, Rc, Tc, ctx->sm_count);
     // SELL grids: one thread per row, or the windows' one-wave grid
     const unsigned grS = w->wr.smem ? w->wr.G : gr, gcS = w->wc.smem ? w->wc.G : gc;
-    const int Lkr = pick_lanes(L.mean_row_len, 0), Lkc = pick_lanes(L.mean_col_len, 0);
-    unsigned gkr = iter_grid(m, Lkr, 1, TB, ctx->sm_count), gkc = iter_grid(n, Lkc, 1, TB, ctx->sm_count);
     Ctrl* ctrl = w->ctrl.p;
     const IterArgs<MT, MT> pa = primal_args<MT>(L, w, p, w->sell_c);
     const IterArgs<MT, MT> da = dual_args<MT>(L, w, p, w->sell_r);
@@ -1776,7 +1856,7 @@ int run_chunks(Ctx* ctx, HalpernWork* w, const b2p_params* p, double time_limit_
         }
         const KktMap map = w->recenter ? KktMap{w->xbar.p, w->ybar.p, w->axbar.p, w->atybar.p}
                                        : KktMap{nullptr, nullptr, nullptr, nullptr};
-        launch_kkt<MT>(Lkr, Lkc, gkr, gkc, s, L, w, map, ctrl);
+        launch_kkt<MT>(ctx, L, w, map, ctrl);
         k_control<<<1, 1, 0, s>>>(ctrl);
         const unsigned gv = grid_for(std::max(m, n), TB, ctx->sm_count, 8);
         if (w->recenter) {
@@ -1912,6 +1992,23 @@ int solve_T(Ctx* ctx, HalpernWork* w, const b2p_params* p, const double* x0, con
             if (st) return st;
         }
     }
+    // the check copies: slices of 32 rows where that gives every SM 32 warps, else 16 or 8
+    auto height = [&](int64_t rows) {
+        const int64_t want = 32LL * ctx->sm_count;
+        return rows >= 32 * want ? 32 : (rows >= 16 * want ? 16 : 8);
+    };
+    if (!w->kr.idx_ready) {
+        st = build_sell_layout(ctx, w->kr, m, L.rowptr.p, L.colidx.p, height(m), 2);
+        if (st) return st;
+    }
+    if (!w->kc.idx_ready) {
+        st = build_sell_layout(ctx, w->kc, n, L.t_rowptr.p, L.t_colidx.p, height(n), 2);
+        if (st) return st;
+    }
+    st = fill_sell_vals<double>(ctx, w->kr, m, L.rowptr.p, w->sv64.p, w->kr.v64);
+    if (st) return st;
+    st = fill_sell_vals<double>(ctx, w->kc, n, L.t_rowptr.p, w->stv64.p, w->kc.v64);
+    if (st) return st;
     double sig2 = 0.0;
     st = power_sigma2(ctx, w, &sig2);
     if (st) return st;
@@ -1919,15 +2016,14 @@ int solve_T(Ctx* ctx, HalpernWork* w, const b2p_params* p, const double* x0, con
     double eta = sigma_max > 0 ? p->step_safety / sigma_max : 1.0;
     double omega = p->primal_weight;
     if (!(omega > 0)) {  // ||c_s|| / ||b_s||
-        std::vector<double> hb(m), hc(n);
-        B2P_CUDA(ctx, cudaMemcpyAsync(hb.data(), w->b64.p, sizeof(double) * m, cudaMemcpyDeviceToHost, s));
-        B2P_CUDA(ctx, cudaMemcpyAsync(hc.data(), w->c64.p, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
+        double q[2];
+        B2P_CUDA(ctx, cudaMemsetAsync(w->pw.p, 0, sizeof(q), s));
+        k_norms2<<<grid_for(std::max(m, n), TB, ctx->sm_count, 4), TB, 0, s>>>(m, w->b64.p, n, w->c64.p, w->pw.p);
+        B2P_LAUNCH(ctx);
+        ctx->launches += 1;
+        B2P_CUDA(ctx, cudaMemcpyAsync(q, w->pw.p, sizeof(q), cudaMemcpyDeviceToHost, s));
         B2P_CUDA(ctx, cudaStreamSynchronize(s));
-        double bn = 0, cn = 0;
-        for (double v : hb) bn += v * v;
-        for (double v : hc) cn += v * v;
-        bn = std::sqrt(bn);
-        cn = std::sqrt(cn);
+        const double bn = std::sqrt(q[0]), cn = std::sqrt(q[1]);
         omega = (bn > 1e-10 && cn > 1e-10) ? cn / bn : 1.0;
     }
     // warm start (original space) -> device temporaries
@@ -2139,7 +2235,7 @@ int halpern_engine_solve(Ctx* ctx, const b2p_params* p, const double* x0, const 
         for (auto* b : {&w->c32, &w->l32, &w->u32}) B2P_CUDA(ctx, b->reserve(n));
         for (auto* b : {&w->b32, &w->ylb32}) B2P_CUDA(ctx, b->reserve(m));
     }
-    B2P_CUDA(ctx, w->pw.reserve(64));
+    B2P_CUDA(ctx, w->pw.reserve(1024));
     B2P_CUDA(ctx, w->sv64.reserve(nnz));
     B2P_CUDA(ctx, w->stv64.reserve(nnz));
     B2P_CUDA(ctx, w->ctrl.reserve(1));
