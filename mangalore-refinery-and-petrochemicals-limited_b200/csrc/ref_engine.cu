@@ -22,6 +22,7 @@
 
 #include "b2p_internal.cuh"
 #include "cluster.cuh"
+#include "pdl.cuh"
 
 namespace b2p {
 
@@ -173,6 +174,8 @@ template <bool CHECK, bool SLICED>
 __global__ void __launch_bounds__(128) k_ref_primal(int n, Sell At, const double* __restrict__ c,
                                                     const double* __restrict__ lb, const double* __restrict__ ub,
                                                     RefState st) {
+    pdl_wait();
+    pdl_trigger();
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         double w = row_sum<kBatch, SLICED>(At, j, st.y);
         double xj = st.x[j];
@@ -191,6 +194,8 @@ template <bool CHECK, bool SLICED>
 __global__ void __launch_bounds__(128) k_ref_dual(int m, Sell A, const double* __restrict__ b,
                                                   const uint8_t* __restrict__ is_eq, RefState st) {
     int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
     for (int i = tid; i < m; i += gridDim.x * blockDim.x) {
         double v = row_sum<kBatch, SLICED>(A, i, st.x_hat);
         double yi = st.y[i];
@@ -250,8 +255,9 @@ double bits_to_double(unsigned long long b) {
 // cluster barrier behind the remote stores (about 1 us a phase).  us per iteration, before ->
 // now (two kernels in a graph -> this): 60 x 200 7.9 -> 0.95 and 300 x 1,000 9.0 -> 2.7 (one
 // CTA / cluster), 1,000 x 3,000 10.0 -> 3.9, 2,000 x 6,000 10.1 -> 5.2.  From 3,000 x 9,000 on
-// (54,000 entries) the stores into eight copies cost as much as kernel boundaries: 8.5 here, 8.5
-// with two kernels (12.2 before, over CSR), so the line is drawn at 49,152 entries.
+// (54,000 entries) the stores into eight copies cost more than kernel boundaries: 8.5 here, 7.2
+// with two kernels (12.2 before, over CSR and without their overlap), so the line is drawn at
+// 49,152 entries.
 struct RefOutcome {
     long long iter;
     int converged, failed;
@@ -575,13 +581,11 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
 
     auto primal = [&](auto check) {
         constexpr bool C = decltype(check)::value;
-        if (At.off) k_ref_primal<C, true><<<gn, TB, 0, s>>>(n, At, L.c.p, L.lb.p, L.ub.p, st);
-        else k_ref_primal<C, false><<<gn, TB, 0, s>>>(n, At, L.c.p, L.lb.p, L.ub.p, st);
+        pdl_launch(At.off ? k_ref_primal<C, true> : k_ref_primal<C, false>, gn, TB, 0, s, n, At, L.c.p, L.lb.p, L.ub.p, st);
     };
     auto dual = [&](auto check) {
         constexpr bool C = decltype(check)::value;
-        if (A.off) k_ref_dual<C, true><<<gm, TB, 0, s>>>(m, A, L.b.p, L.is_eq.p, st);
-        else k_ref_dual<C, false><<<gm, TB, 0, s>>>(m, A, L.b.p, L.is_eq.p, st);
+        pdl_launch(A.off ? k_ref_dual<C, true> : k_ref_dual<C, false>, gm, TB, 0, s, m, A, L.b.p, L.is_eq.p, st);
     };
     auto check_xs = [&]() {
         k_ref_check_cols<<<gn, TB, 0, s>>>(n, L.lb.p, L.ub.p, st);
