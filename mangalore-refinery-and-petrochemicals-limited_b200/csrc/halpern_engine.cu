@@ -1694,11 +1694,13 @@ int ensure_sell(Ctx* ctx, HalpernWork* w, bool primal, int k) {
 }
 
 // Times candidate launch shapes of the primal and dual kernels on the uploaded LP
-// (plain iterations from the current iterates, CUDA events on the context stream)
-// and keeps the fastest of each side: the SELL kernel with slice heights 32 / 16 / 8
+// (plain iterations from the current iterates, CUDA events on the context stream: the
+// candidate and the other side's kernel in turn, as in a solve, so that the candidate finds
+// the L2 the other side leaves and overlaps its end; the faster of two bursts of four
+// iterations counts) and keeps the fastest of each side, the dual's next to the chosen primal: the SELL kernel with slice heights 32 / 16 / 8
 // (1 / 2 / 4 lanes per row) and CTA sizes 256 / 512 / 1024, the SELL kernel with
 // gather windows in shared memory (32-row slices, kWinShapes), and the CSR kernel
-// with (L lanes per row, R rows per lane group, CTA size).  The caller
+// with L lanes per row, then R rows per lane group and the CTA size for the best L.  The caller
 // re-initialises the iterates afterwards.  lanes_per_row > 0 forces the CSR kernel
 // with that L, -1 the SELL kernel (32-row slices, CTA size 256), -2 the windowed
 // SELL kernel (CTA size 512, 96 KB), -3 / -4 the SELL kernel with 16- / 8-row slices
@@ -1763,6 +1765,21 @@ int autotune_shapes(Ctx* ctx, HalpernWork* w, const b2p_params* p) {
         float best = 1e30f;
         int bestL = base_L, bestR = 1, bestT = 256, bestWin = -1, bestK = 0;
         bool bestS = false;
+        float last = 1e30f;  // time of the last trial
+        // the other side's kernel: the dual's plain form while the primal is tuned, then the tuned primal
+        if (primal) w->sr = &w->sr_all[0];
+        const IterArgs<MT, MT> oa = primal ? dual_args<MT>(L, w, p, true) : primal_args<MT>(L, w, p, w->sell_c);
+        auto other = [&](int rep) {
+            if (primal)
+                launch_sell<MT, MT, false>(M_PLAIN, w->sr_all[0], iter_grid(m, 1, 1, 256, ctx->sm_count), 256, 0, s, oa, rep);
+            else if (w->sell_c)
+                launch_sell<MT, MT, true>(M_PLAIN, *w->sc,
+                                          w->wc.smem ? w->wc.G : iter_grid(n, w->Lc, 1, w->Tc, ctx->sm_count), w->Tc,
+                                          w->wc.smem, s, oa, rep);
+            else
+                launch_iter<MT, MT, true>(M_PLAIN, w->Lc, w->Rc, iter_grid(n, w->Lc, w->Rc, w->Tc, ctx->sm_count), w->Tc, s,
+                                          oa, rep);
+        };
         // kind 0: CSR (Lc, R, tb); 1: SELL (layout k, tb); 2: windowed SELL (32-row slices, shape k)
         auto trial = [&](int kind, int Lc, int R, int tb, int k) -> int {
             unsigned g;
@@ -1784,23 +1801,27 @@ int autotune_shapes(Ctx* ctx, HalpernWork* w, const b2p_params* p) {
                 win.smem = 0;
                 g = iter_grid(rows, Lc, R, tb, ctx->sm_count);
             }
-            const IterArgs<MT, MT> pa = primal_args<MT>(L, w, p, kind != 0);
-            const IterArgs<MT, MT> da = dual_args<MT>(L, w, p, kind != 0);
-            float tot = 0.f;
-            for (int rep = 0; rep < 4; ++rep) {
+            float tot = 1e30f;
+            const IterArgs<MT, MT> mine = primal ? primal_args<MT>(L, w, p, kind != 0) : dual_args<MT>(L, w, p, kind != 0);
+            for (int burst = 0; burst < 3; ++burst) {  // the first one warms caches
                 cudaEventRecord(e0, s);
-                if (kind != 0 && primal) launch_sell<MT, MT, true>(M_PLAIN, **cur, g, tb, smem, s, pa, rep);
-                else if (kind != 0) launch_sell<MT, MT, false>(M_PLAIN, **cur, g, tb, smem, s, da, rep);
-                else if (primal) launch_iter<MT, MT, true>(M_PLAIN, Lc, R, g, tb, s, pa, rep);
-                else launch_iter<MT, MT, false>(M_PLAIN, Lc, R, g, tb, s, da, rep);
+                for (int rep = 0; rep < (burst ? 4 : 1); ++rep) {
+                    if (!primal) other(rep);
+                    if (kind != 0 && primal) launch_sell<MT, MT, true>(M_PLAIN, **cur, g, tb, smem, s, mine, rep);
+                    else if (kind != 0) launch_sell<MT, MT, false>(M_PLAIN, **cur, g, tb, smem, s, mine, rep);
+                    else if (primal) launch_iter<MT, MT, true>(M_PLAIN, Lc, R, g, tb, s, mine, rep);
+                    else launch_iter<MT, MT, false>(M_PLAIN, Lc, R, g, tb, s, mine, rep);
+                    if (primal) other(rep);
+                }
                 cudaEventRecord(e1, s);
                 B2P_LAUNCH(ctx);
                 B2P_CUDA(ctx, cudaEventSynchronize(e1));
                 float ms = 0.f;
                 cudaEventElapsedTime(&ms, e0, e1);
-                if (rep > 0) tot += ms;  // first launch warms caches
+                if (burst) tot = std::min(tot, ms);
             }
-            ctx->launches += 4;
+            ctx->launches += 18;
+            last = tot;
             if (tot < best) {
                 best = tot;
                 bestS = kind != 0;
@@ -1821,14 +1842,28 @@ int autotune_shapes(Ctx* ctx, HalpernWork* w, const b2p_params* p) {
             int st = trial(2, 1, 1, kWinShapes[k][0], k);
             if (st) return st;
         }
+        int csr_L = 0;
+        float csr_best = 1e30f;
+        auto csr = [&](int Lc, int R, int tb) -> int {
+            int st = trial(0, Lc, R, tb, 0);
+            if (st == B2P_OK && last < csr_best) {
+                csr_best = last;
+                csr_L = Lc;
+            }
+            return st;
+        };
         for (int Lc : {base_L / 2, base_L, base_L * 2}) {
             if (Lc < 2 || Lc > 32) continue;
-            for (int R : {1, 2, 4})
-                for (int tb : {256, 512, 1024}) {
-                    int st = trial(0, Lc, R, tb, 0);
-                    if (st) return st;
-                }
+            int st = csr(Lc, 1, 256);
+            if (st) return st;
         }
+        const int L0 = csr_L;
+        for (int R : {1, 2, 4})
+            for (int tb : {256, 512, 1024}) {
+                if (R == 1 && tb == 256) continue;  // timed above
+                int st = csr(L0, R, tb);
+                if (st) return st;
+            }
         win.smem = 0;
         *cur = &all[bestK];
         if (bestWin >= 0) {
