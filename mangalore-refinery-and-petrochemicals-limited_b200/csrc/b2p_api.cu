@@ -33,6 +33,9 @@ double now_ms() {
 }
 
 // ---------------------------------------------------------------- transpose (setup only)
+// Entries up to which the context keeps the scratch of a transpose (16 bytes each) for the next one.
+constexpr int64_t kKeepTranspose = 1 << 20;
+
 __global__ void k_row_of(int m, const int32_t* __restrict__ rowptr, int32_t* __restrict__ row_of) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
         for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) row_of[k] = i;
@@ -63,7 +66,7 @@ int build_transpose(Ctx* ctx, int m, int n, int64_t nnz, const int32_t* rowptr, 
     cudaStream_t s = ctx->stream;
     B2P_CUDA(ctx, cudaMemsetAsync(t_rowptr, 0, sizeof(int32_t) * (n + 1), s));
     if (nnz == 0) return B2P_OK;
-    DBuf<int32_t> row_of, keys_out, perm_in, perm_out;
+    DBuf<int32_t>&row_of = ctx->tr_row, &keys_out = ctx->tr_keys, &perm_in = ctx->tr_in, &perm_out = ctx->tr_out;
     B2P_CUDA(ctx, row_of.reserve(nnz));
     B2P_CUDA(ctx, keys_out.reserve(nnz));
     B2P_CUDA(ctx, perm_in.reserve(nnz));
@@ -91,8 +94,10 @@ int build_transpose(Ctx* ctx, int m, int n, int64_t nnz, const int32_t* rowptr, 
     k_gather_t<<<gz, 256, 0, s>>>(nnz, perm_out.p, row_of.p, vals, t_colidx, t_vals);
     B2P_LAUNCH(ctx);
     ctx->launches += 4;
-    // temporaries are freed on return; make sure the stream is done with them
+    // a large matrix's temporaries are freed on return; make sure the stream is done with them
     B2P_CUDA(ctx, cudaStreamSynchronize(s));
+    if (nnz > kKeepTranspose)
+        for (auto* d : {&row_of, &keys_out, &perm_in, &perm_out}) d->release();
     return B2P_OK;
 }
 
@@ -125,6 +130,88 @@ __global__ void k_spmv_f64(int m, const int32_t* __restrict__ rowptr, const int3
         for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) sum += vals[k] * x[colidx[k]];
         y[i] = sum;
     }
+}
+
+// y = A x of an unchecked matrix: entries whose column is out of range or not above the one before
+// are not read through and mark *bad (as k_validate_csr does).
+__global__ void k_spmv_checked(int m, int n, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colidx,
+                               const double* __restrict__ vals, const double* __restrict__ x, double* __restrict__ y,
+                               int32_t* __restrict__ bad) {
+    constexpr int B = 8;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+        double sum = 0.0;
+        int prev = -1;
+        const int e1 = rowptr[i + 1];
+        for (int k = rowptr[i]; k < e1; k += B) {
+            int c[B];
+            double v[B], g[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                c[u] = k + u < e1 ? colidx[k + u] : -1;
+                v[u] = k + u < e1 ? vals[k + u] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                const bool ok = c[u] >= 0 && c[u] < n;
+                g[u] = ok ? x[c[u]] : 0.0;
+                if (k + u < e1) {
+                    if (!ok || c[u] <= prev) atomicExch(bad, i + 1);
+                    prev = c[u];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < B; ++u)
+                if (k + u < e1) sum += v[u] * g[u];
+        }
+        y[i] = sum;
+    }
+}
+
+// w = A^T y of a small unchecked matrix in one CTA, without a transpose: the products to shared
+// memory, then one warp adds them row after row, as the reference scatter does (the columns of a
+// row are distinct, so its entries go side by side; a row that is not is refused anyway).
+__global__ void __launch_bounds__(1024, 1) k_spmv_t_small(int m, int n, const int32_t* __restrict__ rowptr,
+                                                          const int32_t* __restrict__ colidx,
+                                                          const double* __restrict__ vals, const double* __restrict__ y,
+                                                          double* __restrict__ w, int32_t* __restrict__ bad,
+                                                          int rows_off) {
+    extern __shared__ double sh[];
+    const int nnz = rowptr[m], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *ws = sh, *prod = ws + n;
+    int16_t* col = reinterpret_cast<int16_t*>(prod + nnz);  // -1: not read through
+    for (int j = threadIdx.x; j < n; j += blockDim.x) ws[j] = 0.0;
+    for (int i = threadIdx.x; i <= m; i += blockDim.x) reinterpret_cast<int*>(sh + rows_off)[i] = rowptr[i];
+    for (int i = warp; i < m; i += blockDim.x >> 5) {
+        const int e0 = rowptr[i], e1 = rowptr[i + 1];
+        const double yi = y[i];
+        for (int e = e0 + lane; e < e1; e += 32) {
+            const int c = colidx[e], before = e > e0 ? colidx[e - 1] : -1;
+            const bool ok = c >= 0 && c < n;
+            if (!ok || c <= before) atomicExch(bad, i + 1);
+            col[e] = ok ? (int16_t)c : (int16_t)-1;
+            prod[e] = vals[e] * yi;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int* rows = reinterpret_cast<int*>(sh + rows_off);
+        int e = lane < rows[1] ? lane : -1;  // this lane's entry of the next step, read ahead
+        int c = e >= 0 ? col[e] : -1;
+        double p = e >= 0 ? prod[e] : 0.0;
+        for (int i = 0, b = 0; i < m;) {
+            const int c0 = c;
+            const double p0 = p;
+            b += 32;
+            if (b >= rows[i + 1]) b = rows[++i];
+            e = i < m && b + lane < rows[i + 1] ? b + lane : -1;
+            c = e >= 0 ? col[e] : -1;
+            p = e >= 0 ? prod[e] : 0.0;
+            if (c0 >= 0) ws[c0] += p0;
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < n; j += blockDim.x) w[j] = ws[j];
 }
 
 __global__ void k_vec(int op, size_t n, double alpha, const double* __restrict__ a, const double* __restrict__ b,
@@ -176,23 +263,24 @@ __global__ void k_sum_partials(int count, const double* __restrict__ partial, do
     }
 }
 
+// Events around the phases of a call, recorded only where the caller asked for its times; the
+// context keeps them.
 struct PhaseTimer {
-    cudaEvent_t e[4];
-    bool ok = false;
-    PhaseTimer() {
-        ok = true;
-        for (auto& x : e)
-            if (cudaEventCreate(&x) != cudaSuccess) ok = false;
+    Ctx* ctx;
+    bool ok;
+    PhaseTimer(Ctx* c, const b2p_timing_t* t) : ctx(c), ok(t != nullptr) {
+        for (auto& x : c->tev)
+            if (ok && !x && cudaEventCreate(&x) != cudaSuccess) ok = false;
     }
-    ~PhaseTimer() {
-        for (auto& x : e) cudaEventDestroy(x);
+    void mark(int phase) {
+        if (ok) cudaEventRecord(ctx->tev[phase], ctx->stream);
     }
     void fill(b2p_timing_t* t, double host_t0) {
         if (!t || !ok) return;
         float a = 0, b = 0, c = 0;
-        cudaEventElapsedTime(&a, e[0], e[1]);
-        cudaEventElapsedTime(&b, e[1], e[2]);
-        cudaEventElapsedTime(&c, e[2], e[3]);
+        cudaEventElapsedTime(&a, ctx->tev[0], ctx->tev[1]);
+        cudaEventElapsedTime(&b, ctx->tev[1], ctx->tev[2]);
+        cudaEventElapsedTime(&c, ctx->tev[2], ctx->tev[3]);
         t->h2d_time_ms = a;
         t->kernel_time_ms = b;
         t->d2h_time_ms = c;
@@ -201,6 +289,95 @@ struct PhaseTimer {
         t->total_gpu_time_ms = total;
     }
 };
+
+// The transfers of one call.  A call of up to kPackBytes packs its inputs into one buffer and gets
+// its outputs back through it: one copy each way instead of one per argument (each costs
+// several microseconds before its first byte).  The buffer is pageable: pinning it took 3 ms
+// in a context's first call and saved less than a microsecond in the others.  A larger call
+// copies argument by argument, as they are.
+struct CallIO {
+    static constexpr size_t kPackBytes = 1 << 20;
+    Ctx* ctx;
+    bool packed = false;
+    size_t used = 0, in_bytes = 0;
+    struct Out {
+        void* host;
+        const void* dev;
+        size_t at, bytes;
+    };
+    std::vector<Out> outs;
+
+    static size_t round(size_t b) { return (b + 15) & ~(size_t)15; }
+    // total: bytes of all arguments, each rounded up
+    int begin(Ctx* c, size_t total) {
+        ctx = c;
+        packed = total <= kPackBytes;
+        if (packed) {
+            B2P_CUDA(ctx, ctx->s_pack.reserve(total));
+            if (ctx->h_pack.size() < total) ctx->h_pack.resize(total);
+        }
+        return B2P_OK;
+    }
+    template <typename T>
+    int in(DBuf<T>& buf, const T* src, size_t n, T** dev) {
+        if (packed) {
+            std::memcpy(ctx->h_pack.data() + used, src, n * sizeof(T));
+            *dev = reinterpret_cast<T*>(ctx->s_pack.p + used);
+            used += round(n * sizeof(T));
+            return B2P_OK;
+        }
+        B2P_CUDA(ctx, buf.reserve(n));
+        *dev = buf.p;
+        if (n) B2P_CUDA(ctx, cudaMemcpyAsync(buf.p, src, n * sizeof(T), cudaMemcpyHostToDevice, ctx->stream));
+        return B2P_OK;
+    }
+    int send() {  // after the last input
+        in_bytes = used;
+        if (packed && used)
+            B2P_CUDA(ctx, cudaMemcpyAsync(ctx->s_pack.p, ctx->h_pack.data(), used, cudaMemcpyHostToDevice, ctx->stream));
+        return B2P_OK;
+    }
+    template <typename T>
+    int out(DBuf<T>& buf, T* dst, size_t n, T** dev) {
+        if (packed) {
+            *dev = reinterpret_cast<T*>(ctx->s_pack.p + used);
+            outs.push_back({dst, *dev, used, n * sizeof(T)});
+            used += round(n * sizeof(T));
+            return B2P_OK;
+        }
+        B2P_CUDA(ctx, buf.reserve(n));
+        *dev = buf.p;
+        outs.push_back({dst, buf.p, 0, n * sizeof(T)});
+        return B2P_OK;
+    }
+    int receive() {  // queues the copies back
+        if (packed) {
+            B2P_CUDA(ctx, cudaMemcpyAsync(ctx->h_pack.data() + in_bytes, ctx->s_pack.p + in_bytes, used - in_bytes,
+                                          cudaMemcpyDeviceToHost, ctx->stream));
+            return B2P_OK;
+        }
+        for (const Out& o : outs)
+            B2P_CUDA(ctx, cudaMemcpyAsync(o.host, o.dev, o.bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        return B2P_OK;
+    }
+    // waits and hands the outputs over; `bad` (the last output) nonzero: only that one
+    int finish(const int32_t* bad = nullptr) {
+        B2P_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        if (packed && bad) {
+            const Out& o = outs.back();
+            std::memcpy(o.host, ctx->h_pack.data() + o.at, o.bytes);
+            if (*bad) return B2P_OK;
+        }
+        if (packed)
+            for (const Out& o : outs) std::memcpy(o.host, ctx->h_pack.data() + o.at, o.bytes);
+        return B2P_OK;
+    }
+};
+#define B2P_DO(call)                 \
+    do {                             \
+        int _st = (call);            \
+        if (_st != B2P_OK) return _st; \
+    } while (0)
 
 }  // namespace b2p
 
@@ -324,6 +501,8 @@ int b2p_ctx_destroy(void* p) {
     mlp_free(ctx);
     ctx->lp.~DevLP();
     new (&ctx->lp) DevLP();
+    for (auto& x : ctx->tev)
+        if (x) cudaEventDestroy(x);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
@@ -348,34 +527,29 @@ int b2p_spmv(void* p, int m, int n, const int32_t* rowptr, const int32_t* colidx
     if (!host_rowptr_ok(m, nnz, rowptr)) return B2P_INVALID_ARGUMENT;
     cudaSetDevice(ctx->device);
     double t0 = now_ms();
-    PhaseTimer pt;
+    PhaseTimer pt(ctx, timing);
     cudaStream_t s = ctx->stream;
-    B2P_CUDA(ctx, ctx->s_rowptr.reserve(m + 1));
-    B2P_CUDA(ctx, ctx->s_colidx.reserve(nnz));
-    B2P_CUDA(ctx, ctx->s_vals.reserve(nnz));
-    B2P_CUDA(ctx, ctx->s_x.reserve(n));
-    B2P_CUDA(ctx, ctx->s_y.reserve(m));
-    B2P_CUDA(ctx, ctx->s_flag.reserve(1));
-    cudaEventRecord(pt.e[0], s);
-    B2P_CUDA(ctx, cudaMemcpyAsync(ctx->s_rowptr.p, rowptr, sizeof(int32_t) * (m + 1), cudaMemcpyHostToDevice, s));
-    if (nnz) {
-        B2P_CUDA(ctx, cudaMemcpyAsync(ctx->s_colidx.p, colidx, sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, s));
-        B2P_CUDA(ctx, cudaMemcpyAsync(ctx->s_vals.p, vals, sizeof(double) * nnz, cudaMemcpyHostToDevice, s));
-    }
-    B2P_CUDA(ctx, cudaMemcpyAsync(ctx->s_x.p, x, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    B2P_CUDA(ctx, cudaMemsetAsync(ctx->s_flag.p, 0, sizeof(int32_t), s));
-    cudaEventRecord(pt.e[1], s);
-    unsigned g = grid_for(m, 256, ctx->sm_count);
-    k_validate_csr<<<g, 256, 0, s>>>(m, n, ctx->s_rowptr.p, ctx->s_colidx.p, ctx->s_flag.p);
-    k_spmv_f64<<<g, 256, 0, s>>>(m, ctx->s_rowptr.p, ctx->s_colidx.p, ctx->s_vals.p, ctx->s_x.p, ctx->s_y.p);
+    int32_t *rp, *ci, *flag, bad = 0;
+    double *va, *xd, *yd;
+    CallIO io;
+    B2P_DO(io.begin(ctx, CallIO::round(4 * ((size_t)m + 1)) + CallIO::round(4 * nnz) + CallIO::round(8 * nnz) + 8 * ((size_t)n + m) + 64));
+    pt.mark(0);
+    B2P_DO(io.in(ctx->s_rowptr, rowptr, (size_t)m + 1, &rp));
+    B2P_DO(io.in(ctx->s_colidx, colidx, nnz, &ci));
+    B2P_DO(io.in(ctx->s_vals, vals, nnz, &va));
+    B2P_DO(io.in(ctx->s_x, x, n, &xd));
+    B2P_DO(io.send());
+    B2P_DO(io.out(ctx->s_y, y, m, &yd));
+    B2P_DO(io.out(ctx->s_flag, &bad, 1, &flag));
+    B2P_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(int32_t), s));
+    pt.mark(1);
+    k_spmv_checked<<<grid_for(m, 128, ctx->sm_count), 128, 0, s>>>(m, n, rp, ci, va, xd, yd, flag);
     B2P_LAUNCH(ctx);
-    ctx->launches += 2;
-    cudaEventRecord(pt.e[2], s);
-    int32_t bad = 0;
-    B2P_CUDA(ctx, cudaMemcpyAsync(y, ctx->s_y.p, sizeof(double) * m, cudaMemcpyDeviceToHost, s));
-    B2P_CUDA(ctx, cudaMemcpyAsync(&bad, ctx->s_flag.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    cudaEventRecord(pt.e[3], s);
-    B2P_CUDA(ctx, cudaStreamSynchronize(s));
+    ctx->launches += 1;
+    pt.mark(2);
+    B2P_DO(io.receive());
+    pt.mark(3);
+    B2P_DO(io.finish());
     pt.fill(timing, t0);
     if (bad) {
         ctx->err = "CSR column indices out of range or not strictly ascending in row " + std::to_string(bad - 1);
@@ -396,49 +570,55 @@ int b2p_spmv_t(void* p, int m, int n, const int32_t* rowptr, const int32_t* coli
     if (!host_rowptr_ok(m, nnz, rowptr)) return B2P_INVALID_ARGUMENT;
     cudaSetDevice(ctx->device);
     double t0 = now_ms();
-    PhaseTimer pt;
+    PhaseTimer pt(ctx, timing);
     cudaStream_t s = ctx->stream;
-    DBuf<int32_t> rp, ci, trp, tci;
-    DBuf<double> va, tva;
-    B2P_CUDA(ctx, rp.reserve(m + 1));
-    B2P_CUDA(ctx, ci.reserve(nnz));
-    B2P_CUDA(ctx, va.reserve(nnz));
-    B2P_CUDA(ctx, trp.reserve(n + 1));
-    B2P_CUDA(ctx, tci.reserve(nnz));
-    B2P_CUDA(ctx, tva.reserve(nnz));
-    B2P_CUDA(ctx, ctx->s_x.reserve(m));
-    B2P_CUDA(ctx, ctx->s_y.reserve(n));
-    B2P_CUDA(ctx, ctx->s_flag.reserve(1));
-    cudaEventRecord(pt.e[0], s);
-    B2P_CUDA(ctx, cudaMemcpyAsync(rp.p, rowptr, sizeof(int32_t) * (m + 1), cudaMemcpyHostToDevice, s));
-    if (nnz) {
-        B2P_CUDA(ctx, cudaMemcpyAsync(ci.p, colidx, sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, s));
-        B2P_CUDA(ctx, cudaMemcpyAsync(va.p, vals, sizeof(double) * nnz, cudaMemcpyHostToDevice, s));
-    }
-    B2P_CUDA(ctx, cudaMemcpyAsync(ctx->s_x.p, yv, sizeof(double) * m, cudaMemcpyHostToDevice, s));
-    B2P_CUDA(ctx, cudaMemsetAsync(ctx->s_flag.p, 0, sizeof(int32_t), s));
-    cudaEventRecord(pt.e[1], s);
-    unsigned g = grid_for(m, 256, ctx->sm_count);
-    k_validate_csr<<<g, 256, 0, s>>>(m, n, rp.p, ci.p, ctx->s_flag.p);
-    int32_t bad = 0;
-    B2P_CUDA(ctx, cudaMemcpyAsync(&bad, ctx->s_flag.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    B2P_CUDA(ctx, cudaStreamSynchronize(s));
-    if (bad) {
+    int32_t *rp, *ci, *flag, bad = 0;
+    double *va, *yd, *wd;
+    CallIO io;
+    B2P_DO(io.begin(ctx, CallIO::round(4 * ((size_t)m + 1)) + CallIO::round(4 * nnz) + CallIO::round(8 * nnz) + 8 * ((size_t)n + m) + 64));
+    pt.mark(0);
+    B2P_DO(io.in(ctx->s_rowptr, rowptr, (size_t)m + 1, &rp));
+    B2P_DO(io.in(ctx->s_colidx, colidx, nnz, &ci));
+    B2P_DO(io.in(ctx->s_vals, vals, nnz, &va));
+    B2P_DO(io.in(ctx->s_x, yv, m, &yd));
+    B2P_DO(io.send());
+    B2P_DO(io.out(ctx->s_y, w, n, &wd));
+    B2P_DO(io.out(ctx->s_flag, &bad, 1, &flag));
+    B2P_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(int32_t), s));
+    pt.mark(1);
+    auto invalid = [&]() {
         ctx->err = "CSR column indices out of range or not strictly ascending in row " + std::to_string(bad - 1);
         return B2P_INVALID_ARGUMENT;
+    };
+    // small: its products and sums fit one CTA, whose one adding warp takes 0.08 us a row (33 us at
+    // 300 rows of 17 entries); the sort, scan and waits of the transpose took 150 us whatever the size
+    if (io.packed && nnz <= 12288 && n <= 8192 && m <= 1024) {
+        const int rows_off = n + (int)nnz + ((int)nnz + 3) / 4;  // in doubles: sums, products, columns, then row pointers
+        const size_t small = 8 * (size_t)rows_off + 4 * ((size_t)m + 1);
+        B2P_CUDA(ctx, cudaFuncSetAttribute(k_spmv_t_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small));
+        k_spmv_t_small<<<1, 1024, small, s>>>(m, n, rp, ci, va, yd, wd, flag, rows_off);
+        B2P_LAUNCH(ctx);
+        ctx->launches += 1;
+    } else {
+        k_validate_csr<<<grid_for(m, 256, ctx->sm_count), 256, 0, s>>>(m, n, rp, ci, flag);
+        B2P_CUDA(ctx, cudaMemcpyAsync(&bad, flag, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        B2P_CUDA(ctx, cudaStreamSynchronize(s));
+        if (bad) return invalid();
+        B2P_CUDA(ctx, ctx->s_t_rowptr.reserve((size_t)n + 1));
+        B2P_CUDA(ctx, ctx->s_t_colidx.reserve(nnz));
+        B2P_CUDA(ctx, ctx->s_t_vals.reserve(nnz));
+        B2P_DO(build_transpose(ctx, m, n, nnz, rp, ci, va, ctx->s_t_rowptr.p, ctx->s_t_colidx.p, ctx->s_t_vals.p));
+        k_spmv_f64<<<grid_for(n, 256, ctx->sm_count), 256, 0, s>>>(n, ctx->s_t_rowptr.p, ctx->s_t_colidx.p, ctx->s_t_vals.p,
+                                                                   yd, wd);
+        B2P_LAUNCH(ctx);
+        ctx->launches += 2;
     }
-    int st = build_transpose(ctx, m, n, nnz, rp.p, ci.p, va.p, trp.p, tci.p, tva.p);
-    if (st) return st;
-    unsigned gn = grid_for(n, 256, ctx->sm_count);
-    k_spmv_f64<<<gn, 256, 0, s>>>(n, trp.p, tci.p, tva.p, ctx->s_x.p, ctx->s_y.p);
-    B2P_LAUNCH(ctx);
-    ctx->launches += 2;
-    cudaEventRecord(pt.e[2], s);
-    B2P_CUDA(ctx, cudaMemcpyAsync(w, ctx->s_y.p, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-    cudaEventRecord(pt.e[3], s);
-    B2P_CUDA(ctx, cudaStreamSynchronize(s));
+    pt.mark(2);
+    B2P_DO(io.receive());
+    pt.mark(3);
+    B2P_DO(io.finish(&bad));
     pt.fill(timing, t0);
-    return B2P_OK;
+    return bad ? invalid() : B2P_OK;
 }
 
 int b2p_vector_op(void* p, int op, size_t n, double alpha, const double* a, const double* bv, double* out,
@@ -451,22 +631,23 @@ int b2p_vector_op(void* p, int op, size_t n, double alpha, const double* a, cons
     if (n == 0) return B2P_OK;
     cudaSetDevice(ctx->device);
     double t0 = now_ms();
-    PhaseTimer pt;
-    cudaStream_t s = ctx->stream;
-    B2P_CUDA(ctx, ctx->s_x.reserve(n));
-    B2P_CUDA(ctx, ctx->s_y.reserve(n));
-    B2P_CUDA(ctx, ctx->s_z.reserve(n));
-    cudaEventRecord(pt.e[0], s);
-    B2P_CUDA(ctx, cudaMemcpyAsync(ctx->s_x.p, a, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    if (needs_b) B2P_CUDA(ctx, cudaMemcpyAsync(ctx->s_y.p, bv, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    cudaEventRecord(pt.e[1], s);
-    k_vec<<<grid_for((int64_t)n, 256, ctx->sm_count), 256, 0, s>>>(op, n, alpha, ctx->s_x.p, ctx->s_y.p, ctx->s_z.p);
+    PhaseTimer pt(ctx, timing);
+    double *ad, *bd = nullptr, *od;
+    CallIO io;
+    B2P_DO(io.begin(ctx, 24 * n + 64));
+    pt.mark(0);
+    B2P_DO(io.in(ctx->s_x, a, n, &ad));
+    if (needs_b) B2P_DO(io.in(ctx->s_y, bv, n, &bd));
+    B2P_DO(io.send());
+    B2P_DO(io.out(ctx->s_z, out, n, &od));
+    pt.mark(1);
+    k_vec<<<grid_for((int64_t)n, 256, ctx->sm_count), 256, 0, ctx->stream>>>(op, n, alpha, ad, bd, od);
     B2P_LAUNCH(ctx);
     ctx->launches += 1;
-    cudaEventRecord(pt.e[2], s);
-    B2P_CUDA(ctx, cudaMemcpyAsync(out, ctx->s_z.p, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-    cudaEventRecord(pt.e[3], s);
-    B2P_CUDA(ctx, cudaStreamSynchronize(s));
+    pt.mark(2);
+    B2P_DO(io.receive());
+    pt.mark(3);
+    B2P_DO(io.finish());
     pt.fill(timing, t0);
     return B2P_OK;
 }
@@ -481,24 +662,27 @@ static int dot_impl(Ctx* ctx, size_t n, const double* a, const double* bv, doubl
     }
     cudaSetDevice(ctx->device);
     double t0 = now_ms();
-    PhaseTimer pt;
+    PhaseTimer pt(ctx, timing);
     cudaStream_t s = ctx->stream;
-    B2P_CUDA(ctx, ctx->s_x.reserve(n));
-    B2P_CUDA(ctx, ctx->s_y.reserve(n));
-    B2P_CUDA(ctx, ctx->s_z.reserve(kRedBlocks + 1));
-    cudaEventRecord(pt.e[0], s);
-    B2P_CUDA(ctx, cudaMemcpyAsync(ctx->s_x.p, a, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    if (bv) B2P_CUDA(ctx, cudaMemcpyAsync(ctx->s_y.p, bv, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    cudaEventRecord(pt.e[1], s);
-    k_dot_partial<<<kRedBlocks, kRedThreads, 0, s>>>(n, ctx->s_x.p, bv ? ctx->s_y.p : nullptr, ctx->s_z.p);
-    k_sum_partials<<<1, kRedThreads, 0, s>>>(kRedBlocks, ctx->s_z.p, ctx->s_z.p + kRedBlocks);
+    double *ad, *bd = nullptr, *rd, r = 0.0;
+    DBuf<double>& sums = ctx->s_t_vals;  // the blocks' partial sums
+    CallIO io;
+    B2P_DO(io.begin(ctx, 16 * n + 64));
+    B2P_CUDA(ctx, sums.reserve(kRedBlocks));
+    pt.mark(0);
+    B2P_DO(io.in(ctx->s_x, a, n, &ad));
+    if (bv) B2P_DO(io.in(ctx->s_y, bv, n, &bd));
+    B2P_DO(io.send());
+    B2P_DO(io.out(ctx->s_z, &r, 1, &rd));
+    pt.mark(1);
+    k_dot_partial<<<kRedBlocks, kRedThreads, 0, s>>>(n, ad, bd, sums.p);
+    k_sum_partials<<<1, kRedThreads, 0, s>>>(kRedBlocks, sums.p, rd);
     B2P_LAUNCH(ctx);
     ctx->launches += 2;
-    cudaEventRecord(pt.e[2], s);
-    double r = 0.0;
-    B2P_CUDA(ctx, cudaMemcpyAsync(&r, ctx->s_z.p + kRedBlocks, sizeof(double), cudaMemcpyDeviceToHost, s));
-    cudaEventRecord(pt.e[3], s);
-    B2P_CUDA(ctx, cudaStreamSynchronize(s));
+    pt.mark(2);
+    B2P_DO(io.receive());
+    pt.mark(3);
+    B2P_DO(io.finish());
     pt.fill(timing, t0);
     *out = sqrt_out ? std::sqrt(r) : r;
     return B2P_OK;

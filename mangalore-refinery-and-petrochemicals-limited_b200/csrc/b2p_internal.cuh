@@ -102,6 +102,13 @@ struct Ctx {
     DBuf<double> s_vals, s_x, s_y, s_z;
     DBuf<unsigned long long> s_red;
     DBuf<int32_t> s_flag;
+    DBuf<int32_t> s_t_rowptr, s_t_colidx;
+    DBuf<double> s_t_vals;
+    DBuf<uint8_t> s_pack;                // small calls: all inputs, then all outputs, one copy each way
+    std::vector<uint8_t> h_pack;         // its host side
+    cudaEvent_t tev[4] = {nullptr, nullptr, nullptr, nullptr};  // phases of a timed call
+    // scratch of build_transpose, kept up to kKeepTranspose entries
+    DBuf<int32_t> tr_row, tr_keys, tr_in, tr_out;
     // CUB temp storage for setup-only sorts / scans
     DBuf<uint8_t> cub_tmp;
     RefWork* rw = nullptr;
