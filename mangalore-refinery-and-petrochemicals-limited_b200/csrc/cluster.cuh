@@ -42,4 +42,76 @@ struct ClusterVec {
     }
 };
 
+// Phases without a barrier: every CTA has one mbarrier per exchanged vector, and an element's
+// owner posts it into every CTA's copy with st.async, which counts its bytes on that CTA's
+// mbarrier.  A CTA goes on when its own copy is complete.  Safe with two vectors that are
+// gathered in turn: a CTA posts elements of one only after its copy of the other is complete,
+// that is, after every CTA has finished its reads of the first.  No thread may fall two phases
+// of a vector behind (parities repeat): the CTA meets once per turn, and every CTA must own
+// elements, so that none is passed by.
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t peer_addr(uint32_t addr, int rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void tx_init(uint64_t* bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+// Opens the next phase of this CTA's mbarrier: it completes when `bytes` have arrived.
+__device__ __forceinline__ void tx_expect(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+// Waits (about a second at most) for the phase of the given parity.
+__device__ __forceinline__ bool tx_wait(uint64_t* bar, uint32_t parity) {
+    const uint32_t addr = smem_addr(bar);
+    for (int spin = 0; spin < (1 << 20); ++spin) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(addr), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if (spin > 256) __nanosleep(128);
+    }
+    return false;
+}
+__device__ __forceinline__ void st_async(uint32_t addr, double v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+                 "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void st_async(uint32_t addr, float v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr),
+                 "r"(__float_as_int(v)), "r"(bar)
+                 : "memory");
+}
+// Element i of a vector into every CTA's copy (NC = 1: this CTA's, ordered by its own barrier).
+template <typename T, int NC>
+struct ClusterPost {
+    uint32_t vec[NC], bar[NC];
+    T* mine;
+    __device__ __forceinline__ ClusterPost(T* v, uint64_t* b) : mine(v) {
+        if constexpr (NC > 1) {
+#pragma unroll
+            for (int r = 0; r < NC; ++r) {
+                vec[r] = peer_addr(smem_addr(v), r);
+                bar[r] = peer_addr(smem_addr(b), r);
+            }
+        }
+    }
+    __device__ __forceinline__ void store(int i, T v) const {
+        if constexpr (NC == 1) {
+            mine[i] = v;
+        } else {
+#pragma unroll
+            for (int r = 0; r < NC; ++r) st_async(vec[r] + i * (uint32_t)sizeof(T), v, bar[r]);
+        }
+    }
+};
+
 }  // namespace b2p

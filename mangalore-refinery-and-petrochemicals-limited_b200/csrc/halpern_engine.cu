@@ -35,11 +35,14 @@
 //   k_iter_sell<...,WIN>  the same, with each CTA's densest window of the gathered
 //                         vector staged in shared memory
 //   k_iter                CSR, L lanes per row, R rows per lane group
+// Small LPs iterate in k_iter_cluster instead: all iterations between two checks in one launch.
 // The engine works on the LP renumbered so that rows and columns are sorted by
 // length inside windows of 4096 (k_len_keys): the 32 rows of a SELL slice then have
 // nearly equal lengths while rows that were neighbours stay near each other.
 // Warm starts and answers are mapped between the caller's and the internal
 // numbering on the device.
+#include <cooperative_groups.h>
+
 #include <cub/cub.cuh>
 
 #include <cmath>
@@ -47,6 +50,7 @@
 #include <algorithm>
 
 #include "b2p_internal.cuh"
+#include "cluster.cuh"
 #include "pdl.cuh"
 
 namespace b2p {
@@ -79,6 +83,13 @@ struct Ctrl {
 
 // private status of a solve that reached its inner tolerance (refinement continues)
 constexpr int kInnerDone = 100;
+// ... and of one whose cluster kernel gave up waiting (an error of the call)
+constexpr int kWaitFailed = 101;
+
+// LPs that iterate in one launch between checks: longest row or column, entries of those that
+// run on one CTA (see cluster_ctas).
+constexpr int64_t kClusterLongest = 256;
+constexpr int64_t kOneCtaNnz = 8192;
 
 // SELL-32 copy of one orientation of the scaled matrix (internal numbering): slice s
 // holds rows 32s..32s+31; its entries are stored in chunks of W per lane -- entry e
@@ -93,6 +104,7 @@ struct Sell {
     DBuf<int32_t> idx;   // total
     DBuf<float> v32;     // total (mixed engine)
     DBuf<double> v64;    // total (FP64 engine)
+    std::vector<int64_t> h_off;  // host copy of off
     bool idx_ready = false;
 };
 
@@ -145,6 +157,7 @@ struct HalpernWork {
     // autotuned launch shape (lanes per row L, rows per lane group R) of the two
     // iteration kernels, keyed by the LP's shape and precision
     long long tuned_key = -1;
+    bool one_launch = false;       // the last solve iterated in k_iter_cluster (the shapes may be untuned)
     int Lc = 8, Rc = 1, Lr = 8, Rr = 1, Tc = 256, Tr = 256;
     Ctrl* host_ctrl = nullptr;     // pinned, 2 slots
     cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -802,6 +815,235 @@ __global__ void __launch_bounds__(1024) k_iter_sell(IterArgs<VT, GT> a, int it) 
     if (MODE == M_CHECK) {
         block_sum_to(acc_r, &a.ctrl->acc[PRIMAL ? A_RX2 : A_RY2]);
         block_sum_to(acc_d, &a.ctrl->acc[PRIMAL ? A_DXA2 : A_DYA2]);
+    }
+}
+
+// Small LPs: all iterations between two checks in one launch, on one CTA or on a cluster of
+// CTAs.  Slices (the 32-row SELL copies) are dealt to the CTAs in turn; a launch first copies
+// its slices' values and 16-bit indices (in groups of four a lane) and
+// its rows' own vectors into shared memory; every CTA holds whole copies of y and xh, into which
+// the owners post (ClusterPost).  A phase ends when a CTA's copy is complete, where the
+// two-kernel form ends a kernel.
+//
+// Bound: latency (index -> gather -> adds, the post to the peers and the wait for theirs); on one
+// CTA also the shared-memory wavefronts of the random gathers (58 % of the cycles at 5,000
+// entries).  us per iteration, checks every 64 included, two kernels -> one launch: FP64
+// 100 x 300, 4 a column 4.5 -> 1.8; 300 x 1,000, 5: 4.4 -> 2.0; 1,000 x 3,000, 5: 4.5 -> 2.9;
+// 1,500 x 5,000, 6: 5.1 -> 3.8; FP32 300 x 1,000 4.7 -> 2.1, 2,000 x 8,000, 6: 4.9 -> 3.9.  With
+// cluster barriers instead of posts, and each row's vectors in L1 (which a cluster barrier
+// empties), 300 x 1,000 FP64 took 4.1.
+struct ClusterLay {
+    int bar, xh, own, wt, tab, val, idx, total;  // byte offsets in dynamic shared memory; y lies at 0
+};
+
+// Place of entry e of a lane in its slice's values: groups of four, each 16-byte load of a warp
+// over neighbouring words (FP64: two loads a group).  Its index lies at that of float.
+template <typename MT>
+__device__ __forceinline__ int group_pos(int e, int lane) {
+    if (sizeof(MT) == 4) return (e >> 2) * 128 + lane * 4 + (e & 3);
+    return (e >> 2) * 128 + ((e >> 1) & 1) * 64 + lane * 2 + (e & 1);
+}
+__device__ __forceinline__ void group_load(const float* v, int q, int lane, float (&a)[4]) {
+    const float4 t = reinterpret_cast<const float4*>(v)[q * 32 + lane];
+    a[0] = t.x, a[1] = t.y, a[2] = t.z, a[3] = t.w;
+}
+__device__ __forceinline__ void group_load(const double* v, int q, int lane, double (&a)[4]) {
+    const double2 t = reinterpret_cast<const double2*>(v)[q * 64 + lane];
+    const double2 u = reinterpret_cast<const double2*>(v)[q * 64 + 32 + lane];
+    a[0] = t.x, a[1] = t.y, a[2] = u.x, a[3] = u.y;
+}
+// Sum of one lane's row of a slice of nq groups; the next group's indices are on their way while
+// this one's gathers are.
+template <typename MT>
+__device__ __forceinline__ MT slice_dot(const MT* v, const uint16_t* ix, const MT* g, int nq, int lane) {
+    const ushort4* ip = reinterpret_cast<const ushort4*>(ix) + lane;
+    MT s0 = (MT)0, s1 = (MT)0;
+    if (nq == 0) return s0;
+    ushort4 c = ip[0];
+    for (int q = 0; q < nq; ++q) {
+        const ushort4 d = ip[32 * min(q + 1, nq - 1)];
+        MT a[4];
+        group_load(v, q, lane, a);
+        const MT b0 = g[c.x], b1 = g[c.y], b2 = g[c.z], b3 = g[c.w];
+        s0 += a[0] * b0;
+        s1 += a[1] * b1;
+        s0 += a[2] * b2;
+        s1 += a[3] * b3;
+        c = d;
+    }
+    return s0 + s1;
+}
+
+template <typename MT, int NC>
+__global__ void __launch_bounds__(NC == 1 ? 1024 : kClusterThreads)
+    k_iter_cluster(IterArgs<MT, MT> pa, IterArgs<MT, MT> da, int K, int wc, int wr, ClusterLay lay) {
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) unsigned char win_raw[];
+    cg::cluster_group cl = cg::this_cluster();
+    Ctrl* ctrl = pa.ctrl;
+    if (ctrl->done) return;  // the same in every CTA
+    const int rank = NC == 1 ? 0 : (int)cl.block_rank();
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+    const int n = pa.rows, m = da.rows;
+    // this CTA's slices: rank, rank + NC, ...; those of the columns first
+    const int ncl = (((n + 31) >> 5) - rank + NC - 1) / NC, nrl = (((m + 31) >> 5) - rank + NC - 1) / NC;
+    MT* ys = reinterpret_cast<MT*>(win_raw);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(win_raw + lay.bar);  // of xh, of y
+    MT* xh = reinterpret_cast<MT*>(win_raw + lay.xh);
+    MT* own_c = reinterpret_cast<MT*>(win_raw + lay.own);  // per column slice: x, anchor, cost, lower, upper
+    MT* own_r = own_c + 160 * ncl;                         // per row slice: anchor, rhs, dual lower bound
+    MT* wt = reinterpret_cast<MT*>(win_raw + lay.wt);
+    int2* tab = reinterpret_cast<int2*>(win_raw + lay.tab);  // per slice {first entry, groups of four per lane}
+    MT* sv = reinterpret_cast<MT*>(win_raw + lay.val);
+    uint16_t* si = reinterpret_cast<uint16_t*>(win_raw + lay.idx);
+    for (int i = tid; i < m; i += nt) ys[i] = da.z[i];
+    if (tid == 0) ys[m] = xh[n] = (MT)0;  // what the padding of a row's last group gathers
+    for (int l = warp; l < ncl; l += nw) {
+        const int j = (rank + NC * l) * 32 + lane;
+        MT* o = own_c + 160 * l + lane;
+        const bool v = j < n;
+        o[0] = v ? pa.z[j] : (MT)0;
+        o[32] = v ? pa.za[j] : (MT)0;
+        o[64] = v ? pa.cost[j] : (MT)0;
+        o[96] = v ? pa.lo[j] : (MT)0;
+        o[128] = v ? pa.hi[j] : (MT)0;
+    }
+    for (int l = warp; l < nrl; l += nw) {
+        const int i = (rank + NC * l) * 32 + lane;
+        MT* o = own_r + 96 * l + lane;
+        const bool v = i < m;
+        o[0] = v ? da.za[i] : (MT)0;
+        o[32] = v ? da.cost[i] : (MT)0;
+        o[64] = (v && !da.is_eq[i]) ? (da.ylb ? da.ylb[i] : (MT)0) : (MT)(-INFINITY);
+    }
+    for (int i = tid; i < K; i += nt) {
+        const double kk = (double)(ctrl->k_base + i);
+        wt[2 * i] = (MT)((kk + 1.0) / (kk + 2.0));
+        wt[2 * i + 1] = (MT)(1.0 / (kk + 2.0));
+    }
+    for (int l = tid; l < ncl + nrl; l += nt) {
+        const int64_t* o = l < ncl ? pa.soff + rank + NC * l : da.soff + rank + NC * (l - ncl);
+        tab[l] = make_int2(0, (int)((o[1] - o[0]) / 32 + 3) / 4);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        int e = 0;
+        for (int l = 0; l < ncl + nrl; ++l) {
+            tab[l].x = e;
+            e += 128 * tab[l].y;
+        }
+        if (NC > 1) {
+            tx_init(bar);
+            tx_init(bar + 1);
+            tx_expect(bar, n * (uint32_t)sizeof(MT));
+            tx_expect(bar + 1, m * (uint32_t)sizeof(MT));
+        }
+    }
+    __syncthreads();
+    for (int l = warp; l < ncl + nrl; l += nw) {
+        const bool col = l < ncl;
+        const int64_t p0 = col ? pa.soff[rank + NC * l] : da.soff[rank + NC * (l - ncl)];
+        const MT* __restrict__ v = (col ? pa.val : da.val) + p0;
+        const int* __restrict__ ix = (col ? pa.idx : da.idx) + p0;
+        const int ws = col ? wc : wr, sh = ws == 4 ? 2 : ws - 1;  // W = 1, 2, 4
+        const int len = (int)((col ? pa.soff[rank + NC * l + 1] : da.soff[rank + NC * (l - ncl) + 1]) - p0) / 32;
+        const int2 t = tab[l];
+#pragma unroll 4
+        for (int e = 0; e < 4 * t.y; ++e) {
+            const int pos = ((((e >> sh) * 32 + lane) << sh) + (e & (ws - 1)));
+            const bool in = e < len;
+            sv[t.x + group_pos<MT>(e, lane)] = in ? v[pos] : (MT)0;
+            si[t.x + group_pos<float>(e, lane)] = (uint16_t)(in ? ix[pos] : (col ? m : n));
+        }
+    }
+    const MT tau = (MT)ctrl->tau, sigma = (MT)ctrl->sigma, rho = (MT)pa.rho;
+    const ClusterPost<MT, NC> xv(xh, bar), yv(ys, bar + 1);
+    bool ok = true;
+    cluster_phase<NC>(cl);  // every CTA has its copies before anyone writes into them
+    // End of a phase: this CTA's copy is complete.  A thread that gave up once waits no more and
+    // runs on to the end (every index is the host's), so that barriers still meet.
+    auto phase_end = [&](int v, int it, uint32_t bytes) {
+        if constexpr (NC == 1) {
+            __syncthreads();
+        } else {
+            if (ok) ok = tx_wait(bar + v, it & 1);
+            if (tid == 0 && it + 1 < K) tx_expect(bar + v, bytes);
+            if (v == 1) __syncthreads();
+        }
+    };
+    for (int it = 0; it < K; ++it) {
+        const int mode = it == 0 ? M_FIRST : (it == K - 1 ? M_CHECK : M_PLAIN);
+        const MT wk = wt[2 * it], wa = wt[2 * it + 1];
+        double acc_r = 0.0, acc_d = 0.0;
+#pragma unroll 1
+        for (int l = warp; l < ncl; l += nw) {
+            const int j = (rank + NC * l) * 32 + lane;
+            MT* o = own_c + 160 * l + lane;
+            const MT zr = o[0], zan = o[32];
+            const int2 t = tab[l];
+            const MT s = slice_dot(sv + t.x, si + t.x, ys, t.y, lane);
+            const MT zt = clampT(zr - tau * (o[64] + s), o[96], o[128]);
+            o[0] = wk * (((MT)1 + rho) * zt - rho * zr) + wa * zan;
+            if (j >= n) continue;
+            xv.store(j, (MT)2 * zt - zr);
+            if (mode != M_PLAIN) {
+                const double d = (double)zr - (double)zt;
+                acc_r += d * d;
+            }
+            if (mode == M_CHECK) {
+                pa.zt[j] = zt;
+                if (pa.zd) pa.zd[j] = (double)zt - (double)zr;
+                const double e = (double)zt - (double)zan;
+                acc_d += e * e;
+            }
+        }
+        if (mode != M_PLAIN) block_sum_to(acc_r, &ctrl->acc[mode == M_FIRST ? A_RX2_FIRST : A_RX2]);
+        if (mode == M_CHECK) block_sum_to(acc_d, &ctrl->acc[A_DXA2]);
+        phase_end(0, it, n * (uint32_t)sizeof(MT));
+        acc_r = acc_d = 0.0;
+#pragma unroll 1
+        for (int l = warp; l < nrl; l += nw) {
+            const int i = (rank + NC * l) * 32 + lane;
+            const bool valid = i < m;
+            const MT* o = own_r + 96 * l + lane;
+            const MT zr = valid ? ys[i] : (MT)0, zan = o[0], lo = o[64];
+            const int2 t = tab[ncl + l];
+            const MT s = slice_dot(sv + t.x, si + t.x, xh, t.y, lane);
+            if (!valid) continue;
+            MT zt = zr + sigma * (s - o[32]);
+            if (zt < lo) zt = lo;  // -inf on equality rows; NaN stays NaN
+            yv.store(i, wk * (((MT)1 + rho) * zt - rho * zr) + wa * zan);
+            if (mode != M_PLAIN) {
+                const double d = (double)zr - (double)zt;
+                acc_r += d * d;
+            }
+            if (mode == M_CHECK) {
+                da.zt[i] = zt;
+                const double dz = (double)zt - (double)zr;
+                if (da.zd) da.zd[i] = lo != (MT)(-INFINITY) ? fmax(dz, 0.0) : dz;
+                const double e = (double)zt - (double)zan;
+                acc_d += e * e;
+            }
+        }
+        if (mode != M_PLAIN) block_sum_to(acc_r, &ctrl->acc[mode == M_FIRST ? A_RY2_FIRST : A_RY2]);
+        if (mode == M_CHECK) block_sum_to(acc_d, &ctrl->acc[A_DYA2]);
+        phase_end(1, it, m * (uint32_t)sizeof(MT));
+    }
+    for (int l = warp; l < ncl; l += nw) {
+        const int j = (rank + NC * l) * 32 + lane;
+        if (j < n) pa.z[j] = own_c[160 * l + lane];
+    }
+    for (int l = warp; l < nrl; l += nw) {
+        const int i = (rank + NC * l) * 32 + lane;
+        if (i < m) da.z[i] = ys[i];
+    }
+    if constexpr (NC > 1) {
+        if (!ok) {
+            ctrl->status = kWaitFailed;
+            ctrl->done = 1;
+            __nanosleep(1000000);  // late elements land before the CTA they go to leaves
+        }
+        cl.sync();
     }
 }
 
@@ -1469,6 +1711,7 @@ int build_sell_layout(Ctx* ctx, Sell& S, int rows, const int32_t* ptr, const int
     S.W = W;
     S.slices = nsl;
     S.total = off[nsl];
+    S.h_off = off;
     B2P_CUDA(ctx, S.off.reserve(nsl + 1));
     B2P_CUDA(ctx, S.idx.reserve(std::max<int64_t>(S.total, 1)));
     B2P_CUDA(ctx, cudaMemcpyAsync(S.off.p, off.data(), sizeof(int64_t) * (nsl + 1), cudaMemcpyHostToDevice, s));
@@ -1884,8 +2127,97 @@ int autotune_shapes(Ctx* ctx, HalpernWork* w, const b2p_params* p) {
     return B2P_OK;
 }
 
+// Shared memory of k_iter_cluster on NC CTAs (every CTA's layout is that of the fullest).
 template <typename MT>
-int run_chunks(Ctx* ctx, HalpernWork* w, const b2p_params* p, double time_limit_ms, double t_start) {
+ClusterLay cluster_lay(const HalpernWork* w, int K, int NC) {
+    const Sell &R = w->sr_all[0], &C = w->sc_all[0];
+    int64_t most = 0, slices = 0;
+    for (int r = 0; r < NC; ++r) {
+        int64_t e = 0, k = 0;
+        for (const Sell* S : {&R, &C})
+            for (int64_t q = r; q < S->slices; q += NC, ++k) e += ((S->h_off[q + 1] - S->h_off[q]) / 32 + 3) / 4 * 128;
+        most = std::max(most, e);
+        slices = std::max(slices, k);
+    }
+    const int64_t m1 = w->ilp.m + 1, n1 = w->ilp.n + 1, sz = sizeof(MT);  // one zero past each vector
+    ClusterLay lay{};
+    int64_t at = (sz * m1 + 15) & ~(int64_t)15;
+    auto put = [&](int& where, int64_t bytes) {
+        where = (int)std::min<int64_t>(at, INT_MAX);
+        at = (at + bytes + 15) & ~(int64_t)15;
+    };
+    put(lay.bar, 16);
+    put(lay.xh, sz * n1);
+    put(lay.own, sz * (160 * ((C.slices + NC - 1) / NC) + 96 * ((R.slices + NC - 1) / NC)));
+    put(lay.wt, 2 * sz * K);
+    put(lay.tab, (int64_t)sizeof(int2) * slices);
+    put(lay.val, sz * most);
+    put(lay.idx, 2 * most);
+    lay.total = (int)std::min<int64_t>(at, INT_MAX);
+    return lay;
+}
+
+template <typename MT>
+void (*cluster_kernel(int NC))(IterArgs<MT, MT>, IterArgs<MT, MT>, int, int, int, ClusterLay) {
+    return NC == 1 ? k_iter_cluster<MT, 1> : k_iter_cluster<MT, kClusterCtas>;
+}
+
+// CTAs of the one-launch form for this LP: 1, kClusterCtas, or 0 -- the two-kernel form.
+// The form wins wherever an LP fits (us per iteration above); what does not fit shared memory on 8
+// CTAs (FP64 about 35,000 entries, FP32 65,000), has 2^16 rows or columns (16-bit indices) or a
+// row or column of more than kClusterLongest entries (one lane's serial sum: at 315 entries 7.9
+// -> 6.5 us, at 500 8.8 -> 8.6) keeps the two kernels, as does a call that asks for one of
+// theirs.  Fewer than 8 column slices run on one CTA (250 columns FP32: 1.7 us against 2.0; FP64
+// 1.9 either way), up to kOneCtaNnz entries (7,600 entries: 3.8 us against 4.5).
+template <typename MT>
+int cluster_ctas(Ctx* ctx, HalpernWork* w, const b2p_params* p) {
+    const DevLP& L = w->ilp;
+    const int K = p->check_every;
+    const int NC = L.n >= 32 * kClusterCtas ? kClusterCtas : 1;  // every CTA owns columns
+    if (p->lanes_per_row != 0 || L.m < 1 || L.n < 1 || L.m > 65534 || L.n > 65534 || K > 4096) return 0;
+    if (NC == 1 && L.nnz > kOneCtaNnz) return 0;
+    for (const Sell* S : {&w->sr_all[0], &w->sc_all[0]})
+        for (int64_t q = 0; q < S->slices; ++q)
+            if (S->h_off[q + 1] - S->h_off[q] > 32 * kClusterLongest) return 0;
+    int max_smem = 0;
+    if (cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess) return 0;
+    const ClusterLay lay = cluster_lay<MT>(w, K, NC);
+    auto fn = cluster_kernel<MT>(NC);
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) return 0;
+    if ((int64_t)lay.total + (int64_t)fa.sharedSizeBytes > max_smem) return 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, lay.total) != cudaSuccess) return 0;
+    return NC;
+}
+
+template <typename MT>
+int launch_cluster(Ctx* ctx, HalpernWork* w, const b2p_params* p, int NC) {
+    cudaLaunchConfig_t lc{};
+    cudaLaunchAttribute dims;
+    dims.id = cudaLaunchAttributeClusterDimension;
+    dims.val.clusterDim.x = NC;
+    dims.val.clusterDim.y = dims.val.clusterDim.z = 1;
+    const ClusterLay lay = cluster_lay<MT>(w, p->check_every, NC);
+    lc.gridDim = dim3(NC);
+    lc.blockDim = dim3(NC == 1 ? 1024 : kClusterThreads);
+    lc.dynamicSmemBytes = lay.total;
+    lc.stream = ctx->stream;
+    lc.attrs = &dims;
+    lc.numAttrs = 1;
+    IterArgs<MT, MT> pa = primal_args<MT>(w->ilp, w, p, false), da = dual_args<MT>(w->ilp, w, p, false);
+    Sell &C = w->sc_all[0], &R = w->sr_all[0];
+    pa.idx = C.idx.p;
+    pa.val = Ops<MT>::sell(C).p;
+    pa.soff = C.off.p;
+    da.idx = R.idx.p;
+    da.val = Ops<MT>::sell(R).p;
+    da.soff = R.off.p;
+    B2P_CUDA(ctx, cudaLaunchKernelEx(&lc, cluster_kernel<MT>(NC), pa, da, p->check_every, C.W, R.W, lay));
+    return B2P_OK;
+}
+
+template <typename MT>
+int run_chunks(Ctx* ctx, HalpernWork* w, const b2p_params* p, int NC, double time_limit_ms, double t_start) {
     DevLP& L = w->ilp;
     cudaStream_t s = ctx->stream;
     const int m = L.m, n = L.n, K = p->check_every;
@@ -1899,8 +2231,12 @@ int run_chunks(Ctx* ctx, HalpernWork* w, const b2p_params* p, double time_limit_
     Ctrl* ctrl = w->ctrl.p;
     const IterArgs<MT, MT> pa = primal_args<MT>(L, w, p, w->sell_c);
     const IterArgs<MT, MT> da = dual_args<MT>(L, w, p, w->sell_r);
-    auto chunk = [&]() {
-        for (int i = 0; i < K; ++i) {
+    auto chunk = [&]() -> int {
+        if (NC > 0) {
+            const int st = launch_cluster<MT>(ctx, w, p, NC);
+            if (st) return st;
+        }
+        for (int i = 0; i < K && NC == 0; ++i) {
             int mode = (i == 0) ? M_FIRST : (i == K - 1 ? M_CHECK : M_PLAIN);
             if (w->sell_c) launch_sell<MT, MT, true>(mode, *w->sc, gcS, Tc, w->wc.smem, s, pa, i);
             else if (mode == M_PLAIN) launch_iter<MT, MT, true>(mode, Lc, Rc, gcR, Tc, s, pa, i);
@@ -1933,12 +2269,17 @@ int run_chunks(Ctx* ctx, HalpernWork* w, const b2p_params* p, double time_limit_
             k_restart<MT><<<gv, TB, 0, s>>>(m, n, ctrl, zbuf<MT>(w->x), zbuf<MT>(w->xa), zbuf<MT>(w->xt),
                                             zbuf<MT>(w->y), zbuf<MT>(w->ya), zbuf<MT>(w->yt));
         }
+        return B2P_OK;
     };
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     B2P_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    chunk();
+    const int cst = chunk();
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
+    if (cst) {
+        if (ce == cudaSuccess) cudaGraphDestroy(graph);
+        return cst;
+    }
     if (ce != cudaSuccess) {
         ctx->err = std::string("graph capture: ") + cudaGetErrorString(ce);
         return B2P_EXECUTION_FAILED;
@@ -1949,7 +2290,7 @@ int run_chunks(Ctx* ctx, HalpernWork* w, const b2p_params* p, double time_limit_
         ctx->err = std::string("graph instantiate: ") + cudaGetErrorString(ce);
         return B2P_EXECUTION_FAILED;
     }
-    const int64_t per_chunk = 2 * K + 4;
+    const int64_t per_chunk = NC > 0 ? 5 : 2 * K + 4;
     int64_t launched = 0;
     int slot = 0;
     bool timed_out = false;
@@ -2126,7 +2467,9 @@ int solve_T(Ctx* ctx, HalpernWork* w, const b2p_params* p, const double* x0, con
     hc.inner_tol = 0.0;
     hc.r_first = 0.0;
     B2P_CUDA(ctx, cudaMemcpyAsync(w->ctrl.p, &hc, sizeof(Ctrl), cudaMemcpyHostToDevice, s));
-    {
+    const int NC = cluster_ctas<MT>(ctx, w, p);
+    w->one_launch = NC > 0;
+    if (NC == 0) {
         const long long before = w->tuned_key;
         st = autotune_shapes<MT>(ctx, w, p);  // returns at once when this LP shape is already tuned
         if (st) return st;
@@ -2142,7 +2485,7 @@ int solve_T(Ctx* ctx, HalpernWork* w, const b2p_params* p, const double* x0, con
     w->solved_gen = ctx->lp_gen;
     w->solved_precision = p->precision;
     B2P_CUDA(ctx, cudaEventRecord(ctx->ev0, s));
-    st = run_chunks<MT>(ctx, w, p, p->time_limit_s * 1000.0, t_start);
+    st = run_chunks<MT>(ctx, w, p, NC, p->time_limit_s * 1000.0, t_start);
     B2P_CUDA(ctx, cudaEventRecord(ctx->ev1, s));
     if (st != B2P_OK && st != B2P_TIMEOUT) return st;
     Ctrl fin;
@@ -2150,6 +2493,10 @@ int solve_T(Ctx* ctx, HalpernWork* w, const b2p_params* p, const double* x0, con
     B2P_CUDA(ctx, cudaStreamSynchronize(s));
     float kms = 0.f;
     cudaEventElapsedTime(&kms, ctx->ev0, ctx->ev1);
+    if (fin.status == kWaitFailed) {
+        ctx->err = "the iteration cluster's exchange did not complete";
+        return B2P_EXECUTION_FAILED;
+    }
     r->kernel_time_ms = kms;
     r->status = st == B2P_TIMEOUT ? B2P_STATUS_INTERRUPTED : fin.status;
     r->iterations = fin.total;
@@ -2187,11 +2534,6 @@ int kernel_timing_T(Ctx* ctx, HalpernWork* w, const b2p_params* p, int reps, dou
     DevLP& L = w->ilp;
     cudaStream_t s = ctx->stream;
     const int m = L.m, n = L.n;
-    const int Lr = w->Lr, Lc = w->Lc, Rr = w->Rr, Rc = w->Rc, Tr = w->Tr, Tc = w->Tc;
-    unsigned gr = iter_grid(m, Lr, w->sell_r ? 1 : Rr, Tr, ctx->sm_count);
-    unsigned gc = iter_grid(n, Lc, w->sell_c ? 1 : Rc, Tc, ctx->sm_count);
-    if (w->sell_r && w->wr.smem) gr = w->wr.G;
-    if (w->sell_c && w->wc.smem) gc = w->wc.G;
     Ctrl* ctrl = w->ctrl.p;
     // re-open the (finished) control block for plain iterations, restore it afterwards
     Ctrl saved;
@@ -2200,6 +2542,15 @@ int kernel_timing_T(Ctx* ctx, HalpernWork* w, const b2p_params* p, int reps, dou
     Ctrl open = saved;
     open.done = 0;
     B2P_CUDA(ctx, cudaMemcpyAsync(ctrl, &open, sizeof(Ctrl), cudaMemcpyHostToDevice, s));
+    if (w->one_launch) {  // the solve needed no tuned shapes; the kernels timed here do
+        const int st = autotune_shapes<MT>(ctx, w, p);
+        if (st) return st;
+    }
+    const int Lr = w->Lr, Lc = w->Lc, Rr = w->Rr, Rc = w->Rc, Tr = w->Tr, Tc = w->Tc;
+    unsigned gr = iter_grid(m, Lr, w->sell_r ? 1 : Rr, Tr, ctx->sm_count);
+    unsigned gc = iter_grid(n, Lc, w->sell_c ? 1 : Rc, Tc, ctx->sm_count);
+    if (w->sell_r && w->wr.smem) gr = w->wr.G;
+    if (w->sell_c && w->wc.smem) gc = w->wc.G;
     const IterArgs<MT, MT> pa = primal_args<MT>(L, w, p, w->sell_c);
     const IterArgs<MT, MT> da = dual_args<MT>(L, w, p, w->sell_r);
     cudaEvent_t e[3];
