@@ -1,8 +1,9 @@
-// Thread-block clusters as one small machine: every CTA owns a contiguous range of 32-row
-// slices of each orientation, and keeps a full copy of the gathered vectors in its shared
-// memory.  The owner of an element stores it into every CTA's copy (distributed shared
-// memory), and a cluster barrier ends each phase -- a fraction of a microsecond, where a
-// kernel boundary with its first loads from L2 costs three or four.
+// Thread-block clusters as one small machine: every CTA owns 32-row slices of each orientation
+// and keeps a full copy of the gathered vectors in its shared memory.  The owner of an element
+// stores it into every CTA's copy (distributed shared memory).  A phase ends with a cluster
+// barrier (ClusterVec, cluster_phase: about 1 us with the stores before it) or, in the loops that
+// run by the thousand, when the CTA's own copy is complete (ClusterPost: half of that) -- where
+// a kernel boundary with its first loads from L2 costs three or four.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -90,26 +91,30 @@ __device__ __forceinline__ void st_async(uint32_t addr, float v, uint32_t bar) {
                  "r"(__float_as_int(v)), "r"(bar)
                  : "memory");
 }
+// The CTAs' shared memory: where an address of this CTA's lies in CTA r's.
+template <int NC>
+struct ClusterPeers {
+    uint32_t origin, base[NC];
+    __device__ __forceinline__ explicit ClusterPeers(const void* any) : origin(smem_addr(any)) {
+#pragma unroll
+        for (int r = 0; r < NC; ++r) base[r] = NC == 1 ? origin : peer_addr(origin, r);
+    }
+};
 // Element i of a vector into every CTA's copy (NC = 1: this CTA's, ordered by its own barrier).
+// One base address a peer serves all vectors: two a vector and peer spilled.
 template <typename T, int NC>
 struct ClusterPost {
-    uint32_t vec[NC], bar[NC];
+    uint32_t vec, bar;  // from the peers' origin
     T* mine;
-    __device__ __forceinline__ ClusterPost(T* v, uint64_t* b) : mine(v) {
-        if constexpr (NC > 1) {
-#pragma unroll
-            for (int r = 0; r < NC; ++r) {
-                vec[r] = peer_addr(smem_addr(v), r);
-                bar[r] = peer_addr(smem_addr(b), r);
-            }
-        }
-    }
-    __device__ __forceinline__ void store(int i, T v) const {
+    __device__ __forceinline__ ClusterPost(const ClusterPeers<NC>& to, T* v, uint64_t* b)
+        : vec(smem_addr(v) - to.origin), bar(smem_addr(b) - to.origin), mine(v) {}
+    __device__ __forceinline__ void store(const ClusterPeers<NC>& to, int i, T v) const {
         if constexpr (NC == 1) {
             mine[i] = v;
         } else {
+            const uint32_t at = vec + i * (uint32_t)sizeof(T);
 #pragma unroll
-            for (int r = 0; r < NC; ++r) st_async(vec[r] + i * (uint32_t)sizeof(T), v, bar[r]);
+            for (int r = 0; r < NC; ++r) st_async(to.base[r] + at, v, to.base[r] + bar);
         }
     }
 };

@@ -957,7 +957,8 @@ __global__ void __launch_bounds__(NC == 1 ? 1024 : kClusterThreads)
         }
     }
     const MT tau = (MT)ctrl->tau, sigma = (MT)ctrl->sigma, rho = (MT)pa.rho;
-    const ClusterPost<MT, NC> xv(xh, bar), yv(ys, bar + 1);
+    const ClusterPeers<NC> peers(win_raw);
+    const ClusterPost<MT, NC> xv(peers, xh, bar), yv(peers, ys, bar + 1);
     bool ok = true;
     cluster_phase<NC>(cl);  // every CTA has its copies before anyone writes into them
     // End of a phase: this CTA's copy is complete.  A thread that gave up once waits no more and
@@ -985,7 +986,7 @@ __global__ void __launch_bounds__(NC == 1 ? 1024 : kClusterThreads)
             const MT zt = clampT(zr - tau * (o[64] + s), o[96], o[128]);
             o[0] = wk * (((MT)1 + rho) * zt - rho * zr) + wa * zan;
             if (j >= n) continue;
-            xv.store(j, (MT)2 * zt - zr);
+            xv.store(peers, j, (MT)2 * zt - zr);
             if (mode != M_PLAIN) {
                 const double d = (double)zr - (double)zt;
                 acc_r += d * d;
@@ -1012,7 +1013,7 @@ __global__ void __launch_bounds__(NC == 1 ? 1024 : kClusterThreads)
             if (!valid) continue;
             MT zt = zr + sigma * (s - o[32]);
             if (zt < lo) zt = lo;  // -inf on equality rows; NaN stays NaN
-            yv.store(i, wk * (((MT)1 + rho) * zt - rho * zr) + wa * zan);
+            yv.store(peers, i, wk * (((MT)1 + rho) * zt - rho * zr) + wa * zan);
             if (mode != M_PLAIN) {
                 const double d = (double)zr - (double)zt;
                 acc_r += d * d;

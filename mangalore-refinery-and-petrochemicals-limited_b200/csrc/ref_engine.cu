@@ -38,6 +38,9 @@ constexpr int kBatchSmall = 8;   // ... and the cluster form
 constexpr int kGraphIters = 20;  // plain iterations per captured graph
 // LPs of at most this many entries (and whose vectors fit shared memory) run on one cluster
 constexpr int64_t kClusterNnz = 49152;
+// ... and of at most this many on one CTA: 1.50 us against 1.64 on eight at 2,500 entries, 2.6 against
+// 1.8 at 5,000
+constexpr int64_t kOneCtaNnz = 3072;
 
 // Slots of the per-check reduction block.
 enum { R_DPRIMAL = 0, R_DDUAL, R_VIOL_X, R_VIOL_AVG, R_BOUND, R_COUNT };
@@ -252,22 +255,22 @@ double bits_to_double(unsigned long long b) {
 // failure, or iteration `stop`.
 //
 // Bound: latency -- the additions of a row (8.6 cycles each), shared-memory gathers, and the
-// cluster barrier behind the remote stores (about 1 us a phase).  us per iteration, before ->
-// now (two kernels in a graph -> this): 60 x 200 7.9 -> 0.95 and 300 x 1,000 9.0 -> 2.7 (one
-// CTA / cluster), 1,000 x 3,000 10.0 -> 3.9, 2,000 x 6,000 10.1 -> 5.2.  From 3,000 x 9,000 on
-// (54,000 entries) the stores into eight copies cost more than kernel boundaries: 8.5 here, 7.2
+// posts to the peers with the wait for theirs.  us per iteration: two kernels in a graph -> this
+// with cluster barriers -> now: 60 x 200 7.9 -> 0.95 (one CTA), 300 x 1,000 9.0 -> 2.7 -> 1.8,
+// 1,000 x 3,000 10.0 -> 3.9 -> 2.6, 2,000 x 6,000 10.1 -> 5.2 -> 4.3.  From 3,000 x 9,000 on
+// (54,000 entries) the posts to eight copies cost more than kernel boundaries: 8.4 here, 7.2
 // with two kernels (12.2 before, over CSR and without their overlap), so the line is drawn at
 // 49,152 entries.
 struct RefOutcome {
     long long iter;
-    int converged, failed;
+    int converged, failed, wait_failed;
     double viol_x, viol_avg, bound, dprimal, ddual;
 };
 
 // Shared memory of one CTA (bytes from the start of the dynamic array), the same in all.
 struct RefLayout {
     int cols, rows;      // most owned columns / rows of any CTA
-    int y, xh, x, xsum, tau, c, lb, ub, sigma, b, eq, cval, rval, cidx, ridx, total;
+    int y, xh, x, xsum, tau, c, lb, ub, sigma, b, eq, cval, rval, cidx, ridx, coff, roff, total;
 };
 
 // entries in shared memory by slices: entry q of lane l of the CTA's slice s at off + 32 q + l
@@ -315,6 +318,8 @@ k_ref_cluster(int m, int n, Sell A, Sell At, const double* __restrict__ c, const
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char sh[];
     __shared__ unsigned long long red[R_COUNT];
+    __shared__ uint64_t bar[2];  // arrivals of x_hat, of y
+    __shared__ double token;     // where CTAs without columns post
     auto at = [&](int off) { return reinterpret_cast<double*>(sh + off); };
     double *ys = at(lay.y), *xh = at(lay.xh), *xs = at(lay.x), *sums = at(lay.xsum), *ts = at(lay.tau), *cs = at(lay.c);
     double *ls = at(lay.lb), *us = at(lay.ub), *ss = at(lay.sigma), *bs = at(lay.b);
@@ -323,7 +328,22 @@ k_ref_cluster(int m, int n, Sell A, Sell At, const double* __restrict__ c, const
     const int ncs = (n + 31) >> 5, nrs = (m + 31) >> 5;
     const int c0 = cluster_slice<NC>(ncs, rank), c1 = cluster_slice<NC>(ncs, rank + 1);
     const int r0 = cluster_slice<NC>(nrs, rank), r1 = cluster_slice<NC>(nrs, rank + 1);
-    const ClusterVec<double, NC> yc(cl, ys), xc(cl, xh);
+    const ClusterPeers<NC> peers(sh);
+    const ClusterPost<double, NC> xv(peers, xh, bar), yv(peers, ys, bar + 1), tv(peers, &token, bar);
+    // a CTA without columns posts a token, so that no iteration passes it by
+    int empty = 0;
+    for (int r = 0; r < NC; ++r) empty += cluster_slice<NC>(ncs, r) == cluster_slice<NC>(ncs, r + 1);
+    const uint32_t x_bytes = 8u * (uint32_t)(n + empty), y_bytes = 8u * (uint32_t)m;
+    if (NC > 1 && tid == 0) {
+        tx_init(bar);
+        tx_init(bar + 1);
+        tx_expect(bar, x_bytes);
+        tx_expect(bar + 1, y_bytes);
+    }
+    // the first entries of the owned slices, from the CTA's first
+    int *co = reinterpret_cast<int*>(sh + lay.coff), *ro = reinterpret_cast<int*>(sh + lay.roff);
+    for (int q = tid; q <= c1 - c0; q += blockDim.x) co[q] = (int)(At.off[c0 + q] - At.off[c0]);
+    for (int q = tid; q <= r1 - r0; q += blockDim.x) ro[q] = (int)(A.off[r0 + q] - A.off[r0]);
     // full copies, owned vectors, owned part of the matrix
     for (int i = tid; i <= m; i += blockDim.x) ys[i] = st.y[i];
     if (tid == 0) xh[n] = 0.0;
@@ -359,13 +379,26 @@ k_ref_cluster(int m, int n, Sell A, Sell At, const double* __restrict__ c, const
         rv = SliceView<MAT_SMEM>{vr - rb, ir - rb};
     }
     cluster_phase<NC>(cl);
+    // End of a phase: this CTA's copy is complete.  A thread that gave up once waits no more and
+    // runs on, so that barriers still meet.
+    bool ok = true;
+    uint32_t parity = 0;
+    auto phase_end = [&](int v, uint32_t bytes) {
+        if constexpr (NC == 1) {
+            __syncthreads();
+        } else {
+            if (ok) ok = tx_wait(bar + v, parity);
+            if (tid == 0) tx_expect(bar + v, bytes);
+            if (v == 1) __syncthreads();
+        }
+    };
     long long it = out->iter;
     bool finished = out->converged || out->failed;
     // max row violation of the vector whose copies are in xh, into slot
     auto violation = [&](int slot) {
         for (int sl = r0 + warp; sl < r1; sl += nw) {
-            const int64_t p0 = A.off[sl];
-            const double v = rv.sum(p0, (int)((A.off[sl + 1] - p0) >> 5), lane, xh);
+            const int p0 = ro[sl - r0];
+            const double v = rv.sum(rb + p0, (ro[sl - r0 + 1] - p0) >> 5, lane, xh);
             const int i = (sl << 5) + lane, o = i - (r0 << 5);
             if (i < m) {
                 const double d = v - bs[o];
@@ -382,8 +415,8 @@ k_ref_cluster(int m, int n, Sell A, Sell At, const double* __restrict__ c, const
                 __syncthreads();
             }
             for (int sl = c0 + warp; sl < c1; sl += nw) {
-                const int64_t p0 = __ldg(At.off + sl);
-                const double w = cv.sum(p0, (int)((__ldg(At.off + sl + 1) - p0) >> 5), lane, ys);
+                const int p0 = co[sl - c0];
+                const double w = cv.sum(cb + p0, (co[sl - c0 + 1] - p0) >> 5, lane, ys);
                 const int j = (sl << 5) + lane, o = j - (c0 << 5);
                 if (j < n) {
                     double xj = xs[o];
@@ -392,25 +425,28 @@ k_ref_cluster(int m, int n, Sell A, Sell At, const double* __restrict__ c, const
                     double new_x = ref_clamp(next_x, ls[o], us[o]);
                     if (check) atomic_max_nonneg(&red[R_DPRIMAL], fabs(new_x - xj));
                     sums[o] += new_x;
-                    xc.store(j, 2.0 * new_x - xj);
+                    xv.store(peers, j, 2.0 * new_x - xj);
                     xs[o] = new_x;
                 }
             }
-            cluster_phase<NC>(cl);
+            if (NC > 1 && c0 == c1 && tid == 0) tv.store(peers, 0, 0.0);
+            phase_end(0, x_bytes);
             for (int sl = r0 + warp; sl < r1; sl += nw) {
-                const int64_t p0 = __ldg(A.off + sl);
-                const double v = rv.sum(p0, (int)((__ldg(A.off + sl + 1) - p0) >> 5), lane, xh);
+                const int p0 = ro[sl - r0];
+                const double v = rv.sum(rb + p0, (ro[sl - r0 + 1] - p0) >> 5, lane, xh);
                 const int i = (sl << 5) + lane, o = i - (r0 << 5);
                 if (i < m) {
                     double yi = ys[i];
                     double next_y = yi + ss[o] * (v - bs[o]);
                     double new_y = (!eq[o]) ? ((0.0 < next_y) ? next_y : 0.0) : next_y;
                     if (check) atomic_max_nonneg(&red[R_DDUAL], fabs(new_y - yi));
-                    yc.store(i, new_y);
+                    yv.store(peers, i, new_y);
                 }
             }
-            cluster_phase<NC>(cl);
+            phase_end(1, y_bytes);
+            parity ^= 1;
         }
+        const ClusterVec<double, NC> xc(cl, xh);
         for (int j = (c0 << 5) + tid; j < min(n, c1 << 5); j += blockDim.x) {
             const int o = j - (c0 << 5);
             const double xj = xs[o];
@@ -459,6 +495,10 @@ k_ref_cluster(int m, int n, Sell A, Sell At, const double* __restrict__ c, const
         st.x[j] = xs[j - (c0 << 5)];
         st.x_sum[j] = sums[j - (c0 << 5)];
     }
+    if (!ok) {
+        out->wait_failed = 1;
+        __nanosleep(1000000);  // late elements land before the CTA they go to leaves
+    }
     cluster_phase<NC>(cl);  // no CTA leaves while another may still store into its copies
 }
 
@@ -488,6 +528,8 @@ RefLayout ref_layout(int m, int n, int64_t ce, int64_t re) {
     L.rval = take(8 * re);
     L.cidx = take(2 * ce);
     L.ridx = take(2 * re);
+    L.coff = take(4 * (L.cols / 32 + 1));
+    L.roff = take(4 * (L.rows / 32 + 1));
     L.total = (int)std::min<int64_t>(o, 1 << 30);
     return L;
 }
@@ -608,7 +650,7 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
     int max_smem = 0;
     B2P_CUDA(ctx, cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     max_smem -= 1024;  // static part
-    // One CTA where the vectors and the matrix fit its shared memory (no cluster barrier), else a
+    // One CTA for up to kOneCtaNnz entries that fit its shared memory with the vectors, else a
     // cluster where the vectors do, with the owned parts of the matrix in shared memory if
     // they fit as well.
     RefLayout lay{};
@@ -616,7 +658,7 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
     if (A.off && At.off && L.nnz <= kClusterNnz && m < 65535 && n < 65535) {
         const int ncs = (n + 31) >> 5, nrs = (m + 31) >> 5;
         lay = ref_layout<1>(m, n, h_toff[ncs], h_off[nrs]);
-        if (lay.total <= max_smem) form = 1;
+        if (L.nnz <= kOneCtaNnz && lay.total <= max_smem) form = 1;
         if (!form) {
             int64_t ce = 0, re = 0;
             for (int r = 0; r < kClusterCtas; ++r) {
@@ -692,6 +734,10 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
             RefOutcome o;
             B2P_CUDA(ctx, cudaMemcpyAsync(&o, B.outcome.p, sizeof(o), cudaMemcpyDeviceToHost, s));
             B2P_CUDA(ctx, cudaStreamSynchronize(s));
+            if (o.wait_failed) {
+                ctx->err = "the cluster's exchange did not complete";
+                return B2P_EXECUTION_FAILED;
+            }
             iter = o.iter;
             converged = o.converged != 0;
             failed = o.failed != 0;

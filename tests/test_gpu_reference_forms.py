@@ -51,3 +51,15 @@ def test_reference_forms_diverge_like_the_oracle(ctx, lpgen, oracle, m, n):
     o = oracle.ref_pdhg(s, max_iterations=1000, adaptive=False, primal_step=0.5, dual_step=0.5)
     assert res["iterations"] == o["iterations"]
     assert res["status"] == o["status"]
+
+
+@pytest.mark.parametrize("m,n,k", [(2000, 100, 60), (3000, 33, 100), (180, 600, 5), (205, 615, 5)])
+def test_cluster_ctas_without_columns_match_oracle(ctx, lpgen, oracle, m, n, k):
+    """A cluster with fewer column slices than CTAs (the empty ones post a token), and the two sides of
+    one CTA / cluster (3,072 entries): bit for bit over two check intervals and a remainder."""
+    s = lpgen.random_sparse(m=m, n=n, nnz_per_col=k, seed=m + n).standard()
+    ctx.upload(s)
+    res, x, y = ctx.solve(engine="reference", max_iterations=230)
+    o = oracle.ref_pdhg(s, max_iterations=230)
+    assert res["iterations"] == o["iterations"] and res["status"] == o["status"]
+    assert np.array_equal(x, o["x_final"]) and np.array_equal(y, o["y_last"])
