@@ -69,6 +69,7 @@
 #include <string>
 
 #include "b2p_internal.cuh"
+#include "cluster.cuh"
 
 namespace b2p {
 
@@ -1369,14 +1370,17 @@ __global__ void k_batch_power(int nmat, const int32_t* __restrict__ mat_m, const
 }
 
 // The matrices of at least kPowerCluster entries, where a batch has few of them: a cluster of
-// kPowerCtas CTAs each.  One CTA's
-// step is a chain of dependent loads over its whole share of rows and columns (41 us a step
-// on a 2,000 x 8,000 matrix of 47,984 entries, up to 1,000 steps); eight CTAs walk an eighth
-// of it between two cluster barriers (9 us a step: 41 -> 9.2 ms for the planning matrix).  Rows and columns are
-// summed over the FP64 SELL copies (entry order W = 1), one lane each, in the order of the
-// one-CTA kernel; the vectors live in L2 (loads bypass L1, which other CTAs' stores do not
-// reach).  The kernel's clusters loop over the matrices; every CTA of a cluster makes the
-// same decisions from the same sums.
+// kPowerCtas CTAs each.  One CTA's step is a chain of dependent loads over its whole share of
+// rows and columns (41 us a step on a 2,000 x 8,000 matrix of 47,984 entries, up to 1,000
+// steps); eight CTAs walk an eighth of it.  Rows and columns are summed over the FP64 SELL
+// copies (entry order W = 1), one lane each, in the order of the one-CTA kernel.  SM: every CTA
+// holds whole copies of both vectors in shared memory, into which the owners post
+// (ClusterPost), and its share of the matrix where `room` bytes are left for it (4.6 us a
+// step on that matrix); otherwise the vectors lie in L2 (loads bypass L1, which other CTAs'
+// stores do not reach) and a cluster barrier ends each half step (9 us).  The kernel's
+// clusters loop over the matrices; every CTA of a cluster makes the same decisions from the
+// same sums.  Every step ends with a cluster barrier, so no thread falls a phase behind.
+template <bool SM>
 __global__ void __cluster_dims__(kPowerCtas, 1, 1) __launch_bounds__(512)
 k_batch_power_cluster(int nmat, const int32_t* __restrict__ mat_m, const int32_t* __restrict__ mat_n,
                       const int64_t* __restrict__ row_off, const int64_t* __restrict__ col_off,
@@ -1384,15 +1388,29 @@ k_batch_power_cluster(int nmat, const int32_t* __restrict__ mat_m, const int32_t
                       const int64_t* __restrict__ cs_off, const int64_t* __restrict__ r_sptr,
                       const int64_t* __restrict__ c_sptr, const uint16_t* __restrict__ r_eidx,
                       const uint16_t* __restrict__ c_eidx, const double* __restrict__ r_ev,
-                      const double* __restrict__ c_ev, double* pv, double* pu, double safety,
-                      double* __restrict__ eta_out) {
+                      const double* __restrict__ c_ev, double* pv, double* pu, double safety, int max_m, int max_n,
+                      int room, int* __restrict__ wait_failed, double* __restrict__ eta_out) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     __shared__ double red[32];
     __shared__ double part[2];  // this CTA's share of ||v||^2, by step parity
-    const int rank = (int)cl.block_rank();
-    const int lane = threadIdx.x & 31, warp = rank * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int warps = kPowerCtas * (blockDim.x >> 5);
+    __shared__ uint64_t bar[2];  // arrivals of v, of u
+    __shared__ int s_fits;
+    double* vs = smem_at<double>(0);
+    double* us = smem_at<double>(8 * max_n);
+    int2* tab = smem_at<int2>(8 * (max_n + max_m));  // per owned slice {first entry, entries per lane}
+    const int tabs = (((max_n + 31) >> 5) + kPowerCtas - 1) / kPowerCtas + (((max_m + 31) >> 5) + kPowerCtas - 1) / kPowerCtas;
+    double* sv = smem_at<double>(8 * (max_n + max_m + tabs));
+    const int rank = (int)cl.block_rank(), tid = threadIdx.x;
+    const int lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    const ClusterPeers<SM ? kPowerCtas : 1> peers(smem_at<double>(0));
+    const ClusterPost<double, SM ? kPowerCtas : 1> vp(peers, vs, bar), up(peers, us, bar + 1);
+    uint32_t parity = 0;
+    bool ok = true;
+    if (SM && tid == 0) {
+        tx_init(bar);
+        tx_init(bar + 1);
+    }
     // the whole cluster's ||v||^2 from the CTAs' shares, in rank order
     auto total = [&](double share, int slot) -> double {
         double w[1] = {share};
@@ -1404,7 +1422,7 @@ k_batch_power_cluster(int nmat, const int32_t* __restrict__ mat_m, const int32_t
         return t;
     };
     // entries of one row (column) of a slice, 8 in flight
-    auto dot = [&](const double* __restrict__ v, const uint16_t* __restrict__ ix, int len, const double* g) -> double {
+    auto dot = [&](const double* v, const uint16_t* ix, int len, auto g) -> double {
         double s = 0.0;
         for (int q = 0; q < len; q += 8) {
             double vv[8];
@@ -1417,7 +1435,7 @@ k_batch_power_cluster(int nmat, const int32_t* __restrict__ mat_m, const int32_t
             }
             double gg[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) gg[u] = q + u < len ? __ldcg(g + ii[u]) : 0.0;
+            for (int u = 0; u < 8; ++u) gg[u] = q + u < len ? g(ii[u]) : 0.0;
 #pragma unroll
             for (int u = 0; u < 8; ++u)
                 if (q + u < len) s += vv[u] * gg[u];
@@ -1431,40 +1449,104 @@ k_batch_power_cluster(int nmat, const int32_t* __restrict__ mat_m, const int32_t
         const int64_t* rsp = r_sptr + rs_off[k];
         const int64_t* csp = c_sptr + cs_off[k];
         const int nrs = (m + 31) >> 5, ncs = (n + 31) >> 5;
+        // this CTA's slices: rank, rank + kPowerCtas, ...; those of the columns first
+        const int ncl = (ncs - rank + kPowerCtas - 1) / kPowerCtas, nrl = (nrs - rank + kPowerCtas - 1) / kPowerCtas;
+        bool fits = false;
+        uint16_t* si = nullptr;
+        if constexpr (SM) {
+            for (int l = tid; l < ncl + nrl; l += blockDim.x) {
+                const int64_t* o = l < ncl ? csp + rank + kPowerCtas * l : rsp + rank + kPowerCtas * (l - ncl);
+                tab[l] = make_int2(0, (int)((o[1] - o[0]) >> 5));
+            }
+            __syncthreads();
+            if (tid == 0) {
+                int64_t e = 0;
+                for (int l = 0; l < ncl + nrl; ++l) {
+                    tab[l].x = (int)min(e, (int64_t)INT_MAX);
+                    e += 32 * (int64_t)tab[l].y;
+                }
+                s_fits = 10 * e <= room ? (int)e : -1;
+            }
+            __syncthreads();
+            fits = s_fits >= 0;
+            if (fits) {
+                si = reinterpret_cast<uint16_t*>(sv + s_fits);
+                for (int l = warp; l < ncl + nrl; l += nw) {
+                    const int2 t = tab[l];
+                    const int64_t p0 = l < ncl ? csp[rank + kPowerCtas * l] : rsp[rank + kPowerCtas * (l - ncl)];
+                    const double* v = (l < ncl ? c_ev : r_ev) + p0;
+                    const uint16_t* ix = (l < ncl ? c_eidx : r_eidx) + p0;
+                    for (int e = lane; e < 32 * t.y; e += 32) {
+                        sv[t.x + e] = v[e];
+                        si[t.x + e] = ix[e];
+                    }
+                }
+            }
+            for (int j = tid; j < n; j += blockDim.x) vs[j] = power_start(j);
+        }
         double sum = 0.0;
-        for (int sl = warp; sl < ncs; sl += warps) {
-            const int j = (sl << 5) + lane;
+        for (int l = warp; l < ncl; l += nw) {
+            const int j = (rank + kPowerCtas * l) * 32 + lane;
             if (j < n) {
                 const double v = power_start(j);
-                pv[co + j] = v;
+                if (!SM) pv[co + j] = v;
                 sum += v * v;
             }
         }
+        // the sum of slice l's rows (columns) over the gathered vector
+        auto slice = [&](int l, int64_t p0, int64_t p1, const double* gv, const uint16_t* gi, auto g) -> double {
+            if (SM && fits) {
+                const int2 t = tab[l];
+                return dot(sv + t.x + lane, si + t.x + lane, t.y, g);
+            }
+            return dot(gv + p0 + lane, gi + p0 + lane, (int)((p1 - p0) >> 5), g);
+        };
         double norm = sqrt(total(sum, 0)), prev = 0.0;
         for (int t = 0; t < 1000; ++t) {
             const double inv = 1.0 / norm;
-            for (int sl = warp; sl < nrs; sl += warps) {
-                const int i = (sl << 5) + lane;
-                const int64_t p0 = rsp[sl];
-                const double s = dot(r_ev + p0 + lane, r_eidx + p0 + lane, (int)((rsp[sl + 1] - p0) >> 5), pv + co);
-                if (i < m) pu[ro + i] = s * inv;
+            if (SM && tid == 0) {
+                tx_expect(bar, 8u * (uint32_t)n);
+                tx_expect(bar + 1, 8u * (uint32_t)m);
             }
-            cl.sync();
+            for (int l = warp; l < nrl; l += nw) {
+                const int sl = rank + kPowerCtas * l, i = (sl << 5) + lane;
+                const double s = slice(ncl + l, rsp[sl], rsp[sl + 1], r_ev, r_eidx,
+                                       [&](unsigned c) { return SM ? vs[c] : __ldcg(pv + co + c); });
+                if (i < m) {
+                    if constexpr (SM) up.store(peers, i, s * inv);
+                    else pu[ro + i] = s * inv;
+                }
+            }
+            if constexpr (SM) {
+                if (ok) ok = tx_wait(bar + 1, parity);
+            } else {
+                cl.sync();
+            }
             sum = 0.0;
-            for (int sl = warp; sl < ncs; sl += warps) {
-                const int j = (sl << 5) + lane;
-                const int64_t p0 = csp[sl];
-                const double s = dot(c_ev + p0 + lane, c_eidx + p0 + lane, (int)((csp[sl + 1] - p0) >> 5), pu + ro);
+            for (int l = warp; l < ncl; l += nw) {
+                const int sl = rank + kPowerCtas * l, j = (sl << 5) + lane;
+                const double s = slice(l, csp[sl], csp[sl + 1], c_ev, c_eidx,
+                                       [&](unsigned c) { return SM ? us[c] : __ldcg(pu + ro + c); });
                 if (j < n) {
-                    pv[co + j] = s;
+                    if constexpr (SM) vp.store(peers, j, s);
+                    else pv[co + j] = s;
                     sum += s * s;
                 }
             }
             const double nn = sqrt(total(sum, (t + 1) & 1));
+            if constexpr (SM) {
+                if (ok) ok = tx_wait(bar, parity);
+                parity ^= 1;
+                __syncthreads();  // the copies are whole for every warp before tid 0 opens the next phases
+            }
             const bool stop = nn <= 0.0 || fabs(nn - prev) <= 1e-7 * nn;
             prev = nn;
             norm = nn > 0.0 ? nn : 1.0;
             if (stop) break;
+        }
+        if (!ok) {
+            *wait_failed = 1;
+            __nanosleep(1000000);  // late elements land before the CTA they go to leaves
         }
         if (rank == 0 && threadIdx.x == 0) {
             const double sig = sqrt(fmax(prev, 0.0));
@@ -1792,8 +1874,8 @@ BArgs make_args(BatchWork* w, const b2p_params* p, const int32_t* active) {
     return a;
 }
 
-// dynamic shared memory of one CTA: y and xh (MT) of the largest instance, or of two
-// instances of the shared matrix in the paired form
+// dynamic shared memory of one CTA: per-instance blocks, slice table, y and xh (MT) of the largest
+// instance, or of ni instances of the shared matrix
 size_t smem_bytes(BatchWork* w, size_t mt_size, int ni = 1) {
     const size_t tab = sizeof(int2) * slice_tab_len((w->max_m + 31) >> 5, (w->max_n + 31) >> 5);
     const size_t m4 = (size_t)((w->max_m + 3) & ~3), n4 = (size_t)((w->max_n + 3) & ~3);
@@ -2537,16 +2619,37 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
     k_batch_power<<<gmat, 256, 0, s>>>(nmat, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->rowptr.p,
                                         w->colidx.p, w->sv64.p, w->t_rowptr.p, w->t_colidx.p, w->stv64.p, w->pv.p,
                                         w->pu.p, 0.998, use_clusters ? kPowerCluster : INT_MAX, w->mat_eta.p);
+    int wait_failed = 0;
+    DBuf<int> failed;
     if (use_clusters) {
-        k_batch_power_cluster<<<std::min(nmat, clusters) * kPowerCtas, 512, 0, s>>>(
+        int max_smem = 0;
+        B2P_CUDA(ctx, cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+        cudaFuncAttributes fa;
+        B2P_CUDA(ctx, cudaFuncGetAttributes(&fa, k_batch_power_cluster<true>));
+        max_smem -= (int)fa.sharedSizeBytes;
+        const int tabs = (((w->max_n + 31) >> 5) + kPowerCtas - 1) / kPowerCtas + (((w->max_m + 31) >> 5) + kPowerCtas - 1) / kPowerCtas;
+        const int64_t vec = 8ll * ((int64_t)w->max_n + w->max_m + tabs);
+        const bool sm = vec <= max_smem;
+        auto fn = sm ? k_batch_power_cluster<true> : k_batch_power_cluster<false>;
+        if (sm) B2P_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+        B2P_CUDA(ctx, failed.reserve(1));
+        B2P_CUDA(ctx, cudaMemsetAsync(failed.p, 0, sizeof(int), s));
+        // with the copies one CTA per SM is resident; the clusters loop over the matrices
+        const int grid = std::min(nmat, sm ? std::max(clusters / 2, 1) : clusters) * kPowerCtas;
+        fn<<<grid, 512, sm ? max_smem : 0, s>>>(
             nmat, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->rowptr.p, w->mat_rs_off.p,
             w->mat_cs_off.p, w->r_sptr.p, w->c_sptr.p, w->r_eidx.p, w->c_eidx.p, w->r_ev64.p, w->c_ev64.p, w->pv.p,
-            w->pu.p, 0.998, w->mat_eta.p);
+            w->pu.p, 0.998, w->max_m, w->max_n, (int)(max_smem - vec), failed.p, w->mat_eta.p);
         ctx->launches += 1;
+        B2P_CUDA(ctx, cudaMemcpyAsync(&wait_failed, failed.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     }
     B2P_LAUNCH(ctx);
     ctx->launches += 5;
     B2P_CUDA(ctx, cudaStreamSynchronize(s));
+    if (wait_failed) {
+        ctx->err = "batch upload: the power iteration's cluster exchange did not complete";
+        return B2P_EXECUTION_FAILED;
+    }
     return B2P_OK;
 }
 
