@@ -739,8 +739,8 @@ def run_learned_workload(args):
     pk, pk_src = peaks()
     peak = pk["hbm_gbs"]
     achieved = it_total * per_iter / (kern_ms / 1e3) / 1e9
-    kname = "k_batch_pair" if ni == 2 else "k_batch_chunk"
-    prof = read_profile(ROOT / "profiles" / f"{kname[2:]}_refinery_planning.txt")
+    kname = "k_batch_chunk"
+    prof = read_profile(ROOT / "profiles" / "batch_group_refinery_planning.txt")
     roofline = {"bound": "l2", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": prof.get("dram_bytes_per_instance_iteration"),
                 "traffic_unit": "DRAM bytes per instance-iteration (ncu dram__bytes_read.sum + write.sum)",
