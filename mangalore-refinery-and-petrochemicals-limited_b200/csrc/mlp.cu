@@ -462,6 +462,15 @@ int gemm_tn(Ctx* ctx, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, i
     const size_t stride = (size_t)M * ldc;
     float* dst = C;
     if (splits > 1) {
+        if (stride * splits > ws->count) {
+            // a captured graph would keep the old address in the nodes it already holds
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            B2P_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
+            if (cap != cudaStreamCaptureStatusNone) {
+                ctx->err = "gemm: the split-K workspace would have to grow inside a stream capture";
+                return B2P_EXECUTION_FAILED;
+            }
+        }
         B2P_CUDA(ctx, ws->reserve(stride * splits));
         dst = ws->p;
     }
@@ -1279,12 +1288,18 @@ int b2p_mlp_train(void* p, int epochs, int batch, float lr_start, float lr_end, 
             cudaGraphExecDestroy(s->epoch_exec);
             s->epoch_exec = nullptr;
         }
-        // outside the capture: kernel attributes and the split-K workspace of every GEMM shape
-        // (one forward / backward of a full batch; no parameter changes)
-        const int rows0 = (std::min(batch, N) + 7) & ~7;
-        if ((r = forward_hidden(ctx, s, rows0, std::min(batch, N), true))) return r;
+        // outside the capture: kernel attributes and the split-K workspace of every GEMM shape (one
+        // forward / backward of a full batch and of the epoch's last, shorter one; no parameter
+        // changes).  The shorter one can want the larger workspace: fewer rows are fewer tiles and
+        // so more splits (1,024 hidden, 10,008 outputs: 512 x 1,024 x 4 floats for a full batch of
+        // 512, 128 x 1,024 x 18 for a remainder of 128).
         B2P_CUDA(ctx, cudaMemcpyAsync(s->perm.p, order.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice, st));
-        if ((r = backward(ctx, s, rows0, std::min(batch, N), s->DT.p, s->perm.p, false))) return r;
+        for (const int valid : {std::min(batch, N), N % batch}) {
+            const int rows = (valid + 7) & ~7;
+            if (valid == 0) continue;
+            if ((r = forward_hidden(ctx, s, rows, valid, true))) return r;
+            if ((r = backward(ctx, s, rows, valid, s->DT.p, s->perm.p, false))) return r;
+        }
         B2P_CUDA(ctx, cudaStreamSynchronize(st));
         const long long launches0 = ctx->launches, step0 = s->step;
         cudaGraph_t graph = nullptr;
