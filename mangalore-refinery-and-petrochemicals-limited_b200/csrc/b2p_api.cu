@@ -595,7 +595,7 @@ int b2p_spmv_t(void* p, int m, int n, const int32_t* rowptr, const int32_t* coli
     if (io.packed && nnz <= 12288 && n <= 8192 && m <= 1024) {
         const int rows_off = n + (int)nnz + ((int)nnz + 3) / 4;  // in doubles: sums, products, columns, then row pointers
         const size_t small = 8 * (size_t)rows_off + 4 * ((size_t)m + 1);
-        B2P_CUDA(ctx, cudaFuncSetAttribute(k_spmv_t_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small));
+        B2P_CUDA(ctx, open_smem(ctx, k_spmv_t_small));
         k_spmv_t_small<<<1, 1024, small, s>>>(m, n, rp, ci, va, yd, wd, flag, rows_off);
         B2P_LAUNCH(ctx);
         ctx->launches += 1;

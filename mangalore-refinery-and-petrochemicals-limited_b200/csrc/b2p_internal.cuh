@@ -129,6 +129,24 @@ inline unsigned grid_for(int64_t threads, int block, int sm_count, int per_sm = 
 
 double now_ms();
 
+// Opens a kernel to as much dynamic shared memory as its blocks can have (in *most, optional).  The
+// limit is state of the function on the device, which all contexts of the process share, and a launch
+// above it is refused: it is always set to this one value and never to what one call needs, or a
+// context on another host thread could lower it between a call's setting and its launch.
+template <typename F>
+cudaError_t open_smem(const Ctx* ctx, F* fn, int* most = nullptr) {
+    int optin = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+    if (e != cudaSuccess) return e;
+    cudaFuncAttributes fa;
+    e = cudaFuncGetAttributes(&fa, fn);
+    if (e != cudaSuccess) return e;
+    const int limit = optin - (int)fa.sharedSizeBytes;
+    if (most) *most = limit;
+    if (fa.maxDynamicSharedSizeBytes >= limit) return cudaSuccess;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+}
+
 // Builds the stable transpose of a CSR matrix on the device (setup only).
 int build_transpose(Ctx* ctx, int m, int n, int64_t nnz, const int32_t* rowptr, const int32_t* colidx,
                     const double* vals, int32_t* t_rowptr, int32_t* t_colidx, double* t_vals);

@@ -1971,8 +1971,6 @@ int autotune(Ctx* ctx, BatchWork* w, const b2p_params* p, TuneCfg* best) {
     const int trial_iters = 128;
     float best_ms = 1e30f;
     *best = TuneCfg();
-    int max_smem = 0;
-    B2P_CUDA(ctx, cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     // one trial launch of `iters` iterations over the sample with `th` threads, entry order W
     // and ni instances per CTA (ms; < 0: the shape does not fit)
     auto trial = [&](int th, int W, int ni, int iters, float* ms, int* rounds) -> int {
@@ -1980,10 +1978,9 @@ int autotune(Ctx* ctx, BatchWork* w, const b2p_params* p, TuneCfg* best) {
         auto fn = chunk_kernel<MT>(w, W, ni, th);
         if (!fn) return B2P_OK;
         const size_t sm = smem_bytes(w, sizeof(MT), ni);
-        cudaFuncAttributes fa;
-        B2P_CUDA(ctx, cudaFuncGetAttributes(&fa, fn));
-        if (sm + fa.sharedSizeBytes > (size_t)max_smem) return B2P_OK;
-        B2P_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        int most = 0;
+        B2P_CUDA(ctx, open_smem(ctx, fn, &most));
+        if (sm > (size_t)most) return B2P_OK;
         int st = refill_ell(ctx, w, W);
         if (st) return st;
         st = init_instances<MT>(ctx, w, &tp, nullptr, nullptr, nullptr);
@@ -2166,16 +2163,13 @@ int batch_run(Ctx* ctx, BatchWork* w, const b2p_params* p, const double* x0_dev,
             if (host_cnt) cudaFreeHost(host_cnt);
         }
     } own;
-    int max_smem = 0;
-    B2P_CUDA(ctx, cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     auto open_form = [&](Form& f, int ni, int threads, double us) -> int {
         auto fn = chunk_kernel<MT>(w, cfg.w, ni, threads);
         const size_t sm = smem_bytes(w, sizeof(MT), ni);
         if (!fn) return B2P_OK;
-        cudaFuncAttributes fa;
-        B2P_CUDA(ctx, cudaFuncGetAttributes(&fa, fn));
-        if (sm + fa.sharedSizeBytes > (size_t)max_smem) return B2P_OK;
-        B2P_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        int most = 0;
+        B2P_CUDA(ctx, open_smem(ctx, fn, &most));
+        if (sm > (size_t)most) return B2P_OK;
         int per_sm = 0;
         B2P_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, sm));
         if (per_sm < 1) return B2P_OK;
@@ -2623,15 +2617,11 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
     DBuf<int> failed;
     if (use_clusters) {
         int max_smem = 0;
-        B2P_CUDA(ctx, cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-        cudaFuncAttributes fa;
-        B2P_CUDA(ctx, cudaFuncGetAttributes(&fa, k_batch_power_cluster<true>));
-        max_smem -= (int)fa.sharedSizeBytes;
+        B2P_CUDA(ctx, open_smem(ctx, k_batch_power_cluster<true>, &max_smem));
         const int tabs = (((w->max_n + 31) >> 5) + kPowerCtas - 1) / kPowerCtas + (((w->max_m + 31) >> 5) + kPowerCtas - 1) / kPowerCtas;
         const int64_t vec = 8ll * ((int64_t)w->max_n + w->max_m + tabs);
         const bool sm = vec <= max_smem;
         auto fn = sm ? k_batch_power_cluster<true> : k_batch_power_cluster<false>;
-        if (sm) B2P_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
         B2P_CUDA(ctx, failed.reserve(1));
         B2P_CUDA(ctx, cudaMemsetAsync(failed.p, 0, sizeof(int), s));
         // with the copies one CTA per SM is resident; the clusters loop over the matrices

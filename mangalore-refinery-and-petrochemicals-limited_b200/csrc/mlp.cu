@@ -447,12 +447,7 @@ int gemm_tn(Ctx* ctx, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, i
         ctx->err = "gemm: tensor map rejected (alignment) or driver entry point missing";
         return B2P_INVALID_ARGUMENT;
     }
-    static bool attr = false;
-    if (!attr) {
-        B2P_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tn_bf16<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM));
-        B2P_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tn_bf16<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM));
-        attr = true;
-    }
+    B2P_CUDA(ctx, open_smem(ctx, le ? k_gemm_tn_bf16<true> : k_gemm_tn_bf16<false>));
     const int tiles = ((N + GBN - 1) / GBN) * ((M + GBM - 1) / GBM);
     const int nkb = (K + GBK - 1) / GBK;
     int splits = 1;

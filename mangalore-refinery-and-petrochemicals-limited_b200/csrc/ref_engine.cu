@@ -710,7 +710,7 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
         B2P_CUDA(ctx, cudaMemsetAsync(B.outcome.p, 0, sizeof(RefOutcome), s));
         auto fn = form == 1 ? k_ref_cluster<1, true>
                             : (form == 2 ? k_ref_cluster<kClusterCtas, true> : k_ref_cluster<kClusterCtas, false>);
-        B2P_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, lay.total));
+        B2P_CUDA(ctx, open_smem(ctx, fn));
         cudaLaunchConfig_t lc{};
         cudaLaunchAttribute dims;
         dims.id = cudaLaunchAttributeClusterDimension;
