@@ -64,10 +64,21 @@ __device__ __forceinline__ void tx_init(uint64_t* bar) {
 __device__ __forceinline__ void tx_expect(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
 }
-// Waits (about a second at most) for the phase of the given parity.
+// How long a wait for the peers' elements may take: thousands of times what they ever need, and within
+// what a caller can wait for an error.
+constexpr unsigned long long kTxWaitNs = 1000000000ull;
+
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+// Waits for the phase of the given parity, kTxWaitNs at most; false: it did not complete.  The limit is
+// one of time, because a single try_wait may suspend the thread for as long as the hardware likes.
 __device__ __forceinline__ bool tx_wait(uint64_t* bar, uint32_t parity) {
     const uint32_t addr = smem_addr(bar);
-    for (int spin = 0; spin < (1 << 20); ++spin) {
+    unsigned long long since = 0;
+    for (int spin = 0; spin < (1 << 24); ++spin) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -77,7 +88,12 @@ __device__ __forceinline__ bool tx_wait(uint64_t* bar, uint32_t parity) {
             : "r"(addr), "r"(parity)
             : "memory");
         if (done) return true;
-        if (spin > 256) __nanosleep(128);
+        if (spin > 256) {
+            const unsigned long long now = global_ns();
+            if (since == 0) since = now;
+            if (now - since > kTxWaitNs) return false;
+            __nanosleep(128);
+        }
     }
     return false;
 }
