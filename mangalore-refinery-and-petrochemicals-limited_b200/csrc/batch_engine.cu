@@ -2609,24 +2609,25 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
     // clusters only while all big matrices' clusters are resident at once (two 512-thread CTAs
     // per SM): 304 big matrices of 1,024 take 130 ms longer on clusters than one CTA each
     const int clusters = 2 * ctx->sm_count / kPowerCtas;
-    const bool use_clusters = big > 0 && big <= clusters;
+    int max_smem = 0;
+    B2P_CUDA(ctx, open_smem(ctx, k_batch_power_cluster<true>, &max_smem));
+    const int tabs = (((w->max_n + 31) >> 5) + kPowerCtas - 1) / kPowerCtas + (((w->max_m + 31) >> 5) + kPowerCtas - 1) / kPowerCtas;
+    const int64_t vec = 8ll * ((int64_t)w->max_n + w->max_m + tabs);
+    const bool sm = vec <= max_smem;  // both vectors fit a CTA's shared memory
+    const auto power_fn = sm ? k_batch_power_cluster<true> : k_batch_power_cluster<false>;
+    const bool use_clusters =
+        big > 0 && big <= clusters && clusters_resident(power_fn, kPowerCtas, 512, sm ? max_smem : 0) > 0;
     k_batch_power<<<gmat, 256, 0, s>>>(nmat, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->rowptr.p,
                                         w->colidx.p, w->sv64.p, w->t_rowptr.p, w->t_colidx.p, w->stv64.p, w->pv.p,
                                         w->pu.p, 0.998, use_clusters ? kPowerCluster : INT_MAX, w->mat_eta.p);
     int wait_failed = 0;
     DBuf<int> failed;
     if (use_clusters) {
-        int max_smem = 0;
-        B2P_CUDA(ctx, open_smem(ctx, k_batch_power_cluster<true>, &max_smem));
-        const int tabs = (((w->max_n + 31) >> 5) + kPowerCtas - 1) / kPowerCtas + (((w->max_m + 31) >> 5) + kPowerCtas - 1) / kPowerCtas;
-        const int64_t vec = 8ll * ((int64_t)w->max_n + w->max_m + tabs);
-        const bool sm = vec <= max_smem;
-        auto fn = sm ? k_batch_power_cluster<true> : k_batch_power_cluster<false>;
         B2P_CUDA(ctx, failed.reserve(1));
         B2P_CUDA(ctx, cudaMemsetAsync(failed.p, 0, sizeof(int), s));
         // with the copies one CTA per SM is resident; the clusters loop over the matrices
         const int grid = std::min(nmat, sm ? std::max(clusters / 2, 1) : clusters) * kPowerCtas;
-        fn<<<grid, 512, sm ? max_smem : 0, s>>>(
+        power_fn<<<grid, 512, sm ? max_smem : 0, s>>>(
             nmat, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->rowptr.p, w->mat_rs_off.p,
             w->mat_cs_off.p, w->r_sptr.p, w->c_sptr.p, w->r_eidx.p, w->c_eidx.p, w->r_ev64.p, w->c_ev64.p, w->pv.p,
             w->pu.p, 0.998, w->max_m, w->max_n, (int)(max_smem - vec), failed.p, w->mat_eta.p);

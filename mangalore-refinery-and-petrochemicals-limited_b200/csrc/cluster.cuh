@@ -135,4 +135,33 @@ struct ClusterPost {
     }
 };
 
+// Launch of one block shape on clusters of `ctas` CTAs (dims must outlive the configuration).
+inline cudaLaunchConfig_t cluster_config(int grid, int ctas, int threads, size_t smem, cudaStream_t s,
+                                         cudaLaunchAttribute* dims) {
+    cudaLaunchConfig_t lc{};
+    dims->id = cudaLaunchAttributeClusterDimension;
+    dims->val.clusterDim.x = ctas;
+    dims->val.clusterDim.y = dims->val.clusterDim.z = 1;
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(threads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = s;
+    lc.attrs = dims;
+    lc.numAttrs = 1;
+    return lc;
+}
+// Clusters of a launch that the device can hold at once.  0 where its SMs cannot be brought together for
+// one (a partition of a GPU): such a device keeps the forms without clusters.
+template <typename F>
+int clusters_resident(F* fn, int ctas, int threads, size_t smem) {
+    cudaLaunchAttribute dims;
+    const cudaLaunchConfig_t lc = cluster_config(ctas, ctas, threads, smem, nullptr, &dims);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, fn, &lc) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
 }  // namespace b2p

@@ -2181,24 +2181,18 @@ int cluster_ctas(Ctx* ctx, HalpernWork* w, const b2p_params* p) {
         for (int64_t q = 0; q < S->slices; ++q)
             if (S->h_off[q + 1] - S->h_off[q] > 32 * kClusterLongest) return 0;
     int most = 0;
-    if (open_smem(ctx, cluster_kernel<MT>(NC), &most) != cudaSuccess) return 0;
-    return cluster_lay<MT>(w, K, NC).total <= most ? NC : 0;
+    const auto fn = cluster_kernel<MT>(NC);
+    if (open_smem(ctx, fn, &most) != cudaSuccess) return 0;
+    const int total = cluster_lay<MT>(w, K, NC).total;
+    if (total > most) return 0;
+    return NC == 1 || clusters_resident(fn, NC, kClusterThreads, total) > 0 ? NC : 0;
 }
 
 template <typename MT>
 int launch_cluster(Ctx* ctx, HalpernWork* w, const b2p_params* p, int NC) {
-    cudaLaunchConfig_t lc{};
-    cudaLaunchAttribute dims;
-    dims.id = cudaLaunchAttributeClusterDimension;
-    dims.val.clusterDim.x = NC;
-    dims.val.clusterDim.y = dims.val.clusterDim.z = 1;
     const ClusterLay lay = cluster_lay<MT>(w, p->check_every, NC);
-    lc.gridDim = dim3(NC);
-    lc.blockDim = dim3(NC == 1 ? 1024 : kClusterThreads);
-    lc.dynamicSmemBytes = lay.total;
-    lc.stream = ctx->stream;
-    lc.attrs = &dims;
-    lc.numAttrs = 1;
+    cudaLaunchAttribute dims;
+    const cudaLaunchConfig_t lc = cluster_config(NC, NC, NC == 1 ? 1024 : kClusterThreads, lay.total, ctx->stream, &dims);
     IterArgs<MT, MT> pa = primal_args<MT>(w->ilp, w, p, false), da = dual_args<MT>(w->ilp, w, p, false);
     Sell &C = w->sc_all[0], &R = w->sr_all[0];
     pa.idx = C.idx.p;

@@ -673,6 +673,10 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
             if (lay.total <= max_smem) form = 3;
         }
     }
+    const auto small_fn = form == 1 ? k_ref_cluster<1, true>
+                                    : (form == 2 ? k_ref_cluster<kClusterCtas, true> : k_ref_cluster<kClusterCtas, false>);
+    if (form != 0) B2P_CUDA(ctx, open_smem(ctx, small_fn));
+    if (form > 1 && clusters_resident(small_fn, kClusterCtas, kClusterThreads, lay.total) < 1) form = 0;
     const bool small = form != 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -708,24 +712,13 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
     if (small) {
         B2P_CUDA(ctx, B.outcome.reserve(1));
         B2P_CUDA(ctx, cudaMemsetAsync(B.outcome.p, 0, sizeof(RefOutcome), s));
-        auto fn = form == 1 ? k_ref_cluster<1, true>
-                            : (form == 2 ? k_ref_cluster<kClusterCtas, true> : k_ref_cluster<kClusterCtas, false>);
-        B2P_CUDA(ctx, open_smem(ctx, fn));
-        cudaLaunchConfig_t lc{};
+        const int ctas = form == 1 ? 1 : kClusterCtas;
         cudaLaunchAttribute dims;
-        dims.id = cudaLaunchAttributeClusterDimension;
-        dims.val.clusterDim.x = form == 1 ? 1 : kClusterCtas;
-        dims.val.clusterDim.y = dims.val.clusterDim.z = 1;
-        lc.gridDim = dim3(form == 1 ? 1 : kClusterCtas);
-        lc.blockDim = dim3(kClusterThreads);
-        lc.dynamicSmemBytes = lay.total;
-        lc.stream = s;
-        lc.attrs = &dims;
-        lc.numAttrs = 1;
+        const cudaLaunchConfig_t lc = cluster_config(ctas, ctas, kClusterThreads, lay.total, s, &dims);
         // one launch runs up to 100,000 iterations (a fraction of a second)
         while (iter < max_it && !converged && !failed) {
             const int64_t stop = std::min<int64_t>(iter + 100000, max_it);
-            B2P_CUDA(ctx, cudaLaunchKernelEx(&lc, fn, m, n, A, At, (const double*)L.c.p, (const double*)L.lb.p,
+            B2P_CUDA(ctx, cudaLaunchKernelEx(&lc, small_fn, m, n, A, At, (const double*)L.c.p, (const double*)L.lb.p,
                                              (const double*)L.ub.p, (const double*)L.b.p, (const uint8_t*)L.is_eq.p, st, lay,
                                              (long long)stop, (long long)max_it, (long long)cf, p->feasibility_tolerance,
                                              B.outcome.p));
