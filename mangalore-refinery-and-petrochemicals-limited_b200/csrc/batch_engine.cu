@@ -1377,15 +1377,15 @@ __global__ void k_batch_power(int nmat, const int32_t* __restrict__ mat_m, const
 // holds whole copies of both vectors in shared memory, into which the owners post
 // (ClusterPost), and its share of the matrix where `room` bytes are left for it (4.6 us a
 // step on that matrix); otherwise the vectors lie in L2 (loads bypass L1, which other CTAs'
-// stores do not reach) and a cluster barrier ends each half step (9 us).  The kernel's
-// clusters loop over the matrices; every CTA of a cluster makes the same decisions from the
-// same sums.  Every step ends with a cluster barrier, so no thread falls a phase behind.
+// stores do not reach) and a cluster barrier ends each half step (9 us).  The `nbig`
+// matrices to take (`bigs`) are dealt to the kernel's clusters in turn: by their place among all
+// matrices, 36 large ones of 648 that lay 18 apart met on two clusters (upload 99 ms with one
+// CTA each, 239 ms; now 65).  Every CTA of a cluster makes the same decisions from the same sums.  Every step ends with a cluster barrier, so no thread falls a phase behind.
 template <bool SM>
 __global__ void __cluster_dims__(kPowerCtas, 1, 1) __launch_bounds__(512)
-k_batch_power_cluster(int nmat, const int32_t* __restrict__ mat_m, const int32_t* __restrict__ mat_n,
+k_batch_power_cluster(int nbig, const int32_t* __restrict__ bigs, const int32_t* __restrict__ mat_m, const int32_t* __restrict__ mat_n,
                       const int64_t* __restrict__ row_off, const int64_t* __restrict__ col_off,
-                      const int32_t* __restrict__ rowptr, const int64_t* __restrict__ rs_off,
-                      const int64_t* __restrict__ cs_off, const int64_t* __restrict__ r_sptr,
+                      const int64_t* __restrict__ rs_off, const int64_t* __restrict__ cs_off, const int64_t* __restrict__ r_sptr,
                       const int64_t* __restrict__ c_sptr, const uint16_t* __restrict__ r_eidx,
                       const uint16_t* __restrict__ c_eidx, const double* __restrict__ r_ev,
                       const double* __restrict__ c_ev, double* pv, double* pu, double safety, int max_m, int max_n,
@@ -1442,10 +1442,10 @@ k_batch_power_cluster(int nmat, const int32_t* __restrict__ mat_m, const int32_t
         }
         return s;
     };
-    for (int k = blockIdx.x / kPowerCtas; k < nmat; k += gridDim.x / kPowerCtas) {
+    for (int q = blockIdx.x / kPowerCtas; q < nbig; q += gridDim.x / kPowerCtas) {
+        const int k = bigs[q];
         const int m = mat_m[k], n = mat_n[k];
         const int64_t ro = row_off[k], co = col_off[k];
-        if (rowptr[ro + m] - rowptr[ro] < kPowerCluster) continue;
         const int64_t* rsp = r_sptr + rs_off[k];
         const int64_t* csp = c_sptr + cs_off[k];
         const int nrs = (m + 31) >> 5, ncs = (n + 31) >> 5;
@@ -2392,8 +2392,10 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
         w->max_n = std::max(w->max_n, mat_n[k]);
     }
     const int64_t nnz = mat_nnz_off[nmat];
-    int big = 0;  // matrices whose power iteration is worth a cluster
-    for (int k = 0; k < nmat; ++k) big += mat_nnz_off[k + 1] - mat_nnz_off[k] >= kPowerCluster;
+    std::vector<int32_t> bigs{0};  // the wait status of the cluster kernel, then the matrices worth a cluster
+    for (int k = 0; k < nmat; ++k)
+        if (mat_nnz_off[k + 1] - mat_nnz_off[k] >= kPowerCluster) bigs.push_back(k);
+    const int big = (int)bigs.size() - 1;
     if (nnz > INT32_MAX || tm > INT32_MAX || tn > INT32_MAX) {
         ctx->err = "b2p_batch_upload: batch exceeds 32-bit index range";
         return B2P_INVALID_ARGUMENT;
@@ -2606,8 +2608,9 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
     k_fill_ell<<<gmat, 256, 0, s>>>(1, nmat, w->mat_n.p, w->mat_col_off.p, w->mat_row_off.p, w->mat_cs_off.p, w->c_sptr.p,
                                      w->t_rowptr.p, w->t_colidx.p, w->stv64.p, w->stv32.p, w->c_eidx.p, w->c_ev64.p,
                                      w->c_ev32.p);
-    // clusters only while all big matrices' clusters are resident at once (two 512-thread CTAs
-    // per SM): 304 big matrices of 1,024 take 130 ms longer on clusters than one CTA each
+    // clusters for up to two large matrices per 8 SMs -- the L2 form's clusters are then resident at once,
+    // the shared-memory form's take two or three turns of a fifth of the time -- beyond that one CTA each
+    // fills the GPU as well: 304 large matrices of 1,024 take 130 ms longer on clusters
     const int clusters = 2 * ctx->sm_count / kPowerCtas;
     int max_smem = 0;
     B2P_CUDA(ctx, open_smem(ctx, k_batch_power_cluster<true>, &max_smem));
@@ -2615,24 +2618,22 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
     const int64_t vec = 8ll * ((int64_t)w->max_n + w->max_m + tabs);
     const bool sm = vec <= max_smem;  // both vectors fit a CTA's shared memory
     const auto power_fn = sm ? k_batch_power_cluster<true> : k_batch_power_cluster<false>;
-    const bool use_clusters =
-        big > 0 && big <= clusters && clusters_resident(power_fn, kPowerCtas, 512, sm ? max_smem : 0) > 0;
+    const int resident = big > 0 && big <= clusters ? clusters_resident(power_fn, kPowerCtas, 512, sm ? max_smem : 0) : 0;
+    const bool use_clusters = resident > 0;
     k_batch_power<<<gmat, 256, 0, s>>>(nmat, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->rowptr.p,
                                         w->colidx.p, w->sv64.p, w->t_rowptr.p, w->t_colidx.p, w->stv64.p, w->pv.p,
                                         w->pu.p, 0.998, use_clusters ? kPowerCluster : INT_MAX, w->mat_eta.p);
     int wait_failed = 0;
-    DBuf<int> failed;
+    DBuf<int32_t> dbigs;
     if (use_clusters) {
-        B2P_CUDA(ctx, failed.reserve(1));
-        B2P_CUDA(ctx, cudaMemsetAsync(failed.p, 0, sizeof(int), s));
-        // with the copies one CTA per SM is resident; the clusters loop over the matrices
-        const int grid = std::min(nmat, sm ? std::max(clusters / 2, 1) : clusters) * kPowerCtas;
-        power_fn<<<grid, 512, sm ? max_smem : 0, s>>>(
-            nmat, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->rowptr.p, w->mat_rs_off.p,
-            w->mat_cs_off.p, w->r_sptr.p, w->c_sptr.p, w->r_eidx.p, w->c_eidx.p, w->r_ev64.p, w->c_ev64.p, w->pv.p,
-            w->pu.p, 0.998, w->max_m, w->max_n, (int)(max_smem - vec), failed.p, w->mat_eta.p);
+        B2P_CUDA(ctx, dbigs.reserve(bigs.size()));
+        B2P_CUDA(ctx, cudaMemcpyAsync(dbigs.p, bigs.data(), sizeof(int32_t) * bigs.size(), cudaMemcpyHostToDevice, s));
+        power_fn<<<std::min(big, resident) * kPowerCtas, 512, sm ? max_smem : 0, s>>>(
+            big, dbigs.p + 1, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->mat_rs_off.p, w->mat_cs_off.p,
+            w->r_sptr.p, w->c_sptr.p, w->r_eidx.p, w->c_eidx.p, w->r_ev64.p, w->c_ev64.p, w->pv.p, w->pu.p, 0.998,
+            w->max_m, w->max_n, (int)(max_smem - vec), dbigs.p, w->mat_eta.p);
         ctx->launches += 1;
-        B2P_CUDA(ctx, cudaMemcpyAsync(&wait_failed, failed.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+        B2P_CUDA(ctx, cudaMemcpyAsync(&wait_failed, dbigs.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     }
     B2P_LAUNCH(ctx);
     ctx->launches += 5;
