@@ -278,7 +278,8 @@ int b2p_batch_upload(void* ctx, int nmat, const int32_t* mat_m, const int32_t* m
  * used_average = 10 * instances per CTA (2 or 4: batches whose instances share
  * one matrix) + SELL entries per lane load.  The shape is tuned
  * once per batch signature and cached in the file B2P_AUTOTUNE_CACHE (default
- * ~/.cache/b2p_autotune.txt); B2P_BATCH_SHAPE="threads,w,ni" pins it. */
+ * ~/.cache/b2p_autotune.txt); B2P_BATCH_SHAPE="threads,w,ni" pins it for the
+ * whole solve. */
 int b2p_batch_solve(void* ctx, const b2p_params* params, const double* x0, const double* y0, const double* omega0,
                     int32_t* status_out, int64_t* iters_out, double* kkt_out, double* omega_out, double* x_out,
                     double* y_out, b2p_result* summary);

@@ -93,6 +93,7 @@ struct TuneCfg {
     // of one round of resident CTAs
     int form_th[3] = {0, 0, 0};
     double form_us[3] = {0, 0, 0};
+    bool pinned = false;  // B2P_BATCH_SHAPE named the shape: no other form runs
 };
 constexpr int kFormNi[3] = {1, 2, 4};
 
@@ -1729,8 +1730,8 @@ __global__ void k_batch_unscale(BArgs a, int count, const double* __restrict__ x
 
 // Candidate shapes of the autotuner: CTA sizes, SELL entry orders and instances per CTA
 // (more than 1 only when every instance shares one matrix; 4 only in FP32).
-// B2P_BATCH_SHAPE="threads,w,ni" pins all three (the chunk length is still tuned); a pinned
-// group on a batch of several matrices falls back to one instance per CTA.
+// B2P_BATCH_SHAPE="threads,w,ni" pins all three for the whole solve (the chunk length is still
+// tuned); a pinned group on a batch of several matrices falls back to one instance per CTA.
 struct ShapeChoices {
     std::vector<int> threads{128, 256, 512}, w{1, 2}, ni{1, 2, 4};
     bool pinned = false;
@@ -2085,6 +2086,7 @@ int batch_run(Ctx* ctx, BatchWork* w, const b2p_params* p, const double* x0_dev,
         }
         int st = autotune<MT>(ctx, w, p, &cfg);
         if (st) return st;
+        cfg.pinned = shape_choices(w).pinned;
         w->tuned[prec] = true;
         w->tuned_cfg[prec] = cfg;
     }
@@ -2142,7 +2144,8 @@ int batch_run(Ctx* ctx, BatchWork* w, const b2p_params* p, const double* x0_dev,
     BArgs a2 = make_args<MT>(w, p, w->active2.p);
     // The forms of this solve: the tuned ones by instances per CTA, and for the tail, when no
     // more than one instance per SM is left, one CTA per SM as wide as the largest instance has
-    // rows or columns to occupy.
+    // rows or columns to occupy.  A pinned shape is the only one: the tail form adds the FP64 sums of a
+    // check in another order, and where a solve goes over to it depends on the chunk.
     struct Form {
         void (*fn)(const BArgs, int) = nullptr;
         int ni = 1, threads = 0, slots = 0;  // instances per CTA, CTA size, resident CTAs
@@ -2186,7 +2189,7 @@ int batch_run(Ctx* ctx, BatchWork* w, const b2p_params* p, const double* x0_dev,
             int st = open_form(own.form[f], kFormNi[f], cfg.form_th[f], cfg.form_us[f]);
             if (st) return st;
         }
-    {
+    if (!cfg.pinned) {
         int st = open_form(own.form[3], 1, tail_threads(w), 0.0);
         if (st) return st;
     }
