@@ -47,6 +47,7 @@
 
 #include <atomic>
 #include <cmath>
+#include <type_traits>
 #include <cstring>
 #include <algorithm>
 
@@ -106,6 +107,9 @@ struct Sell {
     DBuf<float> v32;     // total (mixed engine)
     DBuf<double> v64;    // total (FP64 engine)
     std::vector<int64_t> h_off;  // host copy of off
+    int limit = INT_MAX;         // rows with more entries are not in the copy (empty there) but in `longs`
+    int nlong = 0;
+    DBuf<int32_t> longs;
     bool idx_ready = false;
 };
 
@@ -262,6 +266,61 @@ __device__ __forceinline__ void sell_pair_dot(const int64_t* __restrict__ off, c
         for (int o = C; o < 32; o <<= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
 }
 
+// The rows that a check copy leaves out (Sell::longs), over the CSR arrays of their orientation.
+struct LongRows {
+    const int32_t* ids;
+    int count, limit;
+    const int32_t *ptr, *idx;
+    const double* val;
+    __device__ __forceinline__ bool has(int r) const { return ptr[r + 1] - ptr[r] > limit; }
+};
+
+// Sum of one long row by the whole CTA, for the vectors g (and gd, optional); every thread must call
+// it, thread 0 returns the sums.  Out of line: no registers of the slice loops.
+template <typename GT>
+__device__ __noinline__ double2 long_row_dot(const LongRows& lr, int r, const GT* __restrict__ g,
+                                             const double* __restrict__ gd) {
+    constexpr int U = 8;
+    __shared__ double sh[2][32];
+    const int e1 = lr.ptr[r + 1], nt = blockDim.x;
+    double s = 0.0, sd = 0.0;
+    for (int64_t e = (int64_t)lr.ptr[r] + threadIdx.x; e < e1; e += U * nt) {
+        double v[U], a[U];
+        int c[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool h = e + u * nt < e1;
+            v[u] = h ? lr.val[e + u * nt] : 0.0;
+            c[u] = h ? lr.idx[e + u * nt] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) a[u] = c[u] >= 0 ? (double)g[c[u]] : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) s += v[u] * a[u];
+        if (gd) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) a[u] = c[u] >= 0 ? gd[c[u]] : 0.0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) sd += v[u] * a[u];
+        }
+    }
+    s = warp_sum(s);
+    sd = warp_sum(sd);
+    __syncthreads();  // the sums of the row before this one have been read
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][threadIdx.x >> 5] = s;
+        sh[1][threadIdx.x >> 5] = sd;
+    }
+    __syncthreads();
+    double2 t = make_double2(0.0, 0.0);
+    if (threadIdx.x == 0)
+        for (int i = 0; i < (nt >> 5); ++i) {
+            t.x += sh[0][i];
+            t.y += sh[1][i];
+        }
+    return t;
+}
+
 // ------------------------------------------------------------------ scaling (FP64, setup)
 __global__ void k_fill(int64_t n, double v, double* __restrict__ a) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) a[i] = v;
@@ -325,39 +384,54 @@ __global__ void k_scale_vecs(int m, int n, const double* __restrict__ b, const d
 // before -> now: 100k x 400k, 4.0M nonzeros, power rows 45 -> 22, columns 25 -> 19; 204k x 1M,
 // 8.0M nonzeros, FP32 iterates with certificates, KKT rows 153 -> 64, columns 190 -> 54.  What is
 // left is the gathers: one L1 lookup per entry and SM cycle is 14 us for 4.0M of them.
+// Rows far longer than the others (check_limit) are not in the copy, where one would stall its warp
+// and pad its slice: whole CTAs take them first, over the CSR arrays (LongRows).
 // One step: u = A_s v / ||v||, w = A_s^T u, ||w||^2 -> nrm2[t + 1] (nrm2[t] holds ||v||^2, so
 // ||w|| estimates sigma_max^2).  Both run over the check copies, one warp per slice.
-template <int C>
+template <int C, bool LONG>
 __global__ void __launch_bounds__(256) k_pow_rows(int m, const int64_t* __restrict__ off, const int32_t* __restrict__ idx,
                                                   const double* __restrict__ val, const double* __restrict__ v,
-                                                  const double* __restrict__ nrm2, double* __restrict__ u) {
+                                                  const double* __restrict__ nrm2, double* __restrict__ u,
+                                                  const LongRows lr) {
     pdl_wait();
     pdl_trigger();
     const double nn = sqrt(*nrm2), inv = 1.0 / (nn > 0 ? nn : 1.0);
+    for (int q = blockIdx.x; LONG && q < lr.count; q += gridDim.x) {
+        const double2 t = long_row_dot<double>(lr, lr.ids[q], v, nullptr);
+        if (threadIdx.x == 0) u[lr.ids[q]] = t.x * inv;
+    }
     const int lane = threadIdx.x & 31, nsl = (m + C - 1) / C;
     for (int sl = blockIdx.x * 8 + (threadIdx.x >> 5); sl < nsl; sl += gridDim.x * 8) {
         double s[1];
         const double* g[1] = {v};
         sell_pair_dot<C, 1>(off, idx, val, sl, lane, g, s);
         const int i = sl * C + lane;
-        if (lane < C && i < m) u[i] = s[0] * inv;
+        if (lane < C && i < m && !(LONG && lr.has(i))) u[i] = s[0] * inv;
     }
 }
 
-template <int C>
+template <int C, bool LONG>
 __global__ void __launch_bounds__(256) k_pow_cols(int n, const int64_t* __restrict__ off, const int32_t* __restrict__ idx,
                                                   const double* __restrict__ val, const double* __restrict__ u,
-                                                  double* __restrict__ w, double* __restrict__ nrm2) {
+                                                  double* __restrict__ w, double* __restrict__ nrm2,
+                                                  const LongRows lr) {
     double part = 0.0;
     pdl_wait();
     pdl_trigger();
+    for (int q = blockIdx.x; LONG && q < lr.count; q += gridDim.x) {
+        const double2 t = long_row_dot<double>(lr, lr.ids[q], u, nullptr);
+        if (threadIdx.x == 0) {
+            w[lr.ids[q]] = t.x;
+            part += t.x * t.x;
+        }
+    }
     const int lane = threadIdx.x & 31, nsl = (n + C - 1) / C;
     for (int sl = blockIdx.x * 8 + (threadIdx.x >> 5); sl < nsl; sl += gridDim.x * 8) {
         double s[1];
         const double* g[1] = {u};
         sell_pair_dot<C, 1>(off, idx, val, sl, lane, g, s);
         const int j = sl * C + lane;
-        if (lane < C && j < n) {
+        if (lane < C && j < n && !(LONG && lr.has(j))) {
             w[j] = s[0];
             part += s[0] * s[0];
         }
@@ -1099,12 +1173,18 @@ __global__ void k_scatter_perm(int rows, const int32_t* __restrict__ perm, const
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) dst[perm[i]] = src[i];
 }
 
-// longest row of every C-row slice
-__global__ void k_slice_len(int rows, const int32_t* __restrict__ ptr, int C, int32_t* __restrict__ slen) {
+// longest row of every C-row slice among those of at most `limit` entries; the others into `longs`,
+// their number into slen[number of slices] (zeroed by the caller)
+__global__ void k_slice_len(int rows, const int32_t* __restrict__ ptr, int C, int limit, int32_t* __restrict__ slen,
+                            int32_t* __restrict__ longs) {
     const int nsl = (rows + C - 1) / C;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nsl; s += gridDim.x * blockDim.x) {
         int mx = 0;
-        for (int r = s * C; r < min(rows, s * C + C); ++r) mx = max(mx, ptr[r + 1] - ptr[r]);
+        for (int r = s * C; r < min(rows, s * C + C); ++r) {
+            const int len = ptr[r + 1] - ptr[r];
+            if (len <= limit) mx = max(mx, len);
+            else longs[atomicAdd(slen + nsl, 1)] = r;
+        }
         slen[s] = mx;
     }
 }
@@ -1118,9 +1198,9 @@ __device__ __forceinline__ int64_t sell_pos(const int64_t* off, int W, int C, in
 // slice's first, longest row), so padding stays inside the row's neighbourhood of the
 // gathered vector (its value is 0)
 __global__ void k_sell_idx(int rows, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                           const int64_t* __restrict__ off, int W, int C, int32_t* __restrict__ sidx) {
+                           const int64_t* __restrict__ off, int W, int C, int limit, int32_t* __restrict__ sidx) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
-        const int k0 = ptr[i], len = ptr[i + 1] - k0;
+        const int k0 = ptr[i], len = ptr[i + 1] - k0 <= limit ? ptr[i + 1] - k0 : 0;
         const int s = i / C;
         const int plen = (int)((off[s + 1] - off[s]) / C);
         for (int e = 0; e < len; ++e) sidx[sell_pos(off, W, C, i, e)] = idx[k0 + e];
@@ -1169,9 +1249,10 @@ __global__ void k_win_setup(int rows, const int32_t* __restrict__ ptr, const int
 
 template <typename VT>
 __global__ void k_sell_vals(int rows, const int32_t* __restrict__ ptr, const double* __restrict__ v64,
-                            const int64_t* __restrict__ off, int W, int C, VT* __restrict__ sval) {
+                            const int64_t* __restrict__ off, int W, int C, int limit, VT* __restrict__ sval) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
         const int k0 = ptr[i], len = ptr[i + 1] - k0;
+        if (len > limit) continue;
         for (int e = 0; e < len; ++e) sval[sell_pos(off, W, C, i, e)] = (VT)v64[k0 + e];
     }
 }
@@ -1192,18 +1273,41 @@ struct KktMap {
 // rows: primal residual, b.y, the objective-error sum |y| viol; with xd / yd (the
 // displacement T(z) - z), A xd for the primal ray and the row terms of the dual ray.  Both
 // kernels run over the FP64 check copies, one warp per slice (lane < C: one row each).
-template <int C, typename ZT>
+template <int C, bool LONG, typename ZT>
 __global__ void __launch_bounds__(TB) k_kkt_rows(int m, const int64_t* __restrict__ off, const int32_t* __restrict__ idx,
                                                  const double* __restrict__ val, const ZT* __restrict__ xt,
                                                  const ZT* __restrict__ yt, const double* __restrict__ b,
                                                  const uint8_t* __restrict__ is_eq, const double* __restrict__ dr,
                                                  KktMap map, const double* __restrict__ xd,
-                                                 const double* __restrict__ yd, Ctrl* ctrl) {
+                                                 const double* __restrict__ yd, Ctrl* ctrl, const LongRows lr) {
     if (ctrl->done) return;
     const double ps = ctrl->pscale, ds = ctrl->dscale;
     const int lane = threadIdx.x & 31, nsl = (m + C - 1) / C;
     const bool rays = xd != nullptr;
     double a[7] = {0, 0, 0, 0, 0, 0, 0};  // |rp|^2, b.y, sum |y| viol, y < 0, |A dx viol|^2, b.dy, sum |b dy|
+    auto terms = [&](int r, double s, double sd) {
+        const bool eq = is_eq[r] != 0;
+        double ax = (map.axbar ? map.axbar[r] : 0.0) + ps * (s / dr[r]);
+        double rp = ax - b[r];
+        if (!eq) rp = fmax(rp, 0.0);
+        a[0] += rp * rp;
+        const double yv = (map.ybar ? map.ybar[r] : 0.0) + ds * (dr[r] * (double)yt[r]);
+        a[1] += b[r] * yv;
+        a[2] += fabs(yv) * fabs(rp);
+        if (!eq && yv < 0.0) a[3] += yv * yv;  // y >= 0 on <= rows: part of the dual residual
+        if (rays) {
+            const double adx = sd / dr[r];  // (A dx)_r, original space
+            const double v = eq ? adx : fmax(adx, 0.0);
+            a[4] += v * v;
+            const double dyo = dr[r] * yd[r];
+            a[5] += b[r] * dyo;
+            a[6] += fabs(b[r] * dyo);
+        }
+    };
+    for (int q = blockIdx.x; LONG && q < lr.count; q += gridDim.x) {
+        const double2 t = long_row_dot<ZT>(lr, lr.ids[q], xt, xd);
+        if (threadIdx.x == 0) terms(lr.ids[q], t.x, t.y);
+    }
     for (int sl = blockIdx.x * (TB / 32) + (threadIdx.x >> 5); sl < nsl; sl += gridDim.x * (TB / 32)) {
         double s[1], sd[1] = {0.0};
         const ZT* g[1] = {xt};
@@ -1213,24 +1317,7 @@ __global__ void __launch_bounds__(TB) k_kkt_rows(int m, const int64_t* __restric
             sell_pair_dot<C, 1>(off, idx, val, sl, lane, gd, sd);
         }
         const int r = sl * C + lane;
-        if (lane >= C || r >= m) continue;
-        const bool eq = is_eq[r] != 0;
-        double ax = (map.axbar ? map.axbar[r] : 0.0) + ps * (s[0] / dr[r]);
-        double rp = ax - b[r];
-        if (!eq) rp = fmax(rp, 0.0);
-        a[0] += rp * rp;
-        const double yv = (map.ybar ? map.ybar[r] : 0.0) + ds * (dr[r] * (double)yt[r]);
-        a[1] += b[r] * yv;
-        a[2] += fabs(yv) * fabs(rp);
-        if (!eq && yv < 0.0) a[3] += yv * yv;  // y >= 0 on <= rows: part of the dual residual
-        if (rays) {
-            const double adx = sd[0] / dr[r];  // (A dx)_r, original space
-            const double v = eq ? adx : fmax(adx, 0.0);
-            a[4] += v * v;
-            const double dyo = dr[r] * yd[r];
-            a[5] += b[r] * dyo;
-            a[6] += fabs(b[r] * dyo);
-        }
+        if (lane < C && r < m && !(LONG && lr.has(r))) terms(r, s[0], sd[0]);
     }
     double* const slots[7] = {&ctrl->acc[A_PRES2], &ctrl->acc[A_BY],  &ctrl->acc[A_EST], &ctrl->acc[A_DRES2],
                               &ctrl->acc[A_PRV2],  &ctrl->acc[A_DRB], &ctrl->acc[A_DRM]};
@@ -1239,32 +1326,23 @@ __global__ void __launch_bounds__(TB) k_kkt_rows(int m, const int64_t* __restric
 
 // columns: reduced cost g = c + A^T y, bound multipliers lambda, dual residual, c.x and the bound
 // terms; with xd / yd, the column terms of the primal ray and A^T yd for the dual ray
-template <int C, typename ZT>
+template <int C, bool LONG, typename ZT>
 __global__ void __launch_bounds__(TB) k_kkt_cols(int n, const int64_t* __restrict__ off, const int32_t* __restrict__ idx,
                                                  const double* __restrict__ val, const ZT* __restrict__ yt,
                                                  const ZT* __restrict__ xt, const double* __restrict__ c,
                                                  const double* __restrict__ lb, const double* __restrict__ ub,
                                                  const double* __restrict__ dc, KktMap map,
                                                  const double* __restrict__ xd, const double* __restrict__ yd,
-                                                 Ctrl* ctrl) {
+                                                 Ctrl* ctrl, const LongRows lr) {
     if (ctrl->done) return;
     const double ps = ctrl->pscale, ds = ctrl->dscale;
     const int lane = threadIdx.x & 31, nsl = (n + C - 1) / C;
     const bool rays = yd != nullptr;
     // |rd|^2, c.x, bound term, |dx recession viol|^2, c.dx, sum |c dx|, bound term of A^T dy, sum |terms|, |viol|^2
     double a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int sl = blockIdx.x * (TB / 32) + (threadIdx.x >> 5); sl < nsl; sl += gridDim.x * (TB / 32)) {
-        double s[1], sd[1] = {0.0};
-        const ZT* g1[1] = {yt};
-        sell_pair_dot<C, 1>(off, idx, val, sl, lane, g1, s);
-        if (rays) {
-            const double* gd[1] = {yd};
-            sell_pair_dot<C, 1>(off, idx, val, sl, lane, gd, sd);
-        }
-        const int j = sl * C + lane;
-        if (lane >= C || j >= n) continue;
+    auto terms = [&](int j, double s, double sd) {
         const double cj = c[j], lj = lb[j], uj = ub[j], dcj = dc[j];
-        double g = cj + (map.atybar ? map.atybar[j] : 0.0) + ds * (s[0] / dcj);
+        double g = cj + (map.atybar ? map.atybar[j] : 0.0) + ds * (s / dcj);
         const bool fl = isfinite(lj), fu = isfinite(uj);
         double lam = (fl && fu) ? g : (fl ? fmax(g, 0.0) : (fu ? fmin(g, 0.0) : 0.0));
         double rd = g - lam;
@@ -1279,13 +1357,28 @@ __global__ void __launch_bounds__(TB) k_kkt_cols(int n, const int64_t* __restric
             a[5] += fabs(cj * dxo);
             const double bv = (fl && dxo < 0.0 ? -dxo : 0.0) + (fu && dxo > 0.0 ? dxo : 0.0);
             a[3] += bv * bv;
-            const double at = sd[0] / dcj;  // (A^T dy)_j, original space
+            const double at = sd / dcj;  // (A^T dy)_j, original space
             const double t = at > 0.0 ? (fl ? at * lj : 0.0) : (at < 0.0 ? (fu ? at * uj : 0.0) : 0.0);
             a[6] += t;
             a[7] += fabs(t);
             const double av = (!fl && at > 0.0 ? at : 0.0) + (!fu && at < 0.0 ? -at : 0.0);
             a[8] += av * av;
         }
+    };
+    for (int q = blockIdx.x; LONG && q < lr.count; q += gridDim.x) {
+        const double2 t = long_row_dot<ZT>(lr, lr.ids[q], yt, yd);
+        if (threadIdx.x == 0) terms(lr.ids[q], t.x, t.y);
+    }
+    for (int sl = blockIdx.x * (TB / 32) + (threadIdx.x >> 5); sl < nsl; sl += gridDim.x * (TB / 32)) {
+        double s[1], sd[1] = {0.0};
+        const ZT* g1[1] = {yt};
+        sell_pair_dot<C, 1>(off, idx, val, sl, lane, g1, s);
+        if (rays) {
+            const double* gd[1] = {yd};
+            sell_pair_dot<C, 1>(off, idx, val, sl, lane, gd, sd);
+        }
+        const int j = sl * C + lane;
+        if (lane < C && j < n && !(LONG && lr.has(j))) terms(j, s[0], sd[0]);
     }
     double* const slots[9] = {&ctrl->acc[A_DRES2], &ctrl->acc[A_PC],  &ctrl->acc[A_LAM],
                               &ctrl->acc[A_PRV2],  &ctrl->acc[A_PRC], &ctrl->acc[A_PRM],
@@ -1488,6 +1581,30 @@ void launch_iter(int mode, int L, int R, unsigned grid, int tb, cudaStream_t s, 
 // CTAs of a kernel over the slices of a check copy, one warp each, at most one resident wave
 unsigned slice_grid(const Sell& S, int sm_count) { return grid_for(S.slices * 32, TB, sm_count, 8); }
 
+// The rows (columns) that the check copies leave out.
+LongRows long_rows(HalpernWork* w, bool rows) {
+    const Sell& S = rows ? w->kr : w->kc;
+    const DevLP& L = w->ilp;
+    if (rows) return {S.longs.p, S.nlong, S.limit, L.rowptr.p, L.colidx.p, w->sv64.p};
+    return {S.longs.p, S.nlong, S.limit, L.t_rowptr.p, L.t_colidx.p, w->stv64.p};
+}
+// Entries from which a row (column) of a check copy counts as long: far more than the others have, so
+// that few are, and more than a warp passes in the time of a short launch.
+int check_limit(double mean_len) { return (int)std::max(256.0, std::min(16.0 * mean_len, 1e9)); }
+
+// f with the slice height of a check copy and whether it leaves rows out (kernels without that code
+// keep their registers).
+template <typename F>
+void with_form(const Sell& S, F f) {
+    const auto height = [&](auto lng) {
+        if (S.C == 32) f(std::integral_constant<int, 32>(), lng);
+        else if (S.C == 16) f(std::integral_constant<int, 16>(), lng);
+        else f(std::integral_constant<int, 8>(), lng);
+    };
+    if (S.nlong > 0) height(std::true_type());
+    else height(std::false_type());
+}
+
 template <typename MT>
 void launch_kkt(Ctx* ctx, const DevLP& lp, HalpernWork* w, const KktMap& map, Ctrl* ctrl) {
     cudaStream_t s = ctx->stream;
@@ -1496,20 +1613,17 @@ void launch_kkt(Ctx* ctx, const DevLP& lp, HalpernWork* w, const KktMap& map, Ct
     const MT* xt = (const MT*)w->xt.p;
     const MT* yt = (const MT*)w->yt.p;
     const unsigned gr = slice_grid(w->kr, ctx->sm_count), gc = slice_grid(w->kc, ctx->sm_count);
+    const LongRows lr = long_rows(w, true), lc = long_rows(w, false);
     auto rows = [&](auto fn) {
         fn<<<gr, TB, 0, s>>>(lp.m, w->kr.off.p, w->kr.idx.p, w->kr.v64.p, xt, yt, lp.b.p, lp.is_eq.p, w->dr.p, map, xd, yd,
-                             ctrl);
+                             ctrl, lr);
     };
     auto cols = [&](auto fn) {
         fn<<<gc, TB, 0, s>>>(lp.n, w->kc.off.p, w->kc.idx.p, w->kc.v64.p, yt, xt, lp.c.p, lp.lb.p, lp.ub.p, w->dc.p, map, xd,
-                             yd, ctrl);
+                             yd, ctrl, lc);
     };
-    if (w->kr.C == 32) rows(k_kkt_rows<32, MT>);
-    else if (w->kr.C == 16) rows(k_kkt_rows<16, MT>);
-    else rows(k_kkt_rows<8, MT>);
-    if (w->kc.C == 32) cols(k_kkt_cols<32, MT>);
-    else if (w->kc.C == 16) cols(k_kkt_cols<16, MT>);
-    else cols(k_kkt_cols<8, MT>);
+    with_form(w->kr, [&](auto c, auto lng) { rows(k_kkt_rows<decltype(c)::value, decltype(lng)::value, MT>); });
+    with_form(w->kc, [&](auto c, auto lng) { cols(k_kkt_cols<decltype(c)::value, decltype(lng)::value, MT>); });
 }
 
 // Scaling, scaled copies and ||A_s||_2 (FP64, once per uploaded LP and ruiz count).
@@ -1550,6 +1664,7 @@ int power_sigma2(Ctx* ctx, HalpernWork* w, double* sigma2) {
     cudaStream_t s = ctx->stream;
     const int m = L.m, n = L.n;
     const unsigned gr = slice_grid(w->kr, ctx->sm_count), gc = slice_grid(w->kc, ctx->sm_count);
+    const LongRows lr = long_rows(w, true), lc = long_rows(w, false);
     const int kMax = 512, kRound = 16;
     double* nrm2 = w->pw.p;  // [t]: the squared norm of the vector step t starts from
     B2P_CUDA(ctx, cudaMemsetAsync(nrm2, 0, sizeof(double) * (kMax + 1), s));
@@ -1557,20 +1672,16 @@ int power_sigma2(Ctx* ctx, HalpernWork* w, double* sigma2) {
     B2P_LAUNCH(ctx);
     ctx->launches += 1;
     auto rows = [&](auto fn, int t) {
-        pdl_launch(fn, gr, TB, 0, s, m, w->kr.off.p, w->kr.idx.p, w->kr.v64.p, w->pv.p, nrm2 + t, w->pu.p);
+        pdl_launch(fn, gr, TB, 0, s, m, w->kr.off.p, w->kr.idx.p, w->kr.v64.p, w->pv.p, nrm2 + t, w->pu.p, lr);
     };
     auto cols = [&](auto fn, int t) {
-        pdl_launch(fn, gc, TB, 0, s, n, w->kc.off.p, w->kc.idx.p, w->kc.v64.p, w->pu.p, w->pv.p, nrm2 + t + 1);
+        pdl_launch(fn, gc, TB, 0, s, n, w->kc.off.p, w->kc.idx.p, w->kc.v64.p, w->pu.p, w->pv.p, nrm2 + t + 1, lc);
     };
     double est = 0.0;
     for (int t = 0; t < kMax; t += kRound) {
         for (int q = t; q < t + kRound; ++q) {
-            if (w->kr.C == 32) rows(k_pow_rows<32>, q);
-            else if (w->kr.C == 16) rows(k_pow_rows<16>, q);
-            else rows(k_pow_rows<8>, q);
-            if (w->kc.C == 32) cols(k_pow_cols<32>, q);
-            else if (w->kc.C == 16) cols(k_pow_cols<16>, q);
-            else cols(k_pow_cols<8>, q);
+            with_form(w->kr, [&](auto c, auto lng) { rows(k_pow_rows<decltype(c)::value, decltype(lng)::value>, q); });
+            with_form(w->kc, [&](auto c, auto lng) { cols(k_pow_cols<decltype(c)::value, decltype(lng)::value>, q); });
         }
         B2P_LAUNCH(ctx);
         ctx->launches += 2 * kRound;
@@ -1685,17 +1796,23 @@ int build_internal(Ctx* ctx, HalpernWork* w) {
 
 // Slice layout and indices of a SELL copy (once per upload): vector width W = 4 or 2
 // when its padding costs at most 3 % over W = 1, which pads only to each slice's
-// longest row.
-int build_sell_layout(Ctx* ctx, Sell& S, int rows, const int32_t* ptr, const int32_t* idx, int C, int force_W = 0) {
+// longest row.  Rows of more than `limit` entries (nnz: of all rows) are listed instead.
+int build_sell_layout(Ctx* ctx, Sell& S, int rows, const int32_t* ptr, const int32_t* idx, int C, int force_W = 0,
+                      int limit = INT_MAX, int64_t nnz = 0) {
     cudaStream_t s = ctx->stream;
     const int nsl = (rows + C - 1) / C;
     DBuf<int32_t> slen;
-    B2P_CUDA(ctx, slen.reserve(nsl));
-    k_slice_len<<<grid_for(nsl, TB, ctx->sm_count), TB, 0, s>>>(rows, ptr, C, slen.p);
+    B2P_CUDA(ctx, slen.reserve(nsl + 1));
+    B2P_CUDA(ctx, cudaMemsetAsync(slen.p + nsl, 0, sizeof(int32_t), s));
+    if (limit < INT_MAX) B2P_CUDA(ctx, S.longs.reserve(nnz / limit + 1));
+    k_slice_len<<<grid_for(nsl, TB, ctx->sm_count), TB, 0, s>>>(rows, ptr, C, limit, slen.p, S.longs.p);
     B2P_LAUNCH(ctx);
-    std::vector<int32_t> h(nsl);
-    B2P_CUDA(ctx, cudaMemcpyAsync(h.data(), slen.p, sizeof(int32_t) * nsl, cudaMemcpyDeviceToHost, s));
+    std::vector<int32_t> h(nsl + 1);
+    B2P_CUDA(ctx, cudaMemcpyAsync(h.data(), slen.p, sizeof(int32_t) * (nsl + 1), cudaMemcpyDeviceToHost, s));
     B2P_CUDA(ctx, cudaStreamSynchronize(s));
+    S.limit = limit;
+    S.nlong = h[nsl];
+    h.pop_back();
     auto padded_total = [&](int W) {
         int64_t t = 0;
         for (int v : h) t += (int64_t)C * ((v + W - 1) / W * W);
@@ -1718,7 +1835,7 @@ int build_sell_layout(Ctx* ctx, Sell& S, int rows, const int32_t* ptr, const int
     B2P_CUDA(ctx, S.idx.reserve(std::max<int64_t>(S.total, 1)));
     B2P_CUDA(ctx, cudaMemcpyAsync(S.off.p, off.data(), sizeof(int64_t) * (nsl + 1), cudaMemcpyHostToDevice, s));
     B2P_CUDA(ctx, cudaMemsetAsync(S.idx.p, 0, sizeof(int32_t) * std::max<int64_t>(S.total, 1), s));
-    k_sell_idx<<<grid_for(rows, TB, ctx->sm_count), TB, 0, s>>>(rows, ptr, idx, S.off.p, W, C, S.idx.p);
+    k_sell_idx<<<grid_for(rows, TB, ctx->sm_count), TB, 0, s>>>(rows, ptr, idx, S.off.p, W, C, limit, S.idx.p);
     B2P_LAUNCH(ctx);
     ctx->launches += 2;
     B2P_CUDA(ctx, cudaStreamSynchronize(s));  // slen is freed on return, h / off are host temporaries
@@ -1736,7 +1853,7 @@ int fill_sell_vals(Ctx* ctx, Sell& S, int rows, const int32_t* ptr, const double
     const bool fresh = out.p == nullptr;
     B2P_CUDA(ctx, out.reserve(std::max<int64_t>(S.total, 1)));
     if (fresh) B2P_CUDA(ctx, cudaMemsetAsync(out.p, 0, sizeof(VT) * std::max<int64_t>(S.total, 1), s));
-    k_sell_vals<VT><<<grid_for(rows, TB, ctx->sm_count), TB, 0, s>>>(rows, ptr, v64, S.off.p, S.W, S.C, out.p);
+    k_sell_vals<VT><<<grid_for(rows, TB, ctx->sm_count), TB, 0, s>>>(rows, ptr, v64, S.off.p, S.W, S.C, S.limit, out.p);
     B2P_LAUNCH(ctx);
     ctx->launches += 1;
     return B2P_OK;
@@ -2010,11 +2127,33 @@ int autotune_shapes(Ctx* ctx, HalpernWork* w, const b2p_params* p) {
         int bestL = base_L, bestR = 1, bestT = 256, bestWin = -1, bestK = 0;
         bool bestS = false;
         float last = 1e30f;  // time of the last trial
-        // the other side's kernel: the dual's plain form while the primal is tuned, then the tuned primal
+        // the other side's kernel: the dual's plain SELL form while the primal is tuned (its CSR form where
+        // that takes less than a quarter of the time: a dense row stalls a slice), then the tuned primal
         if (primal) w->sr = &w->sr_all[0];
-        const IterArgs<MT, MT> oa = primal ? dual_args<MT>(L, w, p, true) : primal_args<MT>(L, w, p, w->sell_c);
+        bool plain_sell = true;
+        if (primal) {
+            const int Lr = pick_lanes(L.mean_row_len, 0);
+            float ms[2] = {0.f, 0.f};
+            for (int burst = 0; burst < 2; ++burst)  // the first one warms caches
+                for (int csr = 0; csr < 2; ++csr) {
+                    cudaEventRecord(e0, s);
+                    const IterArgs<MT, MT> da = dual_args<MT>(L, w, p, !csr);
+                    if (csr) launch_iter<MT, MT, false>(M_PLAIN, Lr, 1, iter_grid(m, Lr, 1, 256, ctx->sm_count), 256, s, da, 0);
+                    else launch_sell<MT, MT, false>(M_PLAIN, w->sr_all[0], iter_grid(m, 1, 1, 256, ctx->sm_count), 256, 0, s, da, 0);
+                    cudaEventRecord(e1, s);
+                    B2P_LAUNCH(ctx);
+                    B2P_CUDA(ctx, cudaEventSynchronize(e1));
+                    cudaEventElapsedTime(&ms[csr], e0, e1);
+                }
+            ctx->launches += 4;
+            plain_sell = ms[0] <= 4.0f * ms[1];
+        }
+        const IterArgs<MT, MT> oa = primal ? dual_args<MT>(L, w, p, plain_sell) : primal_args<MT>(L, w, p, w->sell_c);
         auto other = [&](int rep) {
-            if (primal)
+            if (primal && !plain_sell) {
+                const int Lr = pick_lanes(L.mean_row_len, 0);
+                launch_iter<MT, MT, false>(M_PLAIN, Lr, 1, iter_grid(m, Lr, 1, 256, ctx->sm_count), 256, s, oa, rep);
+            } else if (primal)
                 launch_sell<MT, MT, false>(M_PLAIN, w->sr_all[0], iter_grid(m, 1, 1, 256, ctx->sm_count), 256, 0, s, oa, rep);
             else if (w->sell_c)
                 launch_sell<MT, MT, true>(M_PLAIN, *w->sc,
@@ -2047,9 +2186,13 @@ int autotune_shapes(Ctx* ctx, HalpernWork* w, const b2p_params* p) {
             }
             float tot = 1e30f;
             const IterArgs<MT, MT> mine = primal ? primal_args<MT>(L, w, p, kind != 0) : dual_args<MT>(L, w, p, kind != 0);
+            // a candidate that takes eight times the best's time in its first burst and again alone is
+            // given up (a dense row: 70 ms an iteration in one form, 4 in another)
+            bool behind = false;
             for (int burst = 0; burst < 3; ++burst) {  // the first one warms caches
+                const int reps = burst && !behind ? 4 : 1;
                 cudaEventRecord(e0, s);
-                for (int rep = 0; rep < (burst ? 4 : 1); ++rep) {
+                for (int rep = 0; rep < reps; ++rep) {
                     if (!primal) other(rep);
                     if (kind != 0 && primal) launch_sell<MT, MT, true>(M_PLAIN, **cur, g, tb, smem, s, mine, rep);
                     else if (kind != 0) launch_sell<MT, MT, false>(M_PLAIN, **cur, g, tb, smem, s, mine, rep);
@@ -2062,9 +2205,11 @@ int autotune_shapes(Ctx* ctx, HalpernWork* w, const b2p_params* p) {
                 B2P_CUDA(ctx, cudaEventSynchronize(e1));
                 float ms = 0.f;
                 cudaEventElapsedTime(&ms, e0, e1);
-                if (burst) tot = std::min(tot, ms);
+                ctx->launches += 2 * reps;
+                if (burst) tot = std::min(tot, ms * 4 / reps);
+                behind = 4 * ms / reps > 8 * best;
+                if (burst && behind) break;
             }
-            ctx->launches += 18;
             last = tot;
             if (tot < best) {
                 best = tot;
@@ -2077,15 +2222,6 @@ int autotune_shapes(Ctx* ctx, HalpernWork* w, const b2p_params* p) {
             }
             return B2P_OK;
         };
-        for (int k = 0; k < 3; ++k)
-            for (int tb : {256, 512, 1024}) {
-                int st = trial(1, 1, 1, tb, k);
-                if (st) return st;
-            }
-        for (int k = 0; k < 3; ++k) {
-            int st = trial(2, 1, 1, kWinShapes[k][0], k);
-            if (st) return st;
-        }
         int csr_L = 0;
         float csr_best = 1e30f;
         auto csr = [&](int Lc, int R, int tb) -> int {
@@ -2099,6 +2235,15 @@ int autotune_shapes(Ctx* ctx, HalpernWork* w, const b2p_params* p) {
         for (int Lc : {base_L / 2, base_L, base_L * 2}) {
             if (Lc < 2 || Lc > 32) continue;
             int st = csr(Lc, 1, 256);
+            if (st) return st;
+        }
+        for (int k = 0; k < 3; ++k)
+            for (int tb : {256, 512, 1024}) {
+                int st = trial(1, 1, 1, tb, k);
+                if (st) return st;
+            }
+        for (int k = 0; k < 3; ++k) {
+            int st = trial(2, 1, 1, kWinShapes[k][0], k);
             if (st) return st;
         }
         const int L0 = csr_L;
@@ -2383,11 +2528,11 @@ int solve_T(Ctx* ctx, HalpernWork* w, const b2p_params* p, const double* x0, con
         return rows >= 32 * want ? 32 : (rows >= 16 * want ? 16 : 8);
     };
     if (!w->kr.idx_ready) {
-        st = build_sell_layout(ctx, w->kr, m, L.rowptr.p, L.colidx.p, height(m), 2);
+        st = build_sell_layout(ctx, w->kr, m, L.rowptr.p, L.colidx.p, height(m), 2, check_limit(L.mean_row_len), L.nnz);
         if (st) return st;
     }
     if (!w->kc.idx_ready) {
-        st = build_sell_layout(ctx, w->kc, n, L.t_rowptr.p, L.t_colidx.p, height(n), 2);
+        st = build_sell_layout(ctx, w->kc, n, L.t_rowptr.p, L.t_colidx.p, height(n), 2, check_limit(L.mean_col_len), L.nnz);
         if (st) return st;
     }
     st = fill_sell_vals<double>(ctx, w->kr, m, L.rowptr.p, w->sv64.p, w->kr.v64);
