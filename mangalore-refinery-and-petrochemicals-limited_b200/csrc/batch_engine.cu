@@ -1370,11 +1370,38 @@ __global__ void k_batch_power(int nmat, const int32_t* __restrict__ mat_m, const
     }
 }
 
+// Sum of one row by a whole warp over the CSR arrays (`off` localises the index), eight entries a lane
+// in flight; every lane returns it.  L2: the vector is read past L1.
+template <bool L2>
+__device__ __noinline__ double power_row(const double* __restrict__ val, const int32_t* __restrict__ idx, int64_t e, int64_t e1,
+                                         int64_t off, const double* g, int lane) {
+    constexpr int U = 8;
+    double s = 0.0;
+    for (e += lane; e < e1; e += 32 * U) {
+        double v[U], a[U];
+        int c[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool h = e + 32 * u < e1;
+            v[u] = h ? val[e + 32 * u] : 0.0;
+            c[u] = h ? (int)(idx[e + 32 * u] - off) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) a[u] = c[u] < 0 ? 0.0 : (L2 ? __ldcg(g + c[u]) : g[c[u]]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) s += v[u] * a[u];
+    }
+    return __shfl_sync(0xffffffffu, warp_sum(s), 0);
+}
+
 // The matrices of at least kPowerCluster entries, where a batch has few of them: a cluster of
 // kPowerCtas CTAs each.  One CTA's step is a chain of dependent loads over its whole share of
 // rows and columns (41 us a step on a 2,000 x 8,000 matrix of 47,984 entries, up to 1,000
 // steps); eight CTAs walk an eighth of it.  Rows and columns are summed over the FP64 SELL
-// copies (entry order W = 1), one lane each, in the order of the one-CTA kernel.  SM: every CTA
+// copies (entry order W = 1), one lane each, in the order of the one-CTA kernel; the rows of slices of more
+// than kLongSlice entries are dealt to all warps of the cluster instead, a whole warp each over the CSR
+// arrays (upload of 2,000 x 8,000 with one full row: 1,357 ms with a lane on it, 526 with one thread of
+// a single CTA, now 41).  SM: every CTA
 // holds whole copies of both vectors in shared memory, into which the owners post
 // (ClusterPost), and its share of the matrix where `room` bytes are left for it (4.6 us a
 // step on that matrix); otherwise the vectors lie in L2 (loads bypass L1, which other CTAs'
@@ -1384,10 +1411,14 @@ __global__ void k_batch_power(int nmat, const int32_t* __restrict__ mat_m, const
 // CTA each, 239 ms; now 65).  Every CTA of a cluster makes the same decisions from the same sums.  Every step ends with a cluster barrier, so no thread falls a phase behind.
 template <bool SM>
 __global__ void __cluster_dims__(kPowerCtas, 1, 1) __launch_bounds__(512)
-k_batch_power_cluster(int nbig, const int32_t* __restrict__ bigs, const int32_t* __restrict__ mat_m, const int32_t* __restrict__ mat_n,
+k_batch_power_cluster(int nbig, const int32_t* __restrict__ bigs, const int32_t* __restrict__ mat_m,
+                      const int32_t* __restrict__ mat_n,
                       const int64_t* __restrict__ row_off, const int64_t* __restrict__ col_off,
-                      const int64_t* __restrict__ rs_off, const int64_t* __restrict__ cs_off, const int64_t* __restrict__ r_sptr,
-                      const int64_t* __restrict__ c_sptr, const uint16_t* __restrict__ r_eidx,
+                      const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colidx,
+                      const double* __restrict__ sv64, const int32_t* __restrict__ t_rowptr,
+                      const int32_t* __restrict__ t_colidx, const double* __restrict__ stv64,
+                      const int64_t* __restrict__ rs_off, const int64_t* __restrict__ cs_off,
+                      const int64_t* __restrict__ r_sptr, const int64_t* __restrict__ c_sptr, const uint16_t* __restrict__ r_eidx,
                       const uint16_t* __restrict__ c_eidx, const double* __restrict__ r_ev,
                       const double* __restrict__ c_ev, double* pv, double* pu, double safety, int max_m, int max_n,
                       int room, int* __restrict__ wait_failed, double* __restrict__ eta_out) {
@@ -1397,6 +1428,7 @@ k_batch_power_cluster(int nbig, const int32_t* __restrict__ bigs, const int32_t*
     __shared__ double part[2];  // this CTA's share of ||v||^2, by step parity
     __shared__ uint64_t bar[2];  // arrivals of v, of u
     __shared__ int s_fits;
+    __shared__ int s_long[2];  // slices of more than kLongSlice entries a lane (they come first): columns, rows
     double* vs = smem_at<double>(0);
     double* us = smem_at<double>(8 * max_n);
     int2* tab = smem_at<int2>(8 * (max_n + max_m));  // per owned slice {first entry, entries per lane}
@@ -1452,12 +1484,21 @@ k_batch_power_cluster(int nbig, const int32_t* __restrict__ bigs, const int32_t*
         const int nrs = (m + 31) >> 5, ncs = (n + 31) >> 5;
         // this CTA's slices: rank, rank + kPowerCtas, ...; those of the columns first
         const int ncl = (ncs - rank + kPowerCtas - 1) / kPowerCtas, nrl = (nrs - rank + kPowerCtas - 1) / kPowerCtas;
+        if (tid < 2) s_long[tid] = 0;
+        __syncthreads();
+        for (int sl = tid; sl < ncs + nrs; sl += blockDim.x) {
+            const int64_t* o = sl < ncs ? csp + sl : rsp + (sl - ncs);
+            if (o[1] - o[0] > 32 * kLongSlice) atomicAdd(&s_long[sl < ncs ? 0 : 1], 1);
+        }
+        __syncthreads();
+        const int lcs = s_long[0], lrs = s_long[1];
         bool fits = false;
         uint16_t* si = nullptr;
         if constexpr (SM) {
             for (int l = tid; l < ncl + nrl; l += blockDim.x) {
                 const int64_t* o = l < ncl ? csp + rank + kPowerCtas * l : rsp + rank + kPowerCtas * (l - ncl);
-                tab[l] = make_int2(0, (int)((o[1] - o[0]) >> 5));
+                const bool is_long = l < ncl ? rank + kPowerCtas * l < lcs : rank + kPowerCtas * (l - ncl) < lrs;
+                tab[l] = make_int2(0, is_long ? 0 : (int)((o[1] - o[0]) >> 5));
             }
             __syncthreads();
             if (tid == 0) {
@@ -1509,8 +1550,16 @@ k_batch_power_cluster(int nbig, const int32_t* __restrict__ bigs, const int32_t*
                 tx_expect(bar, 8u * (uint32_t)n);
                 tx_expect(bar + 1, 8u * (uint32_t)m);
             }
+            for (int i = rank + kPowerCtas * warp; i < min(m, 32 * lrs); i += kPowerCtas * nw) {
+                const double s = power_row<!SM>(sv64, colidx, rowptr[ro + i], rowptr[ro + i + 1], co, SM ? vs : pv + co, lane);
+                if (lane == 0) {
+                    if constexpr (SM) up.store(peers, i, s * inv);
+                    else pu[ro + i] = s * inv;
+                }
+            }
             for (int l = warp; l < nrl; l += nw) {
                 const int sl = rank + kPowerCtas * l, i = (sl << 5) + lane;
+                if (sl < lrs) continue;
                 const double s = slice(ncl + l, rsp[sl], rsp[sl + 1], r_ev, r_eidx,
                                        [&](unsigned c) { return SM ? vs[c] : __ldcg(pv + co + c); });
                 if (i < m) {
@@ -1524,8 +1573,17 @@ k_batch_power_cluster(int nbig, const int32_t* __restrict__ bigs, const int32_t*
                 cl.sync();
             }
             sum = 0.0;
+            for (int j = rank + kPowerCtas * warp; j < min(n, 32 * lcs); j += kPowerCtas * nw) {
+                const double s = power_row<!SM>(stv64, t_colidx, t_rowptr[co + j], t_rowptr[co + j + 1], ro, SM ? us : pu + ro, lane);
+                if (lane == 0) {
+                    if constexpr (SM) vp.store(peers, j, s);
+                    else pv[co + j] = s;
+                    sum += s * s;
+                }
+            }
             for (int l = warp; l < ncl; l += nw) {
                 const int sl = rank + kPowerCtas * l, j = (sl << 5) + lane;
+                if (sl < lcs) continue;
                 const double s = slice(l, csp[sl], csp[sl + 1], c_ev, c_eidx,
                                        [&](unsigned c) { return SM ? us[c] : __ldcg(pu + ro + c); });
                 if (j < n) {
@@ -2635,9 +2693,10 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
         B2P_CUDA(ctx, dbigs.reserve(bigs.size()));
         B2P_CUDA(ctx, cudaMemcpyAsync(dbigs.p, bigs.data(), sizeof(int32_t) * bigs.size(), cudaMemcpyHostToDevice, s));
         power_fn<<<std::min(big, resident) * kPowerCtas, 512, sm ? max_smem : 0, s>>>(
-            big, dbigs.p + 1, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->mat_rs_off.p, w->mat_cs_off.p,
-            w->r_sptr.p, w->c_sptr.p, w->r_eidx.p, w->c_eidx.p, w->r_ev64.p, w->c_ev64.p, w->pv.p, w->pu.p, 0.998,
-            w->max_m, w->max_n, (int)(max_smem - vec), dbigs.p, w->mat_eta.p);
+            big, dbigs.p + 1, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->rowptr.p, w->colidx.p,
+            w->sv64.p, w->t_rowptr.p, w->t_colidx.p, w->stv64.p, w->mat_rs_off.p, w->mat_cs_off.p, w->r_sptr.p,
+            w->c_sptr.p, w->r_eidx.p, w->c_eidx.p, w->r_ev64.p, w->c_ev64.p, w->pv.p, w->pu.p, 0.998, w->max_m, w->max_n,
+            (int)(max_smem - vec), dbigs.p, w->mat_eta.p);
         ctx->launches += 1;
         B2P_CUDA(ctx, cudaMemcpyAsync(&wait_failed, dbigs.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     }
