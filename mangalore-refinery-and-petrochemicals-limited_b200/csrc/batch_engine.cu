@@ -1308,21 +1308,22 @@ __device__ __forceinline__ double power_start(int j) {
 }
 
 // sigma_max(A_s)^2 per matrix by power iteration (stops at rel change 1e-7).  Two kernels
-// share the matrices: this one takes those of fewer than cluster_from entries, one CTA
-// each -- a batch of many matrices fills the GPU that way.
+// share the matrices: this one takes one CTA each, all of them or (SMALL) those of fewer than
+// kPowerCluster entries -- a batch of many matrices fills the GPU that way.
+template <bool SMALL>
 __global__ void k_batch_power(int nmat, const int32_t* __restrict__ mat_m, const int32_t* __restrict__ mat_n,
                               const int64_t* __restrict__ row_off, const int64_t* __restrict__ col_off,
                               const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colidx,
                               const double* __restrict__ sv64, const int32_t* __restrict__ t_rowptr,
                               const int32_t* __restrict__ t_colidx, const double* __restrict__ stv64, double* pv,
-                              double* pu, double safety, int cluster_from, double* __restrict__ eta_out) {
+                              double* pu, double safety, double* __restrict__ eta_out) {
     __shared__ double red[32];
     __shared__ double s_norm, s_prev;
     __shared__ int s_stop;
     for (int k = blockIdx.x; k < nmat; k += gridDim.x) {
         const int m = mat_m[k], n = mat_n[k];
         const int64_t ro = row_off[k], co = col_off[k];
-        if (rowptr[ro + m] - rowptr[ro] >= cluster_from) continue;
+        if (SMALL && rowptr[ro + m] - rowptr[ro] >= kPowerCluster) continue;
         double part = 0.0;
         for (int j = threadIdx.x; j < n; j += blockDim.x) {
             const double v = power_start(j);
@@ -2684,9 +2685,10 @@ int b2p_batch_upload(void* p, int nmat, const int32_t* mat_m, const int32_t* mat
     const auto power_fn = sm ? k_batch_power_cluster<true> : k_batch_power_cluster<false>;
     const int resident = big > 0 && big <= clusters ? clusters_resident(power_fn, kPowerCtas, 512, sm ? max_smem : 0) : 0;
     const bool use_clusters = resident > 0;
-    k_batch_power<<<gmat, 256, 0, s>>>(nmat, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->rowptr.p,
-                                        w->colidx.p, w->sv64.p, w->t_rowptr.p, w->t_colidx.p, w->stv64.p, w->pv.p,
-                                        w->pu.p, 0.998, use_clusters ? kPowerCluster : INT_MAX, w->mat_eta.p);
+    const auto one_cta_fn = use_clusters ? k_batch_power<true> : k_batch_power<false>;
+    one_cta_fn<<<gmat, 256, 0, s>>>(nmat, w->mat_m.p, w->mat_n.p, w->mat_row_off.p, w->mat_col_off.p, w->rowptr.p,
+                                    w->colidx.p, w->sv64.p, w->t_rowptr.p, w->t_colidx.p, w->stv64.p, w->pv.p, w->pu.p,
+                                    0.998, w->mat_eta.p);
     int wait_failed = 0;
     DBuf<int32_t> dbigs;
     if (use_clusters) {
