@@ -41,6 +41,9 @@ constexpr int64_t kClusterNnz = 49152;
 // ... and of at most this many on one CTA: 1.50 us against 1.64 on eight at 2,500 entries, 2.6 against
 // 1.8 at 5,000
 constexpr int64_t kOneCtaNnz = 3072;
+// ... and their long rows (of at least kLongRow entries each)
+constexpr int kLongRow = 128;
+constexpr int kMostLong = kClusterNnz / kLongRow;
 
 // Slots of the per-check reduction block.
 enum { R_DPRIMAL = 0, R_DDUAL, R_VIOL_X, R_VIOL_AVG, R_BOUND, R_COUNT };
@@ -55,15 +58,24 @@ struct RefState {
 // row 32 s + l at off[s] + 32 q + l, slices padded to their longest row and to a multiple
 // of kPad entries.  A padding entry has value 0 and the index one past the gathered vector, where
 // a 0 is stored: it adds +0 to a sum that started from +0, which leaves every sum as it was
-// (such a sum is never -0), whatever the iterates hold.  off null: the CSR arrays (a slice with
-// one very long row would pad the others to it).
+// (such a sum is never -0), whatever the iterates hold.  off null: the CSR arrays (slices whose rows
+// differ too much in length).  Rows of more than `limit` entries are not in the slices but in `longs`:
+// a whole warp sums each over the CSR arrays (long_row_sum).
 struct Sell {
     const int64_t* off;
     const int32_t* ptr;  // CSR row pointers
     const int32_t* idx;
     const double* val;
+    const int32_t* csr_idx;
+    const double* csr_val;
+    const int32_t* longs;
+    int nlong, limit;
+    __device__ __forceinline__ bool is_long(int i) const { return ptr[i + 1] - ptr[i] > limit; }
 };
 constexpr int kPad = 2;
+// Entries from which a row is long, kLongRow at least: a lane takes 64 ns an entry there (a thread on the CSR
+// arrays 50), a warp 7 to 10; rows of a usual length, which 32 lanes sum side by side, stay in the slices.
+int long_limit(int64_t nnz, int rows) { return (int)std::max<int64_t>(kLongRow, 8 * nnz / rows); }
 
 // Sum over row i in entry order, products and sums rounded separately.  The products of a
 // batch are independent; only the additions are a chain.
@@ -104,26 +116,79 @@ __device__ __forceinline__ double row_sum(const Sell& S, int i, const double* g)
     return w;
 }
 
-// padded length of every slice, x 32 lanes (the offsets are their sums)
-__global__ void k_ref_slice_len(int rows, const int32_t* __restrict__ ptr, int64_t* __restrict__ off) {
+// Sum over row i in entry order by a whole warp: the lanes load, gather and multiply 128 entries side by
+// side, the next 128 on their way, and every lane adds the products up in order.
+__device__ __noinline__ double long_row_sum(const double* __restrict__ val, const int32_t* __restrict__ idx, int e0, int e1,
+                                            const double* g) {
+    constexpr int U = 4;
+    const int lane = threadIdx.x & 31;
+    double w = 0.0, v[U];
+    int c[U];
+    auto load = [&](int64_t e) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool h = e + 32 * u + lane < e1;
+            v[u] = h ? __ldg(val + e + 32 * u + lane) : 0.0;
+            c[u] = h ? __ldg(idx + e + 32 * u + lane) : -1;
+        }
+    };
+    load(e0);
+    for (int64_t e = e0; e < e1; e += 32 * U) {
+        double p[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) p[u] = c[u] >= 0 ? v[u] * g[c[u]] : 0.0;
+        load(e + 32 * U);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int n = (int)min((int64_t)32, e1 - (e + 32 * u));
+            if (n == 32) {
+#pragma unroll
+                for (int l = 0; l < 32; ++l) w += __shfl_sync(0xffffffffu, p[u], l);
+            } else {
+                for (int l = 0; l < n; ++l) w += __shfl_sync(0xffffffffu, p[u], l);
+            }
+        }
+    }
+    return w;
+}
+
+// update(i, sum) of every long row, by one lane; all warps of the grid take part
+template <typename F>
+__device__ __forceinline__ void for_long_rows(const Sell& S, const double* g, F update) {
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < S.nlong; q += warps) {
+        const int i = S.longs[q];
+        const double w = long_row_sum(S.csr_val, S.csr_idx, S.ptr[i], S.ptr[i + 1], g);
+        if ((threadIdx.x & 31) == 0) update(i, w);
+    }
+}
+
+// padded length of every slice, x 32 lanes (the offsets are their sums), without the long rows; those
+// into `longs`, their number into off[number of slices + 1] (zeroed by the caller)
+__global__ void k_ref_slice_len(int rows, int limit, const int32_t* __restrict__ ptr, int64_t* __restrict__ off,
+                                int32_t* __restrict__ longs) {
     const int nsl = (rows + 31) >> 5;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nsl; s += gridDim.x * blockDim.x) {
         int mx = 0;
-        for (int i = s << 5; i < min(rows, (s + 1) << 5); ++i) mx = max(mx, ptr[i + 1] - ptr[i]);
+        for (int i = s << 5; i < min(rows, (s + 1) << 5); ++i) {
+            const int len = ptr[i + 1] - ptr[i];
+            if (len <= limit) mx = max(mx, len);
+            else longs[atomicAdd(reinterpret_cast<unsigned long long*>(off + nsl + 1), 1ull)] = i;
+        }
         off[s + 1] = 32ll * ((mx + kPad - 1) / kPad * kPad);
         if (s == 0) off[0] = 0;
     }
 }
 
 // every lane slot of every slice; `other`: the length of the gathered vector
-__global__ void k_ref_slice_fill(int rows, int other, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+__global__ void k_ref_slice_fill(int rows, int limit, int other, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                                  const double* __restrict__ val, const int64_t* __restrict__ off,
                                  int32_t* __restrict__ oidx, double* __restrict__ oval) {
     const int padded = (rows + 31) & ~31;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < padded; i += gridDim.x * blockDim.x) {
         const int64_t base = off[i >> 5] + (i & 31);
         const int slen = (int)((off[(i >> 5) + 1] - off[i >> 5]) >> 5);
-        const int p0 = i < rows ? ptr[i] : 0, len = i < rows ? ptr[i + 1] - p0 : 0;
+        const int p0 = i < rows ? ptr[i] : 0, all = i < rows ? ptr[i + 1] - p0 : 0, len = all <= limit ? all : 0;
         for (int q = 0; q < slen; ++q) {
             oidx[base + 32ll * q] = q < len ? idx[p0 + q] : other;
             oval[base + 32ll * q] = q < len ? val[p0 + q] : 0.0;
@@ -173,14 +238,13 @@ __global__ void k_ref_init(int m, int n, const double* __restrict__ lb, const do
 
 // Steps A-C (first_order_solver.cpp:163-180): A^T y, projected primal step,
 // ergodic sum, extrapolation.  x_prev == x at entry, so x_hat = 2 x_new - x.
-template <bool CHECK, bool SLICED>
+template <bool CHECK, bool SLICED, bool LONG>
 __global__ void __launch_bounds__(128) k_ref_primal(int n, Sell At, const double* __restrict__ c,
                                                     const double* __restrict__ lb, const double* __restrict__ ub,
                                                     RefState st) {
     pdl_wait();
     pdl_trigger();
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        double w = row_sum<kBatch, SLICED>(At, j, st.y);
+    auto update = [&](int j, double w) {
         double xj = st.x[j];
         double grad = c[j] + w;
         double next_x = xj - st.tau[j] * grad;
@@ -189,25 +253,30 @@ __global__ void __launch_bounds__(128) k_ref_primal(int n, Sell At, const double
         st.x_sum[j] += new_x;
         st.x_hat[j] = 2.0 * new_x - xj;
         st.x[j] = new_x;
-    }
+    };
+    if (LONG) for_long_rows(At, st.y, update);
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+        if (!LONG || !At.is_long(j)) update(j, row_sum<kBatch, SLICED>(At, j, st.y));
 }
 
 // Steps D-E (first_order_solver.cpp:183-192): A x_hat, dual step, sign projection.
-template <bool CHECK, bool SLICED>
+template <bool CHECK, bool SLICED, bool LONG>
 __global__ void __launch_bounds__(128) k_ref_dual(int m, Sell A, const double* __restrict__ b,
                                                   const uint8_t* __restrict__ is_eq, RefState st) {
     int tid = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_wait();
     pdl_trigger();
-    for (int i = tid; i < m; i += gridDim.x * blockDim.x) {
-        double v = row_sum<kBatch, SLICED>(A, i, st.x_hat);
+    auto update = [&](int i, double v) {
         double yi = st.y[i];
         double next_y = yi + st.sigma[i] * (v - b[i]);
         // std::max(0.0, next_y) == (0.0 < next_y) ? next_y : 0.0
         double new_y = (!is_eq[i]) ? ((0.0 < next_y) ? next_y : 0.0) : next_y;
         if (CHECK) atomic_max_nonneg(&st.red[R_DDUAL], fabs(new_y - yi));
         st.y[i] = new_y;
-    }
+    };
+    if (LONG) for_long_rows(A, st.x_hat, update);
+    for (int i = tid; i < m; i += gridDim.x * blockDim.x)
+        if (!LONG || !A.is_long(i)) update(i, row_sum<kBatch, SLICED>(A, i, st.x_hat));
     if (tid == 0) *st.iter += 1;
 }
 
@@ -227,13 +296,16 @@ __global__ void k_ref_check_cols(int n, const double* __restrict__ lb, const dou
 template <bool SLICED>
 __global__ void __launch_bounds__(128) k_ref_check_rows(int m, Sell A, const double* __restrict__ b,
                                                         const uint8_t* __restrict__ is_eq, RefState st) {
+    auto violation = [&](int i, int slot, double v) {
+        const double d = v - b[i];
+        atomic_max_nonneg(&st.red[slot], (!is_eq[i]) ? ((0.0 < d) ? d : 0.0) : fabs(d));
+    };
+    for_long_rows(A, st.x, [&](int i, double v) { violation(i, R_VIOL_X, v); });
+    for_long_rows(A, st.x_avg, [&](int i, double v) { violation(i, R_VIOL_AVG, v); });
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-        double ax = row_sum<kBatch, SLICED>(A, i, st.x), aa = row_sum<kBatch, SLICED>(A, i, st.x_avg);
-        double d1 = ax - b[i], d2 = aa - b[i];
-        double v1 = (!is_eq[i]) ? ((0.0 < d1) ? d1 : 0.0) : fabs(d1);
-        double v2 = (!is_eq[i]) ? ((0.0 < d2) ? d2 : 0.0) : fabs(d2);
-        atomic_max_nonneg(&st.red[R_VIOL_X], v1);
-        atomic_max_nonneg(&st.red[R_VIOL_AVG], v2);
+        if (A.nlong > 0 && A.is_long(i)) continue;
+        violation(i, R_VIOL_X, row_sum<kBatch, SLICED>(A, i, st.x));
+        violation(i, R_VIOL_AVG, row_sum<kBatch, SLICED>(A, i, st.x_avg));
     }
 }
 
@@ -270,7 +342,7 @@ struct RefOutcome {
 // Shared memory of one CTA (bytes from the start of the dynamic array), the same in all.
 struct RefLayout {
     int cols, rows;      // most owned columns / rows of any CTA
-    int y, xh, x, xsum, tau, c, lb, ub, sigma, b, eq, cval, rval, cidx, ridx, coff, roff, total;
+    int y, xh, x, xsum, tau, c, lb, ub, sigma, b, eq, cval, rval, cidx, ridx, coff, roff, cmask, rmask, total;
 };
 
 // entries in shared memory by slices: entry q of lane l of the CTA's slice s at off + 32 q + l
@@ -309,7 +381,8 @@ struct SliceView {
     }
 };
 
-template <int NC, bool MAT_SMEM>
+// LONG: some rows or columns are long; the warps of the CTA that owns them take them before its slices.
+template <int NC, bool MAT_SMEM, bool LONG>
 __global__ void __launch_bounds__(kClusterThreads, 1)
 k_ref_cluster(int m, int n, Sell A, Sell At, const double* __restrict__ c, const double* __restrict__ lb,
               const double* __restrict__ ub, const double* __restrict__ b, const uint8_t* __restrict__ is_eq, RefState st,
@@ -320,6 +393,7 @@ k_ref_cluster(int m, int n, Sell A, Sell At, const double* __restrict__ c, const
     __shared__ unsigned long long red[R_COUNT];
     __shared__ uint64_t bar[2];  // arrivals of x_hat, of y
     __shared__ double token;     // where CTAs without columns post
+    __shared__ int longs[2][LONG ? kMostLong : 1], nlong[2];  // owned long columns, rows
     auto at = [&](int off) { return reinterpret_cast<double*>(sh + off); };
     double *ys = at(lay.y), *xh = at(lay.xh), *xs = at(lay.x), *sums = at(lay.xsum), *ts = at(lay.tau), *cs = at(lay.c);
     double *ls = at(lay.lb), *us = at(lay.ub), *ss = at(lay.sigma), *bs = at(lay.b);
@@ -344,6 +418,24 @@ k_ref_cluster(int m, int n, Sell A, Sell At, const double* __restrict__ c, const
     int *co = reinterpret_cast<int*>(sh + lay.coff), *ro = reinterpret_cast<int*>(sh + lay.roff);
     for (int q = tid; q <= c1 - c0; q += blockDim.x) co[q] = (int)(At.off[c0 + q] - At.off[c0]);
     for (int q = tid; q <= r1 - r0; q += blockDim.x) ro[q] = (int)(A.off[r0 + q] - A.off[r0]);
+    // owned long columns and rows, and per slice the lanes that have one
+    unsigned *cmask = reinterpret_cast<unsigned*>(sh + lay.cmask), *rmask = reinterpret_cast<unsigned*>(sh + lay.rmask);
+    if (LONG) {
+        for (int q = tid; q < c1 - c0; q += blockDim.x) cmask[q] = 0;
+        for (int q = tid; q < r1 - r0; q += blockDim.x) rmask[q] = 0;
+        if (tid < 2) nlong[tid] = 0;
+        __syncthreads();
+        auto own = [&](const Sell& S, int s0, int s1, int side, unsigned* mask) {
+            for (int q = tid; q < S.nlong; q += blockDim.x) {
+                const int i = S.longs[q];
+                if ((i >> 5) < s0 || (i >> 5) >= s1) continue;
+                longs[side][atomicAdd(&nlong[side], 1)] = i;
+                atomicOr(&mask[(i >> 5) - s0], 1u << (i & 31));
+            }
+        };
+        own(At, c0, c1, 0, cmask);
+        own(A, r0, r1, 1, rmask);
+    }
     // full copies, owned vectors, owned part of the matrix
     for (int i = tid; i <= m; i += blockDim.x) ys[i] = st.y[i];
     if (tid == 0) xh[n] = 0.0;
@@ -394,16 +486,28 @@ k_ref_cluster(int m, int n, Sell A, Sell At, const double* __restrict__ c, const
     };
     long long it = out->iter;
     bool finished = out->converged || out->failed;
+    // update(i, sum) for the owned long rows of one orientation
+    auto long_rows = [&](const Sell& S, int side, const double* g, auto update) {
+        for (int q = warp; LONG && q < nlong[side]; q += nw) {
+            const int i = longs[side][q];
+            const double w = long_row_sum(S.csr_val, S.csr_idx, S.ptr[i], S.ptr[i + 1], g);
+            if (lane == 0) update(i, w);
+        }
+    };
+    auto in_slices = [&](const unsigned* mask, int sl) { return !LONG || !(mask[sl] >> lane & 1u); };
     // max row violation of the vector whose copies are in xh, into slot
     auto violation = [&](int slot) {
+        auto row = [&](int i, double v) {
+            const int o = i - (r0 << 5);
+            const double d = v - bs[o];
+            atomic_max_nonneg(&red[slot], (!eq[o]) ? ((0.0 < d) ? d : 0.0) : fabs(d));
+        };
+        long_rows(A, 1, xh, row);
         for (int sl = r0 + warp; sl < r1; sl += nw) {
             const int p0 = ro[sl - r0];
             const double v = rv.sum(rb + p0, (ro[sl - r0 + 1] - p0) >> 5, lane, xh);
-            const int i = (sl << 5) + lane, o = i - (r0 << 5);
-            if (i < m) {
-                const double d = v - bs[o];
-                atomic_max_nonneg(&red[slot], (!eq[o]) ? ((0.0 < d) ? d : 0.0) : fabs(d));
-            }
+            const int i = (sl << 5) + lane;
+            if (i < m && in_slices(rmask, sl - r0)) row(i, v);
         }
     };
     while (it < stop && !finished) {
@@ -414,34 +518,40 @@ k_ref_cluster(int m, int n, Sell A, Sell At, const double* __restrict__ c, const
                 if (tid < R_COUNT) red[tid] = 0ull;
                 __syncthreads();
             }
+            auto column = [&](int j, double w) {
+                const int o = j - (c0 << 5);
+                double xj = xs[o];
+                double grad = cs[o] + w;
+                double next_x = xj - ts[o] * grad;
+                double new_x = ref_clamp(next_x, ls[o], us[o]);
+                if (check) atomic_max_nonneg(&red[R_DPRIMAL], fabs(new_x - xj));
+                sums[o] += new_x;
+                xv.store(peers, j, 2.0 * new_x - xj);
+                xs[o] = new_x;
+            };
+            long_rows(At, 0, ys, column);
             for (int sl = c0 + warp; sl < c1; sl += nw) {
                 const int p0 = co[sl - c0];
                 const double w = cv.sum(cb + p0, (co[sl - c0 + 1] - p0) >> 5, lane, ys);
-                const int j = (sl << 5) + lane, o = j - (c0 << 5);
-                if (j < n) {
-                    double xj = xs[o];
-                    double grad = cs[o] + w;
-                    double next_x = xj - ts[o] * grad;
-                    double new_x = ref_clamp(next_x, ls[o], us[o]);
-                    if (check) atomic_max_nonneg(&red[R_DPRIMAL], fabs(new_x - xj));
-                    sums[o] += new_x;
-                    xv.store(peers, j, 2.0 * new_x - xj);
-                    xs[o] = new_x;
-                }
+                const int j = (sl << 5) + lane;
+                if (j < n && in_slices(cmask, sl - c0)) column(j, w);
             }
             if (NC > 1 && c0 == c1 && tid == 0) tv.store(peers, 0, 0.0);
             phase_end(0, x_bytes);
+            auto row = [&](int i, double v) {
+                const int o = i - (r0 << 5);
+                double yi = ys[i];
+                double next_y = yi + ss[o] * (v - bs[o]);
+                double new_y = (!eq[o]) ? ((0.0 < next_y) ? next_y : 0.0) : next_y;
+                if (check) atomic_max_nonneg(&red[R_DDUAL], fabs(new_y - yi));
+                yv.store(peers, i, new_y);
+            };
+            long_rows(A, 1, xh, row);
             for (int sl = r0 + warp; sl < r1; sl += nw) {
                 const int p0 = ro[sl - r0];
                 const double v = rv.sum(rb + p0, (ro[sl - r0 + 1] - p0) >> 5, lane, xh);
-                const int i = (sl << 5) + lane, o = i - (r0 << 5);
-                if (i < m) {
-                    double yi = ys[i];
-                    double next_y = yi + ss[o] * (v - bs[o]);
-                    double new_y = (!eq[o]) ? ((0.0 < next_y) ? next_y : 0.0) : next_y;
-                    if (check) atomic_max_nonneg(&red[R_DDUAL], fabs(new_y - yi));
-                    yv.store(peers, i, new_y);
-                }
+                const int i = (sl << 5) + lane;
+                if (i < m && in_slices(rmask, sl - r0)) row(i, v);
             }
             phase_end(1, y_bytes);
             parity ^= 1;
@@ -530,6 +640,8 @@ RefLayout ref_layout(int m, int n, int64_t ce, int64_t re) {
     L.ridx = take(2 * re);
     L.coff = take(4 * (L.cols / 32 + 1));
     L.roff = take(4 * (L.rows / 32 + 1));
+    L.cmask = take(4 * (L.cols / 32));
+    L.rmask = take(4 * (L.rows / 32));
     L.total = (int)std::min<int64_t>(o, 1 << 30);
     return L;
 }
@@ -541,40 +653,47 @@ struct RefBuffers {
     DBuf<long long> iter;
     DBuf<RefOutcome> outcome;
     DBuf<int64_t> off, t_off;
-    DBuf<int32_t> idx, t_idx;
+    DBuf<int32_t> idx, t_idx, longs, t_longs;
     DBuf<double> val, t_val;
 };
 
 // The sliced copy of one orientation, or the CSR arrays where padding would cost more than
 // three times the entries.
 int build_sell(Ctx* ctx, int rows, int other, int64_t nnz, const int32_t* ptr, const int32_t* idx, const double* val,
-               DBuf<int64_t>& off, DBuf<int32_t>& oidx, DBuf<double>& oval, Sell* S, std::vector<int64_t>* h_off) {
+               DBuf<int64_t>& off, DBuf<int32_t>& longs, DBuf<int32_t>& oidx, DBuf<double>& oval, Sell* S,
+               std::vector<int64_t>* h_off) {
     cudaStream_t s = ctx->stream;
-    const int nsl = (rows + 31) >> 5;
-    *S = Sell{nullptr, ptr, idx, val};
-    B2P_CUDA(ctx, off.reserve(nsl + 1));
-    k_ref_slice_len<<<grid_for(nsl, 128, ctx->sm_count), 128, 0, s>>>(rows, ptr, off.p);
+    const int nsl = (rows + 31) >> 5, limit = long_limit(nnz, rows);
+    B2P_CUDA(ctx, off.reserve(nsl + 2));
+    B2P_CUDA(ctx, longs.reserve(nnz / limit + 1));
+    B2P_CUDA(ctx, cudaMemsetAsync(off.p + nsl + 1, 0, sizeof(int64_t), s));
+    k_ref_slice_len<<<grid_for(nsl, 128, ctx->sm_count), 128, 0, s>>>(rows, limit, ptr, off.p, longs.p);
     B2P_LAUNCH(ctx);
     size_t tmp = 0;
     B2P_CUDA(ctx, cub::DeviceScan::InclusiveSum(nullptr, tmp, off.p + 1, off.p + 1, nsl, s));
     B2P_CUDA(ctx, ctx->cub_tmp.reserve(tmp));
     tmp = ctx->cub_tmp.bytes();
     B2P_CUDA(ctx, cub::DeviceScan::InclusiveSum(ctx->cub_tmp.p, tmp, off.p + 1, off.p + 1, nsl, s));
-    // the offsets of an LP that may run on a cluster are wanted on the host, else only the total
-    const size_t want = nnz <= kClusterNnz ? (size_t)nsl + 1 : 1;
+    // the offsets of an LP that may run on a cluster are wanted on the host, else only the total; the number
+    // of long rows lies behind them
+    const size_t want = nnz <= kClusterNnz ? (size_t)nsl + 2 : 2;
     h_off->resize(want);
-    B2P_CUDA(ctx, cudaMemcpyAsync(h_off->data(), off.p + nsl + 1 - want, sizeof(int64_t) * want, cudaMemcpyDeviceToHost, s));
+    B2P_CUDA(ctx, cudaMemcpyAsync(h_off->data(), off.p + nsl + 2 - want, sizeof(int64_t) * want, cudaMemcpyDeviceToHost, s));
     B2P_CUDA(ctx, cudaStreamSynchronize(s));
+    *S = Sell{nullptr, ptr, idx, val, idx, val, longs.p, (int)h_off->back(), limit};
+    h_off->pop_back();
     const int64_t total = h_off->back();
     ctx->launches += 2;
     if (total > 3 * nnz + 4096) return B2P_OK;
     B2P_CUDA(ctx, oidx.reserve(total));
     B2P_CUDA(ctx, oval.reserve(total));
-    k_ref_slice_fill<<<grid_for(rows + 31, 128, ctx->sm_count), 128, 0, s>>>(rows, other, ptr, idx, val, off.p, oidx.p,
+    k_ref_slice_fill<<<grid_for(rows + 31, 128, ctx->sm_count), 128, 0, s>>>(rows, limit, other, ptr, idx, val, off.p, oidx.p,
                                                                             oval.p);
     B2P_LAUNCH(ctx);
     ctx->launches += 1;
-    *S = Sell{off.p, ptr, oidx.p, oval.p};
+    S->off = off.p;
+    S->idx = oidx.p;
+    S->val = oval.p;
     return B2P_OK;
 }
 
@@ -616,18 +735,23 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
     ctx->launches += 2;
     Sell A, At;
     std::vector<int64_t> h_off, h_toff;
-    int bst = build_sell(ctx, m, n, L.nnz, L.rowptr.p, L.colidx.p, L.vals.p, B.off, B.idx, B.val, &A, &h_off);
+    int bst = build_sell(ctx, m, n, L.nnz, L.rowptr.p, L.colidx.p, L.vals.p, B.off, B.longs, B.idx, B.val, &A, &h_off);
     if (bst) return bst;
-    bst = build_sell(ctx, n, m, L.nnz, L.t_rowptr.p, L.t_colidx.p, L.t_vals.p, B.t_off, B.t_idx, B.t_val, &At, &h_toff);
+    bst = build_sell(ctx, n, m, L.nnz, L.t_rowptr.p, L.t_colidx.p, L.t_vals.p, B.t_off, B.t_longs, B.t_idx, B.t_val, &At,
+                     &h_toff);
     if (bst) return bst;
 
     auto primal = [&](auto check) {
         constexpr bool C = decltype(check)::value;
-        pdl_launch(At.off ? k_ref_primal<C, true> : k_ref_primal<C, false>, gn, TB, 0, s, n, At, L.c.p, L.lb.p, L.ub.p, st);
+        const auto fn = At.nlong ? (At.off ? k_ref_primal<C, true, true> : k_ref_primal<C, false, true>)
+                                 : (At.off ? k_ref_primal<C, true, false> : k_ref_primal<C, false, false>);
+        pdl_launch(fn, gn, TB, 0, s, n, At, L.c.p, L.lb.p, L.ub.p, st);
     };
     auto dual = [&](auto check) {
         constexpr bool C = decltype(check)::value;
-        pdl_launch(A.off ? k_ref_dual<C, true> : k_ref_dual<C, false>, gm, TB, 0, s, m, A, L.b.p, L.is_eq.p, st);
+        const auto fn = A.nlong ? (A.off ? k_ref_dual<C, true, true> : k_ref_dual<C, false, true>)
+                                : (A.off ? k_ref_dual<C, true, false> : k_ref_dual<C, false, false>);
+        pdl_launch(fn, gm, TB, 0, s, m, A, L.b.p, L.is_eq.p, st);
     };
     auto check_xs = [&]() {
         k_ref_check_cols<<<gn, TB, 0, s>>>(n, L.lb.p, L.ub.p, st);
@@ -647,37 +771,47 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
 
     const int64_t max_it = p->max_iterations;
     const int64_t cf = std::min<int64_t>(p->check_frequency, 100);  // first_order_solver.cpp:156
-    int max_smem = 0;
-    B2P_CUDA(ctx, cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-    max_smem -= 1024;  // static part
     // One CTA for up to kOneCtaNnz entries that fit its shared memory with the vectors, else a
     // cluster where the vectors do, with the owned parts of the matrix in shared memory if
     // they fit as well.
     RefLayout lay{};
-    int form = 0;  // 1: one CTA, 2: cluster with the matrix in shared memory, 3: cluster without
+    const bool longs = A.nlong > 0 || At.nlong > 0;
+    decltype(&k_ref_cluster<1, true, false>) small_fn = nullptr;
+    int ctas = 1;
     if (A.off && At.off && L.nnz <= kClusterNnz && m < 65535 && n < 65535) {
         const int ncs = (n + 31) >> 5, nrs = (m + 31) >> 5;
-        lay = ref_layout<1>(m, n, h_toff[ncs], h_off[nrs]);
-        if (L.nnz <= kOneCtaNnz && lay.total <= max_smem) form = 1;
-        if (!form) {
+        // the form `fn` with the layout `l` if its CTAs have the shared memory and the device the clusters
+        auto take = [&](auto fn, int nc, const RefLayout& l) -> int {
+            int most = 0;
+            B2P_CUDA(ctx, open_smem(ctx, fn, &most));
+            if (l.total > most || (nc > 1 && clusters_resident(fn, nc, kClusterThreads, l.total) < 1)) return B2P_OK;
+            small_fn = fn;
+            ctas = nc;
+            lay = l;
+            return B2P_OK;
+        };
+        if (L.nnz <= kOneCtaNnz) {
+            const int tst = take(longs ? k_ref_cluster<1, true, true> : k_ref_cluster<1, true, false>, 1,
+                                 ref_layout<1>(m, n, h_toff[ncs], h_off[nrs]));
+            if (tst) return tst;
+        }
+        if (!small_fn) {
             int64_t ce = 0, re = 0;
             for (int r = 0; r < kClusterCtas; ++r) {
                 ce = std::max(ce, h_toff[cluster_slice<kClusterCtas>(ncs, r + 1)] - h_toff[cluster_slice<kClusterCtas>(ncs, r)]);
                 re = std::max(re, h_off[cluster_slice<kClusterCtas>(nrs, r + 1)] - h_off[cluster_slice<kClusterCtas>(nrs, r)]);
             }
-            lay = ref_layout<kClusterCtas>(m, n, ce, re);
-            if (lay.total <= max_smem) form = 2;
+            const int tst = take(longs ? k_ref_cluster<kClusterCtas, true, true> : k_ref_cluster<kClusterCtas, true, false>,
+                                 kClusterCtas, ref_layout<kClusterCtas>(m, n, ce, re));
+            if (tst) return tst;
         }
-        if (!form) {
-            lay = ref_layout<kClusterCtas>(m, n, 0, 0);
-            if (lay.total <= max_smem) form = 3;
+        if (!small_fn) {
+            const int tst = take(longs ? k_ref_cluster<kClusterCtas, false, true> : k_ref_cluster<kClusterCtas, false, false>,
+                                 kClusterCtas, ref_layout<kClusterCtas>(m, n, 0, 0));
+            if (tst) return tst;
         }
     }
-    const auto small_fn = form == 1 ? k_ref_cluster<1, true>
-                                    : (form == 2 ? k_ref_cluster<kClusterCtas, true> : k_ref_cluster<kClusterCtas, false>);
-    if (form != 0) B2P_CUDA(ctx, open_smem(ctx, small_fn));
-    if (form > 1 && clusters_resident(small_fn, kClusterCtas, kClusterThreads, lay.total) < 1) form = 0;
-    const bool small = form != 0;
+    const bool small = small_fn != nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     if (!small && max_it >= kGraphIters && cf > kGraphIters) {
@@ -712,7 +846,6 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
     if (small) {
         B2P_CUDA(ctx, B.outcome.reserve(1));
         B2P_CUDA(ctx, cudaMemsetAsync(B.outcome.p, 0, sizeof(RefOutcome), s));
-        const int ctas = form == 1 ? 1 : kClusterCtas;
         cudaLaunchAttribute dims;
         const cudaLaunchConfig_t lc = cluster_config(ctas, ctas, kClusterThreads, lay.total, s, &dims);
         // one launch runs up to 100,000 iterations (a fraction of a second)
