@@ -646,7 +646,9 @@ RefLayout ref_layout(int m, int n, int64_t ce, int64_t re) {
     return L;
 }
 
-// Grow-only device buffers of the engine, kept by the context between solves.
+// Device buffers of the engine, kept by the context between solves of LPs of at most kKeepEntries
+// entries and as many rows and columns (up to 72 bytes an entry of sliced copies).
+constexpr int64_t kKeepEntries = 1 << 20;
 struct RefBuffers {
     DBuf<double> tau, sigma, x, y, x_hat, x_sum, x_avg;
     DBuf<unsigned long long> red;
@@ -713,6 +715,14 @@ int ref_engine_solve(Ctx* ctx, const b2p_params* p, b2p_result* r, double* x_out
     const int m = L.m, n = L.n;
     cudaStream_t s = ctx->stream;
     if (!ctx->rw) ctx->rw = new RefWork();
+    // a large LP's buffers go back when the solve ends (freeing waits for what is in flight)
+    struct Keep {
+        Ctx* ctx;
+        bool keep;
+        ~Keep() {
+            if (!keep) ref_free(ctx);
+        }
+    } keep{ctx, L.nnz <= kKeepEntries && (int64_t)m + n <= kKeepEntries};
     RefBuffers& B = ctx->rw->b;
     B2P_CUDA(ctx, B.tau.reserve(n));
     B2P_CUDA(ctx, B.sigma.reserve(m));
