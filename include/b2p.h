@@ -275,8 +275,10 @@ int b2p_batch_upload(void* ctx, int nmat, const int32_t* mat_m, const int32_t* m
  * Outputs (optional): per-instance status, iterations, rel KKT and final primal
  * weight; concatenated x, y.  The summary reports the autotuned kernel shape:
  * step_size = CTA size * 1e5 + chunk length (iterations per persistent launch),
- * used_average = 10 * instances per CTA (2 or 4: batches whose instances share
- * one matrix) + SELL entries per lane load.  The shape is tuned
+ * used_average = 10 * instances per CTA + SELL entries per lane load.  The
+ * instances per CTA are those of the solve's first launch (2 or 4: batches whose
+ * instances share one matrix; 1 for a batch of at most one instance per SM);
+ * later launches go over to fewer as instances finish.  The shape is tuned
  * once per batch signature and cached in the file B2P_AUTOTUNE_CACHE (default
  * ~/.cache/b2p_autotune.txt); B2P_BATCH_SHAPE="threads,w,ni" pins it for the
  * whole solve. */

@@ -2305,6 +2305,7 @@ int batch_run(Ctx* ctx, BatchWork* w, const b2p_params* p, const double* x0_dev,
     int32_t*& host_cnt = own.host_cnt;
     B2P_CUDA(ctx, cudaMallocHost(&host_cnt, 2 * sizeof(int32_t)));
     host_cnt[1] = n_act;
+    const int first_ni = pick_form(n_act).ni;  // instances per CTA of the first launch
     const int64_t max_graphs = p->max_iterations / (2LL * cfg.chunk) + 3;
     int64_t graphs = 0;
     bool timed_out = false;
@@ -2360,7 +2361,10 @@ int batch_run(Ctx* ctx, BatchWork* w, const b2p_params* p, const double* x0_dev,
     w->solved = true;
     if (timed_out_out) *timed_out_out = timed_out;
     if (kms_out) *kms_out = kms;
-    if (cfg_out) *cfg_out = cfg;
+    if (cfg_out) {
+        *cfg_out = cfg;
+        cfg_out->ni = first_ni;
+    }
     return B2P_OK;
 }
 
@@ -2402,7 +2406,7 @@ void fill_summary(b2p_result* sum, int count, bool timed_out, int64_t tot_it, in
     sum->kernel_time_ms = kms;
     sum->primal_weight = 0.0;
     sum->step_size = cfg.threads * 100000.0 + cfg.chunk;  // tuned block size * 1e5 + chunk length
-    sum->used_average = 10 * cfg.ni + cfg.w;                // 10 * instances per CTA + SELL entries per lane load
+    sum->used_average = 10 * cfg.ni + cfg.w;                // 10 * instances per CTA at first + SELL entries per lane load
 }
 
 // All instances of the batch share one shape (required by the learned warm start).
@@ -2867,9 +2871,10 @@ int b2p_batch_solve_learned(void* p, const b2p_params* params, const float* feat
         if (!ok && warm_iters[i] < pp->max_iterations) failed.push_back(i);
     }
     if (fallback && !failed.empty() && !timed_out) {
-        st = f64 ? batch_run<double>(ctx, w, pp, nullptr, nullptr, nullptr, &failed, &timed_out, &kms2, &cfg,
+        // the summary names the shape of the warm run
+        st = f64 ? batch_run<double>(ctx, w, pp, nullptr, nullptr, nullptr, &failed, &timed_out, &kms2, nullptr,
                                      &warm_iters)
-                 : batch_run<float>(ctx, w, pp, nullptr, nullptr, nullptr, &failed, &timed_out, &kms2, &cfg,
+                 : batch_run<float>(ctx, w, pp, nullptr, nullptr, nullptr, &failed, &timed_out, &kms2, nullptr,
                                     &warm_iters);
         if (st) return st;
     }
