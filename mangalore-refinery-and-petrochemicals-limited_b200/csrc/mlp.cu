@@ -88,7 +88,9 @@ struct MlpState {
     // one training epoch captured as a CUDA graph (for this data-set size and batch)
     cudaGraphExec_t epoch_exec = nullptr;
     int epoch_n = 0, epoch_batch = 0;
-    std::vector<const void*> epoch_bufs;  // the buffers it works on (a larger request elsewhere may have moved them)
+    // every buffer it works on that a larger request elsewhere may have moved (each by itself: one of two
+    // that grow together can come back at its old address)
+    std::vector<const void*> epoch_bufs;
     long long epoch_launches = 0;  // kernels one replay launches
     ~MlpState() {
         if (epoch_exec) cudaGraphExecDestroy(epoch_exec);
@@ -1274,8 +1276,8 @@ int b2p_mlp_train(void* p, int epochs, int batch, float lr_start, float lr_end, 
         return B2P_OK;
     };
     auto buffers = [&]() -> std::vector<const void*> {
-        return {s->Xf.p, s->Xh.p, s->Z1.p, s->H1.p, s->dY.p, s->dZ.p, s->G.p, s->ws.p, s->ws1.p, s->ws2.p, s->DX.p, s->DT.p,
-                s->perm.p};
+        return {s->Xf.p,  s->Xh.p,  s->Xt.p, s->Z1.p,  s->Z2.p, s->H1.p, s->H1t.p, s->H2.p,  s->H2t.p, s->dY.p,
+                s->dYt.p, s->dZ.p,  s->dZt.p, s->G.p,  s->ws.p, s->ws1.p, s->ws2.p, s->DX.p, s->DT.p,  s->perm.p};
     };
     const int steps_per_epoch = (N + batch - 1) / batch;
     if (!s->epoch_exec || s->epoch_bufs != buffers() || s->epoch_n != N || s->epoch_batch != batch) {
