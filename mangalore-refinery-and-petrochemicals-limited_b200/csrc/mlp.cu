@@ -1291,7 +1291,7 @@ int b2p_mlp_train(void* p, int epochs, int batch, float lr_start, float lr_end, 
         // so more splits (1,024 hidden, 10,008 outputs: 512 x 1,024 x 4 floats for a full batch of
         // 512, 128 x 1,024 x 18 for a remainder of 128).
         B2P_CUDA(ctx, cudaMemcpyAsync(s->perm.p, order.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice, st));
-        for (const int valid : {std::min(batch, N), N % batch}) {
+        for (const int valid : {std::min(batch, N), N > batch ? N % batch : 0}) {
             const int rows = (valid + 7) & ~7;
             if (valid == 0) continue;
             if ((r = forward_hidden(ctx, s, rows, valid, true))) return r;
