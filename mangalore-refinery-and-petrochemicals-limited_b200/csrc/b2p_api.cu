@@ -590,8 +590,9 @@ int b2p_spmv_t(void* p, int m, int n, const int32_t* rowptr, const int32_t* coli
         ctx->err = "CSR column indices out of range or not strictly ascending in row " + std::to_string(bad - 1);
         return B2P_INVALID_ARGUMENT;
     };
-    // small: its products and sums fit one CTA, whose one adding warp takes 0.08 us a row (33 us at
-    // 300 rows of 17 entries); the sort, scan and waits of the transpose took 150 us whatever the size
+    // small: its products and sums fit one CTA, whose one adding warp takes 0.1 us for a row of up to 32
+    // entries (the kernel by device events: 38 us at 300 rows of 17 entries, 109 at 1,000 of 12 or of 5);
+    // the sort, scan and waits of the transpose took 150 us whatever the size
     if (io.packed && nnz <= 12288 && n <= 8192 && m <= 1024) {
         const int rows_off = n + (int)nnz + ((int)nnz + 3) / 4;  // in doubles: sums, products, columns, then row pointers
         const size_t small = 8 * (size_t)rows_off + 4 * ((size_t)m + 1);
