@@ -680,7 +680,7 @@ def run_learned_workload(args):
             launches = int(summ["kernel_launches"]) * k
             it_total = float(per["iterations"].sum())
             kern_ms = summ["kernel_time_ms"]
-            ni = max(1, int(round(summ["used_average"])) // 10)  # instances per CTA of the tuned shape
+            ni = max(1, int(round(summ["used_average"])) // 10)  # instances per CTA of the first launch
     # end to end through the public API: pinned host parameter vectors and instance
     # data -> upload -> learned solve -> answers to host
     _, B, Cc, LB, UB, EQ = fam.standard_batch(P)
@@ -732,8 +732,9 @@ def run_learned_workload(args):
     # algorithmic bytes of every instance-iteration of the value leg over its kernel time --
     # the SELL matrix (12 B per nonzero, both orientations) once per CTA-iteration, so once
     # per ni instances, plus each instance's vectors.  The shared matrix and the vectors are
-    # served from L2 and shared memory, so the bound that applies is the on-chip one; the
-    # DRAM share comes from the committed ncu capture.
+    # served from L2 and shared memory; what bounds the kernel is the shared-memory pipe, which
+    # its gathers from random addresses keep at 73 % of its wavefronts (L2: 24 % of its
+    # throughput).  The DRAM share comes from the committed ncu capture.
     nnz = int(fam.rowptr[-1])
     per_iter = 12 * nnz / ni + 24 * fam.n + 16 * fam.m
     pk, pk_src = peaks()
@@ -741,7 +742,7 @@ def run_learned_workload(args):
     achieved = it_total * per_iter / (kern_ms / 1e3) / 1e9
     kname = "k_batch_chunk"
     prof = read_profile(ROOT / "profiles" / "batch_group_refinery_planning.txt")
-    roofline = {"bound": "l2", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+    roofline = {"bound": "smem", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": prof.get("dram_bytes_per_instance_iteration"),
                 "traffic_unit": "DRAM bytes per instance-iteration (ncu dram__bytes_read.sum + write.sum)",
                 "dram_frac": (prof["dram_bytes_per_instance_iteration"] / per_iter
@@ -750,11 +751,11 @@ def run_learned_workload(args):
                 "lts_throughput_pct": prof.get("lts_throughput_pct"),
                 "kernel": f"{kname}<float> (SELL, {ni} instance(s) per CTA, learned leg)",
                 "algorithmic_bytes_per_instance_iteration": per_iter,
-                "peak_source": "hbm_gbs: " + pk_src + "; no measured L2 peak exists, so the fraction is against HBM",
+                "peak_source": "hbm_gbs: " + pk_src + "; no measured on-chip peak exists, so the fraction is against HBM",
                 "note": f"12 B per nonzero (FP32 value + 16-bit index, both orientations) shared by the {ni} "
-                        "instance(s) of a CTA, 24 B per column, 16 B per row; bound 'l2': the shared matrix and "
-                        "the instances' vectors stay in L2 / shared memory (ncu: DRAM carries dram_frac of these "
-                        "bytes)"}
+                        "instance(s) of a CTA, 24 B per column, 16 B per row; bound 'smem': shared-memory wavefronts of "
+                        "the random gathers; the shared matrix and the instances' vectors stay in L2 / shared "
+                        "memory (ncu: DRAM carries dram_frac of these bytes)"}
     # training on the tensor cores: GEMM FLOPs of all epochs (per sample: layer 1 forward +
     # weight gradient, layers 2 and 3 forward + weight gradient + input gradient) over the
     # training time, against the sustained BF16 peak
